@@ -219,17 +219,21 @@ int tcs_plan_set_coeffs(tcs_plan plan, const float *coeffs);
  * engine).  Results are bit-identical either way; the autotuner picks. */
 int tcs_plan_set_temporal_depth(tcs_plan plan, int depth);
 /* Tensor engine (FP16 or split, temporal depth 1): run(steps >= 2) as ONE
- * launch whose tiles of step j wait only for the neighbouring tile rows of
- * step j-1 (per-row completion counts), instead of one launch per step.
- * mode -1 (default): FP16 when a step has more than two tiles per SM, split
- * when it has more than one and at most eight (where each measured
- * faster); 0: never; 1: always.  Results are bit-identical either way.
- * TCS_MULTI=0 in the environment turns it off for the process. */
+ * launch instead of one launch per step.  FP16 tiles take up to eight
+ * (radius 1) or four (radius 2) steps each time they are loaded and wait for
+ * the neighbouring tiles' previous visit; split tiles of step j wait for the
+ * neighbouring tile rows of step j-1.  mode -1 (default): FP16 grids of more
+ * than 16 tiles of 128 x 128, split grids of more than one and at most 20
+ * tiles per SM; 0: never; 1: always.  Results are bit-identical either way
+ * for grids of finite values (an infinity or NaN spreads by whole 16-column
+ * windows a step, and over several steps of a visit not past its tile's
+ * halo).  TCS_MULTI=0 in the environment turns it off for the process. */
 int tcs_plan_set_multistep(tcs_plan plan, int mode);
 /* Tile shape of the plain FP16 tensor sweeps: 128 rows by tile_w = 128
  * (default), 96 or 64 columns.  Narrower tiles give a grid more tiles: on
  * grids with few tiles per SM more SMs share a step, and each tile's MMAs and
- * epilogue shrink with its width.  Results are bit-identical at every width;
+ * epilogue shrink with its width.  One-launch runs at the default choose
+ * their width (32 to 128) by the grid; a width set here holds for them too.  Results are bit-identical at every width;
  * the autotuner picks the width per size class (it replaces the reference's
  * TILE_SIZE sweep, script/param.py:5).  TCS_ERR_UNSUPPORTED for widths below
  * 128 on other engines and precisions. */

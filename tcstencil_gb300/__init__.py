@@ -316,6 +316,8 @@ class Plan:
             if temporal_depth is None:
                 temporal_depth = tuned_depth
             tuned_launch = best_launch(stencil, precision, ny, nx)
+            if tuned_launch < 0 and precision == "f16":
+                tuned_launch = 1  # every tuned FP16 class takes one launch for all steps
             if tile_w is None and engine == "tensor" and precision == "f16":
                 tile_w = best_tile_width(stencil, ny, nx)
         self._c = _coeffs(coeffs, stencil)

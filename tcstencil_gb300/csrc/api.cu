@@ -185,6 +185,9 @@ int tcs_device_error(int *code) {
     st = cuda_status(tb_take_error(&cb), "reading the blocked-sweep error word");
     if (st) return st;
     if (!c) c = cb;
+    st = cuda_status(visit_take_error(&cb), "reading the visit-sweep error word");
+    if (st) return st;
+    if (!c) c = cb;
     st = cuda_status(cc_take_error(&cb), "reading the CUDA-core error word");
     if (st) return st;
     if (!c) c = cb;
@@ -363,7 +366,7 @@ struct tcs_plan_s {
     cudaEvent_t band_ev[kBands + 1] = {};
     cudaStream_t capture_stream = nullptr;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (steps, start state)
-    unsigned *rows_done = nullptr;  // plain tensor form: per tile row, for multi-step launches
+    unsigned *rows_done = nullptr;  // tensor form: counters of the multi-step launches
 
     int planes() const { return prob.precision == TCS_PREC_SPLIT ? 2 : 1; }
 
@@ -435,12 +438,10 @@ struct tcs_plan_s {
             "blocked sweep launch");
     }
     // Tensor-engine plans (FP16 or split, temporal depth 1) run all steps of
-    // a call in one launch, whose tiles of step j wait only for the
-    // neighbouring tile rows of step j-1 (tcs_plan_set_multistep; TCS_MULTI=0
-    // in the environment: one launch per step).  Measured on GB300 (FP16 box2d2r, us per step, one
-    // launch per step -> one launch): 8196² 49.8 -> 42.2, 4096² 13.2 -> 10.4,
-    // 2048² 6.8 -> 6.9, 1026² 5.5 -> 6.3: small grids are latency-bound, and
-    // a step boundary between launches is quicker than the counters.
+    // a call in one launch (tcs_plan_set_multistep; TCS_MULTI=0 in the
+    // environment: one launch per step): FP16 tiles take several steps per
+    // visit (sweep_visit.cu), split tiles one, and wait only for the
+    // neighbouring tiles or tile rows of the visit or step before.
     int multistep = -1;
     bool multi() const {
         static const bool on = [] {
@@ -459,28 +460,41 @@ struct tcs_plan_s {
         // the multi-step kernel spends a little more per tile, which the step
         // overheads repay up to about 20 tiles per SM.
         if (prob.precision == TCS_PREC_SPLIT) return tiles > sms && tiles <= 20 * sms;
-        return tiles > 2 * sms;
+        // FP16: one launch is faster at every size (visit_shape), but its CTAs
+        // must all be resident and take an SM each, so the smallest grids,
+        // of which a program may step several side by side on its streams,
+        // keep to ordinary launches unless the caller asks (mode 1; the
+        // autotuned plans do)
+        return tiles > 16;
+    }
+    bool visits() const { return prob.precision == TCS_PREC_F16; }
+    VisitShape visit_shape(int steps) const {
+        return tcs::visit_shape(g.ny, g.nx, prob.stencil, steps, tile_w, device_sms());
     }
     int steps_in_one(int steps, int from, cudaStream_t s) {
+        if (visits())
+            return cuda_status(
+                launch_tc_f16_visits(g, prob.stencil, coeffs, static_cast<uint16_t *>(buf[from][0]),
+                                     static_cast<uint16_t *>(buf[1 - from][0]), steps,
+                                     visit_shape(steps), rows_done, s, device_sms()),
+                "multi-step sweep launch");
         const int tiles_y = (g.ny + kTile - 1) / kTile;
         int st = cuda_status(
             cudaMemsetAsync(rows_done, 0, (size_t)tiles_y * kRowCounterStride * sizeof(unsigned), s),
             "row counter reset");
         if (st) return st;
-        const cudaError_t e =
-            prob.precision == TCS_PREC_SPLIT
-                ? launch_tc_split_steps(g, prob.stencil, coeffs, static_cast<const uint16_t *>(buf[from][0]),
-                                        static_cast<const uint16_t *>(buf[from][1]),
-                                        static_cast<uint16_t *>(buf[1 - from][0]),
-                                        static_cast<uint16_t *>(buf[1 - from][1]), steps, rows_done, s,
-                                        d_scale, 0)
-                : launch_tc_f16_steps(g, prob.stencil, coeffs, static_cast<const uint16_t *>(buf[from][0]),
-                                      static_cast<uint16_t *>(buf[1 - from][0]), steps, rows_done, s,
-                                      tile_w);
-        return cuda_status(e, "multi-step sweep launch");
+        return cuda_status(
+            launch_tc_split_steps(g, prob.stencil, coeffs, static_cast<const uint16_t *>(buf[from][0]),
+                                  static_cast<const uint16_t *>(buf[from][1]),
+                                  static_cast<uint16_t *>(buf[1 - from][0]),
+                                  static_cast<uint16_t *>(buf[1 - from][1]), steps, rows_done, s,
+                                  d_scale, 0),
+            "multi-step sweep launch");
     }
-    // The state `steps` steps from `from` ends in: one flip per step.
+    // The state `steps` steps from `from` ends in: one flip per step, step
+    // pair or visit.
     int final_state(int steps, int from) const {
+        if (steps >= 2 && multi() && visits()) return from ^ (visit_shape(steps).visits & 1);
         const int launches = pairs() ? steps / 2 + steps % 2 : steps;
         return from ^ (launches & 1);
     }
@@ -490,7 +504,7 @@ struct tcs_plan_s {
     int enqueue(int steps, int from, cudaStream_t s, int *to) {
         int st = TCS_OK;
         if (steps >= 2 && multi()) {
-            *to = from ^ (steps & 1);
+            *to = final_state(steps, from);
             st = steps_in_one(steps, from, s);
         } else {
             for (int t = 0; t < steps && !st;) {
@@ -554,11 +568,15 @@ int tcs_plan_create(const tcs_problem *pr, tcs_plan *out) {
     if (pr->engine == TCS_ENGINE_TENSOR) {
         st = cuda_status(tc_prepare(pr->stencil, pr->precision == TCS_PREC_SPLIT), "tensor kernel set-up");
         if (st) return st;
-        {
-            const int tiles_y = (pr->ny + kTile - 1) / kTile;
-            st = dev_alloc_t(&p->rows_done, (size_t)tiles_y * kRowCounterStride * sizeof(unsigned), "row counters");
+        size_t words = (size_t)((pr->ny + kTile - 1) / kTile) * kRowCounterStride;
+        if (pr->precision == TCS_PREC_F16) {
+            st = cuda_status(visit_prepare(pr->stencil), "multi-step kernel set-up");
             if (st) return st;
+            words = visit_counter_words(pr->ny, pr->nx);
         }
+        st = dev_alloc_t(&p->rows_done, words * sizeof(unsigned), "row counters");
+        if (!st) st = cuda_status(cudaMemset(p->rows_done, 0, words * sizeof(unsigned)), "cudaMemset(counters)");
+        if (st) return st;
     }
     *out = p.release();
     return TCS_OK;

@@ -333,14 +333,15 @@ EncodeTiledFn encode_tiled() {
 
 }  // namespace
 
-cudaError_t encode_panel_map(const uint16_t *plane, const PlaneGeom &pg, CUtensorMap *map) {
+cudaError_t encode_panel_map(const uint16_t *plane, const PlaneGeom &pg, CUtensorMap *map,
+                             int panels, int rows) {
     const EncodeTiledFn enc = encode_tiled();
     if (!enc) return cudaErrorNotSupported;
     if (reinterpret_cast<uintptr_t>(plane) % 16 || pg.nyp % 8 || pg.cpp != 8)
         return cudaErrorInvalidValue;
-    const cuuint64_t dims[3] = {16, (cuuint64_t)pg.nyp / 8, (cuuint64_t)pg.npan};
-    const cuuint64_t strides[2] = {128, (cuuint64_t)pg.nyp * 16};  // bytes, dims 1 and 2
-    const cuuint32_t box[3] = {16, (kTile + 8) / 8, kTile / 8 + 2};
+    const cuuint64_t dims[3] = {(cuuint64_t)(2 * rows), (cuuint64_t)(pg.nyp / rows), (cuuint64_t)pg.npan};
+    const cuuint64_t strides[2] = {(cuuint64_t)(16 * rows), (cuuint64_t)pg.nyp * 16};  // bytes, dims 1 and 2
+    const cuuint32_t box[3] = {(cuuint32_t)(2 * rows), (cuuint32_t)((kTile + 8) / rows), (cuuint32_t)panels};
     const cuuint32_t es[3] = {1, 1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<uint16_t *>(plane),
                            dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -47,17 +47,16 @@
 //                for radius-2 stencils (warp 1 also owns TMEM)
 //   next 8       epilogue (two warpgroups, one per column half):
 //                TMEM -> registers -> FP16 -> global
-//   last         signal: with several steps per launch, publishes finished
-//                tile rows (see "several steps per launch" below)
 // One accumulator slot per issuer lets the epilogue of one tile overlap the
 // MMAs of the next; tile i uses slot i % I, issued by warp 1 + i % I.  Every
 // wait is bounded; on timeout the kernel records an error word, stops,
 // drains its own copies and MMAs, frees TMEM and returns.
 //
 // Launches: one step per launch, overlapped with the next step's set-up by
-// programmatic dependent launch; or, for a plan's multi-step call on a large
-// grid, all steps in one cooperative launch whose tiles of step j wait only
-// for the neighbouring tile rows of step j-1.
+// programmatic dependent launch; or, for a split plan's multi-step call on a
+// mid-size grid, all steps in one cooperative launch whose tiles of step j
+// wait only for the neighbouring tile rows of step j-1.  (Several plain steps
+// per launch: sweep_visit.cu.)
 #include "tc_core.cuh"
 #include "tile_walk.h"
 
@@ -195,8 +194,7 @@ struct Sweep {
     static constexpr int ISSUERS = stencil_r(S) == 1 ? 3 : 2;
     static constexpr int SLOTS = ISSUERS;
     static constexpr int STAGES = ISSUERS == 2 ? 4 : 3;
-    static constexpr int SIGNAL_WARP = 1 + ISSUERS + kEpiWarps;  // several steps: row counts
-    static constexpr int THREADS = 32 * (SIGNAL_WARP + 1);
+    static constexpr int THREADS = 32 * (1 + ISSUERS + kEpiWarps);
     static_assert(SLOTS * Mode<false>::ACC <= kTmemCols, "accumulator slots fit TMEM");
     static_assert(STAGES % ISSUERS == 0, "each stage holds one issuer's tiles");
 };
@@ -215,12 +213,12 @@ struct Cfg {
 
 struct TcParams {
     CUtensorMap map_hi, map_lo;     // input planes (encode_panel_map)
-    CUtensorMap map_out, map_out_lo;  // several steps: the output planes (odd steps' input)
+    CUtensorMap map_out, map_out_lo;  // several split steps: the output planes (odd steps' input)
     GridGeom g;
     int tiles_x, n_tiles;
     int tile_w;                     // plain: tile columns, 64, 96 or 128 (split: 128)
-    int steps;                      // plain: steps of this launch (1 for the split kernels)
-    unsigned *rows_done;            // plain, several steps: per tile row (every
+    int steps;                      // steps of this launch
+    unsigned *rows_done;            // several split steps: per tile row (every
                                     // kRowCounterStride), epilogue-warp completions
                                     // over the launch (zeroed before it)
     const uint16_t *in_hi, *in_lo;  // input planes
@@ -286,8 +284,7 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
     uint64_t *acc_empty = acc_full + NSL;       // [NSL]
     uint64_t *drain = acc_empty + NSL;          // [1]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
-    uint32_t *warp_done = tmem_slot + 2;        // [kEpiWarps] several steps: items stored
-    static_assert((2 * NS + 2 * NSL + 1) * 8 + (2 + kEpiWarps) * 4 <= 256, "barrier area");
+    static_assert((2 * NS + 2 * NSL + 1) * 8 + 2 * 4 <= 256, "barrier area");
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -305,7 +302,6 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
             mbar_init(&acc_empty[b], kEpiWarps);
         }
         mbar_init(drain, Sweep<S>::ISSUERS);
-        for (int w = 0; w < kEpiWarps; w++) warp_done[w] = 0;
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -328,36 +324,26 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
     const int tiles_x = p.tiles_x;
     const int n_tiles = p.n_tiles;
     const int tiles_y = n_tiles / tiles_x;
-    const int n_items = p.steps * n_tiles;  // (step, tile), step-major; CTA b takes b, b + grid, ...
+    const int n_items = n_tiles;  // CTA b takes b, b + grid, ...
 
     if (warp == 0) {
         // ------------------------------------------------------ producer ---
         if (lane == 0) {
             int i = 0;
             int last_issued = -1;
-            RowDeps deps;
-            const unsigned per_row = (unsigned)(kEpiWarps * tiles_x);
             TileWalk w;
             w.init(blockIdx.x, gridDim.x, tiles_x, tiles_y);
             for (int k = blockIdx.x; k < n_items; k += gridDim.x, i++, w.advance()) {
-                const int step = w.step;
-                const int ty = w.ty;
                 const int s = i % NS;
                 const uint32_t ph = (i / NS) & 1;
-                if (step > 0 && !deps.wait(p.rows_done, step, ty, tiles_y, per_row)) {
-                    record_error(&g_tc_error, kErrWaitDep);
-                    *abort_flag = 1;
-                    break;
-                }
-                // (the poll above overlaps the wait for a free stage)
                 if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) {
                     record_error(&g_tc_error, kErrWaitEmpty);
                     *abort_flag = 1;
                     break;
                 }
                 mbar_arrive_expect_tx(&full[s], NP * SG::PLANE);
-                load_tile_map((step & 1) ? &p.map_out : &p.map_hi, &p.map_lo, NP, ty * kTile,
-                              w.tx * p.tile_w, stage_base + (size_t)s * NP * SG::PLANE, &full[s]);
+                load_tile_map(&p.map_hi, &p.map_lo, NP, w.ty * kTile, w.tx * p.tile_w,
+                              stage_base + (size_t)s * NP * SG::PLANE, &full[s]);
                 last_issued = i;
             }
             // Drain: every stage armed last must have landed before exit.
@@ -421,10 +407,6 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
                 }
             }
         }
-    } else if (warp == Sweep<S>::SIGNAL_WARP) {
-        // -------------------------------------------------------- signal ---
-        if (p.rows_done && lane == 0)
-            signal_rows<kEpiWarps>(p.rows_done, n_items, n_tiles, tiles_x, warp_done, abort_flag);
     } else {
         // ------------------------------------------------------ epilogue ---
         const int q = warp & 3;            // TMEM lane quarter of this warp
@@ -447,12 +429,8 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
         const int G = W / 32;  // output blocks per warpgroup
         const int j0 = half * G;
         for (int k = blockIdx.x; k < n_items && !stop; k += gridDim.x, i++, w.advance()) {
-            const int step = w.step;
             const int Y0 = w.ty * kTile;
             const int X0 = w.tx * W;
-            // odd steps run from the output plane back into the input plane
-            o.in_hi = (step & 1) ? p.out_hi : p.in_hi;
-            o.out_hi = (step & 1) ? const_cast<uint16_t *>(p.in_hi) : p.out_hi;
             const int sl = i % NSL;  // tile i's accumulator slot
             bool ok = mbar_wait(&acc_full[sl], (i / NSL) & 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
@@ -484,7 +462,6 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
                 else if (G == 3) plain_epilogue<3>(o, lc, j0, nblk, y, X0, fast, row_in, release);
                 else plain_epilogue<2>(o, lc, j0, nblk, y, X0, fast, row_in, release);
             }
-            if (p.rows_done) count_item(warp_done, warp - 1 - Sweep<S>::ISSUERS, (uint32_t)(i + 1));
         }
     }
 
@@ -903,7 +880,7 @@ cudaError_t launch_tc(const GridGeom &g, const float *B, const uint16_t *in_hi,
                       int steps = 1, unsigned *rows_done = nullptr, int tile_w = kTile,
                       SplitScale *scale = nullptr, int t0 = 0) {
     using C = Cfg<S, SPLIT>;
-    if (!valid_tile_width(tile_w) || (SPLIT && tile_w != kTile)) return cudaErrorInvalidValue;
+    if (!valid_tile_width(tile_w) || (SPLIT ? tile_w != kTile : steps != 1)) return cudaErrorInvalidValue;
     cudaError_t pe = prepare_tc<S, SPLIT>();
     if (pe != cudaSuccess) return pe;
     TcParams p;
@@ -942,8 +919,7 @@ cudaError_t launch_tc(const GridGeom &g, const float *B, const uint16_t *in_hi,
                    ? launch_step(tc_split_ring_kernel<S, true>, grid, Ring<true>::THREADS, C::SMEM, s, p, true)
                    : launch_step(tc_split_ring_kernel<S, false>, grid, Ring<false>::THREADS, C::SMEM, s, p);
     else
-        return launch_step(tc_sweep_kernel<S, SPLIT>, grid, Sweep<S>::THREADS, C::SMEM, s, p,
-                           p.steps > 1);
+        return launch_step(tc_sweep_kernel<S, SPLIT>, grid, Sweep<S>::THREADS, C::SMEM, s, p);
 }
 
 template <bool SPLIT>
@@ -982,12 +958,6 @@ cudaError_t tc_take_error(int *code) {
 cudaError_t launch_tc_f16(const GridGeom &g, int stencil, const float *B, const uint16_t *in,
                           uint16_t *out, cudaStream_t s, int tile_w) {
     return dispatch_tc<false>(g, stencil, B, in, nullptr, out, nullptr, s, 1, nullptr, tile_w);
-}
-
-cudaError_t launch_tc_f16_steps(const GridGeom &g, int stencil, const float *B, const uint16_t *in,
-                                uint16_t *out, int steps, unsigned *rows_done, cudaStream_t s,
-                                int tile_w) {
-    return dispatch_tc<false>(g, stencil, B, in, nullptr, out, nullptr, s, steps, rows_done, tile_w);
 }
 
 cudaError_t launch_tc_split_steps(const GridGeom &g, int stencil, const float *B,

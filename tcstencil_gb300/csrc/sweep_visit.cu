@@ -1,0 +1,648 @@
+// Plain FP16 sweeps of several steps per tile visit: a tile is loaded once,
+// stepped T times in shared memory and stored once.
+//
+// A step that reads and writes every plane moves 4 bytes per point update,
+// which at 8196² takes as long as the two issuers of tc_sweep_kernel need for
+// the radius-2 MMAs and 1.6 times as long as the radius-1 MMAs; a small grid's
+// step is a launch boundary, a load and a store around about a microsecond of
+// MMAs.  Both come down to one load and one store per T steps here.
+//
+// Tile.  As in tc_sweep_kernel (sweep_tc.cu): the stage holds rows
+// Yb-4 .. Yb+131 of the panels X0-8 .. X0+W+7, an MMA step gives rows
+// Yb .. Yb+127 of the columns X0-16 .. X0+W+15, and the windows and their
+// order are the same, so every cell sums the same products in the same order
+// as in a single-step launch.  After a step the epilogue warps write the new
+// values back over the staged image (all MMAs that read it are complete),
+// X0-8 .. X0+W+7 included, and the next step's MMAs run on the image.  Cells
+// whose neighbourhood is not all of the previous step are not written: r more
+// rows at the image's top and bottom and r more columns at its sides with
+// every step (r(t-1) rows, r t columns after t steps), so the image only ever
+// holds values of the field.  The halo columns are the staged panels on
+// either side, which bounds r T by 8; an incomplete halo column lacks only
+// windows whose products with it are all zero.  Tile rows overlap by 2 halo
+// rows, halo = 2, 4 or 8 (>= r(T-1)): the tile at Yb = ty (128 - 2 halo) owns rows
+// Yb+halo .. Yb+127-halo (from row 0, to the last row, for the first and last
+// tile rows), stored to the other plane after the visit's last step.
+//
+// Pipeline.  Two MMA issuers, each with its own accumulator slot and its own
+// eight epilogue warps (a lane quarter and a column half each): while one
+// slot's tile is in its epilogue, the other's MMAs run.  Each slot walks its
+// tiles in order and never waits for the other, because with few tiles per SM
+// the other slot's tile may be of the next visit and wait for this one's
+// result.  Stage i % 4 holds tile i, so each stage belongs to one issuer.
+// A tile's visit j needs visit j-1 of itself and its eight neighbours: they
+// hold its input, and they were the last readers of the plane it overwrites.
+// Every tile has a counter of its finished visits, added to with one release
+// reduction by the last of its epilogue warps; nine lanes of the producer
+// warp poll the nine counters at once.  (Counters per tile row, as the split
+// kernel's several-step form has, made a visit's boundary 3.3 us on a
+// 333 x 1517 grid: a tile waited for its rows' slowest CTA, and 192 reductions
+// met on one word.  A reduction by each of a tile's eight warps: 8196²
+// star2d1r 28.3 us per step, 26.9 with one.)  The launch is cooperative: all
+// CTAs are resident at once.  Every wait is bounded.
+//
+// Cells that are not finite: an MMA multiplies all 16 columns of a window, so
+// one infinity or NaN makes every output of its windows in the reaching rows
+// NaN, here as in single steps; which further cells it reaches over several
+// steps depends on the visit's halo.
+#include "tc_core.cuh"
+#include "tile_walk.h"
+
+namespace tcs {
+
+namespace {
+
+using namespace tc;
+using SG = StageLines;
+
+__device__ int g_visit_error = 0;
+
+constexpr int kVisitSlots = 2;
+constexpr int kVisitStages = 4;                 // a multiple of the slots
+constexpr int kVisitEpi0 = 1 + kVisitSlots;     // first epilogue warp
+constexpr int kVisitEpi = 8;                    // epilogue warps per slot
+constexpr int kVisitThreads = 32 * (kVisitEpi0 + kVisitSlots * kVisitEpi);
+constexpr int kVisitSlotCols = 256;             // TMEM columns per slot (160 used)
+
+struct VisitParams {
+    CUtensorMap map[2];  // the planes; visit j reads map[j & 1]
+    GridGeom g;
+    int tiles_x, tiles_y, halo;
+    int map_rows;             // rows of a panel per box line (encode_panel_map)
+    int visits, base, extra;  // visit j takes base + (j < extra) steps
+    unsigned *ended;          // CTAs at the end of the launch (zero at its start)
+    unsigned *done;           // [tiles] the tile's finished visits (zeros)
+    uint16_t *plane[2];
+    float coef[25];
+};
+
+__host__ __device__ constexpr int visit_stage_bytes(int W) { return (W / 8 + 2) * SG::CHUNK; }
+
+__device__ __forceinline__ void sts128(uint32_t addr, const uint4 &v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y),
+                 "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
+
+// 8 accumulators as a panel row of FP16 cells.
+__device__ __forceinline__ uint4 pack_panel(const uint32_t *v) {
+    uint32_t w[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) w[c] = pack_h2(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Masks of a panel row's cells in shared memory, 16 bytes each: entry n is the
+// cells c >= n (n = 0 .. 8), entry 9 + n the cells c < n.
+constexpr int kMaskBytes = 18 * 16;
+constexpr int kBarBytes = 256;  // barriers and flags, before the masks
+__device__ __forceinline__ void build_masks(uint32_t *mask, int tid) {
+    if (tid < 72) {
+        const int n = (tid / 4) % 9, c = 2 * (tid % 4);
+        const uint32_t ge = (c >= n ? 0x0000ffffu : 0u) | (c + 1 >= n ? 0xffff0000u : 0u);
+        mask[tid] = tid < 36 ? ge : ~ge;
+    }
+}
+__device__ __forceinline__ uint4 blend(const uint4 &w, const uint4 &old, const uint4 &m) {
+    return make_uint4((w.x & m.x) | (old.x & ~m.x), (w.y & m.y) | (old.y & ~m.y),
+                      (w.z & m.z) | (old.z & ~m.z), (w.w & m.w) | (old.w & ~m.w));
+}
+// The mask of cells [a, b), 0 <= a, b <= 8 (none if b <= a).
+__device__ __forceinline__ uint4 cells_mask(uint32_t mask, int a, int b) {
+    const uint4 x = lds128(mask + 16 * a), y = lds128(mask + 16 * (9 + b));
+    return make_uint4(x.x & y.x, x.y & y.y, x.z & y.z, x.w & y.w);
+}
+__device__ __forceinline__ int clamp8(int v) { return v < 0 ? 0 : v > 8 ? 8 : v; }
+
+// This warp's G blocks of 16 columns of a step's accumulators, two blocks at
+// a time: sink(p, w) takes panel row p = 0 .. 2G-1.  (A TMEM load takes about
+// 25 cycles; holding all blocks at once would spill registers, which cost
+// ten times that, as little L1 is left beside the stages.)
+template <int G, typename Sink>
+__device__ __forceinline__ void walk_blocks(uint32_t col, Sink &&sink) {
+#pragma unroll
+    for (int g = 0; g < G; g += 2) {
+        uint32_t v[2][16];
+        tmem_ld_x16(col + 16 * g, v[0]);
+        if (g + 1 < G) tmem_ld_x16(col + 16 * (g + 1), v[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int p = 2 * g; p < 2 * g + 4 && p < 2 * G; p++)
+            sink(p, pack_panel(v[(p >> 1) - g] + 8 * (p & 1)));
+    }
+}
+
+// A tile's MMAs: the windows its grid cells need (tile_windows), rounded up
+// to a sequence of 5 or of all.  (In a loop over the coefficient rows instead
+// of unrolled, the issuing thread took 87 cycles per MMA instead of 67.)
+template <int R, int NWIN>
+__device__ __forceinline__ void issue_visit_tile(uint64_t a0, uint32_t band, uint32_t d, int nwin) {
+    if (NWIN > 5 && nwin <= 5) issue_subtile<R, false, SG, 5>(a0, band, d, 0);
+    else issue_subtile<R, false, SG, NWIN>(a0, band, d, 0);
+}
+
+// What one epilogue warp does with a tile: fixed over the tile's steps.
+struct WarpTile {
+    uint32_t col, ecol;  // TMEM: its blocks' first column, its halo panel's
+    uint32_t img, eimg;  // image: this row of its blocks' first panel, of its halo panel
+    uint32_t mask;       // the mask table
+    int xf, ex;          // first column of its blocks, of its halo panel
+    int tmax;            // the row may be written up to this step (0: never)
+    bool inner;          // its blocks' and halo panel's columns all lie in the rectangle
+    // otherwise: panels [p0, p1) of its blocks lie in the rectangle, the others
+    // of [q0, q1) in part, and cells [ea, eb) of the halo panel
+    int p0, p1, q0, q1, ea, eb;
+};
+
+// An intermediate step t: the new values go back into the image.  A step's
+// MMAs wait for this chain, so it is kept to TMEM loads, conversions and
+// predicated stores; only columns at the rectangle's edge take the blends of
+// the second branch.
+template <int G, int R>
+__device__ __forceinline__ void step_to_image(const WarpTile &c, int half, int t, int x0, int x1) {
+    const bool row = t <= c.tmax;
+    // halo cells whose neighbourhood is all of step t-1: R t fewer
+    const int ea = half ? 0 : R * t, eb = half ? 8 - R * t : 8;
+    if (c.inner) {
+        uint32_t e[8];
+        tmem_ld_x8(c.ecol, e);
+        const uint4 old = lds128(c.eimg);
+        const uint4 m = lds128(c.mask + 16 * (half ? 9 + eb : ea));
+        tmem_ld_wait();
+        if (row) sts128(c.eimg, blend(pack_panel(e), old, m));
+        walk_blocks<G>(c.col, [&](int p, const uint4 &w) {
+            if (row) sts128(c.img + p * SG::CHUNK, w);
+        });
+    } else {
+        if (c.ea < c.eb) {
+            uint32_t e[8];
+            tmem_ld_x8(c.ecol, e);
+            const uint4 old = lds128(c.eimg);
+            const uint4 m = cells_mask(c.mask, max(ea, c.ea), min(eb, c.eb));
+            tmem_ld_wait();
+            if (row) sts128(c.eimg, blend(pack_panel(e), old, m));
+        }
+        walk_blocks<G>(c.col, [&](int p, const uint4 &w) {
+            const uint32_t at = c.img + p * SG::CHUNK;
+            if (p >= c.p0 && p < c.p1) {
+                if (row) sts128(at, w);
+            } else if (p >= c.q0 && p < c.q1) {
+                const int xb = c.xf + 8 * p;
+                if (row) sts128(at, blend(w, lds128(at), cells_mask(c.mask, clamp8(x0 - xb), clamp8(x1 - xb))));
+            }
+        });
+    }
+}
+
+// The visit's last step: the new values go to the output plane (dst: the
+// blocks' first panel in this row), and the image's where they may not be
+// written (every grid cell of an owned row is stored: the fixed border has to
+// be in both planes).
+template <int G>
+__device__ __forceinline__ void step_to_plane(const WarpTile &c, int t, int x0, int x1, int nx,
+                                              bool owned, uint4 *dst, int nyp) {
+    const bool row = t <= c.tmax;
+    if (c.inner && __all_sync(0xffffffffu, row || !owned)) {
+        walk_blocks<G>(c.col, [&](int p, const uint4 &w) {
+            if (owned) dst[(size_t)p * nyp] = w;
+        });
+    } else {
+        walk_blocks<G>(c.col, [&](int p, const uint4 &w) {
+            const int xb = c.xf + 8 * p;
+            if (!owned || xb >= nx) return;
+            const int a = row ? clamp8(x0 - xb) : 8, b = row ? clamp8(x1 - xb) : 0;
+            dst[(size_t)p * nyp] =
+                a == 0 && b == 8 ? w : blend(w, lds128(c.img + p * SG::CHUNK), cells_mask(c.mask, a, b));
+        });
+    }
+}
+
+// Waits (bounded) for visit w.step - 1 of the tile and its neighbours: lane l
+// < 9 acquires the counter of neighbour l.  Called by a whole warp.
+__device__ __forceinline__ bool wait_neighbours(const unsigned *done, const TileWalk &w, int lane,
+                                                const volatile int *abort_flag) {
+    const int y = w.ty + lane / 3 - 1, x = w.tx + lane % 3 - 1;
+    const bool mine = lane < 9 && y >= 0 && y < w.tiles_y && x >= 0 && x < w.tiles_x;
+    const unsigned *ctr = done + (mine ? y * w.tiles_x + x : 0);
+    const unsigned target = (unsigned)w.step;
+    const uint64_t t0 = global_timer_ns();
+    // the error word and the clock, which take as long as a poll each, are
+    // read only now and then
+    for (int n = 1; !__all_sync(0xffffffffu, !mine || ld_acquire(ctr) >= target); n++) {
+        if (n % 32) continue;
+        const bool stop = *abort_flag || *(volatile int *)&g_visit_error != 0 ||
+                          global_timer_ns() - t0 > kWaitLimitNs;
+        if (__any_sync(0xffffffffu, stop)) return false;
+    }
+    return true;
+}
+
+// mbar_wait that polls for a while before it sleeps between polls: a step's
+// waits end within a microsecond, and a sleep that outlasts one costs a
+// quarter of a step.
+__device__ __forceinline__ bool mbar_wait_soon(uint64_t *bar, uint32_t parity,
+                                               const volatile int *abort_flag) {
+#pragma unroll 1
+    for (int n = 0; n < 64; n++)
+        if (mbar_try_wait(bar, parity)) return true;
+    return mbar_wait(bar, parity, abort_flag);
+}
+
+// G: a tile is W = 32 G columns wide, G blocks of 16 for each column half.
+template <int S, int G>
+__global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid_constant__ VisitParams p) {
+    constexpr int R = stencil_r(S);
+    constexpr int W = 32 * G;
+    constexpr int stage_bytes = visit_stage_bytes(W);
+    constexpr int NS = kVisitStages;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                                ~static_cast<uintptr_t>(1023));
+    uint8_t *stage_base = smem;                          // [NS]
+    uint8_t *band_base = smem + (size_t)NS * stage_bytes;  // [2R+1]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(band_base + (2 * R + 1) * kBandBytes);
+    uint64_t *full = bars;                        // [NS] tile loaded
+    uint64_t *empty = full + NS;                  // [NS] tile stored
+    uint64_t *acc_full = empty + NS;              // [slots] a step's MMAs complete
+    uint64_t *step_done = acc_full + kVisitSlots; // [slots] its results in the image (or registers)
+    uint64_t *drain = step_done + kVisitSlots;    // [1]
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    unsigned *stored = tmem_slot + 2;             // [slots] warps that stored their last step
+    static_assert((2 * NS + 2 * kVisitSlots + 1) * 8 + 8 + 4 * kVisitSlots <= kBarBytes, "barrier area");
+    uint32_t *masks = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(bars) + kBarBytes);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NS; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], kVisitEpi);
+        }
+        for (int b = 0; b < kVisitSlots; b++) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&step_done[b], kVisitEpi);
+            stored[b] = 0;
+        }
+        mbar_init(drain, kVisitSlots);
+        *abort_flag = 0;
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        __syncwarp();
+        tmem_alloc(tmem_slot, kTmemCols);
+        tmem_relinquish();
+    }
+    build_bands(reinterpret_cast<uint16_t *>(band_base), p.coef, R, stencil_box(S), false,
+                threadIdx.x, kVisitThreads);
+    build_masks(masks, threadIdx.x);
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const int tiles_x = p.tiles_x, tiles_y = p.tiles_y;
+    const int n_items = p.visits * tiles_x * tiles_y;  // (visit, tile), visit-major
+    const int H = kTile - 2 * p.halo;                  // rows from one tile row to the next
+    const int grid = (int)gridDim.x;
+    auto fail = [&](int code) {
+        record_error(&g_visit_error, code);
+        *abort_flag = 1;
+    };
+
+    if (warp == 0) {
+        // ------------------------------------------------------ producer ---
+        int i = 0, last_issued = -1;
+        TileWalk w;
+        w.init(blockIdx.x, grid, tiles_x, tiles_y);
+        for (int k = blockIdx.x; k < n_items; k += grid, i++, w.advance()) {
+            const int s = i % NS;
+            if (w.step > 0 && !wait_neighbours(p.done, w, lane, abort_flag)) {
+                if (lane == 0) fail(kErrWaitDep);
+                break;
+            }
+            int ok = 1;
+            if (lane == 0) {
+                ok = mbar_wait(&empty[s], ((i / NS) & 1) ^ 1, abort_flag);
+                if (ok) {
+                    fence_proxy_async_global();  // the copy reads what other SMs stored
+                    mbar_arrive_expect_tx(&full[s], (uint32_t)stage_bytes);
+                    tma_load_3d(stage_base + (size_t)s * stage_bytes, &p.map[w.step & 1], &full[s],
+                                0, w.ty * H / p.map_rows, w.tx * W / 8);
+                } else {
+                    fail(kErrWaitEmpty);
+                }
+            }
+            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+            last_issued = i;
+        }
+        // every stage armed last must have landed before exit
+        if (lane == 0) {
+            for (int k = 0; k < NS && last_issued - k >= 0; k++) {
+                const int ii = last_issued - k;
+                const uint64_t t0 = global_timer_ns();
+                while (!mbar_try_wait(&full[ii % NS], (ii / NS) & 1)) {
+                    if (global_timer_ns() - t0 > kWaitLimitNs) {
+                        record_error(&g_visit_error, kErrWaitDrain);
+                        break;
+                    }
+                }
+            }
+        }
+    } else if (warp < kVisitEpi0) {
+        // --------------------------------------------------- MMA issuers ---
+        if (lane == 0) {
+            const int id = warp - 1;  // its slot: tiles i with i % slots == id
+            const uint32_t band = smem_u32(band_base);
+            const uint32_t d = tmem_base + (uint32_t)(id * kVisitSlotCols);
+            bool stop = false;
+            uint32_t e = 0;  // the slot's steps so far
+            TileWalk w;
+            w.init(blockIdx.x + id * grid, kVisitSlots * grid, tiles_x, tiles_y);
+            int i = id;
+            for (int k = blockIdx.x + id * grid; k < n_items && !stop;
+                 k += kVisitSlots * grid, i += kVisitSlots, w.advance()) {
+                const int s = i % NS;
+                if (!mbar_wait_soon(&full[s], (i / NS) & 1, abort_flag)) {
+                    fail(kErrWaitFull);
+                    break;
+                }
+                const uint64_t a0 = smem_desc(smem_u32(stage_base + (size_t)s * stage_bytes), SG::CHUNK, 128);
+                const int T = p.base + (w.step < p.extra ? 1 : 0);
+                const int nwin = tile_windows(p.g.nx, w.tx * W, W);
+                for (int t = 0; t < T; t++, e++) {
+                    // the slot's previous step has been read out (and, within
+                    // a visit, written to the image)
+                    if (e > 0 && !mbar_wait_soon(&step_done[id], (e - 1) & 1, abort_flag)) {
+                        fail(kErrWaitAccum);
+                        stop = true;
+                        break;
+                    }
+                    tc_fence_after();
+                    issue_visit_tile<R, W / 16 + 1>(a0, band, d, nwin);
+                    umma_commit(&acc_full[id]);
+                }
+            }
+            umma_commit(drain);  // completes at once if nothing is in flight
+            const uint64_t t0 = global_timer_ns();
+            while (!mbar_try_wait(drain, 0)) {
+                if (global_timer_ns() - t0 > kWaitLimitNs) {
+                    record_error(&g_visit_error, kErrWaitDrain);
+                    break;
+                }
+            }
+        }
+    } else {
+        // ------------------------------------------------------ epilogue ---
+        const int slot = (warp - kVisitEpi0) / kVisitEpi;
+        const int half = ((warp - kVisitEpi0) >> 2) & 1;
+        const int q = warp & 3;       // TMEM lane quarter
+        const int m = q * 32 + lane;  // tile row
+        const uint32_t lane_col =
+            tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(slot * kVisitSlotCols);
+        const GridGeom &g = p.g;
+        uint32_t e = 0;  // the slot's steps so far
+        bool stop = false;
+        WarpTile c;
+        c.col = lane_col + 16 * (half * G + 1);
+        c.ecol = lane_col + (half ? 16 + W : 8);
+        c.mask = smem_u32(masks);
+        TileWalk w;
+        w.init(blockIdx.x + slot * grid, kVisitSlots * grid, tiles_x, tiles_y);
+        int i = slot;
+        for (int k = blockIdx.x + slot * grid; k < n_items && !stop;
+             k += kVisitSlots * grid, i += kVisitSlots, w.advance()) {
+            const int s = i % NS;
+            const int T = p.base + (w.step < p.extra ? 1 : 0);
+            const int X0 = w.tx * W;
+            const int y = w.ty * H + m;
+            const bool top = w.ty == 0, bottom = w.ty == tiles_y - 1;
+            c.xf = X0 + 16 * half * G;
+            c.ex = half ? X0 + W : X0 - 8;
+            const uint32_t row0 = smem_u32(stage_base) + (uint32_t)(s * stage_bytes + (m + SG::TOP) * 16);
+            c.img = row0 + (uint32_t)((1 + 2 * half * G) * SG::CHUNK);
+            c.eimg = row0 + (uint32_t)((half ? 4 * G + 1 : 0) * SG::CHUNK);
+            c.inner = min(c.xf, c.ex) >= g.x0 && max(c.xf + 16 * G, c.ex + 8) <= g.x1;
+            if (!c.inner) {
+                c.q0 = (g.x0 - c.xf) >> 3;
+                c.p0 = (g.x0 - c.xf + 7) >> 3;
+                c.p1 = (g.x1 - c.xf) >> 3;
+                c.q1 = (g.x1 - c.xf + 7) >> 3;
+                c.ea = clamp8(g.x0 - c.ex);
+                c.eb = clamp8(g.x1 - c.ex);
+            }
+            // rows whose neighbourhood is all of step t-1: R fewer a step,
+            // except at the grid's own top and bottom
+            c.tmax = y >= g.y0 && y < g.y1
+                         ? min(top ? kTile : m / R + 1, bottom ? kTile : (kTile - 1 - m) / R + 1)
+                         : 0;
+            for (int t = 1; t <= T; t++, e++) {
+                bool ok = mbar_wait_soon(&acc_full[slot], e & 1, abort_flag);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    if (lane == 0) fail(kErrWaitResult);
+                    stop = true;
+                    break;
+                }
+                tc_fence_after();
+                if (t < T) {
+                    step_to_image<G, R>(c, half, t, g.x0, g.x1);
+                    fence_proxy_async_smem();  // the next step's MMAs read the image
+                } else {
+                    const bool owned = y < g.ny && (top || m >= p.halo) && (bottom || m < kTile - p.halo);
+                    uint4 *dst = reinterpret_cast<uint4 *>(p.plane[(w.step & 1) ^ 1] +
+                                                           plane_index16(g.p16, owned ? y : 0, c.xf));
+                    step_to_plane<G>(c, t, g.x0, g.x1, g.nx, owned, dst, g.p16.nyp);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&step_done[slot]);
+                    if (t == T) {
+                        mbar_arrive(&empty[s]);
+                        // the tile's last warp publishes it: the warps' stores
+                        // are ordered by the barrier above and this count, and
+                        // visible to whoever acquires the tile's counter
+                        if (w.step + 1 < p.visits &&
+                            add_acq_rel_cta(&stored[slot], 1u) % kVisitEpi == kVisitEpi - 1)
+                            red_release_add(p.done + w.ty * tiles_x + w.tx, 1u);
+                    }
+                }
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) {
+        __syncwarp();
+        tmem_dealloc(tmem_base, kTmemCols);
+    }
+    // The last CTA to end leaves the counters zero for the next launch (a
+    // memset before each launch took a tenth of a 256², 10-step run).
+    if (p.visits > 1) {
+        if (threadIdx.x == 0) {
+            fence_acq_rel_gpu();
+            *tmem_slot = atomicAdd(p.ended, 1u) == (unsigned)grid - 1;
+            fence_acq_rel_gpu();
+        }
+        __syncthreads();
+        if (*tmem_slot) {
+            for (int t = threadIdx.x; t < tiles_x * tiles_y; t += kVisitThreads) p.done[t] = 0;
+            if (threadIdx.x == 0) *p.ended = 0;
+        }
+    }
+}
+
+// One CTA per SM: two would share TMEM, of which each takes all, and the CTAs
+// of a launch wait on one another.
+size_t visit_smem(int R, int W) {
+    const size_t need = 1024 + (size_t)kVisitStages * visit_stage_bytes(W) + (2 * R + 1) * kBandBytes + kBarBytes + kMaskBytes;
+    return need > 120 * 1024 ? need : 120 * 1024;
+}
+
+template <int S, int G>
+cudaError_t launch_visit_w(VisitParams &p, int sms, cudaStream_t s) {
+    const int tiles = p.tiles_x * p.tiles_y;
+    const int grid = tiles < sms ? tiles : sms;
+    return launch_step(tc_visit_kernel<S, G>, grid, kVisitThreads, visit_smem(stencil_r(S), 32 * G),
+                       s, p, true);
+}
+template <int S>
+cudaError_t launch_visit(VisitParams &p, int w, int sms, cudaStream_t s) {
+    return w == 128  ? launch_visit_w<S, 4>(p, sms, s)
+           : w == 96 ? launch_visit_w<S, 3>(p, sms, s)
+           : w == 64 ? launch_visit_w<S, 2>(p, sms, s)
+                     : launch_visit_w<S, 1>(p, sms, s);
+}
+
+template <int S, int G>
+cudaError_t prepare_visit_w() {
+    return cudaFuncSetAttribute(tc_visit_kernel<S, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)visit_smem(stencil_r(S), 32 * G));
+}
+template <int S>
+cudaError_t prepare_visit() {
+    static bool configured = false;
+    if (configured) return cudaSuccess;
+    cudaError_t e = prepare_visit_w<S, 1>();
+    if (e == cudaSuccess) e = prepare_visit_w<S, 2>();
+    if (e == cudaSuccess) e = prepare_visit_w<S, 3>();
+    if (e == cudaSuccess) e = prepare_visit_w<S, 4>();
+    configured = e == cudaSuccess;
+    return e;
+}
+
+}  // namespace
+
+// The tile width and halo of a sweep, from a model of a step's SM cycles that
+// was fitted to sweeps of 128² to 16386² (M: a tile's MMAs; L: from the last
+// MMA of a step to the slot's next one; B: from a visit's last step to the
+// next visit's first MMA; n tiles per SM):
+//   step = max(n M, M + L, n (M + L) / 2),  visit = T step + B (2 B / n, n > 2)
+// Narrow tiles have short steps and more SMs, wide ones fewer MMAs per cell;
+// halo 8 takes more steps per visit, halo 4 fewer rows twice, and halo 2
+// (whose copies move half lines) pays only for radius 2 with many tiles,
+// where T = 2 already takes the sweep off the memory bound.  The model's
+// choice measured within 3 % of the best of W = 32, 64, 96, 128 with every
+// halo at all but one of 30 grids (6 % at 1026², 10 steps, box2d2r); box2d2r,
+// us per step, W 32 / 64 / 96 / 128: 256² 1.47 / 1.90 / 2.34 / 2.88, 1026²
+// 1.70 / 2.13 / 2.36 / 2.82, 2048² 4.05 / 3.08 / 3.15 / 3.41, 8196² - / - /
+// 40.0 / 40.7.  The best form against one launch per step (radius 1 star /
+// radius 2 box): 256² 3.50 -> 1.03 / 3.79 -> 1.47, 1026² 4.09 -> 1.32 /
+// 4.52 -> 1.70, 4096² 11.2 -> 6.96 / 12.7 -> 10.0; against one step per tile
+// visit in one launch: 8196² 42.1 -> 26.9 / 41.5 -> 40.0, 16386² 169 -> 107 /
+// 167 -> 158 (5792², radius 2, whose planes nearly fit L2: 19.75 -> 20.0).
+VisitShape visit_shape(int ny, int nx, int stencil, int steps, int tile_w, int sms) {
+    const int r = stencil_r(stencil);
+    VisitShape best{};
+    double best_cost = 0.0;
+    for (int w = 32; w <= kTile; w += 32) {
+        if (tile_w != kTile && w != tile_w) continue;  // a width the caller set stays
+        for (int halo = 2; halo <= 8; halo *= 2) {
+            const int h = kTile - 2 * halo;
+            VisitShape v;
+            v.tile_w = w;
+            v.halo = halo;
+            v.tiles_x = (nx + w - 1) / w;
+            v.tiles_y = ny <= kTile ? 1 : (ny - 2 * halo + h - 1) / h;
+            const int by_rows = halo / r + 1, by_cols = 8 / r;
+            const int depth = by_rows < by_cols ? by_rows : by_cols;
+            v.visits = (steps + depth - 1) / depth;
+            double n = (double)v.tiles_x * v.tiles_y / sms;
+            if (n < 1.0) n = 1.0;
+            if (halo == 2 && (r == 1 || n <= 4.0)) continue;
+            const double per_mma = r == 1 ? 66.0 : w == 96 ? 61.0 : 64.0;
+            const double m = per_mma * (w / 16 + 1) * (2 * r + 1), l = 800.0 + 9.0 * w;
+            double step = n * m;
+            if (step < m + l) step = m + l;
+            if (step < n * (m + l) / 2) step = n * (m + l) / 2;
+            const double cost = steps * step + v.visits * 4750.0 * (n > 2.0 ? 2.0 / n : 1.0);
+            if (!best.visits || cost < best_cost) {
+                best = v;
+                best_cost = cost;
+            }
+        }
+    }
+    return best;
+}
+
+cudaError_t visit_prepare(int stencil) {
+    switch (stencil) {
+    case TCS_STAR2D1R: return prepare_visit<TCS_STAR2D1R>();
+    case TCS_STAR2D2R: return prepare_visit<TCS_STAR2D2R>();
+    case TCS_BOX2D1R: return prepare_visit<TCS_BOX2D1R>();
+    case TCS_BOX2D2R: return prepare_visit<TCS_BOX2D2R>();
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_tc_f16_visits(const GridGeom &g, int stencil, const float *B, uint16_t *in,
+                                 uint16_t *out, int steps, const VisitShape &v,
+                                 unsigned *counters, cudaStream_t s, int sms) {
+    if (steps < 1 || v.visits < 1 || !counters) return cudaErrorInvalidValue;
+    VisitParams p;
+    p.g = g;
+    p.tiles_x = v.tiles_x;
+    p.tiles_y = v.tiles_y;
+    p.halo = v.halo;
+    p.map_rows = v.halo == 2 ? 4 : 8;  // tile rows start at multiples of 124, 120 or 112
+    p.visits = v.visits;
+    p.base = steps / v.visits;
+    p.extra = steps % v.visits;
+    p.ended = counters;
+    p.done = counters + kRowCounterStride;  // a line of its own each
+    p.plane[0] = in;
+    p.plane[1] = out;
+    cudaError_t e = encode_panel_map(in, g.p16, &p.map[0], v.tile_w / 8 + 2, p.map_rows);
+    if (e == cudaSuccess) e = encode_panel_map(out, g.p16, &p.map[1], v.tile_w / 8 + 2, p.map_rows);
+    if (e != cudaSuccess) return e;
+    const int n = 2 * stencil_r(stencil) + 1;
+    for (int k = 0; k < 25; k++) p.coef[k] = k < n * n ? B[k] : 0.0f;
+    switch (stencil) {
+    case TCS_STAR2D1R: return launch_visit<TCS_STAR2D1R>(p, v.tile_w, sms, s);
+    case TCS_STAR2D2R: return launch_visit<TCS_STAR2D2R>(p, v.tile_w, sms, s);
+    case TCS_BOX2D1R: return launch_visit<TCS_BOX2D1R>(p, v.tile_w, sms, s);
+    case TCS_BOX2D2R: return launch_visit<TCS_BOX2D2R>(p, v.tile_w, sms, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t visit_take_error(int *code) {
+    int zero = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(code, g_visit_error, sizeof(int));
+    if (e != cudaSuccess) return e;
+    return *code ? cudaMemcpyToSymbol(g_visit_error, &zero, sizeof(int)) : cudaSuccess;
+}
+
+}  // namespace tcs

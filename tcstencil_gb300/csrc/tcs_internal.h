@@ -96,8 +96,11 @@ struct GridGeom {
 // (16 words = 8 rows of a panel, nyp / 8 row groups, npan panels), box
 // (16, 17, 18) = the 136 rows from Y0 - 4 of the 18 panels a 128 x 128 tile
 // reads, landing in shared memory as 18 row-contiguous 2176-byte runs (one
-// load instruction per plane and tile instead of 18 bulk copies).
-cudaError_t encode_panel_map(const uint16_t *plane, const PlaneGeom &pg, CUtensorMap *map);
+// load instruction per plane and tile instead of 18 bulk copies); or the
+// `panels` = W/8 + 2 panels of a tile W columns wide, and lines of `rows` = 4
+// rows (64 bytes) for tile rows that start at multiples of 4.
+cudaError_t encode_panel_map(const uint16_t *plane, const PlaneGeom &pg, CUtensorMap *map,
+                             int panels = kTile / 8 + 2, int rows = 8);
 
 // Sets the thread's last-error message and returns `status`.
 int fail(int status, const char *fmt, ...);
@@ -165,14 +168,27 @@ cudaError_t tc_prepare(int stencil, bool split);
 
 cudaError_t launch_tc_f16(const GridGeom &g, int stencil, const float *B, const uint16_t *in,
                           uint16_t *out, cudaStream_t s, int tile_w = kTile);
-// Several plain steps in one launch (in -> out -> in ...); rows_done: one
+// Several split steps in one launch (in -> out -> in ...); rows_done: one
 // counter per tile row (ceil(ny / 128)) every kRowCounterStride unsigneds,
 // zeroed before the launch.  Each counter has its own 128-byte line: every SM
 // polls and counts them, and on shared lines those accesses serialise.
 constexpr int kRowCounterStride = 32;
-cudaError_t launch_tc_f16_steps(const GridGeom &g, int stencil, const float *B, const uint16_t *in,
-                                uint16_t *out, int steps, unsigned *rows_done, cudaStream_t s,
-                                int tile_w = kTile);
+// Several plain steps per tile visit (sweep_visit.cu): `visits` loads and
+// stores of every tile carry `steps` steps between them, in one launch
+// (in -> out -> in ..., one flip per visit); counters: visit_counter_words of
+// zeros, which a launch leaves zero again.
+struct VisitShape {
+    int tile_w, tiles_x, tiles_y, halo, visits;
+};
+VisitShape visit_shape(int ny, int nx, int stencil, int steps, int tile_w, int sms);
+constexpr size_t visit_counter_words(int ny, int nx) {
+    return kRowCounterStride + (size_t)(ny / (kTile - 16) + 2) * ((nx + 31) / 32);
+}
+cudaError_t visit_prepare(int stencil);
+cudaError_t launch_tc_f16_visits(const GridGeom &g, int stencil, const float *B, uint16_t *in,
+                                 uint16_t *out, int steps, const VisitShape &v,
+                                 unsigned *counters, cudaStream_t s, int sms);
+cudaError_t visit_take_error(int *code);
 cudaError_t launch_tc_split_steps(const GridGeom &g, int stencil, const float *B,
                                   const uint16_t *in_hi, const uint16_t *in_lo, uint16_t *out_hi,
                                   uint16_t *out_lo, int steps, unsigned *rows_done, cudaStream_t s,
