@@ -357,7 +357,7 @@ struct tcs_plan_s {
     void *buf[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [state][hi, lo]
     int cur = 0;
     SplitScale *d_scale = nullptr;  // split form: per-step scale; the planes hold x 2^-E
-    unsigned *d_max = nullptr;      // split form: max |x| scratch (float bits)
+    unsigned *d_upload = nullptr;   // split form: launch_split_upload scratch
     float *staging = nullptr;   // ny*nx FP32, for host/row-major transfers
     // host transfers in row bands: packing (unpacking) of one band on `aux`
     // while the next band's copy runs on the caller's stream
@@ -381,7 +381,7 @@ struct tcs_plan_s {
             for (auto &p : s)
                 if (p) dev_free(p);
         if (staging) dev_free(staging);
-        if (d_max) dev_free(d_max);
+        if (d_upload) dev_free(d_upload);
         if (d_scale) dev_free(d_scale);
         if (rows_done) dev_free(rows_done);
         for (cudaEvent_t e : band_ev)
@@ -563,6 +563,8 @@ int tcs_plan_create(const tcs_problem *pr, tcs_plan *out) {
     if (pr->precision == TCS_PREC_SPLIT) {
         st = dev_alloc_t(&p->d_scale, sizeof(SplitScale), "scale");
         if (!st) st = cuda_status(cudaMemset(p->d_scale, 0, sizeof(SplitScale)), "cudaMemset(scale)");
+        if (!st) st = dev_alloc_t(&p->d_upload, kUploadScratch * sizeof(unsigned), "max");
+        if (!st) st = cuda_status(cudaMemset(p->d_upload, 0, kUploadScratch * sizeof(unsigned)), "cudaMemset(max)");
         if (st) return st;
     }
     if (pr->engine == TCS_ENGINE_TENSOR) {
@@ -640,21 +642,10 @@ int tcs_plan_upload(tcs_plan p, const float *grid, int on_host, void *stream) {
     if (p->prob.precision == TCS_PREC_F32)
         e = launch_pack_f32(src, p->prob.ny, p->prob.nx, 0, 0.0f, static_cast<float *>(p->buf[0][0]), s);
     else if (p->prob.precision == TCS_PREC_SPLIT) {
-        // scale so that max |x| 2^-E < 1, all on the device: the maximum, the
-        // packing with its exponent, and the scale record's starting history
-        int st = TCS_OK;
-        if (!p->d_max) st = dev_alloc_t(&p->d_max, sizeof(unsigned), "max");
-        if (!st) st = cuda_status(cudaMemsetAsync(p->d_max, 0, sizeof(unsigned), s), "memset(max)");
-        if (!st) st = cuda_status(launch_max_abs(src, (size_t)p->prob.ny * p->prob.nx, p->d_max, s), "max_abs launch");
-        if (!st)
-            st = cuda_status(launch_pack_split_dev(src, p->prob.ny, p->prob.nx, p->d_max, nullptr,
-                                                   static_cast<uint16_t *>(p->buf[0][0]),
-                                                   static_cast<uint16_t *>(p->buf[0][1]), s),
-                             "pack launch");
-        if (st) return st;
-        e = launch_split_scale_init(p->d_scale, p->d_max, p->g,
-                                    static_cast<const uint16_t *>(p->buf[0][0]),
-                                    static_cast<const uint16_t *>(p->buf[0][1]), s);
+        // scaled so that max |x| 2^-E < 1, all on the device
+        e = launch_split_upload(src, p->g, p->d_upload, p->d_scale,
+                                static_cast<uint16_t *>(p->buf[0][0]),
+                                static_cast<uint16_t *>(p->buf[0][1]), s);
     }
     else
         e = launch_pack_f16(src, p->prob.ny, p->prob.nx, 0, 0.0f, static_cast<uint16_t *>(p->buf[0][0]), s);

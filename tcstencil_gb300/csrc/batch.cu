@@ -798,7 +798,7 @@ struct tcs_batch_s {
     float *d_coefs = nullptr;
     float *d_staging = nullptr;
     size_t staging_elems = 0;
-    unsigned *d_max = nullptr;
+    unsigned *d_upload = nullptr;    // [entry] launch_split_upload scratch
     SplitScale *d_scales = nullptr;  // [entry] the split grids' per-step scales
     long long point_updates = 0;
     bool built = false;
@@ -814,7 +814,7 @@ struct tcs_batch_s {
         for (void *p : {(void *)pool, (void *)d_grids, (void *)d_maps, (void *)part[0].d_layout,
                         (void *)part[0].d_counters, (void *)part[1].d_layout,
                         (void *)part[1].d_counters, (void *)d_bands, (void *)d_coefs,
-                        (void *)d_staging, (void *)d_max, (void *)d_scales})
+                        (void *)d_staging, (void *)d_upload, (void *)d_scales})
             if (p) dev_free(p);
     }
 
@@ -857,6 +857,9 @@ int batch_build(tcs_batch b) {
     }
     if (!st) st = dev_alloc_t(&b->d_scales, b->entries.size() * sizeof(SplitScale), "scales");
     if (!st) st = cuda_status(cudaMemset(b->d_scales, 0, b->entries.size() * sizeof(SplitScale)), "cudaMemset(scales)");
+    const size_t upload_bytes = b->entries.size() * kUploadScratch * sizeof(unsigned);
+    if (!st) st = dev_alloc_t(&b->d_upload, upload_bytes, "max");
+    if (!st) st = cuda_status(cudaMemset(b->d_upload, 0, upload_bytes), "cudaMemset(max)");
     if (st) return st;
     b->pool_elems = total;
     // descriptors (FP16 grids then split grids, each sorted by steps,
@@ -1043,15 +1046,10 @@ int tcs_batch_upload(tcs_batch b, int index, const float *grid, int on_host, voi
     const int cur = b->state_of(e);
     uint16_t *hi = b->pool + e.offset[cur][0];
     if (e.prob.precision == TCS_PREC_SPLIT) {
-        // scale so that max |x| 2^-E < 1, on the device: the maximum, the
-        // packing with its exponent, and the scale record's starting history
-        if (!b->d_max) st = dev_alloc_t(&b->d_max, sizeof(unsigned), "max");
-        if (!st) st = cuda_status(cudaMemsetAsync(b->d_max, 0, sizeof(unsigned), s), "memset(max)");
-        if (!st) st = cuda_status(launch_max_abs(src, cells, b->d_max, s), "max_abs launch");
-        if (!st) st = cuda_status(launch_pack_split_dev(src, e.g.ny, e.g.nx, b->d_max, nullptr, hi,
-                                                        b->pool + e.offset[cur][1], s), "pack launch");
-        if (!st) st = cuda_status(launch_split_scale_init(b->d_scales + index, b->d_max, e.g, hi,
-                                                          b->pool + e.offset[cur][1], s), "scale init");
+        // scaled so that max |x| 2^-E < 1, all on the device
+        st = cuda_status(launch_split_upload(src, e.g, b->d_upload + kUploadScratch * (size_t)index,
+                                             b->d_scales + index, hi, b->pool + e.offset[cur][1], s),
+                         "pack launch");
     } else {
         st = cuda_status(launch_pack_f16(src, e.g.ny, e.g.nx, 0, 0.0f, hi, s), "pack launch");
     }

@@ -5,9 +5,8 @@
 //    device kernels (16 x 16 bricks, row-major inside a brick).
 //  - pack / unpack between FP32 row-major grids and the engine's panel
 //    planes: array_float2half (common/common.hpp:146-160) + padding_2D +
-//    layout change in one pass, and the inverse.  One thread writes or reads
-//    one 16-byte panel row, so plane-side accesses are 128-bit and
-//    consecutive threads touch consecutive bytes of a panel.
+//    layout change in one pass, and the inverse, by blocks of 32 rows by 32
+//    panels through shared memory.
 #include "tcs_device.cuh"
 #include "tcs_internal.h"
 
@@ -27,71 +26,25 @@ __device__ __forceinline__ float h2f_bits(uint16_t b) {
     return __half2float(h);
 }
 
-// Value of padded-grid cell (Y, X) of a (ny+2pad) x (nx+2pad) grid whose
-// interior is the FP32 row-major input; 0 outside the padded grid.
-__device__ __forceinline__ float padded_cell(const float *in, int ny, int nx, int pad,
-                                             float pad_value, int Y, int X) {
-    if (Y < 0 || X < 0 || Y >= ny + 2 * pad || X >= nx + 2 * pad) return 0.0f;
-    const int iy = Y - pad, ix = X - pad;
-    return (iy >= 0 && iy < ny && ix >= 0 && ix < nx) ? in[(size_t)iy * nx + ix] : pad_value;
-}
+// pack and unpack move a block of kBlkRows plane rows by kBlkPans panels
+// through shared memory, so that both sides are contiguous: a warp's accesses
+// of the FP32 grid are runs of 32 cells of one row, its accesses of a plane
+// 32 rows of one panel (512 bytes).  (With one 16-byte panel row per thread
+// straight to the plane, each was half a 32-byte sector, a plane row apart:
+// 16386² split up- and download took 2.25 ms of a 50-step solve's 19.9 ms,
+// 0.8 ms at the memory rate.)  The grid side uses 4-byte accesses, so a grid
+// and its rows may start at any float.
+constexpr int kBlkRows = 32, kBlkPans = 32;
+constexpr int kBlkPitch = kBlkPans * 16 + 16;  // bytes of a staged plane row (16: no bank conflicts)
+enum PackMode { kPackF16, kPackF32, kPackSplit };
 
-// A panel row: thread id -> (plane row, panel) -> first cell (Y, X0) of the
-// padded grid and the row's index q in the plane.  Consecutive threads take
-// consecutive panels of one plane row, so that the row-major FP32 side of a
-// warp's accesses is one contiguous run (the plane side is one 16-byte panel
-// row per thread; the next plane row of a panel follows a few warps later).
-struct PanelRow {
-    int Y, X0;
-    size_t q;
+struct BlockPos {
+    int row, pan;  // first plane row and panel
 };
-__device__ __forceinline__ PanelRow panel_row(size_t id, const PlaneGeom &p, int q0 = 0) {
-    PanelRow r;
-    const int yl = static_cast<int>(id / p.npan);  // row within the range
-    const int yq = q0 + yl;
-    const int pan = static_cast<int>(id - (size_t)yl * p.npan);
-    r.Y = yq - kPadTop;
-    r.X0 = (pan - 1) * p.cpp;
-    r.q = (size_t)pan * p.nyp + yq;
-    return r;
-}
-
-// The N cells (Y, X0 .. X0+N-1) of the padded grid (padded_cell), by 16-byte
-// loads where they are all interior and 16-byte aligned.
-template <int N>
-__device__ __forceinline__ void load_cells(const float *__restrict__ in, int ny, int nx, int pad,
-                                           float pad_value, int Y, int X0, float (&c)[N]) {
-    const int iy = Y - pad, ix = X0 - pad;
-    const size_t e = (size_t)iy * nx + ix;
-    if (iy >= 0 && iy < ny && ix >= 0 && ix + N <= nx && (e & 3) == 0) {
-#pragma unroll
-        for (int k = 0; k < N; k += 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(in + e + k);
-            c[k] = v.x; c[k + 1] = v.y; c[k + 2] = v.z; c[k + 3] = v.w;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < N; i++) c[i] = padded_cell(in, ny, nx, pad, pad_value, Y, X0 + i);
-    }
-}
-
-// Stores the grid cells among (Y, X0 .. X0+N-1) of the padded grid into the
-// ny x nx row-major output, by 16-byte stores where all N are and aligned.
-template <int N>
-__device__ __forceinline__ void store_cells(float *__restrict__ out, int ny, int nx, int pad,
-                                            int Y, int X0, const float (&c)[N]) {
-    const int iy = Y - pad, ix = X0 - pad;
-    if (iy < 0 || iy >= ny) return;
-    const size_t e = (size_t)iy * nx + ix;
-    if (ix >= 0 && ix + N <= nx && (e & 3) == 0) {
-#pragma unroll
-        for (int k = 0; k < N; k += 4)
-            *reinterpret_cast<float4 *>(out + e + k) = make_float4(c[k], c[k + 1], c[k + 2], c[k + 3]);
-    } else {
-#pragma unroll
-        for (int i = 0; i < N; i++)
-            if (ix + i >= 0 && ix + i < nx) out[(size_t)iy * nx + (ix + i)] = c[i];
-    }
+__device__ __forceinline__ BlockPos block_pos(const PlaneGeom &p, int q0) {
+    const int npb = (p.npan + kBlkPans - 1) / kBlkPans;
+    const int rb = (int)(blockIdx.x / npb);
+    return BlockPos{q0 + rb * kBlkRows, (int)(blockIdx.x - (unsigned)rb * npb) * kBlkPans};
 }
 
 // Split storage of x: x' = x 2^-E, hi = fp16(rint(x' 2^11) 2^-11) (fixed
@@ -103,56 +56,163 @@ __device__ __forceinline__ void split_value(float x, float scale, uint16_t &h, u
     l = f2h_bits((xs - h2f_bits(h)) * 2048.0f);
 }
 
-__global__ void pack_f16_kernel(const float *__restrict__ in, int ny, int nx, int pad,
-                                float pad_value, uint16_t *__restrict__ out, PlaneGeom p,
-                                size_t n_rows, int q0) {
-    const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n_rows) return;
-    const PanelRow r = panel_row(id, p, q0);
-    float c[8];
-    load_cells<8>(in, ny, nx, pad, pad_value, r.Y, r.X0, c);
-    uint32_t w[4];
+// Plane rows [q0, q1) of the padded grid.  Split: scaled by 2^-E, E from
+// `sc` when given (and the largest |x'| of the cells outside the update
+// rectangle [y0, y1) x [x0, x1) added to its border maximum), else `scale`.
+struct PackArgs {
+    const float *in;
+    int ny, nx, pad;
+    float pad_value;
+    void *out, *out_lo;
+    PlaneGeom p;
+    int q0, q1;
+    float scale;
+    SplitScale *sc;
+    int y0, y1, x0, x1;
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads) pack_kernel(const PackArgs a) {
+    constexpr int CPP = MODE == kPackF32 ? 4 : 8;
+    constexpr int CELLS = kBlkPans * CPP;  // of a block's row
+    constexpr int N = CELLS / 32, K = kBlkRows / 8;
+    __shared__ __align__(16) uint8_t buf[MODE == kPackSplit ? 2 : 1][kBlkRows][kBlkPitch];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const BlockPos b = block_pos(a.p, a.q0);
+    const int X = (b.pan - 1) * CPP + lane;  // this lane's first cell: X, X + 32, ...
+    pdl_launch_dependents();
+    pdl_wait();
+    float v[K][N];
 #pragma unroll
-    for (int i = 0; i < 4; i++) w[i] = f2h_bits(c[2 * i]) | ((uint32_t)f2h_bits(c[2 * i + 1]) << 16);
-    reinterpret_cast<uint4 *>(out)[r.q] = make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-__global__ void unpack_f16_kernel(const uint16_t *__restrict__ in, int ny, int nx, int pad,
-                                  float *__restrict__ out, PlaneGeom p, size_t n_rows, int q0) {
-    const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n_rows) return;
-    const PanelRow r = panel_row(id, p, q0);
-    const int iy = r.Y - pad;
-    if (iy < 0 || iy >= ny) return;
-    const uint4 v = reinterpret_cast<const uint4 *>(in)[r.q];
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    float c[8];
+    for (int k = 0; k < K; k++) {
+        const int Y = b.row + warp + 8 * k - kPadTop;
+        const int iy = Y - a.pad, ix = X - lane - a.pad;
+        // (rows from q1 on belong to a later range: not read)
+        const bool row_in = iy >= 0 && iy < a.ny && b.row + warp + 8 * k < a.q1;
+        const float *src = a.in + (size_t)(row_in ? iy : 0) * a.nx;
+        if (row_in && ix >= 0 && ix + CELLS <= a.nx) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) c[i] = h2f_bits((uint16_t)(w[i >> 1] >> (16 * (i & 1))));
-    store_cells<8>(out, ny, nx, pad, r.Y, r.X0, c);
+            for (int i = 0; i < N; i++) v[k][i] = src[ix + lane + 32 * i];
+        } else {
+            // border and padding cells: the loads clamped to the row and the
+            // values selected, so that they all are in flight at once
+            const bool row_pad = Y >= 0 && Y < a.ny + 2 * a.pad;
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const int x = ix + lane + 32 * i;
+                const float c = row_in ? src[min(max(x, 0), a.nx - 1)] : 0.0f;
+                const bool pad_in = row_pad && x >= -a.pad && x < a.nx + a.pad;
+                v[k][i] = row_in && x >= 0 && x < a.nx ? c : pad_in ? a.pad_value : 0.0f;
+            }
+        }
+    }
+    float scale = a.scale;
+    bool border = false;  // the block may hold cells outside the update rectangle
+    if (MODE == kPackSplit && a.sc) {
+        scale = ldexpf(1.0f, -a.sc->bexp);
+        const int ya = b.row - kPadTop, xa = X - lane;
+        border = ya < a.y0 || ya + kBlkRows > a.y1 || xa < a.x0 || xa + CELLS > a.x1;
+    }
+    float m = 0.0f;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const int r = warp + 8 * k;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int c = lane + 32 * i;
+            if (MODE == kPackF32) {
+                reinterpret_cast<float *>(buf[0][r])[c] = v[k][i];
+            } else if (MODE == kPackF16) {
+                reinterpret_cast<uint16_t *>(buf[0][r])[c] = f2h_bits(v[k][i]);
+            } else {
+                uint16_t h, l;
+                split_value(v[k][i], scale, h, l);
+                reinterpret_cast<uint16_t *>(buf[0][r])[c] = h;
+                reinterpret_cast<uint16_t *>(buf[MODE == kPackSplit][r])[c] = l;
+                if (border) {
+                    const int y = b.row + r - kPadTop, x = X + 32 * i;
+                    const bool in_grid = y >= 0 && y < a.ny && x >= 0 && x < a.nx && b.row + r < a.q1;
+                    if (in_grid && !(y >= a.y0 && y < a.y1 && x >= a.x0 && x < a.x1))
+                        m = fmaxf(m, fabsf(fmaf(h2f_bits(h), 2048.0f, h2f_bits(l))));
+                }
+            }
+        }
+    }
+    if (border) {  // |x'| 2^11 = |hi 2^11 + lo|, rounded once to FP32
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0 && m > 0.0f) atomicMax(&a.sc->bmax, __float_as_uint(m * (1.0f / 2048.0f)));
+    }
+    __syncthreads();
+    const int row = b.row + lane;
+    if (row >= a.q1) return;
+#pragma unroll
+    for (int k = 0; k < kBlkPans / 8; k++) {
+        const int j = warp + 8 * k, pan = b.pan + j;
+        if (pan >= a.p.npan) continue;
+        const size_t q = (size_t)pan * a.p.nyp + row;
+        static_cast<uint4 *>(a.out)[q] = *reinterpret_cast<const uint4 *>(&buf[0][lane][16 * j]);
+        if (MODE == kPackSplit)
+            static_cast<uint4 *>(a.out_lo)[q] = *reinterpret_cast<const uint4 *>(&buf[MODE == kPackSplit][lane][16 * j]);
+    }
 }
 
-__global__ void pack_f32_kernel(const float *__restrict__ in, int ny, int nx, int pad,
-                                float pad_value, float *__restrict__ out, PlaneGeom p,
-                                size_t n_rows, int q0) {
-    const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n_rows) return;
-    const PanelRow r = panel_row(id, p, q0);
-    float v[4];
-    load_cells<4>(in, ny, nx, pad, pad_value, r.Y, r.X0, v);
-    reinterpret_cast<float4 *>(out)[r.q] = make_float4(v[0], v[1], v[2], v[3]);
-}
+// The grid cells of plane rows [q0, q1), as FP32.  Split: scaled by 2^E, E
+// from *exp when given, else `scale`.
+struct UnpackArgs {
+    const void *in, *in_lo;
+    int ny, nx, pad;
+    float *out;
+    PlaneGeom p;
+    int q0, q1;
+    float scale;
+    const int *exp;
+};
 
-__global__ void unpack_f32_kernel(const float *__restrict__ in, int ny, int nx, int pad,
-                                  float *__restrict__ out, PlaneGeom p, size_t n_rows, int q0) {
-    const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n_rows) return;
-    const PanelRow r = panel_row(id, p, q0);
-    const int iy = r.Y - pad;
-    if (iy < 0 || iy >= ny) return;
-    const float4 v = reinterpret_cast<const float4 *>(in)[r.q];
-    const float c[4] = {v.x, v.y, v.z, v.w};
-    store_cells<4>(out, ny, nx, pad, r.Y, r.X0, c);
+template <int MODE>
+__global__ void __launch_bounds__(kThreads) unpack_kernel(const UnpackArgs a) {
+    constexpr int CPP = MODE == kPackF32 ? 4 : 8;
+    constexpr int CELLS = kBlkPans * CPP;
+    constexpr int N = CELLS / 32, K = kBlkPans / 8;
+    __shared__ __align__(16) uint8_t buf[MODE == kPackSplit ? 2 : 1][kBlkRows][kBlkPitch];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const BlockPos b = block_pos(a.p, a.q0);
+    const int row = min(b.row + lane, a.q1 - 1);
+    pdl_launch_dependents();
+    pdl_wait();
+    uint4 v[K], l[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const int pan = min(b.pan + warp + 8 * k, a.p.npan - 1);
+        const size_t q = (size_t)pan * a.p.nyp + row;
+        v[k] = static_cast<const uint4 *>(a.in)[q];
+        if (MODE == kPackSplit) l[k] = static_cast<const uint4 *>(a.in_lo)[q];
+    }
+    float scale = a.scale;
+    if (MODE == kPackSplit && a.exp) scale = ldexpf(1.0f, *a.exp);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        *reinterpret_cast<uint4 *>(&buf[0][lane][16 * (warp + 8 * k)]) = v[k];
+        if (MODE == kPackSplit) *reinterpret_cast<uint4 *>(&buf[MODE == kPackSplit][lane][16 * (warp + 8 * k)]) = l[k];
+    }
+    __syncthreads();
+    const int ix0 = (b.pan - 1) * CPP - a.pad;
+#pragma unroll
+    for (int k = 0; k < kBlkRows / 8; k++) {
+        const int r = warp + 8 * k, iy = b.row + r - kPadTop - a.pad;
+        if (b.row + r >= a.q1 || iy < 0 || iy >= a.ny) continue;
+        float *dst = a.out + (size_t)iy * a.nx;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int c = lane + 32 * i, ix = ix0 + c;
+            float x;
+            if (MODE == kPackF32) x = reinterpret_cast<const float *>(buf[0][r])[c];
+            else if (MODE == kPackF16) x = h2f_bits(reinterpret_cast<const uint16_t *>(buf[0][r])[c]);
+            else
+                x = fmaf(h2f_bits(reinterpret_cast<const uint16_t *>(buf[MODE == kPackSplit][r])[c]), 1.0f / 2048.0f,
+                         h2f_bits(reinterpret_cast<const uint16_t *>(buf[0][r])[c])) * scale;
+            if (ix >= 0 && ix < a.nx) dst[ix] = x;
+        }
+    }
 }
 
 // Scale exponent E of a grid whose max |x| has float bits `bits`: the
@@ -165,67 +225,70 @@ __device__ __forceinline__ int scale_exp_of(unsigned bits) {
     return e;
 }
 
-// With max_bits set, the scale comes from the device-side maximum (and E is
-// written to exp_out), so that packing needs no host round trip.
-__global__ void pack_split_kernel(const float *__restrict__ in, int ny, int nx, int pad,
-                                  float pad_value, float scale, const unsigned *max_bits,
-                                  int *exp_out, uint16_t *__restrict__ hi,
-                                  uint16_t *__restrict__ lo, PlaneGeom p, size_t n_rows) {
+// The largest |x| of this block's share of n floats, as FP32 bits in every
+// thread of warp 0: 16-byte loads from the first aligned element on, four in
+// flight (one 4-byte load at a time ran at a third of the memory rate).
+__device__ __forceinline__ unsigned block_max_abs(const float *__restrict__ in, size_t n) {
     const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (max_bits) {
-        const int e = scale_exp_of(*max_bits);
-        scale = ldexpf(1.0f, -e);
-        if (id == 0 && exp_out) *exp_out = e;
-    }
-    if (id >= n_rows) return;
-    const PanelRow r = panel_row(id, p);
-    float c[8];
-    load_cells<8>(in, ny, nx, pad, pad_value, r.Y, r.X0, c);
-    uint32_t wh[4], wl[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        uint16_t h[2], l[2];
-#pragma unroll
-        for (int j = 0; j < 2; j++) split_value(c[2 * i + j], scale, h[j], l[j]);
-        wh[i] = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
-        wl[i] = (uint32_t)l[0] | ((uint32_t)l[1] << 16);
-    }
-    reinterpret_cast<uint4 *>(hi)[r.q] = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-    reinterpret_cast<uint4 *>(lo)[r.q] = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-}
-
-__global__ void unpack_split_kernel(const uint16_t *__restrict__ hi,
-                                    const uint16_t *__restrict__ lo, int ny, int nx, int pad,
-                                    float scale, const int *exp_in, float *__restrict__ out,
-                                    PlaneGeom p, size_t n_rows) {
-    const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n_rows) return;
-    if (exp_in) scale = ldexpf(1.0f, *exp_in);
-    const PanelRow r = panel_row(id, p);
-    const int iy = r.Y - pad;
-    if (iy < 0 || iy >= ny) return;
-    const uint4 vh = reinterpret_cast<const uint4 *>(hi)[r.q];
-    const uint4 vl = reinterpret_cast<const uint4 *>(lo)[r.q];
-    const uint32_t wh[4] = {vh.x, vh.y, vh.z, vh.w};
-    const uint32_t wl[4] = {vl.x, vl.y, vl.z, vl.w};
-    float c[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const float h = h2f_bits((uint16_t)(wh[i >> 1] >> (16 * (i & 1))));
-        const float l = h2f_bits((uint16_t)(wl[i >> 1] >> (16 * (i & 1))));
-        c[i] = fmaf(l, 1.0f / 2048.0f, h) * scale;
-    }
-    store_cells<8>(out, ny, nx, pad, r.Y, r.X0, c);
-}
-
-// max |x| as float bits (non-negative floats order like their bit patterns).
-__global__ void max_abs_kernel(const float *__restrict__ in, size_t n, unsigned *out_bits) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    size_t head = ((16 - (reinterpret_cast<uintptr_t>(in) & 15)) & 15) / sizeof(float);
+    if (head > n) head = n;
+    const size_t n4 = (n - head) / 4;
+    const float4 *v = reinterpret_cast<const float4 *>(in + head);
     float m = 0.0f;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x)
-        m = fmaxf(m, fabsf(in[i]));
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out_bits, __float_as_uint(m));
+    auto take = [&](const float4 &x) {
+        m = fmaxf(fmaxf(fmaxf(m, fabsf(x.x)), fmaxf(fabsf(x.y), fabsf(x.z))), fabsf(x.w));
+    };
+    size_t i = id;
+    for (; i + 3 * stride < n4; i += 4 * stride) {
+        const float4 a = v[i], b = v[i + stride], c = v[i + 2 * stride], d = v[i + 3 * stride];
+        take(a);
+        take(b);
+        take(c);
+        take(d);
+    }
+    for (; i < n4; i += stride) take(v[i]);
+    if (id < head) m = fmaxf(m, fabsf(in[id]));
+    for (size_t j = head + 4 * n4 + id; j < n; j += stride) m = fmaxf(m, fabsf(in[j]));
+    __shared__ unsigned part[kThreads / 32];
+    // (non-negative floats order like their bit patterns)
+    unsigned u = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = u;
+    __syncthreads();
+    u = threadIdx.x < kThreads / 32 ? part[threadIdx.x] : 0u;
+    return __reduce_max_sync(0xffffffffu, u);
+}
+
+// max |x| into *out_bits (which starts at 0).
+__global__ void __launch_bounds__(kThreads) max_abs_kernel(const float *__restrict__ in, size_t n,
+                                                           unsigned *out_bits) {
+    const unsigned u = block_max_abs(in, n);
+    if (threadIdx.x == 0) atomicMax(out_bits, u);
+}
+
+// The same for a split grid's upload: the last block to finish starts the
+// grid's scale record from the maximum (E_0 = E_B = its exponent, steps -1
+// and 0 unmeasured, no border yet) and leaves scratch[0] (the maximum) and
+// scratch[1] (blocks done) zero for the next use.
+__global__ void __launch_bounds__(kThreads) max_abs_scale_kernel(const float *__restrict__ in, size_t n,
+                                                                 unsigned *scratch, SplitScale *sc) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const unsigned u = block_max_abs(in, n);
+    if (threadIdx.x != 0) return;
+    atomicMax(&scratch[0], u);
+    __threadfence();
+    if (atomicAdd(&scratch[1], 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const int e = scale_exp_of(atomicExch(&scratch[0], 0u));
+    scratch[1] = 0u;
+    for (int i = 0; i < kScaleRing; i++) {
+        sc->maxbits[i] = 0;
+        sc->exp[i] = e;
+    }
+    sc->maxbits[0] = sc->maxbits[kScaleRing - 1] = kScaleNoMax;
+    sc->bmax = 0u;
+    sc->bexp = e;
 }
 
 // ------------------------------------------- reference layout16 helpers ---
@@ -296,17 +359,6 @@ __global__ void unbrick_2d_kernel(const uint16_t *__restrict__ in, uint16_t *__r
 inline unsigned blocks_for(size_t n) { return static_cast<unsigned>((n + kThreads - 1) / kThreads); }
 inline int nb(int n) { return (n + 15) / 16; }
 
-struct PackShape {
-    PlaneGeom p;
-    size_t rows;
-};
-inline PackShape pack_shape(int ny, int nx, int pad, int cpp) {
-    PackShape s;
-    s.p = plane_geom(ny + 2 * pad, nx + 2 * pad, cpp);
-    s.rows = (size_t)s.p.nyp * s.p.npan;
-    return s;
-}
-
 }  // namespace
 
 namespace {
@@ -350,62 +402,82 @@ cudaError_t encode_panel_map(const uint16_t *plane, const PlaneGeom &pg, CUtenso
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+namespace {
+
+// Layout kernels launch with programmatic stream serialization (pdl_enabled):
+// a kernel's launch overlaps its predecessor's run, and it waits for it
+// before its first access.  A batch's or a small grid's transfers are a row
+// of such launches of a few microseconds each.
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), unsigned blocks, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <int MODE>
+cudaError_t launch_pack(PackArgs a, cudaStream_t s) {
+    const unsigned blocks = (unsigned)((a.q1 - a.q0 + kBlkRows - 1) / kBlkRows) *
+                            (unsigned)((a.p.npan + kBlkPans - 1) / kBlkPans);
+    return launch_pdl(pack_kernel<MODE>, blocks, s, a);
+}
+template <int MODE>
+cudaError_t launch_unpack(UnpackArgs a, cudaStream_t s) {
+    const unsigned blocks = (unsigned)((a.q1 - a.q0 + kBlkRows - 1) / kBlkRows) *
+                            (unsigned)((a.p.npan + kBlkPans - 1) / kBlkPans);
+    return launch_pdl(unpack_kernel<MODE>, blocks, s, a);
+}
+
+PackArgs pack_args(const float *in, int ny, int nx, int pad, float pad_value, void *out, int cpp) {
+    PackArgs a{};
+    a.in = in;
+    a.ny = ny;
+    a.nx = nx;
+    a.pad = pad;
+    a.pad_value = pad_value;
+    a.out = out;
+    a.p = plane_geom(ny + 2 * pad, nx + 2 * pad, cpp);
+    a.q1 = a.p.nyp;
+    a.scale = 1.0f;
+    return a;
+}
+UnpackArgs unpack_args(const void *in, int ny, int nx, int pad, float *out, int cpp) {
+    UnpackArgs a{};
+    a.in = in;
+    a.ny = ny;
+    a.nx = nx;
+    a.pad = pad;
+    a.out = out;
+    a.p = plane_geom(ny + 2 * pad, nx + 2 * pad, cpp);
+    // only the plane rows that hold the grid's
+    a.q0 = kPadTop + pad;
+    a.q1 = a.q0 + ny;
+    a.scale = 1.0f;
+    return a;
+}
+
+unsigned max_abs_blocks(size_t n) {
+    const size_t want = (n + 16 * kThreads - 1) / (16 * kThreads);
+    return static_cast<unsigned>(want < 1216 ? (want ? want : 1) : 1216);  // eight per SM
+}
+
+}  // namespace
+
 cudaError_t launch_pack_f16(const float *in, int ny, int nx, int pad, float pad_value,
                             uint16_t *plane, cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, pad, 8);
-    pack_f16_kernel<<<blocks_for(ps.rows), kThreads, 0, s>>>(in, ny, nx, pad, pad_value, plane,
-                                                             ps.p, ps.rows, 0);
-    return cudaGetLastError();
+    return launch_pack<kPackF16>(pack_args(in, ny, nx, pad, pad_value, plane, 8), s);
 }
 
 cudaError_t launch_unpack_f16(const uint16_t *plane, int ny, int nx, int pad, float *out,
                               cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, pad, 8);
-    unpack_f16_kernel<<<blocks_for(ps.rows), kThreads, 0, s>>>(plane, ny, nx, pad, out, ps.p,
-                                                               ps.rows, 0);
-    return cudaGetLastError();
-}
-
-__global__ void split_scale_init_kernel(SplitScale *sc, const unsigned *max_bits) {
-    const int e = scale_exp_of(*max_bits);
-    for (int i = 0; i < kScaleRing; i++) {
-        sc->maxbits[i] = 0;
-        sc->exp[i] = e;
-    }
-    sc->maxbits[0] = sc->maxbits[kScaleRing - 1] = kScaleNoMax;
-    sc->bmax = 0u;
-    sc->bexp = e;
-}
-
-// B: the largest |x'| 2^-11 stored in the grid's cells outside the update
-// rectangle, as FP32 bits, over the index space of the rows outside
-// [y0, y1) (every column) followed by the rows inside (the columns outside
-// [x0, x1)).  |x'| 2^11 = |hi 2^11 + lo| rounded once to FP32.
-__global__ void split_border_max_kernel(SplitScale *sc, GridGeom g, const uint16_t *__restrict__ hi,
-                                        const uint16_t *__restrict__ lo) {
-    const int out_rows = g.y0 + (g.ny - g.y1);
-    const int out_cols = g.x0 + (g.nx - g.x1);
-    const size_t na = (size_t)out_rows * g.nx;
-    const size_t n = na + (size_t)(g.y1 - g.y0) * out_cols;
-    float m = 0.0f;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x) {
-        int y, x;
-        if (i < na) {
-            const int r = (int)(i / g.nx);
-            x = (int)(i - (size_t)r * g.nx);
-            y = r < g.y0 ? r : g.y1 + (r - g.y0);
-        } else {
-            const size_t j = i - na;
-            const int r = (int)(j / out_cols), c = (int)(j - (size_t)r * out_cols);
-            y = g.y0 + r;
-            x = c < g.x0 ? c : g.x1 + (c - g.x0);
-        }
-        const size_t idx = plane_index(g.p16, y, x);
-        m = fmaxf(m, fabsf(fmaf(h2f_bits(hi[idx]), 2048.0f, h2f_bits(lo[idx]))));
-    }
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(&sc->bmax, __float_as_uint(m * (1.0f / 2048.0f)));
+    return launch_unpack<kPackF16>(unpack_args(plane, ny, nx, pad, out, 8), s);
 }
 
 __global__ void split_scale_end_run_kernel(SplitScale *sc, int steps) {
@@ -420,19 +492,6 @@ __global__ void split_scale_end_run_kernel(SplitScale *sc, int steps) {
     sc->exp[0] = e0;
 }
 
-cudaError_t launch_split_scale_init(SplitScale *sc, const unsigned *max_bits, const GridGeom &g,
-                                    const uint16_t *hi, const uint16_t *lo, cudaStream_t s) {
-    split_scale_init_kernel<<<1, 1, 0, s>>>(sc, max_bits);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const size_t n = (size_t)g.ny * g.nx - (size_t)(g.y1 - g.y0) * (g.x1 - g.x0);
-    if (n == 0) return cudaSuccess;
-    const size_t want = blocks_for(n);
-    split_border_max_kernel<<<static_cast<unsigned>(want < 1024 ? want : 1024), kThreads, 0, s>>>(
-        sc, g, hi, lo);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_split_scale_end_run(SplitScale *sc, int steps, cudaStream_t s) {
     if (steps <= 0) return cudaSuccess;
     split_scale_end_run_kernel<<<1, 1, 0, s>>>(sc, steps);
@@ -441,18 +500,12 @@ cudaError_t launch_split_scale_end_run(SplitScale *sc, int steps, cudaStream_t s
 
 cudaError_t launch_pack_f32(const float *in, int ny, int nx, int pad, float pad_value,
                             float *plane, cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, pad, 4);
-    pack_f32_kernel<<<blocks_for(ps.rows), kThreads, 0, s>>>(in, ny, nx, pad, pad_value, plane,
-                                                             ps.p, ps.rows, 0);
-    return cudaGetLastError();
+    return launch_pack<kPackF32>(pack_args(in, ny, nx, pad, pad_value, plane, 4), s);
 }
 
 cudaError_t launch_unpack_f32(const float *plane, int ny, int nx, int pad, float *out,
                               cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, pad, 4);
-    unpack_f32_kernel<<<blocks_for(ps.rows), kThreads, 0, s>>>(plane, ny, nx, pad, out, ps.p,
-                                                               ps.rows, 0);
-    return cudaGetLastError();
+    return launch_unpack<kPackF32>(unpack_args(plane, ny, nx, pad, out, 4), s);
 }
 
 // Plane rows [q0, q1) only (every panel), pad 0: the grid rows they hold are
@@ -460,71 +513,60 @@ cudaError_t launch_unpack_f32(const float *plane, int ny, int nx, int pad, float
 // to the first and last ranges.
 cudaError_t launch_pack_rows(const float *in, int ny, int nx, bool f32, void *plane, int q0,
                              int q1, cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, 0, f32 ? 4 : 8);
-    if (q0 < 0 || q1 > ps.p.nyp || q0 >= q1) return cudaErrorInvalidValue;
-    const size_t rows = (size_t)(q1 - q0) * ps.p.npan;
-    if (f32)
-        pack_f32_kernel<<<blocks_for(rows), kThreads, 0, s>>>(in, ny, nx, 0, 0.0f,
-                                                              static_cast<float *>(plane), ps.p,
-                                                              rows, q0);
-    else
-        pack_f16_kernel<<<blocks_for(rows), kThreads, 0, s>>>(in, ny, nx, 0, 0.0f,
-                                                              static_cast<uint16_t *>(plane),
-                                                              ps.p, rows, q0);
-    return cudaGetLastError();
+    PackArgs a = pack_args(in, ny, nx, 0, 0.0f, plane, f32 ? 4 : 8);
+    if (q0 < 0 || q1 > a.p.nyp || q0 >= q1) return cudaErrorInvalidValue;
+    a.q0 = q0;
+    a.q1 = q1;
+    return f32 ? launch_pack<kPackF32>(a, s) : launch_pack<kPackF16>(a, s);
 }
 
 cudaError_t launch_unpack_rows(const void *plane, int ny, int nx, bool f32, float *out, int q0,
                                int q1, cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, 0, f32 ? 4 : 8);
-    if (q0 < 0 || q1 > ps.p.nyp || q0 >= q1) return cudaErrorInvalidValue;
-    const size_t rows = (size_t)(q1 - q0) * ps.p.npan;
-    if (f32)
-        unpack_f32_kernel<<<blocks_for(rows), kThreads, 0, s>>>(static_cast<const float *>(plane),
-                                                                ny, nx, 0, out, ps.p, rows, q0);
-    else
-        unpack_f16_kernel<<<blocks_for(rows), kThreads, 0, s>>>(
-            static_cast<const uint16_t *>(plane), ny, nx, 0, out, ps.p, rows, q0);
-    return cudaGetLastError();
+    UnpackArgs a = unpack_args(plane, ny, nx, 0, out, f32 ? 4 : 8);
+    if (q0 < 0 || q1 > a.p.nyp || q0 >= q1) return cudaErrorInvalidValue;
+    a.q0 = q0;
+    a.q1 = q1;
+    return f32 ? launch_unpack<kPackF32>(a, s) : launch_unpack<kPackF16>(a, s);
 }
 
 cudaError_t launch_pack_split(const float *in, int ny, int nx, int pad, float pad_value,
                               int scale_exp, uint16_t *hi, uint16_t *lo, cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, pad, 8);
-    pack_split_kernel<<<blocks_for(ps.rows), kThreads, 0, s>>>(
-        in, ny, nx, pad, pad_value, ldexpf(1.0f, -scale_exp), nullptr, nullptr, hi, lo, ps.p,
-        ps.rows);
-    return cudaGetLastError();
+    PackArgs a = pack_args(in, ny, nx, pad, pad_value, hi, 8);
+    a.out_lo = lo;
+    a.scale = ldexpf(1.0f, -scale_exp);
+    return launch_pack<kPackSplit>(a, s);
 }
 
-cudaError_t launch_pack_split_dev(const float *in, int ny, int nx, const unsigned *max_bits,
-                                  int *exp_out, uint16_t *hi, uint16_t *lo, cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, 0, 8);
-    pack_split_kernel<<<blocks_for(ps.rows), kThreads, 0, s>>>(
-        in, ny, nx, 0, 0.0f, 1.0f, max_bits, exp_out, hi, lo, ps.p, ps.rows);
-    return cudaGetLastError();
+cudaError_t launch_split_upload(const float *in, const GridGeom &g, unsigned *scratch,
+                                SplitScale *sc, uint16_t *hi, uint16_t *lo, cudaStream_t s) {
+    const size_t n = (size_t)g.ny * g.nx;
+    cudaError_t e = launch_pdl(max_abs_scale_kernel, max_abs_blocks(n), s, in, n, scratch, sc);
+    if (e != cudaSuccess) return e;
+    PackArgs a = pack_args(in, g.ny, g.nx, 0, 0.0f, hi, 8);
+    a.out_lo = lo;
+    a.sc = sc;
+    a.y0 = g.y0; a.y1 = g.y1; a.x0 = g.x0; a.x1 = g.x1;
+    return launch_pack<kPackSplit>(a, s);
 }
 
 cudaError_t launch_unpack_split(const uint16_t *hi, const uint16_t *lo, int ny, int nx, int pad,
                                 int scale_exp, float *out, cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, pad, 8);
-    unpack_split_kernel<<<blocks_for(ps.rows), kThreads, 0, s>>>(
-        hi, lo, ny, nx, pad, ldexpf(1.0f, scale_exp), nullptr, out, ps.p, ps.rows);
-    return cudaGetLastError();
+    UnpackArgs a = unpack_args(hi, ny, nx, pad, out, 8);
+    a.in_lo = lo;
+    a.scale = ldexpf(1.0f, scale_exp);
+    return launch_unpack<kPackSplit>(a, s);
 }
 
 cudaError_t launch_unpack_split_dev(const uint16_t *hi, const uint16_t *lo, int ny, int nx,
                                     const int *exp_in, float *out, cudaStream_t s) {
-    const PackShape ps = pack_shape(ny, nx, 0, 8);
-    unpack_split_kernel<<<blocks_for(ps.rows), kThreads, 0, s>>>(hi, lo, ny, nx, 0, 1.0f, exp_in,
-                                                                 out, ps.p, ps.rows);
-    return cudaGetLastError();
+    UnpackArgs a = unpack_args(hi, ny, nx, 0, out, 8);
+    a.in_lo = lo;
+    a.exp = exp_in;
+    return launch_unpack<kPackSplit>(a, s);
 }
 
 cudaError_t launch_max_abs(const float *in, size_t n, unsigned *out_bits, cudaStream_t s) {
-    const size_t want = (n + kThreads - 1) / kThreads;
-    const unsigned blocks = static_cast<unsigned>(want < 2048 ? (want ? want : 1) : 2048);
-    max_abs_kernel<<<blocks, kThreads, 0, s>>>(in, n, out_bits);
+    max_abs_kernel<<<max_abs_blocks(n), kThreads, 0, s>>>(in, n, out_bits);
     return cudaGetLastError();
 }
 

@@ -152,7 +152,7 @@ struct tcs_server_s {
     CUtensorMap *d_maps = nullptr;  // per slot: tensor maps of the request's planes
     CUtensorMap *h_maps = nullptr;  // pinned staging of d_maps (a slot's entry is
                                     // rewritten only after its request retired)
-    unsigned *d_maxbits = nullptr;
+    unsigned *d_upload = nullptr;  // per slot: launch_split_upload scratch
     SplitScale *d_scale = nullptr;  // per slot: a split request's per-step scale
     int *d_err = nullptr;       // sticky: the first failed wait of any round
     int *h_slot_err = nullptr;  // pinned, per slot: d_err as seen at completion
@@ -402,15 +402,11 @@ void tcs_server_s::admit() {
         }
         const size_t cells = (size_t)q->g.ny * q->g.nx;
         float *stg = staging(q);
-        unsigned *mx = d_maxbits + q->slot;
         int st = cuda_status(cudaMemcpyAsync(stg, q->h_in, cells * sizeof(float), cudaMemcpyHostToDevice, upload), "request upload");
         // state-1 planes: padding cells must be finite (pack writes all of state 0)
         if (!st) st = cuda_status(cudaMemsetAsync(plane(q, 1, 0), 0, 2 * q->plane_bytes, upload), "plane clear");
         if (!st && q->split) {
-            st = cuda_status(cudaMemsetAsync(mx, 0, sizeof(unsigned), upload), "max clear");
-            if (!st) st = cuda_status(launch_max_abs(stg, cells, mx, upload), "max_abs launch");
-            if (!st) st = cuda_status(launch_pack_split_dev(stg, q->g.ny, q->g.nx, mx, nullptr, plane(q, 0, 0), plane(q, 0, 1), upload), "pack launch");
-            if (!st) st = cuda_status(launch_split_scale_init(d_scale + q->slot, mx, q->g, plane(q, 0, 0), plane(q, 0, 1), upload), "scale init");
+            st = cuda_status(launch_split_upload(stg, q->g, d_upload + kUploadScratch * (size_t)q->slot, d_scale + q->slot, plane(q, 0, 0), plane(q, 0, 1), upload), "pack launch");
         } else if (!st) {
             st = cuda_status(launch_pack_f16(stg, q->g.ny, q->g.nx, 0, 0.0f, plane(q, 0, 0), upload), "pack launch");
         }
@@ -699,7 +695,8 @@ int tcs_server_create(const tcs_server_config *config, tcs_server *out) {
     if (!st) st = dev_alloc_t(&s->d_bands, (size_t)slots * kBatchMaxBandElems * sizeof(uint16_t), "bands");
     if (!st) st = dev_alloc_t(&s->d_maps, (size_t)slots * 4 * sizeof(CUtensorMap), "maps");
     if (!st) st = host_alloc_t(&s->h_maps, (size_t)slots * 4 * sizeof(CUtensorMap), "maps");
-    if (!st) st = dev_alloc_t(&s->d_maxbits, slots * sizeof(unsigned), "max");
+    if (!st) st = dev_alloc_t(&s->d_upload, kUploadScratch * (size_t)slots * sizeof(unsigned), "max");
+    if (!st) st = cuda_status(cudaMemset(s->d_upload, 0, kUploadScratch * (size_t)slots * sizeof(unsigned)), "cudaMemset(max)");
     if (!st) st = dev_alloc_t(&s->d_scale, slots * sizeof(SplitScale), "scales");
     if (!st) st = dev_alloc_t(&s->d_err, sizeof(int), "error");
     if (!st) st = cuda_status(cudaMemset(s->d_err, 0, sizeof(int)), "cudaMemset(error)");
@@ -765,7 +762,7 @@ int tcs_server_destroy(tcs_server s) {
     for (cudaEvent_t e : s->event_pool) cudaEventDestroy(e);
     for (void *p : s->retired.host) host_free(p);
     for (void *p : s->retired.dev) dev_free(p);
-    for (void *p : {(void *)s->pool, (void *)s->d_bands, (void *)s->d_maps, (void *)s->d_maxbits,
+    for (void *p : {(void *)s->pool, (void *)s->d_bands, (void *)s->d_maps, (void *)s->d_upload,
                     (void *)s->d_scale, (void *)s->d_err})
         if (p) dev_free(p);
     if (s->h_slot_err) host_free(s->h_slot_err);

@@ -213,13 +213,18 @@ cudaError_t launch_pack_split(const float *in, int ny, int nx, int pad, float pa
                               int scale_exp, uint16_t *hi, uint16_t *lo, cudaStream_t s);
 cudaError_t launch_unpack_split(const uint16_t *hi, const uint16_t *lo, int ny, int nx, int pad,
                                 int scale_exp, float *out, cudaStream_t s);
-// max |x| over n floats into *out_bits (float bits; *out_bits must start at 0)
-// Split pack/unpack (pad 0) with the scale exponent kept in device memory:
-// pack derives E from the max-|x| bits that launch_max_abs left and stores it.
-cudaError_t launch_pack_split_dev(const float *in, int ny, int nx, const unsigned *max_bits,
-                                  int *exp_out, uint16_t *hi, uint16_t *lo, cudaStream_t s);
+// A split grid's upload (pad 0): the scale record from max |x| (E_0 = E_B = its
+// exponent, steps -1 and 0 marked as unmeasured), the planes packed with that
+// exponent, and the record's B from the packed cells outside the update
+// rectangle.  scratch: kUploadScratch words, zero before the first use (each
+// leaves them zero again).
+constexpr int kUploadScratch = 2;
+cudaError_t launch_split_upload(const float *in, const GridGeom &g, unsigned *scratch,
+                                SplitScale *sc, uint16_t *hi, uint16_t *lo, cudaStream_t s);
+// Unpack with the scale exponent kept in device memory.
 cudaError_t launch_unpack_split_dev(const uint16_t *hi, const uint16_t *lo, int ny, int nx,
                                     const int *exp_in, float *out, cudaStream_t s);
+// max |x| over n floats into *out_bits (float bits; *out_bits must start at 0).
 cudaError_t launch_max_abs(const float *in, size_t n, unsigned *out_bits, cudaStream_t s);
 // FP16 (f32 false) or FP32 plane rows [q0, q1) from / to an ny x nx
 // row-major grid, no padding; the grid rows involved are [q0 - 4, q1 - 4)
@@ -260,11 +265,6 @@ struct SplitScale {
     unsigned bmax;                 // B as FP32 bits
     int bexp;                      // E_B
 };
-// From the max-|x| bits launch_max_abs left for a grid's input: E_0 = E_B =
-// the pack's exponent, steps -1 and 0 marked as unmeasured, and B from the
-// packed planes (hi, lo) of the grid g.
-cudaError_t launch_split_scale_init(SplitScale *sc, const unsigned *max_bits, const GridGeom &g,
-                                    const uint16_t *hi, const uint16_t *lo, cudaStream_t s);
 // After a run of `steps` steps: steps T-1 and T become slots 7 and 0, the
 // maxima of slots 1..6 are cleared.
 cudaError_t launch_split_scale_end_run(SplitScale *sc, int steps, cudaStream_t s);
