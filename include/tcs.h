@@ -214,9 +214,10 @@ int tcs_plan_state(tcs_plan plan, void **hi, void **lo, size_t *plane_bytes);
 int tcs_plan_scale_exp(tcs_plan plan, int *scale_exp);
 /* Replaces the coefficients (host n*n). */
 int tcs_plan_set_coeffs(tcs_plan plan, const float *coeffs);
-/* Temporal blocking depth: 1 (one launch per step, the default) or 2 (two
- * steps per launch, intermediate kept on chip; split precision on the tensor
- * engine).  Results are bit-identical either way; the autotuner picks. */
+/* Temporal blocking depth: 1 (single steps, the default) or 2 (two steps per
+ * launch, intermediate kept on chip; split precision on the tensor engine,
+ * faster there at every size measured).  Results are bit-identical either
+ * way; the autotuner picks, tcs_sweep_host and pipes take depth 2 for split. */
 int tcs_plan_set_temporal_depth(tcs_plan plan, int depth);
 /* Tensor engine (FP16 or split, temporal depth 1): run(steps >= 2) as ONE
  * launch instead of one launch per step.  FP16 tiles take up to eight

@@ -313,9 +313,9 @@ class Plan:
             from .autotune import best_config, best_launch, best_tile_width
 
             engine, tuned_depth = best_config(stencil, precision, ny, nx)
-            if temporal_depth is None:
-                temporal_depth = tuned_depth
             tuned_launch = best_launch(stencil, precision, ny, nx)
+            if temporal_depth is None:  # (every tuned split class takes pairs)
+                temporal_depth = 2 if precision == "split" and tuned_launch < 0 else tuned_depth
             if tuned_launch < 0 and precision == "f16":
                 tuned_launch = 1  # every tuned FP16 class takes one launch for all steps
             if tile_w is None and engine == "tensor" and precision == "f16":

@@ -426,9 +426,17 @@ struct tcs_plan_s {
     }
 
     // Temporal depth 2 (split precision on the tensor engine): steps run in
-    // blocked pairs, with the same bits as single steps.
+    // blocked pairs, with the same bits as single steps.  The one-call form,
+    // pipes and autotuned plans take it for every split grid: faster than
+    // either form of single steps at every size measured (box2d1r / box2d2r,
+    // us per step, best single form -> pairs: 256² 6.65 -> 6.26 / 6.88 -> 6.46,
+    // 1026² 7.49 -> 6.53 / 8.91 -> 6.64, 4096² 26.5 -> 22.2 / 27.2 -> 25.1,
+    // 16386² 356 -> 264 / 371 -> 312).
     int temporal_depth = 1;
     bool pairs() const { return temporal_depth == 2; }
+    void take_pairs() {
+        if (prob.engine == TCS_ENGINE_TENSOR && prob.precision == TCS_PREC_SPLIT) temporal_depth = 2;
+    }
     int step2(int from, cudaStream_t s, int t0) {
         return cuda_status(
             launch_tc_split2(g, prob.stencil, coeffs, static_cast<const uint16_t *>(buf[from][0]),
@@ -831,6 +839,7 @@ int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *pr, int s
     if (it == t_cache.plans.end()) {
         int st = tcs_plan_create(pr, &p);
         if (st) return st;
+        p->take_pairs();
         t_cache.plans.emplace(key, p);
     } else {
         p = it->second;
@@ -882,6 +891,7 @@ int tcs_pipe_create(const tcs_problem *pr, tcs_pipe *out) {
     int st = TCS_OK;
     for (int k = 0; k < 2 && !st; k++) {
         st = tcs_plan_create(pr, &q->plan[k]);
+        if (!st) q->plan[k]->take_pairs();
         if (!st) st = cuda_status(cudaStreamCreateWithFlags(&q->stream[k], cudaStreamNonBlocking), "cudaStreamCreate");
         if (!st) st = cuda_status(cudaEventCreateWithFlags(&q->done[k], cudaEventDisableTiming), "cudaEventCreate");
         if (!st) st = cuda_status(cudaEventCreateWithFlags(&q->swept[k], cudaEventDisableTiming), "cudaEventCreate");

@@ -452,8 +452,8 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                         const uint32_t d = tmem_base + col;
                         // all windows: FP16 items are bound by the producer, and a
                         // second MMA sequence for edge tiles measured slower
-                        if (g.r == 1) issue_subtile<1, false, SG>(a_hi0, band, d, 0);
-                        else issue_subtile<2, false, SG>(a_hi0, band, d, 0);
+                        if (g.r == 1) issue_plain_windows<1, SG>(a_hi0, band, d);
+                        else issue_plain_windows<2, SG>(a_hi0, band, d);
                         slots.commit(acc_full, mask);
                         slots.used(mask);
                     }
@@ -620,16 +620,17 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                         return;
                     }
                     tc_fence_after();
-                    float f[16];
+                    float u[16];
                     split_block_load(lane_base + (Ga % kBatchRingSlots) * kBatchRegion,
-                                     lane_base + (Gb % kBatchRingSlots) * kBatchRegion, f);
+                                     lane_base + (Gb % kBatchRingSlots) * kBatchRegion, u);
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
                         mbar_arrive(&acc_empty[Ga % kBatchRingSlots]);
                         mbar_arrive(&acc_empty[Gb % kBatchRingSlots]);
                     }
-                    store_block_split(o, f, y, X0 + 16 * jb, fast, row_in, ss, mx);
+                    shift_block(u, ss);
+                    store_block_split(o, u, y, X0 + 16 * jb, fast, row_in, mx);
                 });
                 if (ok && ss.k != 0 && !fast && !rows_out)
                     resplit_border(o, y, X0, grp, C::GROUPS, nwin - 1, ss);
@@ -661,11 +662,11 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                 } else {
                     tc_fence_after();
                     float f[Mode<false>::SUB_BLOCKS / 2][16];
-                    epilogue_load<false>(lane_base + col, grp, f);
+                    epilogue_load(lane_base + col, grp, f);
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) slots.release(acc_empty, mask);
-                    epilogue_store<false>(o, f, 0, grp, m, Y0, X0);
+                    epilogue_store(o, f, grp, m, Y0, X0);
                     slots.used(mask);
                 }
             }

@@ -1,30 +1,40 @@
 // Temporally blocked split-precision sweep: TWO Jacobi steps per HBM round
-// trip.  The single-step split kernel is bound by the bytes an SM can keep in
-// flight (two 76 KB stages for ~140 KB of traffic per tile and step);
-// blocking two steps cuts the traffic per step to ~5.4 B per point-update
-// for ~25 % more MMA work.
+// trip.  A split step moves 8 bytes per point update, which at the memory
+// rate takes twice as long as a radius-1 tile's MMAs and as long as a
+// radius-2 tile's; two steps per load and store halve the traffic.
 //
-// Tile.  Outputs are rows [Y0, Y0 + 128 - 2r) x columns [X0, X0 + 80) (X0 a
-// multiple of 80).  The producer stages input rows [Y0 - r - 2, Y0 - r + 130)
-// and columns [X0 - 24, X0 + 104): 16 panels, hi and lo, 66 KB.
-//   Step 1: eight windows (input columns X0 - 24 + 16w .. +16) give the
-//     128-row intermediate over columns [X0 - 16, X0 + 96) (seven blocks), of
-//     which columns [X0 - 8, X0 + 88) (12 panels) go, as hi/lo FP16 panels,
-//     into a shared-memory intermediate image.  The input stage is released
-//     as soon as these MMAs are done, so the next tile loads during step 2.
-//   Step 2: six windows over the intermediate (columns X0 - 8 + 16w .. +16)
-//     give the 80 output columns; rows r .. 127 - r of the 128 are valid.
-// Windows sit at the same absolute columns (8 mod 16) as in the single-step
-// kernel and each block sums the same two windows, so two blocked steps give
-// exactly the bits of two single steps.
+// Tile.  As in the single-step split kernel (sweep_tc.cu): the stage holds
+// rows Yb-4 .. Yb+131 of the panels X0-8 .. X0+135, hi and lo, and one step's
+// nine windows give rows Yb .. Yb+127 of the columns X0-16 .. X0+143.  The
+// first step's values go back over the staged image (X0-8 .. X0+135: the
+// halo panels lack only windows whose products with their valid cells are all
+// zero), the second step's nine windows run on it, and the rows Yb+2 ..
+// Yb+125 (from row 0 / to the last row for the first and last tile rows) go
+// to the output planes.  Windows, their order and the split are the
+// single-step kernel's, so two blocked steps give exactly the bits of two
+// single steps.  Tile rows start at multiples of 124, so their copies move
+// half lines (encode_panel_map with rows = 4; 120 and whole lines: 3 % more
+// rows, the same time per tile).
 //
 // Pipeline.  Window accumulators stream through the ring of five 96-column
-// TMEM regions of the single-step split kernel; per tile the issuer runs step
-// 1, waits for the epilogue's intermediate, then runs step 2.  There is one
-// intermediate image: the epilogue writes tile t+1's only after consuming
-// every step-2 window of tile t, i.e. after those MMAs have read it.  Panels
-// outside the plane come from a zero panel; row copies are clipped to the
-// plane; stores are clipped to the grid.
+// TMEM regions of the single-step kernel, 18 windows per tile.  A block's new
+// values overwrite its two panels as soon as its two windows are complete
+// (no other window reads those panels), and window w of the second step
+// waits for its two blocks: the second step follows the first a few windows
+// behind, and the tensor pipe does not drain between them.  Radius 2 runs at
+// the tensor pipe's 60 cycles per MMA (16386²: 371 -> 312 us per step against
+// one step per launch); radius 1 (356 -> 264) at 490 cycles per window of 360
+// cycles' MMAs, the five regions' turnaround.  An epilogue warp
+// waits once per block, on a barrier that both windows' commits arrive at.
+// (Waiting for windows, each released by all warps read or not, cost a warp
+// 800 of 2200 cycles per block: 16386² box2d1r 399 us per step, 336 with the
+// barriers per block; one range check per panel row instead of per pair
+// -> 292; both panels summed before the first is split -> 272; the groups
+// taking turns over both steps' blocks -> 264.  Reading each window the moment
+// it completes, for three groups of 128 registers, was slower: 309.)  (The form this
+// replaces, with 80-column tiles, a second image for the intermediate and a
+// handoff per step, took 140 / 156 us per step at 8196², box2d1r / box2d2r.)
+// Two stages: the next tile loads while a tile runs both its steps.
 #include "tc_core.cuh"
 
 namespace tcs {
@@ -32,47 +42,45 @@ namespace tcs {
 namespace {
 
 using namespace tc;
+using SG = StageLines;
 
 __device__ int g_tb_error = 0;
 
-// One staged panel of zeros, the source for panels outside the plane.
-__device__ __align__(256) uint16_t g_zero_panel[kRowsStaged * 8] = {0};
-
-constexpr int kTbCols = 80;  // output columns per tile
 constexpr int kTbStages = 2;
 constexpr int kTbRing = 5;
 constexpr int kTbRegion = 96;
-constexpr int kS1Windows = 8;  // step 1: intermediate columns [X0 - 16, X0 + 96)
-constexpr int kS2Windows = 6;  // step 2: output columns [X0, X0 + 80)
-constexpr int kInPanels = 16;  // input columns [X0 - 24, X0 + 104)
-constexpr int kMidPanels = 12; // intermediate columns [X0 - 8, X0 + 88)
-constexpr int kInPlane = kInPanels * kChunkBytes;    // one staged input plane
-constexpr int kMidPlane = kMidPanels * kChunkBytes;  // one intermediate plane
-constexpr int kTbGroups = 3;                          // epilogue block groups
-constexpr int kTbEpiWarps = 4 * kTbGroups;            // a lane quarter each
-// MMA issuer warps 1 and 2 take alternate windows (G % 2), as in the
-// single-step split kernel: both wait for every stage fill and every
-// intermediate, in order, and commit the stage after step 1 (the stage is
-// free when both have); an issuer's previous region wait, two windows back,
-// already covered the release before the one it now needs.
-constexpr int kTbIssuers = 2;
-constexpr int kTbThreads = 32 * (1 + kTbIssuers + kTbEpiWarps);
+constexpr int kTbWindows = kTile / 16 + 1;  // of one step
+constexpr int kTbBlocks = kTile / 16 + 2;   // blocks -1 .. 8: the halo panels are -1 and 8
+constexpr int kTbHalo = 2;                  // rows given up at the top and bottom
+constexpr int kTbRows = kTile - 2 * kTbHalo;
+constexpr int kTbMapRows = 4;
+constexpr int kTbGroups = 4;                // epilogue block groups
+constexpr int kTbEpiWarps = 4 * kTbGroups;  // a lane quarter each
+// MMA issuer warps 1 .. 3 take the windows w with w % 3 == id of every step;
+// each waits for every stage fill, in order, and for the phases of its own
+// windows' blocks.  A region's barrier completes a phase per window that used
+// it; an issuer waits for window G's region only once window G - 5, whose
+// issuer saw the release of window G - 10, has been issued (`issued`), so the
+// parity it waits for cannot be that of an older phase.
+constexpr int kTbIssuers = 3;
+constexpr int kTbEpi0 = 1 + kTbIssuers;
+constexpr int kTbThreads = 32 * (kTbEpi0 + kTbEpiWarps);
 
 template <int S>
 struct TbCfg {
     static constexpr int R = stencil_r(S);
     static constexpr bool BOX = stencil_box(S);
     static constexpr int NDY = 2 * R + 1;
-    static constexpr int H = kTile - 2 * R;  // output rows per tile
     static constexpr size_t BAND = (size_t)4 * NDY * kBandBytes;
-    static constexpr size_t SMEM =
-        1024 + (size_t)kTbStages * 2 * kInPlane + 2 * kMidPlane + BAND + 256;
+    static constexpr int BARS = 512;
+    static constexpr size_t SMEM = 1024 + (size_t)kTbStages * 2 * SG::PLANE + BAND + BARS;
     static_assert(SMEM <= 232448, "shared memory budget");
 };
 
 struct TbParams {
+    CUtensorMap map_hi, map_lo;  // input planes
     GridGeom g;
-    int tiles_x, n_tiles;
+    int tiles_x, tiles_y, n_tiles;
     const uint16_t *in_hi, *in_lo;
     uint16_t *out_hi, *out_lo;
     SplitScale *scale;  // the grid's per-step scale (null: fixed scale)
@@ -80,43 +88,100 @@ struct TbParams {
     float coef[25];
 };
 
-// 8 cells of panel row (y, x0) of a plane (x0 a multiple of 8), or zeros when
-// the row or panel is outside the plane.
-__device__ __forceinline__ uint4 load_panel_row(const uint16_t *plane, const PlaneGeom &pg, int y,
-                                                int x0) {
-    const int row = y + kPadTop, pan = (x0 >> 3) + 1;
-    if (row < 0 || row >= pg.nyp || pan < 0 || pan >= pg.npan) return make_uint4(0, 0, 0, 0);
-    return *reinterpret_cast<const uint4 *>(plane + ((size_t)pan * pg.nyp + row) * 8);
+// Eight columns of a split block from its two windows' regions (TMEM columns
+// `a` and `b` of each part; b is ignored for the halo panels, which one window
+// alone reaches): the loads, and after tmem_ld_wait their sum u as
+// split_block_load forms it.
+__device__ __forceinline__ void panel_load(uint32_t a, uint32_t b, bool two, uint32_t (&v)[6][8]) {
+#pragma unroll
+    for (int part = 0; part < 3; part++) {
+        tmem_ld_x8(a + 32 * part, v[2 * part]);
+        if (two) tmem_ld_x8(b + 32 * part, v[2 * part + 1]);
+    }
+}
+__device__ __forceinline__ void panel_sum(const uint32_t (&v)[6][8], bool two, const StepScale &ss,
+                                          float (&u)[8]) {
+    auto pr = [&](int part, int c) {
+        return make_float2(__uint_as_float(v[part][c]), __uint_as_float(v[part][c + 1]));
+    };
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+        float2 main = pr(0, c), c1 = pr(2, c), c2 = pr(4, c);
+        if (two) {
+            main = __fadd2_rn(main, pr(1, c));
+            c1 = __fadd2_rn(c1, pr(3, c));
+            c2 = __fadd2_rn(c2, pr(5, c));
+        }
+        const float2 x = __ffma2_rn(main, make_float2(2048.0f, 2048.0f), __fadd2_rn(c1, c2));
+        u[c] = x.x;
+        u[c + 1] = x.y;
+    }
+    if (ss.k != 0) {
+        const float f = ss.s * (1.0f / 2048.0f);
+#pragma unroll
+        for (int c = 0; c < 8; c++) u[c] *= f;
+    }
+}
+
+// split_panel where not every cell is updated: cells outside [x0, x1) or of a
+// row outside the rectangle keep the old pair (re-split when `move`s scale
+// shifts).
+__device__ __forceinline__ PanelPair split_panel_edge(const float (&u)[8], const PanelPair &old, int xb,
+                                                   bool row_in, int x0, int x1, const StepScale &move,
+                                                   float &mx) {
+    const uint32_t ih[4] = {old.hi.x, old.hi.y, old.hi.z, old.hi.w};
+    const uint32_t il[4] = {old.lo.x, old.lo.y, old.lo.z, old.lo.w};
+    uint32_t hw[4], lw[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        uint16_t hh[2], ll[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int x = xb + 2 * c + k;
+            if (row_in && x >= x0 && x < x1) {
+                split_fixed_u(u[2 * c + k], hh[k], ll[k], mx);
+            } else {
+                hh[k] = (uint16_t)(ih[c] >> (16 * k));
+                ll[k] = (uint16_t)(il[c] >> (16 * k));
+                if (move.k != 0) resplit_pair(hh[k], ll[k], move);
+            }
+        }
+        hw[c] = (uint32_t)hh[0] | ((uint32_t)hh[1] << 16);
+        lw[c] = (uint32_t)ll[0] | ((uint32_t)ll[1] << 16);
+    }
+    return PanelPair{make_uint4(hw[0], hw[1], hw[2], hw[3]), make_uint4(lw[0], lw[1], lw[2], lw[3])};
 }
 
 template <int S>
-__global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const TbParams p) {
+__global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid_constant__ TbParams p) {
     using C = TbCfg<S>;
+    constexpr int R = C::R;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                 ~static_cast<uintptr_t>(1023));
-    uint8_t *stage_base = smem;  // [stage][hi, lo][16 panels]
-    uint8_t *mid_base = smem + (size_t)kTbStages * 2 * kInPlane;  // [hi, lo][12 panels]
-    uint8_t *band_base = mid_base + 2 * kMidPlane;
+    uint8_t *stage_base = smem;  // [stage][hi, lo]
+    uint8_t *band_base = smem + (size_t)kTbStages * 2 * SG::PLANE;
     uint64_t *bars = reinterpret_cast<uint64_t *>(band_base + C::BAND);
-    uint64_t *full = bars;                         // [2]
-    uint64_t *empty = bars + 2;                    // [2]
-    uint64_t *inter_ready = bars + 4;              // [1] intermediate written
-    uint64_t *win_full = bars + 5;                 // [kTbRing]
-    uint64_t *win_empty = bars + 5 + kTbRing;      // [kTbRing]
-    uint64_t *drain = bars + 5 + 2 * kTbRing;      // [1]
-    CtaScale cs;                                   // the CTA's side of the scale
-    cs.bar = drain + 1;                            // [2]
+    uint64_t *full = bars;                          // [stages]
+    uint64_t *empty = full + kTbStages;             // [stages]
+    uint64_t *win_empty = empty + kTbStages;        // [kTbRing] region read by its blocks' groups
+    uint64_t *blk_full = win_empty + kTbRing;       // [2][kTbBlocks] a step's block: its windows complete
+    uint64_t *blk_ready = blk_full + 2 * kTbBlocks; // [kTbBlocks] first-step values in the image
+    uint64_t *drain = blk_ready + kTbBlocks;        // [1]
+    CtaScale cs;                                    // the CTA's side of the scale
+    cs.bar = drain + 1;                             // [2]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(cs.bar + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    cs.max = tmem_slot + 2;                        // [2]
-    cs.cnt = cs.max + 2;                           // [2]
+    cs.max = tmem_slot + 2;                         // [2]
+    cs.cnt = cs.max + 2;                            // [2]
     cs.ss = reinterpret_cast<StepScale *>(cs.cnt + 2);  // [2]
-    static_assert((8 + 2 * kTbRing) * 8 + 8 + 16 + 2 * sizeof(StepScale) <= 256, "barrier area");
+    uint32_t *issued = reinterpret_cast<uint32_t *>(cs.ss + 2);  // [kTbIssuers] 1 + its last window
+    static_assert((2 * kTbStages + kTbRing + 3 * kTbBlocks + 3) * 8 + 24 + 2 * sizeof(StepScale) +
+                          4 * kTbIssuers <= C::BARS,
+                  "barrier area");
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const PlaneGeom pg = p.g.p16;
     const int n_mine = (p.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
     if (threadIdx.x == 0) {
@@ -124,11 +189,14 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const TbPara
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], kTbIssuers);
         }
-        mbar_init(inter_ready, kTbEpiWarps);
-        for (int r = 0; r < kTbRing; r++) {
-            mbar_init(&win_full[r], 1);
-            mbar_init(&win_empty[r], kTbEpiWarps);
+        for (int r = 0; r < kTbRing; r++) mbar_init(&win_empty[r], 8);  // two groups
+        for (int b = 0; b < kTbBlocks; b++) {
+            // the halo blocks have one window
+            for (int st = 0; st < 2; st++)
+                mbar_init(&blk_full[st * kTbBlocks + b], b == 0 || b == kTbBlocks - 1 ? 1 : 2);
+            mbar_init(&blk_ready[b], 4);
         }
+        for (int k = 0; k < kTbIssuers; k++) issued[k] = 0;
         mbar_init(drain, kTbIssuers);
         cta_scale_init(cs);
         *abort_flag = 0;
@@ -139,7 +207,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const TbPara
         tmem_alloc(tmem_slot, kTmemCols);
         tmem_relinquish();
     }
-    build_bands(reinterpret_cast<uint16_t *>(band_base), p.coef, C::R, C::BOX, true, threadIdx.x,
+    build_bands(reinterpret_cast<uint16_t *>(band_base), p.coef, R, C::BOX, true, threadIdx.x,
                 kTbThreads);
     fence_proxy_async_smem();
     tc_fence_before();
@@ -150,10 +218,9 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const TbPara
     pdl_launch_dependents();
     pdl_wait();
 
-    auto tile_origin = [&](int i, int &Y0, int &X0) {
-        const int t = (int)blockIdx.x + i * (int)gridDim.x;
-        Y0 = (t / p.tiles_x) * C::H;
-        X0 = (t % p.tiles_x) * kTbCols;
+    auto fail = [&](int code) {
+        record_error(&g_tb_error, code);
+        *abort_flag = 1;
     };
 
     if (warp == 0) {
@@ -163,35 +230,16 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const TbPara
             for (int i = 0; i < n_mine; i++) {
                 const int s = i % kTbStages;
                 if (!mbar_wait(&empty[s], ((i / kTbStages) & 1) ^ 1, abort_flag)) {
-                    record_error(&g_tb_error, kErrWaitEmpty);
-                    *abort_flag = 1;
+                    fail(kErrWaitEmpty);
                     break;
                 }
-                int Y0, X0;
-                tile_origin(i, Y0, X0);
-                const int row0 = Y0 - C::R - 2 + kPadTop;  // >= 0
-                const int rows = min(kRowsStaged, pg.nyp - row0);
-                const int pan0 = (X0 >> 3) - 2;  // plane panel of column X0 - 24
-                uint32_t bytes = 0;
-                for (int q = 0; q < kInPanels; q++) {
-                    const int pan = pan0 + q;
-                    bytes += (pan >= 0 && pan < pg.npan) ? rows * 16 : kChunkBytes;
-                }
-                mbar_arrive_expect_tx(&full[s], 2 * bytes);
-                uint8_t *st = stage_base + (size_t)s * 2 * kInPlane;
-                for (int pl = 0; pl < 2; pl++) {
-                    const uint16_t *src = pl ? p.in_lo : p.in_hi;
-#pragma unroll 1
-                    for (int q = 0; q < kInPanels; q++) {
-                        const int pan = pan0 + q;
-                        uint8_t *dst = st + (size_t)pl * kInPlane + q * kChunkBytes;
-                        if (pan >= 0 && pan < pg.npan)
-                            bulk_load(dst, src + ((size_t)pan * pg.nyp + row0) * 8, rows * 16,
-                                      &full[s]);
-                        else
-                            bulk_load(dst, g_zero_panel, kChunkBytes, &full[s]);
-                    }
-                }
+                const int t = (int)blockIdx.x + i * (int)gridDim.x;
+                const int ty = t / p.tiles_x, tx = t - ty * p.tiles_x;
+                uint8_t *st = stage_base + (size_t)s * 2 * SG::PLANE;
+                mbar_arrive_expect_tx(&full[s], 2 * SG::PLANE);
+                tma_load_3d(st, &p.map_hi, &full[s], 0, ty * kTbRows / kTbMapRows, tx * (kTile / 8));
+                tma_load_3d(st + SG::PLANE, &p.map_lo, &full[s], 0, ty * kTbRows / kTbMapRows,
+                            tx * (kTile / 8));
                 last_issued = i;
             }
             for (int k = 0; k < kTbStages && last_issued - k >= 0; k++) {
@@ -205,58 +253,61 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const TbPara
                 }
             }
         }
-    } else if (warp <= kTbIssuers) {
-        // ---------------------------------------------------- MMA issuer ---
+    } else if (warp < kTbEpi0) {
+        // --------------------------------------------------- MMA issuers ---
         if (lane == 0) {
-            const int id = warp - 1;  // takes the windows G with G % 2 == id
+            const int id = warp - 1;
             const uint32_t band = smem_u32(band_base);
-            int G = 0;
-            bool issued_any = false, stop = false;
-            // the windows of one step of tile i, from stage panel slot0 + 2w
-            // the windows of one step from an image (hi at a_hi0, lo lo_bytes on)
-            auto run_step = [&](uint64_t a_hi0, int lo_bytes, int nwin) {
-#pragma unroll 1
-                for (int w = 0; w < nwin; w++, G++) {
-                    if (G % kTbIssuers != id) continue;
-                    const int r = G % kTbRing;
-                    if (!mbar_wait(&win_empty[r], ((G / kTbRing) & 1) ^ 1, abort_flag)) {
-                        record_error(&g_tb_error, kErrWaitAccum);
-                        *abort_flag = 1;
-                        stop = true;
-                        return;
-                    }
-                    tc_fence_after();
-                    issue_split_window_at<C::R>(a_hi0, band, tmem_base + r * kTbRegion, 2 * w,
-                                                lo_bytes);
-                    umma_commit(&win_full[r]);
-                    issued_any = true;
-                }
+            bool stop = false;
+            // global window, its region, the region's uses before it
+            int G = id, r = id % kTbRing, uses = id / kTbRing;
+            static_assert(2 * kTbWindows % kTbIssuers == 0, "an issuer's windows are the same in every tile");
+            const int before = (id + kTbIssuers - kTbRing % kTbIssuers) % kTbIssuers;  // issuer of G - 5
+            // bounded wait until issuer k has issued window G
+            auto issued_by = [&](int k, int G) {
+                if (ld_acquire_cta(&issued[k]) > (uint32_t)G) return true;
+                const uint64_t t0 = global_timer_ns();
+                while (ld_acquire_cta(&issued[k]) <= (uint32_t)G)
+                    if (*abort_flag || global_timer_ns() - t0 > kWaitLimitNs) return false;
+                return true;
             };
-            const uint64_t mid_desc = smem_desc(smem_u32(mid_base), kChunkBytes, 128);
             for (int i = 0; i < n_mine && !stop; i++) {
                 const int s = i % kTbStages;
                 if (!mbar_wait(&full[s], (i / kTbStages) & 1, abort_flag)) {
-                    record_error(&g_tb_error, kErrWaitFull);
-                    *abort_flag = 1;
+                    fail(kErrWaitFull);
                     break;
                 }
-                tc_fence_after();
-                run_step(smem_desc(smem_u32(stage_base + (size_t)s * 2 * kInPlane), kChunkBytes, 128),
-                         kInPlane, kS1Windows);
-                if (stop) break;
-                umma_commit(&empty[s]);  // the input stage is free once step 1 is done
-                if (!mbar_wait(inter_ready, i & 1, abort_flag)) {
-                    record_error(&g_tb_error, kErrWaitFull);
-                    *abort_flag = 1;
-                    break;
+                const uint64_t a_hi0 =
+                    smem_desc(smem_u32(stage_base + (size_t)s * 2 * SG::PLANE), SG::CHUNK, 128);
+                for (int sw = id; sw < 2 * kTbWindows; sw += kTbIssuers) {
+                    const bool second = sw >= kTbWindows;
+                    const int w = second ? sw - kTbWindows : sw;
+                    // window w's blocks are w and w + 1
+                    if ((G >= kTbRing && !issued_by(before, G - kTbRing)) ||
+                        !mbar_wait(&win_empty[r], (uses & 1) ^ 1, abort_flag) ||
+                        (second && (!mbar_wait(&blk_ready[w], i & 1, abort_flag) ||
+                                    !mbar_wait(&blk_ready[w + 1], i & 1, abort_flag)))) {
+                        fail(kErrWaitAccum);
+                        stop = true;
+                        break;
+                    }
+                    tc_fence_after();
+                    issue_split_window<R, SG>(a_hi0, band, tmem_base + r * kTbRegion, w);
+                    st_release_cta(&issued[id], (uint32_t)G + 1);
+                    // the window's two blocks (the second step has no halo blocks)
+                    uint64_t *bf = blk_full + (second ? kTbBlocks : 0);
+                    if (!second || w > 0) umma_commit(&bf[w]);
+                    if (!second || w < kTbWindows - 1) umma_commit(&bf[w + 1]);
+                    G += kTbIssuers;
+                    r += kTbIssuers;
+                    while (r >= kTbRing) {
+                        r -= kTbRing;
+                        uses++;
+                    }
                 }
-                tc_fence_after();
-                run_step(mid_desc, kMidPlane, kS2Windows);
+                if (!stop) umma_commit(&empty[s]);  // both steps' MMAs have read the stage
             }
-            // both issuers commit (one with nothing in flight completes at
-            // once), so the drain phase always completes
-            (void)issued_any;
-            umma_commit(drain);
+            umma_commit(drain);  // completes at once if nothing is in flight
             const uint64_t t0 = global_timer_ns();
             while (!mbar_try_wait(drain, 0)) {
                 if (global_timer_ns() - t0 > kWaitLimitNs) {
@@ -268,151 +319,147 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const TbPara
     } else {
         // ------------------------------------------------------ epilogue ---
         const int q = warp & 3;
-        const int grp = (warp - 1 - kTbIssuers) >> 2;  // block group
-        const int m = q * 32 + lane;  // M row of the step (intermediate row Y0 - r + m)
+        // A tile's 18 blocks in order: blocks 0 .. 9 of the first step (block
+        // b: columns X0-16+16b ..; 0 and 9 are the halo panels), then 1 .. 8
+        // of the second; this group takes every fourth.
+        const int grp = (warp - kTbEpi0) >> 2;
+        const int m = q * 32 + lane;            // tile row
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
-        TileOut o;
-        o.in_hi = p.in_hi;
-        o.in_lo = p.in_lo;
-        o.out_hi = p.out_hi;
-        o.out_lo = p.out_lo;
-        o.pg = pg;
-        o.y0 = p.g.y0; o.y1 = p.g.y1; o.x0 = p.g.x0; o.x1 = p.g.x1;
-        o.ny = p.g.ny; o.nx = p.g.nx;
-        int G0 = 0;
+        const GridGeom &g = p.g;
         bool stop = false;
-        // bounded wait for window w of the current step (from G0)
-        auto ready = [&](int w) {
-            const int Gw = G0 + w;
-            bool ok = mbar_wait(&win_full[Gw % kTbRing], (Gw / kTbRing) & 1, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok && lane == 0) {
-                record_error(&g_tb_error, kErrWaitResult);
-                *abort_flag = 1;
-            }
-            return ok;
-        };
-        auto release = [&](int w) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&win_empty[(G0 + w) % kTbRing]);
-        };
-        // Blocks of one step: block j sums windows j and j+1 and belongs to
-        // group j mod 3; every window is released by all twelve warps.
-        auto run_step = [&](int nwin, auto &&store) {
-            const bool ok = walk_windows(grp, kTbGroups, nwin, ready, release, [&](int j) {
-                const int Ga = G0 + j, Gb = Ga + 1;
-                tc_fence_after();
-                float f[16];
-                split_block_load(lane_base + (Ga % kTbRing) * kTbRegion,
-                                 lane_base + (Gb % kTbRing) * kTbRegion, f);
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&win_empty[Ga % kTbRing]);
-                    mbar_arrive(&win_empty[Gb % kTbRing]);
-                }
-                store(j, f);
-            });
-            if (!ok) stop = true;
-            G0 += nwin;
-        };
         // The pair's two scales, both from steps finished before the launch
         // (step t reads steps t-2 and t-3), read by the first epilogue warp;
         // the second step's copies come from the input, two steps back, so
         // they take both shifts.
-        if (warp == 1 + kTbIssuers && lane == 0) {
+        if (warp == kTbEpi0 && lane == 0) {
             cta_scale_publish(cs, 0, step_scale(p.scale, p.t0 + 1));
             cta_scale_publish(cs, 1, step_scale(p.scale, p.t0 + 2));
         }
         StepScale ss1, ss2;
         if (!cta_scale_take(cs, 0, ss1, abort_flag) || !cta_scale_take(cs, 1, ss2, abort_flag)) {
-            if (lane == 0) {
-                record_error(&g_tb_error, kErrWaitResult);
-                *abort_flag = 1;
-            }
+            if (lane == 0) fail(kErrWaitResult);
             stop = true;
         }
         StepScale cs2 = ss2;
         cs2.k = ss1.k + ss2.k;
         cs2.s = __int_as_float((127 + 11 + cs2.k) << 23);
         float mx1 = 0.0f, mx2 = 0.0f;
-        for (int i = 0; i < n_mine && !stop; i++) {
-            int Y0, X0;
-            tile_origin(i, Y0, X0);
-            {
-                // step 1 -> the intermediate image
-                const int y = Y0 - C::R + m;
-                const int xi = X0 - 16;  // first column of step 1's blocks
-                const bool fast = Y0 - C::R >= o.y0 && Y0 - C::R + kTile <= o.y1 &&
-                                  xi >= o.x0 && xi + 112 <= o.x1;
-                const bool row_in = y >= o.y0 && y < o.y1;
-                run_step(kS1Windows, [&](int j, const float (&f)[16]) {
-                    const int xb = xi + 16 * j;
-                    uint32_t hw[8], lw[8];
-                    if (fast) {
-#pragma unroll
-                        for (int c = 0; c < 8; c++)
-                            split_pair_s(f[2 * c], f[2 * c + 1], ss1.s, hw[c], lw[c], mx1);
-                    } else {
-                        const uint4 a0 = load_panel_row(o.in_hi, pg, y, xb);
-                        const uint4 a1 = load_panel_row(o.in_hi, pg, y, xb + 8);
-                        const uint4 b0 = load_panel_row(o.in_lo, pg, y, xb);
-                        const uint4 b1 = load_panel_row(o.in_lo, pg, y, xb + 8);
-                        const uint32_t iw[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                        const uint32_t il[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-                        for (int c = 0; c < 8; c++) {
-                            uint16_t hh[2], ll[2];
-#pragma unroll
-                            for (int u2 = 0; u2 < 2; u2++) {
-                                const int x = xb + 2 * c + u2;
-                                if (row_in && x >= o.x0 && x < o.x1) {
-                                    split_fixed_s(f[2 * c + u2], ss1.s, hh[u2], ll[u2], mx1);
-                                } else {
-                                    hh[u2] = (uint16_t)(iw[c] >> (16 * u2));
-                                    ll[u2] = (uint16_t)(il[c] >> (16 * u2));
-                                    if (ss1.k != 0) resplit_pair(hh[u2], ll[u2], ss1);
-                                }
-                            }
-                            hw[c] = (uint32_t)hh[0] | ((uint32_t)hh[1] << 16);
-                            lw[c] = (uint32_t)ll[0] | ((uint32_t)ll[1] << 16);
-                        }
-                    }
-                    // block j = intermediate panels 2j-1, 2j (those of the
-                    // 12 kept), image row m + 2
-#pragma unroll
-                    for (int hlf = 0; hlf < 2; hlf++) {
-                        const int pnl = 2 * j - 1 + hlf;
-                        if (pnl < 0 || pnl >= kMidPanels) continue;
-                        uint8_t *h0 = mid_base + (size_t)pnl * kChunkBytes + (m + 2) * 16;
-                        const int c0 = 4 * hlf;
-                        *reinterpret_cast<uint4 *>(h0) =
-                            make_uint4(hw[c0], hw[c0 + 1], hw[c0 + 2], hw[c0 + 3]);
-                        *reinterpret_cast<uint4 *>(h0 + kMidPlane) =
-                            make_uint4(lw[c0], lw[c0 + 1], lw[c0 + 2], lw[c0 + 3]);
-                    }
-                });
-                if (stop) break;
-                // the intermediate is an MMA operand next
-                fence_proxy_async_smem();
+        int r0 = 0;  // ring region of the tile's window 0
+        // One block: wait for its windows, load and sum its panels, give the
+        // windows back, and sink each panel (its index in the image, its
+        // eight values).  rb: region of the step's window 0, at most 4.
+        auto take_block = [&](int st, int b, int rb, int i, const StepScale &ss, auto &&sink) {
+            bool ok = mbar_wait(&blk_full[st * kTbBlocks + b], i & 1, abort_flag);
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0) fail(kErrWaitResult);
+                return false;
+            }
+            tc_fence_after();
+            auto region = [&](int w) {
+                const int x = rb + w;  // < 14
+                return x >= 10 ? x - 10 : x >= 5 ? x - 5 : x;
+            };
+            const int wa = region(b - 1), wb = region(b);
+            const uint32_t ta = lane_base + (uint32_t)(wa * kTbRegion) + 16;  // its second half
+            const uint32_t tb = lane_base + (uint32_t)(wb * kTbRegion);       // its first half
+            auto release = [&]() {
+                tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(inter_ready);
+                if (lane == 0) {
+                    // in the second step the outer windows have one block
+                    if (b > 0) mbar_arrive_n(&win_empty[wa], st == 1 && b == 1 ? 2 : 1);
+                    if (b < kTbBlocks - 1) mbar_arrive_n(&win_empty[wb], st == 1 && b == kTbBlocks - 2 ? 2 : 1);
+                }
+            };
+            float u[8];
+            uint32_t v[6][8];
+            if (b == 0 || b == kTbBlocks - 1) {
+                // halo panel: the inner one of the block; cells that lack a
+                // column of the input are zero (nothing valid reads them)
+                panel_load(b == 0 ? tb + 8 : ta, 0, false, v);
+                tmem_ld_wait();
+                release();
+                panel_sum(v, false, ss, u);
+#pragma unroll
+                for (int c = 0; c < 8; c++)
+                    if (b == 0 ? c < R : c >= 8 - R) u[c] = 0.0f;
+                sink(b == 0 ? 0 : 2 * b - 1, u);
+            } else {
+                // (both panels are summed before the first is split: with
+                // five regions the windows wait for this release)
+                float u2[8];
+                panel_load(ta, tb, true, v);
+                tmem_ld_wait();
+                panel_sum(v, true, ss, u);
+                panel_load(ta + 8, tb + 8, true, v);
+                tmem_ld_wait();
+                release();
+                panel_sum(v, true, ss, u2);
+                sink(2 * b - 1, u);
+                sink(2 * b, u2);
             }
-            {
-                // step 2 -> the output plane
-                const int y = Y0 - C::R + m;
-                const bool mine = m >= C::R && m < kTile - C::R && y < p.g.ny;
-                const bool fast = Y0 >= o.y0 && Y0 + C::H <= o.y1 && X0 >= o.x0 &&
-                                  X0 + kTbCols <= o.x1;
-                const bool row_in = y >= o.y0 && y < o.y1;
-                run_step(kS2Windows, [&](int j, const float (&f)[16]) {
-                    const int xb = X0 + 16 * j;
-                    if (mine && xb < p.g.nx) store_block_split(o, f, y, xb, fast, row_in, ss2, mx2);
-                });
-                if (!stop && mine && cs2.k != 0 && !fast)
-                    resplit_border(o, y, X0, grp, kTbGroups, kS2Windows - 1, cs2);
+            return true;
+        };
+        for (int i = 0; i < n_mine && !stop; i++) {
+            const int t = (int)blockIdx.x + i * (int)gridDim.x;
+            const int ty = t / p.tiles_x, tx = t - ty * p.tiles_x;
+            const int Yb = ty * kTbRows, X0 = tx * kTile;
+            const int y = Yb + m;
+            const bool top = ty == 0, bottom = ty == p.tiles_y - 1;
+            const bool row_in = y >= g.y0 && y < g.y1;
+            // first step: all of the image's rows may be updated; second: the
+            // rows this tile owns
+            const bool rows1 = Yb >= g.y0 && Yb + kTile <= g.y1;
+            const bool rows2 = !top && !bottom && Yb + kTbHalo >= g.y0 && Yb + kTile - kTbHalo <= g.y1;
+            const bool mine = (top || m >= kTbHalo) && (bottom || m < kTile - kTbHalo) && y < g.ny;
+            const uint32_t img = smem_u32(stage_base) +
+                                 (uint32_t)((i % kTbStages) * 2 * SG::PLANE + (m + SG::TOP) * 16);
+            const size_t row0 = plane_index16(g.p16, mine ? y : 0, X0 - 8);
+            for (int idx = grp; idx < 2 * kTbWindows && !stop; idx += kTbGroups) {
+                if (idx < kTbBlocks) {
+                    // first step -> the image
+                    const bool ok = take_block(0, idx, r0, i, ss1, [&](int pan, const float (&u)[8]) {
+                        const int xb = X0 - 8 + 8 * pan;
+                        const uint32_t a = img + (uint32_t)(pan * SG::CHUNK);
+                        PanelPair w;
+                        if (rows1 && xb >= g.x0 && xb + 8 <= g.x1) {
+                            w = split_panel(u, mx1);
+                        } else {
+                            const PanelPair old{lds128(a), lds128(a + SG::PLANE)};
+                            w = split_panel_edge(u, old, xb, row_in, g.x0, g.x1, ss1, mx1);
+                        }
+                        sts128(a, w.hi);
+                        sts128(a + SG::PLANE, w.lo);
+                    });
+                    if (!ok) {
+                        stop = true;
+                        break;
+                    }
+                    fence_proxy_async_smem();  // an MMA operand next
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&blk_ready[idx]);
+                } else {
+                    // second step -> the output planes
+                    const int rb = r0 + 4 >= 5 ? r0 - 1 : r0 + 4;  // nine windows on
+                    const bool ok = take_block(1, idx - kTbWindows, rb, i, ss2, [&](int pan, const float (&u)[8]) {
+                        const int xb = X0 - 8 + 8 * pan;
+                        if (!mine || xb >= g.nx) return;
+                        const size_t off = row0 + (size_t)pan * g.p16.nyp * 8;
+                        PanelPair w;
+                        if (rows2 && xb >= g.x0 && xb + 8 <= g.x1) {
+                            w = split_panel(u, mx2);
+                        } else {
+                            const PanelPair old{*reinterpret_cast<const uint4 *>(p.in_hi + off),
+                                                *reinterpret_cast<const uint4 *>(p.in_lo + off)};
+                            w = split_panel_edge(u, old, xb, row_in, g.x0, g.x1, cs2, mx2);
+                        }
+                        *reinterpret_cast<uint4 *>(p.out_hi + off) = w.hi;
+                        *reinterpret_cast<uint4 *>(p.out_lo + off) = w.lo;
+                    });
+                    if (!ok) stop = true;
+                }
             }
+            r0 = r0 + 3 >= 5 ? r0 - 2 : r0 + 3;  // 18 windows on
         }
         if (!stop && p.scale) {  // tile 0 is CTA 0's
             cta_scale_flush<kTbEpiWarps>(cs, 0, p.scale, p.t0 + 1, ss1, mx1, blockIdx.x == 0);
@@ -452,8 +499,12 @@ cudaError_t launch_tb(const GridGeom &g, const float *B, const uint16_t *in_hi,
     }
     TbParams p;
     p.g = g;
-    p.tiles_x = (g.nx + kTbCols - 1) / kTbCols;
-    p.n_tiles = p.tiles_x * ((g.ny + C::H - 1) / C::H);
+    cudaError_t e = encode_panel_map(in_hi, g.p16, &p.map_hi, kTile / 8 + 2, kTbMapRows);
+    if (e == cudaSuccess) e = encode_panel_map(in_lo, g.p16, &p.map_lo, kTile / 8 + 2, kTbMapRows);
+    if (e != cudaSuccess) return e;
+    p.tiles_x = (g.nx + kTile - 1) / kTile;
+    p.tiles_y = g.ny <= kTile ? 1 : (g.ny - 2 * kTbHalo + kTbRows - 1) / kTbRows;
+    p.n_tiles = p.tiles_x * p.tiles_y;
     p.in_hi = in_hi;
     p.in_lo = in_lo;
     p.out_hi = out_hi;

@@ -268,7 +268,6 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
     using M = Mode<SPLIT>;
     constexpr int NS = C::STAGES;
     constexpr int NP = M::PLANES;
-    constexpr int NSUB = M::NSUB;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
         }
     } else if (warp <= Sweep<S>::ISSUERS) {
         // --------------------------------------------------- MMA issuers ---
-        static_assert(!SPLIT && NSUB == 1, "one plain sub-tile per tile");
+        static_assert(!SPLIT, "plain tiles");
         if (lane == 0) {
             const int id = warp - 1;  // issues the tiles i with i % Sweep<S>::ISSUERS == id
             bool stop = false;
@@ -801,16 +800,17 @@ __global__ void __launch_bounds__(Ring<MULTI>::THREADS, 1) tc_split_ring_kernel(
             const bool ok = walk_windows(grp, kRingGroups, kTileWindows, ready, release, [&](int j) {
                 const int Ga = G0 + j, Gb = Ga + 1;
                 tc_fence_after();
-                float f[16];
+                float u[16];
                 split_block_load(lane_base + (Ga % kRingSlots) * kRegionCols,
-                                 lane_base + (Gb % kRingSlots) * kRegionCols, f);
+                                 lane_base + (Gb % kRingSlots) * kRegionCols, u);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(&win_empty[Ga % kRingSlots]);
                     mbar_arrive(&win_empty[Gb % kRingSlots]);
                 }
-                store_block_split(o, f, y, X0 + 16 * j, fast, row_in, ss, mx);
+                shift_block(u, ss);
+                store_block_split(o, u, y, X0 + 16 * j, fast, row_in, mx);
             });
             if (!ok) break;
             if (ss.k != 0 && !fast) resplit_border(o, y, X0, grp, kRingGroups, kTileWindows - 1, ss);

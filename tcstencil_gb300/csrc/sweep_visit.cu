@@ -78,20 +78,6 @@ struct VisitParams {
 
 __host__ __device__ constexpr int visit_stage_bytes(int W) { return (W / 8 + 2) * SG::CHUNK; }
 
-__device__ __forceinline__ void sts128(uint32_t addr, const uint4 &v) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y),
-                 "r"(v.z), "r"(v.w)
-                 : "memory");
-}
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "r"(addr)
-                 : "memory");
-    return v;
-}
-
 // 8 accumulators as a panel row of FP16 cells.
 __device__ __forceinline__ uint4 pack_panel(const uint32_t *v) {
     uint32_t w[4];
@@ -145,8 +131,8 @@ __device__ __forceinline__ void walk_blocks(uint32_t col, Sink &&sink) {
 // of unrolled, the issuing thread took 87 cycles per MMA instead of 67.)
 template <int R, int NWIN>
 __device__ __forceinline__ void issue_visit_tile(uint64_t a0, uint32_t band, uint32_t d, int nwin) {
-    if (NWIN > 5 && nwin <= 5) issue_subtile<R, false, SG, 5>(a0, band, d, 0);
-    else issue_subtile<R, false, SG, NWIN>(a0, band, d, 0);
+    if (NWIN > 5 && nwin <= 5) issue_plain_windows<R, SG, 5>(a0, band, d);
+    else issue_plain_windows<R, SG, NWIN>(a0, band, d);
 }
 
 // What one epilogue warp does with a tile: fixed over the tile's steps.

@@ -12,10 +12,7 @@
 namespace tcs {
 namespace tc {
 
-constexpr int kRowsStaged = kTile + 4;          // two halo rows above and below
-constexpr int kChunkBytes = kRowsStaged * 16;   // one panel of a stage
 constexpr int kSlots = kTile / 8 + 2;           // 16 panels + one each side
-constexpr int kPlaneStage = kSlots * kChunkBytes;
 
 // Staged-panel geometry: CHUNK bytes per panel (rows at a 16-byte stride),
 // TOP rows staged above the tile, PLANE bytes per staged plane.
@@ -25,8 +22,6 @@ struct Staging {
     static constexpr int TOP = TOP_;
     static constexpr int PLANE = kSlots * CHUNK_;
 };
-// 132 rows from Y0 - 2: the two halo rows each side a radius-2 stencil needs.
-using StageHalo2 = Staging<kChunkBytes, 2>;
 // 136 rows from Y0 - 4: every panel run starts on a 128-byte line (tile rows
 // are multiples of 128 and the plane's top padding is 4 rows), so a tile's
 // copies move 17 whole lines per panel instead of 17 partial ones.
@@ -39,29 +34,22 @@ constexpr int kSlotCols = 256;                  // AccSlots: two slots of the ba
 constexpr uint32_t kIdesc = idesc_f16_f32(128, 32);
 constexpr uint32_t kIdescStack = idesc_f16_f32(128, 96);
 
-// Accumulator layout.
-//  plain: one 128-column tile; window w adds into columns [16w, 16w+32) of a
-//    160-column accumulator (overlapping windows accumulate in place); it
-//    occupies one slot, so two sub-tiles double-buffer.
-//  split: 64-column sub-tiles of five windows.  Each window has its own
-//    96-column region [ch.hi | cl.hi + cf.lo | c3.hi] (three products of the
-//    stacked band in one N=96 MMA, the lo product accumulated into the middle
-//    part), even windows at 96e, odd windows at 288 + 96o: 480 columns, both
-//    slots.  Neighbouring windows then never share columns, and an output
-//    block sums the second half of window j with the first half of window j+1.
+// Plain accumulators: one 128-column tile, window w adding into columns
+// [16w, 16w+32) of a 160-column slot (overlapping windows accumulate in
+// place).  Split accumulators: each window has its own 96-column region
+// [ch.hi | cl.hi + cf.lo | c3.hi] (three products of the stacked band in one
+// N=96 MMA, the lo product accumulated into the middle part) in a ring;
+// neighbouring windows then never share columns, and an output block sums the
+// second half of window j with the first half of window j+1.
 template <bool SPLIT>
 struct Mode {
-    static constexpr int NSUB = SPLIT ? 2 : 1;            // sub-tiles per tile
-    static constexpr int SUB_BLOCKS = kTile / 16 / NSUB;  // 16-column blocks per sub-tile
-    static constexpr int SUB_WIN = SUB_BLOCKS + 1;        // input windows per sub-tile
-    static constexpr int ACC = SPLIT ? 480 : 16 * (SUB_BLOCKS + 2);  // TMEM columns used
+    static constexpr int SUB_BLOCKS = kTile / 16;         // 16-column blocks per tile
+    static constexpr int SUB_WIN = SUB_BLOCKS + 1;        // input windows per tile
+    static constexpr int ACC = 16 * (SUB_BLOCKS + 2);     // TMEM columns of a plain tile
     static constexpr int PLANES = SPLIT ? 2 : 1;          // hi (and lo) data planes
     static constexpr int BAND_PLANES = SPLIT ? 4 : 1;     // band bytes per row, in kBandBytes
 };
-static_assert(Mode<false>::ACC <= kSlotCols && Mode<true>::ACC <= kTmemCols, "TMEM layout");
-
-// First TMEM column of split window w's region.
-__host__ __device__ constexpr int split_region(int w) { return (w & 1) ? 288 + 96 * (w >> 1) : 96 * (w >> 1); }
+static_assert(Mode<false>::ACC <= kSlotCols, "TMEM layout");
 
 // Which accumulator slots a sub-tile holds: plain sub-tiles alternate between
 // the two slots, a split sub-tile takes both.  The MMA issuer and the
@@ -154,8 +142,8 @@ __device__ __forceinline__ int split_exp_of(unsigned mbits, unsigned bbits, int 
 }
 
 // Scale of step t (the step index within the run, from 1): s = 2^(11 + k_t)
-// turns the step's value v (units of 2^E_{t-1}) into u = v s, the new state
-// in units of 2^-11 of 2^E_t.  Without a scale record (sc null) k = 0.
+// turns a value v in units of 2^E_{t-1} into u = v s, the new state in units
+// of 2^-11 of 2^E_t.  Without a scale record (sc null) k = 0.
 struct StepScale {
     float s;
     int k, e;
@@ -274,19 +262,9 @@ __device__ __forceinline__ void cta_scale_flush(const CtaScale &c, int n, SplitS
     }
 }
 
-// Fixed-point split of a value v (|v| about 1 or below): hi = fp16 of
-// rint(v 2^11) 2^-11, lo = fp16((v - hi) 2^11).
-__device__ __forceinline__ void split_fixed(float v, uint16_t &hi, uint16_t &lo) {
-    hi = h_bits(rintf(v * 2048.0f) * (1.0f / 2048.0f));
-    lo = h_bits((v - h_val(hi)) * 2048.0f);
-}
-
-// split_fixed of the value v 2^k, with s = 2^(11 + k) (StepScale): u = v s,
-// hi = fp16(rint(u) 2^-11), lo = fp16(u - hi 2^11), the same bits as
-// split_fixed(v) when k = 0; the largest |u| is kept in mx.
-__device__ __forceinline__ void split_fixed_s(float v, float s, uint16_t &hi, uint16_t &lo,
-                                              float &mx) {
-    const float u = v * s;
+// The split form's epilogue works on u, the new value in units of 2^-11: hi =
+// fp16(rint(u) 2^-11), lo = fp16(u - hi 2^11); the largest |u| is kept in mx.
+__device__ __forceinline__ void split_fixed_u(float u, uint16_t &hi, uint16_t &lo, float &mx) {
     hi = h_bits(rintf(u) * (1.0f / 2048.0f));
     lo = h_bits(u - h_val(hi) * 2048.0f);
     mx = fmaxf(mx, fabsf(u));
@@ -312,57 +290,78 @@ __device__ __forceinline__ uint32_t pack_h2(float v0, float v1) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// split_fixed of two values into packed hi and lo words, with the same bits
-// and less conversion work: u = v 2^11 is exact, t = rint(u) is formed by the
-// add-and-subtract of 1.5 * 2^23 (round to nearest even for |u| < 2^22; the
-// sign copy keeps rint's -0 for small negative u).  While |t| <= 2^11, hi =
-// t 2^-11 is exact in FP16 and lo = u - t = (v - hi) 2^11 is exact; past that
-// (|v| slightly above 1, or NaN) hi rounds in FP16 and split_fixed's rule is
-// taken.
-// With s = 2^(11 + k) the pair is of v 2^k (StepScale), and the largest |u|
-// is kept in mx.
-__device__ __forceinline__ void split_pair_s(float v0, float v1, float s, uint32_t &hw,
-                                             uint32_t &lw, float &mx) {
+// split_fixed_u of two values into packed hi and lo words, with the same
+// values and less conversion work: t = rint(u) is formed by the
+// add-and-subtract of 1.5 * 2^23 (round to nearest even for |u| < 2^22; a zero
+// t is +0).  While |t| <= 2^11, hi = t 2^-11 is exact in FP16 and lo = u - t is
+// exact; past that (|u| above 2048.5: the value slightly above 1, or NaN) hi
+// rounds in FP16 and split_fixed_u's rule is taken.  One comparison serves
+// both values, on the maximum that mx needs anyway.
+__device__ __forceinline__ void split_pair_u(float u0, float u1, uint32_t &hw, uint32_t &lw,
+                                             float &mx) {
     constexpr float kRound = 12582912.0f;  // 1.5 * 2^23
-    // packed FP32 operations on the pair: each lane rounds as the scalar
-    // operation would, so the bits are split_pair's
-    const float2 u = __fmul2_rn(make_float2(v0, v1), make_float2(s, s));
-    const float u0 = u.x, u1 = u.y;
-    mx = fmaxf(mx, fmaxf(fabsf(u0), fabsf(u1)));
-    const float2 r = __fadd2_rn(__fadd2_rn(u, make_float2(kRound, kRound)),
+    const float2 u = make_float2(u0, u1);
+    const float m = fmaxf(fabsf(u0), fabsf(u1));
+    mx = fmaxf(mx, m);
+    // packed FP32 operations: each lane rounds as the scalar one would
+    const float2 t = __fadd2_rn(__fadd2_rn(u, make_float2(kRound, kRound)),
                                 make_float2(-kRound, -kRound));
-    const float t0 = copysignf(r.x, u0);
-    const float t1 = copysignf(r.y, u1);
-    if (fabsf(t0) <= 2048.0f && fabsf(t1) <= 2048.0f) {
-        const float2 t = make_float2(t0, t1);
+    if (m <= 2048.5f) {
         const float2 h = __fmul2_rn(t, make_float2(1.0f / 2048.0f, 1.0f / 2048.0f));
         const float2 l = __ffma2_rn(t, make_float2(-1.0f, -1.0f), u);  // u - t, exact
         hw = pack_h2(h.x, h.y);
         lw = pack_h2(l.x, l.y);
     } else {
         uint16_t h0, l0, h1, l1;
-        split_fixed_s(v0, s, h0, l0, mx);
-        split_fixed_s(v1, s, h1, l1, mx);
+        split_fixed_u(u0, h0, l0, mx);
+        split_fixed_u(u1, h1, l1, mx);
         hw = (uint32_t)h0 | ((uint32_t)h1 << 16);
         lw = (uint32_t)l0 | ((uint32_t)l1 << 16);
     }
 }
 
-__device__ __forceinline__ void split_pair(float v0, float v1, uint32_t &hw, uint32_t &lw) {
+// split_pair_u of a panel row's eight values, with one range check for all
+// (a check per pair is a branch per pair: 550 cycles per panel row in the
+// blocked kernel, whose warps wait on each).
+struct PanelPair {
+    uint4 hi, lo;
+};
+__device__ __forceinline__ PanelPair split_panel(const float (&u)[8], float &mx) {
     constexpr float kRound = 12582912.0f;  // 1.5 * 2^23
-    const float u0 = v0 * 2048.0f, u1 = v1 * 2048.0f;
-    const float t0 = copysignf(__fsub_rn(__fadd_rn(u0, kRound), kRound), u0);
-    const float t1 = copysignf(__fsub_rn(__fadd_rn(u1, kRound), kRound), u1);
-    if (fabsf(t0) <= 2048.0f && fabsf(t1) <= 2048.0f) {
-        hw = pack_h2(t0 * (1.0f / 2048.0f), t1 * (1.0f / 2048.0f));
-        lw = pack_h2(__fsub_rn(u0, t0), __fsub_rn(u1, t1));
-    } else {
-        uint16_t h0, l0, h1, l1;
-        split_fixed(v0, h0, l0);
-        split_fixed(v1, h1, l1);
-        hw = (uint32_t)h0 | ((uint32_t)h1 << 16);
-        lw = (uint32_t)l0 | ((uint32_t)l1 << 16);
+    uint32_t hw[4], lw[4];
+    float m = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const float2 v = make_float2(u[2 * c], u[2 * c + 1]);
+        m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+        const float2 t = __fadd2_rn(__fadd2_rn(v, make_float2(kRound, kRound)),
+                                    make_float2(-kRound, -kRound));
+        const float2 h = __fmul2_rn(t, make_float2(1.0f / 2048.0f, 1.0f / 2048.0f));
+        const float2 l = __ffma2_rn(t, make_float2(-1.0f, -1.0f), v);  // exact
+        hw[c] = pack_h2(h.x, h.y);
+        lw[c] = pack_h2(l.x, l.y);
     }
+    mx = fmaxf(mx, m);
+    if (m > 2048.5f) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            uint16_t h0, l0, h1, l1;
+            split_fixed_u(u[2 * c], h0, l0, mx);
+            split_fixed_u(u[2 * c + 1], h1, l1, mx);
+            hw[c] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+            lw[c] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+        }
+    }
+    return PanelPair{make_uint4(hw[0], hw[1], hw[2], hw[3]), make_uint4(lw[0], lw[1], lw[2], lw[3])};
+}
+
+// A block's values in the units of the step's new scale (StepScale): 2^k of
+// them, exactly; most steps move no scale.
+__device__ __forceinline__ void shift_block(float (&u)[16], const StepScale &ss) {
+    if (ss.k == 0) return;
+    const float f = ss.s * (1.0f / 2048.0f);
+#pragma unroll
+    for (int c = 0; c < 16; c++) u[c] *= f;
 }
 
 // Band element (n, k) of coefficient row dy: input column k of a 16-column
@@ -432,9 +431,11 @@ __device__ __forceinline__ void load_tile_map(const CUtensorMap *hi, const CUten
 
 // One 16-column output block of the split form from the regions of its two
 // windows (TMEM addresses of this warp's lane quarter at each region): the
-// second half of window a plus the first half of window b, per part.
+// second half of window a plus the first half of window b, per part, as u
+// (units of 2^-11 of the input's scale).  main (the exact sum of ch.hi) times
+// 2^11 is exact, so u rounds once, as main + corr 2^-11 would.
 __device__ __forceinline__ void split_block_load(uint32_t region_a, uint32_t region_b,
-                                                 float (&f)[16]) {
+                                                 float (&u)[16]) {
     uint32_t v[6][16];
 #pragma unroll
     for (int part = 0; part < 3; part++) {
@@ -442,8 +443,8 @@ __device__ __forceinline__ void split_block_load(uint32_t region_a, uint32_t reg
         tmem_ld_x16(region_b + 32 * part, v[2 * part + 1]);
     }
     tmem_ld_wait();
-    // main (exact sum of ch.hi), correction in units of 2^-11; two columns
-    // per packed FP32 operation (each lane rounds as the scalar one would)
+    // two columns per packed FP32 operation (each lane rounds as the scalar
+    // one would)
     auto pr = [&](int part, int c) {
         return make_float2(__uint_as_float(v[part][c]), __uint_as_float(v[part][c + 1]));
     };
@@ -451,38 +452,30 @@ __device__ __forceinline__ void split_block_load(uint32_t region_a, uint32_t reg
     for (int c = 0; c < 16; c += 2) {
         const float2 main = __fadd2_rn(pr(0, c), pr(1, c));
         const float2 corr = __fadd2_rn(__fadd2_rn(pr(2, c), pr(3, c)), __fadd2_rn(pr(4, c), pr(5, c)));
-        const float2 r = __ffma2_rn(corr, make_float2(1.0f / 2048.0f, 1.0f / 2048.0f), main);
-        f[c] = r.x;
-        f[c + 1] = r.y;
+        const float2 r = __ffma2_rn(main, make_float2(2048.0f, 2048.0f), corr);
+        u[c] = r.x;
+        u[c + 1] = r.y;
     }
 }
 
-// MMAs of one split window, whose K panels are stage slots `slot` and
-// `slot`+1 (the lo image lo_bytes after the hi image), into the 96-column
-// region at d: per coefficient row, the stacked hi MMA (which
-// initialises the region on the first row) and the lo MMA into its middle
-// part.
-template <int R, class SG = StageHalo2>
-__device__ __forceinline__ void issue_split_window_at(uint64_t a_hi0, uint32_t band, uint32_t d,
-                                                      int slot, int lo_bytes = SG::PLANE) {
+// MMAs of window wg of a staged split tile (its panels 2wg, 2wg+1; the lo
+// image SG::PLANE bytes after the hi image) into the 96-column region at d:
+// per coefficient row, the stacked hi MMA (which initialises the region on
+// the first row) and the lo MMA into its middle part.
+template <int R, class SG>
+__device__ __forceinline__ void issue_split_window(uint64_t a_hi0, uint32_t band, uint32_t d,
+                                                   int wg) {
     constexpr int NDY = 2 * R + 1;
-    const uint64_t a_lo0 = a_hi0 + (uint64_t)(lo_bytes >> 4);
+    const uint64_t a_lo0 = a_hi0 + (uint64_t)(SG::PLANE >> 4);
     const uint64_t bs0 = smem_desc(band, 1536, 128);
     const uint64_t bf0 = smem_desc(band + NDY * 3072, 512, 128);
 #pragma unroll
     for (int dy = 0; dy < NDY; dy++) {
-        const uint64_t a_off = (uint64_t)((slot * SG::CHUNK + (SG::TOP - R + dy) * 16) >> 4);
+        const uint64_t a_off = (uint64_t)((2 * wg * SG::CHUNK + (SG::TOP - R + dy) * 16) >> 4);
         umma_f16(d, a_hi0 + a_off, bs0 + (uint64_t)((dy * 3072) >> 4), kIdescStack,
                  dy > 0 ? 1u : 0u);
         umma_f16(d + 32, a_lo0 + a_off, bf0 + (uint64_t)((dy * kBandBytes) >> 4), kIdesc, 1u);
     }
-}
-
-// The same for window wg of a staged tile (its panels 2wg, 2wg+1).
-template <int R, class SG = StageHalo2>
-__device__ __forceinline__ void issue_split_window(uint64_t a_hi0, uint32_t band, uint32_t d,
-                                                   int wg) {
-    issue_split_window_at<R, SG>(a_hi0, band, d, 2 * wg);
 }
 
 // Windows a tile needs: output block j (columns X0 + 16j .. +15) takes
@@ -497,41 +490,29 @@ __device__ __forceinline__ int tile_windows(int nx, int X0, int W = kTile) {
     return (nb < W / 16 ? nb : W / 16) + 1;
 }
 
-// MMAs of sub-tile h of a staged tile into accumulator columns from d.
-// a_hi0 is the descriptor of the stage's hi plane (lo follows at
-// +kPlaneStage); band is the shared-memory address of the stencil's bands.
-// Descriptors for base + offset are the base descriptor plus offset >> 4 (the
-// start-address field holds address >> 4 in its low bits).
-//  plain: even windows (disjoint outputs, the first of them initialising)
-//    before odd windows, which add into the overlaps; NWIN windows (all, or
-//    the first half's, issue_plain_tile).
-//  split: per window and coefficient row, one N=96 MMA of hi with the stacked
-//    band (initialising its region on the first row) and one N=32 MMA of lo
-//    with cf into the region's middle part.
-template <int R, bool SPLIT, class SG = StageHalo2, int NWIN = Mode<SPLIT>::SUB_WIN>
-__device__ __forceinline__ void issue_subtile(uint64_t a_hi0, uint32_t band, uint32_t d, int h) {
-    using M = Mode<SPLIT>;
+// MMAs of the first NWIN windows of a staged plain tile into accumulator
+// columns from d.  a_hi0 is the descriptor of the stage's plane; band is the
+// shared-memory address of the stencil's bands.  Descriptors for base +
+// offset are the base descriptor plus offset >> 4 (the start-address field
+// holds address >> 4 in its low bits).  Even windows (disjoint outputs, the
+// first of them initialising) come before odd windows, which add into the
+// overlaps.
+template <int R, class SG, int NWIN = Mode<false>::SUB_WIN>
+__device__ __forceinline__ void issue_plain_windows(uint64_t a_hi0, uint32_t band, uint32_t d) {
     constexpr int NDY = 2 * R + 1;
-    if (!SPLIT) {
-        const uint64_t b0 = smem_desc(band, 512, 128);
+    const uint64_t b0 = smem_desc(band, 512, 128);
 #pragma unroll
-        for (int parity = 0; parity < 2; parity++) {
+    for (int parity = 0; parity < 2; parity++) {
 #pragma unroll
-            for (int dy = 0; dy < NDY; dy++) {
-                const uint64_t b = b0 + (uint64_t)((dy * kBandBytes) >> 4);
-                const uint32_t acc = (parity == 1 || dy > 0) ? 1u : 0u;
+        for (int dy = 0; dy < NDY; dy++) {
+            const uint64_t b = b0 + (uint64_t)((dy * kBandBytes) >> 4);
+            const uint32_t acc = (parity == 1 || dy > 0) ? 1u : 0u;
 #pragma unroll
-                for (int w = parity; w < NWIN; w += 2) {
-                    const int wg = h * M::SUB_BLOCKS + w;  // window in the tile
-                    const uint64_t a_off = (uint64_t)((2 * wg * SG::CHUNK + (SG::TOP - R + dy) * 16) >> 4);
-                    umma_f16(d + 16 * w, a_hi0 + a_off, b, kIdesc, acc);
-                }
+            for (int w = parity; w < NWIN; w += 2) {
+                const uint64_t a_off = (uint64_t)((2 * w * SG::CHUNK + (SG::TOP - R + dy) * 16) >> 4);
+                umma_f16(d + 16 * w, a_hi0 + a_off, b, kIdesc, acc);
             }
         }
-    } else {
-#pragma unroll
-        for (int w = 0; w < M::SUB_WIN; w++)
-            issue_split_window<R, SG>(a_hi0, band, d + split_region(w), h * M::SUB_BLOCKS + w);
     }
 }
 
@@ -543,40 +524,28 @@ __device__ __forceinline__ void issue_subtile(uint64_t a_hi0, uint32_t band, uin
 template <int R, class SG>
 __device__ __forceinline__ void issue_plain_tile(uint64_t a_hi0, uint32_t band, uint32_t d,
                                                  int nwin) {
-    if (nwin <= 5) issue_subtile<R, false, SG, 5>(a_hi0, band, d, 0);
-    else if (nwin <= 7) issue_subtile<R, false, SG, 7>(a_hi0, band, d, 0);
-    else issue_subtile<R, false, SG>(a_hi0, band, d, 0);
+    if (nwin <= 5) issue_plain_windows<R, SG, 5>(a_hi0, band, d);
+    else if (nwin <= 7) issue_plain_windows<R, SG, 7>(a_hi0, band, d);
+    else issue_plain_windows<R, SG>(a_hi0, band, d);
 }
 
-// Epilogue, first half: this warp's accumulators of a sub-tile into
+// Epilogue of a whole plain tile, first half: this warp's accumulators into
 // registers, one FP32 value per output (lanes = tile rows of the warp's lane
-// quarter, `half` = which half of the sub-tile's column blocks).  lane_col is
-// the TMEM address of the warp's lane quarter at the sub-tile's first column.
-// After it returns the accumulator may be reused.
-template <bool SPLIT>
+// quarter, `half` = which half of the tile's column blocks).  lane_col is the
+// TMEM address of the warp's lane quarter at the tile's first column.  After
+// it returns the accumulator may be reused.
 __device__ __forceinline__ void epilogue_load(uint32_t lane_col, int half,
-                                              float (&f)[Mode<SPLIT>::SUB_BLOCKS / 2][16]) {
-    using M = Mode<SPLIT>;
-    constexpr int G = M::SUB_BLOCKS / 2;
-    const int j0 = half * G;
-    if (!SPLIT) {
-        // output block jl is accumulator columns 16(jl+1) .. 16(jl+1)+15
-        uint32_t v[G][16];
+                                              float (&f)[Mode<false>::SUB_BLOCKS / 2][16]) {
+    constexpr int G = Mode<false>::SUB_BLOCKS / 2;
+    // output block j is accumulator columns 16(j+1) .. 16(j+1)+15
+    uint32_t v[G][16];
 #pragma unroll
-        for (int gg = 0; gg < G; gg++) tmem_ld_x16(lane_col + 16 * (j0 + gg + 1), v[gg]);
-        tmem_ld_wait();
+    for (int gg = 0; gg < G; gg++) tmem_ld_x16(lane_col + 16 * (half * G + gg + 1), v[gg]);
+    tmem_ld_wait();
 #pragma unroll
-        for (int gg = 0; gg < G; gg++)
+    for (int gg = 0; gg < G; gg++)
 #pragma unroll
-            for (int c = 0; c < 16; c++) f[gg][c] = __uint_as_float(v[gg][c]);
-    } else {
-        // block jl = second half of window jl + first half of window jl+1
-#pragma unroll
-        for (int gg = 0; gg < G; gg++) {
-            const int jl = j0 + gg;
-            split_block_load(lane_col + split_region(jl), lane_col + split_region(jl + 1), f[gg]);
-        }
-    }
+        for (int c = 0; c < 16; c++) f[gg][c] = __uint_as_float(v[gg][c]);
 }
 
 // Output of one tile: planes, geometry and the update rectangle.
@@ -614,74 +583,35 @@ __device__ __forceinline__ bool walk_windows(int g, int ng, int nwin, Ready &&re
     return true;
 }
 
-// Converts and stores one 16-column output block of tile row y (cells xb ..
-// xb+15).  fast: the whole tile is inside the update rectangle; otherwise
-// cells outside it copy the input.
-//  split: fast blocks take the paired split (split_pair), others split each
-//    updated cell alone (split_fixed: the same bits) and copy the rest.
-//  plain: every cell is converted in pairs (pack_h2, the same bits as h_bits
-//    per cell); where a thread's 16 cells are not all inside, the input
-//    words are blended back in under a per-cell mask.
-// (Measured on GB300: the blend is faster for plain blocks, the separate
-// per-cell path faster for split ones, whose epilogue is sensitive to code
-// size.)
-template <bool SPLIT>
+// Converts and stores one 16-column plain output block of tile row y (cells
+// xb .. xb+15).  fast: the whole tile is inside the update rectangle;
+// otherwise cells outside it copy the input: every cell is converted in pairs
+// (pack_h2, the same bits as h_bits per cell), and where a thread's 16 cells
+// are not all inside, the input words are blended back in under a per-cell
+// mask.  (Measured on GB300: the blend is faster for plain blocks, the
+// separate per-cell path of store_block_split faster for split ones, whose
+// epilogue is sensitive to code size.)
 __device__ __forceinline__ void store_block(const TileOut &o, const float (&f)[16], int y, int xb,
                                             bool fast, bool row_in) {
     const size_t off0 = plane_index16(o.pg, y, xb);     // cells xb .. xb+7
     const size_t off1 = off0 + (size_t)o.pg.nyp * 8;  // cells xb+8 .. xb+15
-    uint32_t hw[8], lw[8];
-    if constexpr (SPLIT) {
-        if (fast) {
+    uint32_t hw[8];
 #pragma unroll
-            for (int c = 0; c < 8; c++) split_pair(f[2 * c], f[2 * c + 1], hw[c], lw[c]);
-        } else {
-            const uint4 i0 = *reinterpret_cast<const uint4 *>(o.in_hi + off0);
-            const uint4 i1 = *reinterpret_cast<const uint4 *>(o.in_hi + off1);
-            const uint4 l0 = *reinterpret_cast<const uint4 *>(o.in_lo + off0);
-            const uint4 l1 = *reinterpret_cast<const uint4 *>(o.in_lo + off1);
-            const uint32_t iw[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
-            const uint32_t il[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+    for (int c = 0; c < 8; c++) hw[c] = pack_h2(f[2 * c], f[2 * c + 1]);
+    if (!fast && !(row_in && xb >= o.x0 && xb + 16 <= o.x1)) {
+        const uint4 i0 = *reinterpret_cast<const uint4 *>(o.in_hi + off0);
+        const uint4 i1 = *reinterpret_cast<const uint4 *>(o.in_hi + off1);
+        const uint32_t iw[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
 #pragma unroll
-            for (int c = 0; c < 8; c++) {
-                uint16_t hh[2], ll[2];
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const int x = xb + 2 * c + u;
-                    if (row_in && x >= o.x0 && x < o.x1) {
-                        split_fixed(f[2 * c + u], hh[u], ll[u]);
-                    } else {
-                        hh[u] = (uint16_t)(iw[c] >> (16 * u));
-                        ll[u] = (uint16_t)(il[c] >> (16 * u));
-                    }
-                }
-                hw[c] = (uint32_t)hh[0] | ((uint32_t)hh[1] << 16);
-                lw[c] = (uint32_t)ll[0] | ((uint32_t)ll[1] << 16);
-            }
+        for (int c = 0; c < 8; c++) {
+            const int x = xb + 2 * c;
+            const uint32_t m = (row_in && x >= o.x0 && x < o.x1 ? 0x0000ffffu : 0u) |
+                               (row_in && x + 1 >= o.x0 && x + 1 < o.x1 ? 0xffff0000u : 0u);
+            hw[c] = (hw[c] & m) | (iw[c] & ~m);
         }
-        *reinterpret_cast<uint4 *>(o.out_hi + off0) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-        *reinterpret_cast<uint4 *>(o.out_hi + off1) = make_uint4(hw[4], hw[5], hw[6], hw[7]);
-        *reinterpret_cast<uint4 *>(o.out_lo + off0) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-        *reinterpret_cast<uint4 *>(o.out_lo + off1) = make_uint4(lw[4], lw[5], lw[6], lw[7]);
-    } else {
-        (void)lw;
-#pragma unroll
-        for (int c = 0; c < 8; c++) hw[c] = pack_h2(f[2 * c], f[2 * c + 1]);
-        if (!fast && !(row_in && xb >= o.x0 && xb + 16 <= o.x1)) {
-            const uint4 i0 = *reinterpret_cast<const uint4 *>(o.in_hi + off0);
-            const uint4 i1 = *reinterpret_cast<const uint4 *>(o.in_hi + off1);
-            const uint32_t iw[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                const int x = xb + 2 * c;
-                const uint32_t m = (row_in && x >= o.x0 && x < o.x1 ? 0x0000ffffu : 0u) |
-                                   (row_in && x + 1 >= o.x0 && x + 1 < o.x1 ? 0xffff0000u : 0u);
-                hw[c] = (hw[c] & m) | (iw[c] & ~m);
-            }
-        }
-        *reinterpret_cast<uint4 *>(o.out_hi + off0) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-        *reinterpret_cast<uint4 *>(o.out_hi + off1) = make_uint4(hw[4], hw[5], hw[6], hw[7]);
     }
+    *reinterpret_cast<uint4 *>(o.out_hi + off0) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+    *reinterpret_cast<uint4 *>(o.out_hi + off1) = make_uint4(hw[4], hw[5], hw[6], hw[7]);
 }
 
 // After a warp has stored its blocks of a tile (row y, blocks X0 + 16 j for
@@ -733,20 +663,20 @@ __device__ __forceinline__ void resplit_border(const TileOut &o, int y, int X0, 
     }
 }
 
-// store_block<true> of the values v 2^k (StepScale ss): fast blocks split in
-// pairs, others split each updated cell alone and copy the rest (on a step
-// whose copies change scale, resplit_border then rewrites the grid's copied
-// cells).  The largest |u| of the updated cells is kept in mx (the border's
-// share of the step maximum is the record's B; padding cells never count).
-__device__ __forceinline__ void store_block_split(const TileOut &o, const float (&f)[16], int y,
-                                                  int xb, bool fast, bool row_in,
-                                                  const StepScale &ss, float &mx) {
+// Splits and stores one 16-column block of u (units of the step's scale):
+// fast blocks split in pairs, others split each updated cell alone and copy
+// the rest (on a step whose copies change scale, resplit_border then rewrites
+// the grid's copied cells).  The largest |u| of the updated cells is kept in
+// mx (the border's share of the step maximum is the record's B; padding cells
+// never count).
+__device__ __forceinline__ void store_block_split(const TileOut &o, const float (&u)[16], int y,
+                                                  int xb, bool fast, bool row_in, float &mx) {
     const size_t off0 = plane_index16(o.pg, y, xb);     // cells xb .. xb+7
     const size_t off1 = off0 + (size_t)o.pg.nyp * 8;  // cells xb+8 .. xb+15
     uint32_t hw[8], lw[8];
     if (fast) {
 #pragma unroll
-        for (int c = 0; c < 8; c++) split_pair_s(f[2 * c], f[2 * c + 1], ss.s, hw[c], lw[c], mx);
+        for (int c = 0; c < 8; c++) split_pair_u(u[2 * c], u[2 * c + 1], hw[c], lw[c], mx);
     } else {
         const uint4 i0 = *reinterpret_cast<const uint4 *>(o.in_hi + off0);
         const uint4 i1 = *reinterpret_cast<const uint4 *>(o.in_hi + off1);
@@ -758,13 +688,13 @@ __device__ __forceinline__ void store_block_split(const TileOut &o, const float 
         for (int c = 0; c < 8; c++) {
             uint16_t hh[2], ll[2];
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const int x = xb + 2 * c + u;
+            for (int k = 0; k < 2; k++) {
+                const int x = xb + 2 * c + k;
                 if (row_in && x >= o.x0 && x < o.x1) {
-                    split_fixed_s(f[2 * c + u], ss.s, hh[u], ll[u], mx);
+                    split_fixed_u(u[2 * c + k], hh[k], ll[k], mx);
                 } else {
-                    hh[u] = (uint16_t)(iw[c] >> (16 * u));
-                    ll[u] = (uint16_t)(il[c] >> (16 * u));
+                    hh[k] = (uint16_t)(iw[c] >> (16 * k));
+                    ll[k] = (uint16_t)(il[c] >> (16 * k));
                 }
             }
             hw[c] = (uint32_t)hh[0] | ((uint32_t)hh[1] << 16);
@@ -781,21 +711,18 @@ __device__ __forceinline__ bool tile_inside(const TileOut &o, int Y0, int X0) {
     return Y0 >= o.y0 && Y0 + kTile <= o.y1 && X0 >= o.x0 && X0 + kTile <= o.x1;
 }
 
-// Epilogue, second half: converts and stores this warp's outputs of sub-tile
-// h (tile row m).
-template <bool SPLIT>
+// Epilogue of a whole plain tile, second half: converts and stores this
+// warp's outputs (tile row m).
 __device__ __forceinline__ void epilogue_store(const TileOut &o,
-                                               const float (&f)[Mode<SPLIT>::SUB_BLOCKS / 2][16],
-                                               int h, int half, int m, int Y0, int X0) {
-    using M = Mode<SPLIT>;
-    constexpr int G = M::SUB_BLOCKS / 2;
-    const int j0 = half * G;
+                                               const float (&f)[Mode<false>::SUB_BLOCKS / 2][16],
+                                               int half, int m, int Y0, int X0) {
+    constexpr int G = Mode<false>::SUB_BLOCKS / 2;
     const int y = Y0 + m;
     const bool fast = tile_inside(o, Y0, X0);
     const bool row_in = y >= o.y0 && y < o.y1;
 #pragma unroll
     for (int gg = 0; gg < G; gg++)
-        store_block<SPLIT>(o, f[gg], y, X0 + 16 * (h * M::SUB_BLOCKS + j0 + gg), fast, row_in);
+        store_block(o, f[gg], y, X0 + 16 * (half * G + gg), fast, row_in);
 }
 
 // Plain tiles of W = 64, 96 or 128 columns (the plain sweep kernel's
@@ -827,7 +754,7 @@ __device__ __forceinline__ void plain_epilogue(const TileOut &o, uint32_t lane_c
             float f[16];
 #pragma unroll
             for (int c = 0; c < 16; c++) f[c] = __uint_as_float(v[gg][c]);
-            store_block<false>(o, f, y, X0 + 16 * (j0 + gg), fast, row_in);
+            store_block(o, f, y, X0 + 16 * (j0 + gg), fast, row_in);
         }
     }
 }
