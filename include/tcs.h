@@ -216,26 +216,31 @@ int tcs_plan_scale_exp(tcs_plan plan, int *scale_exp);
 int tcs_plan_set_coeffs(tcs_plan plan, const float *coeffs);
 /* Temporal blocking depth: 1 (single steps, the default) or 2 (two steps per
  * launch, intermediate kept on chip; split precision on the tensor engine,
- * faster there at every size measured).  Results are bit-identical either
- * way; the autotuner picks, tcs_sweep_host and pipes take depth 2 for split. */
+ * faster there but for 2000 to 3000 columns and rows, where the one-launch form
+ * of single steps is).  Results are bit-identical either way; the autotuner
+ * picks, tcs_sweep_host and pipes take depth 2 for split. */
 int tcs_plan_set_temporal_depth(tcs_plan plan, int depth);
 /* Tensor engine (FP16 or split, temporal depth 1): run(steps >= 2) as ONE
  * launch instead of one launch per step.  FP16 tiles take up to eight
  * (radius 1) or four (radius 2) steps each time they are loaded and wait for
  * the neighbouring tiles' previous visit; split tiles of step j wait for the
  * neighbouring tile rows of step j-1.  mode -1 (default): FP16 grids of more
- * than 16 tiles of 128 x 128, split grids of more than one and at most 20
- * tiles per SM; 0: never; 1: always.  Results are bit-identical either way
- * for grids of finite values (an infinity or NaN spreads by whole 16-column
- * windows a step, and over several steps of a visit not past its tile's
- * halo).  TCS_MULTI=0 in the environment turns it off for the process. */
+ * than nine tiles of 128 x 128 or calls of more than ten steps, split grids of
+ * more than one and at most 20 tiles per SM; 0: never; 1: always.  CUDA-core
+ * plans take the one-launch form in mode -1 too, by the FP16 rule where it is
+ * faster (the radius-2 box up to about seven tiles per SM), not in mode 1.
+ * Results are bit-identical either way for grids of finite values (on the
+ * tensor engine an infinity or NaN spreads by whole 16-column windows a step,
+ * and over several steps of a visit not past its tile's halo).  TCS_MULTI=0 in
+ * the environment turns it off for the process. */
 int tcs_plan_set_multistep(tcs_plan plan, int mode);
 /* Tile shape of the plain FP16 tensor sweeps: 128 rows by tile_w = 128
  * (default), 96 or 64 columns.  Narrower tiles give a grid more tiles: on
  * grids with few tiles per SM more SMs share a step, and each tile's MMAs and
  * epilogue shrink with its width.  One-launch runs at the default choose
- * their width (32 to 128) by the grid; a width set here holds for them too.  Results are bit-identical at every width;
- * the autotuner picks the width per size class (it replaces the reference's
+ * their width (32 to 128) by the grid; a width set here holds for them too.
+ * Results are bit-identical at every width; the autotuner picks the width per
+ * size class (it replaces the reference's
  * TILE_SIZE sweep, script/param.py:5).  TCS_ERR_UNSUPPORTED for widths below
  * 128 on other engines and precisions. */
 int tcs_plan_set_tile_width(tcs_plan plan, int tile_w);

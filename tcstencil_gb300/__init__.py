@@ -314,7 +314,7 @@ class Plan:
 
             engine, tuned_depth = best_config(stencil, precision, ny, nx)
             tuned_launch = best_launch(stencil, precision, ny, nx)
-            if temporal_depth is None:  # (every tuned split class takes pairs)
+            if temporal_depth is None:  # untuned split sizes take pairs
                 temporal_depth = 2 if precision == "split" and tuned_launch < 0 else tuned_depth
             if tuned_launch < 0 and precision == "f16":
                 tuned_launch = 1  # every tuned FP16 class takes one launch for all steps

@@ -427,11 +427,13 @@ struct tcs_plan_s {
 
     // Temporal depth 2 (split precision on the tensor engine): steps run in
     // blocked pairs, with the same bits as single steps.  The one-call form,
-    // pipes and autotuned plans take it for every split grid: faster than
-    // either form of single steps at every size measured (box2d1r / box2d2r,
-    // us per step, best single form -> pairs: 256² 6.65 -> 6.26 / 6.88 -> 6.46,
-    // 1026² 7.49 -> 6.53 / 8.91 -> 6.64, 4096² 26.5 -> 22.2 / 27.2 -> 25.1,
-    // 16386² 356 -> 264 / 371 -> 312).
+    // pipes and autotuned plans of untuned sizes take it for every split grid:
+    // box2d1r / box2d2r, us per step, best form of single steps -> pairs:
+    // 256² 6.65 -> 6.26 / 6.88 -> 6.46, 1026² 7.49 -> 6.53 / 8.91 -> 6.64, 4096²
+    // 26.5 -> 22.2 / 27.2 -> 25.1, 16386² 356 -> 264 / 371 -> 312.  Only around
+    // 2048² to 2900² is the one-launch form of single steps faster (2048² 10.3
+    // -> 11.3, 2896² 14.5 -> 15.5), where a pair's launches still weigh; the
+    // tuned table takes it there.
     int temporal_depth = 1;
     bool pairs() const { return temporal_depth == 2; }
     void take_pairs() {
@@ -449,17 +451,20 @@ struct tcs_plan_s {
     // a call in one launch (tcs_plan_set_multistep; TCS_MULTI=0 in the
     // environment: one launch per step): FP16 tiles take several steps per
     // visit (sweep_visit.cu), split tiles one, and wait only for the
-    // neighbouring tiles or tile rows of the visit or step before.
+    // neighbouring tiles or tile rows of the visit or step before.  CUDA-core
+    // plans do the same by size, in mode -1 only (sweep_cc.cu).
     int multistep = -1;
-    bool multi() const {
+    bool multi(int steps) const {
         static const bool on = [] {
             const char *e = getenv("TCS_MULTI");
             return !(e && e[0] == '0');
         }();
-        if (!on || !rows_done || prob.engine != TCS_ENGINE_TENSOR || pairs()) return false;
-        if (multistep >= 0) return multistep == 1;
+        if (!on || !rows_done || pairs() || steps < 2) return false;
         const long long tiles = this->tiles();
         const long long sms = device_sms();
+        if (prob.engine == TCS_ENGINE_CUDACORE)
+            return multistep < 0 && several(steps) && cc_shape(steps).visits > 0;
+        if (multistep >= 0) return multistep == 1;
         // Split, us per step, one launch per step -> one launch (box2d1r /
         // box2d2r): 2400² 16.5 -> 11.8 / 16.5 -> 12.6, 3200² 22.2 -> 16.3 /
         // 23.0 -> 17.2, 4800² 51.8 -> 46.2 / 53.0 -> 47.0, 6400² 65.9 -> 60.5
@@ -468,18 +473,29 @@ struct tcs_plan_s {
         // the multi-step kernel spends a little more per tile, which the step
         // overheads repay up to about 20 tiles per SM.
         if (prob.precision == TCS_PREC_SPLIT) return tiles > sms && tiles <= 20 * sms;
-        // FP16: one launch is faster at every size (visit_shape), but its CTAs
-        // must all be resident and take an SM each, so the smallest grids,
-        // of which a program may step several side by side on its streams,
-        // keep to ordinary launches unless the caller asks (mode 1; the
-        // autotuned plans do)
-        return tiles > 16;
+        return several(steps);
     }
+    // One launch for all steps is faster at every size where its tiles take
+    // several steps per visit (visit_shape, cc_visit_shape), but it is a
+    // cooperative launch, which starts only when all its CTAs can be resident:
+    // short calls on the smallest grids keep to ordinary launches, which get
+    // onto a busy device sooner, unless the caller asks (mode 1; the autotuned
+    // plans do).
+    bool several(int steps) const { return tiles() > 9 || steps > 10; }
     bool visits() const { return prob.precision == TCS_PREC_F16; }
+    CcVisitShape cc_shape(int steps) const {
+        return cc_visit_shape(g, prob.stencil, prob.precision == TCS_PREC_F32, steps, device_sms());
+    }
     VisitShape visit_shape(int steps) const {
         return tcs::visit_shape(g.ny, g.nx, prob.stencil, steps, tile_w, device_sms());
     }
     int steps_in_one(int steps, int from, cudaStream_t s) {
+        if (prob.engine == TCS_ENGINE_CUDACORE)
+            return cuda_status(
+                launch_cc_visits(g, prob.stencil, prob.precision == TCS_PREC_F32,
+                                 tap_coeffs(prob.stencil, coeffs), buf[from][0], buf[1 - from][0],
+                                 steps, cc_shape(steps), rows_done, s, device_sms()),
+                "multi-step sweep launch");
         if (visits())
             return cuda_status(
                 launch_tc_f16_visits(g, prob.stencil, coeffs, static_cast<uint16_t *>(buf[from][0]),
@@ -502,7 +518,9 @@ struct tcs_plan_s {
     // The state `steps` steps from `from` ends in: one flip per step, step
     // pair or visit.
     int final_state(int steps, int from) const {
-        if (steps >= 2 && multi() && visits()) return from ^ (visit_shape(steps).visits & 1);
+        if (multi(steps) && prob.engine == TCS_ENGINE_CUDACORE)
+            return from ^ (cc_shape(steps).visits & 1);
+        if (multi(steps) && visits()) return from ^ (visit_shape(steps).visits & 1);
         const int launches = pairs() ? steps / 2 + steps % 2 : steps;
         return from ^ (launches & 1);
     }
@@ -511,7 +529,7 @@ struct tcs_plan_s {
     // records into the places the next run starts from.
     int enqueue(int steps, int from, cudaStream_t s, int *to) {
         int st = TCS_OK;
-        if (steps >= 2 && multi()) {
+        if (multi(steps)) {
             *to = final_state(steps, from);
             st = steps_in_one(steps, from, s);
         } else {
@@ -575,19 +593,23 @@ int tcs_plan_create(const tcs_problem *pr, tcs_plan *out) {
         if (!st) st = cuda_status(cudaMemset(p->d_upload, 0, kUploadScratch * sizeof(unsigned)), "cudaMemset(max)");
         if (st) return st;
     }
+    size_t words = cc_visit_counter_words(pr->ny, pr->nx);
     if (pr->engine == TCS_ENGINE_TENSOR) {
         st = cuda_status(tc_prepare(pr->stencil, pr->precision == TCS_PREC_SPLIT), "tensor kernel set-up");
         if (st) return st;
-        size_t words = (size_t)((pr->ny + kTile - 1) / kTile) * kRowCounterStride;
+        words = (size_t)((pr->ny + kTile - 1) / kTile) * kRowCounterStride;
         if (pr->precision == TCS_PREC_F16) {
             st = cuda_status(visit_prepare(pr->stencil), "multi-step kernel set-up");
             if (st) return st;
             words = visit_counter_words(pr->ny, pr->nx);
         }
-        st = dev_alloc_t(&p->rows_done, words * sizeof(unsigned), "row counters");
-        if (!st) st = cuda_status(cudaMemset(p->rows_done, 0, words * sizeof(unsigned)), "cudaMemset(counters)");
+    } else {
+        st = cuda_status(cc_visit_prepare(pr->stencil, pr->precision == TCS_PREC_F32), "multi-step kernel set-up");
         if (st) return st;
     }
+    st = dev_alloc_t(&p->rows_done, words * sizeof(unsigned), "row counters");
+    if (!st) st = cuda_status(cudaMemset(p->rows_done, 0, words * sizeof(unsigned)), "cudaMemset(counters)");
+    if (st) return st;
     *out = p.release();
     return TCS_OK;
 }
@@ -747,7 +769,7 @@ int tcs_plan_tile_width(tcs_plan p, int *tile_w) {
 
 int tcs_plan_launches(tcs_plan p, int steps, int *launches) {
     if (!p || steps < 0 || !launches) return fail(TCS_ERR_INVALID, "tcs_plan_launches: bad arguments");
-    if (steps >= 2 && p->multi()) *launches = 1;
+    if (p->multi(steps)) *launches = 1;
     else *launches = p->pairs() ? steps / 2 + steps % 2 : steps;
     return TCS_OK;
 }

@@ -150,6 +150,18 @@ cudaError_t launch_cc_f16(const GridGeom &g, int stencil, const TapCoeffs &c, co
 cudaError_t launch_cc_f32(const GridGeom &g, int stencil, const TapCoeffs &c, const float *in,
                           float *out, cudaStream_t s);
 
+// Several CUDA-core steps per tile visit, in one launch (in -> out -> in ...,
+// one flip per visit; visits = 0: single steps are faster); counters:
+// cc_visit_counter_words of zeros, which a launch leaves zero again.
+struct CcVisitShape {
+    int ppl, warps, halo, tiles_x, tiles_y, visits;
+};
+CcVisitShape cc_visit_shape(const GridGeom &g, int stencil, bool f32, int steps, int sms);
+cudaError_t cc_visit_prepare(int stencil, bool f32);
+cudaError_t launch_cc_visits(const GridGeom &g, int stencil, bool f32, const TapCoeffs &c, void *in,
+                             void *out, int steps, const CcVisitShape &v, unsigned *counters,
+                             cudaStream_t s, int sms);
+
 // Reads and clears the tensor kernels' device error word.
 cudaError_t tc_take_error(int *code);
 struct SplitScale;
@@ -183,6 +195,9 @@ struct VisitShape {
 VisitShape visit_shape(int ny, int nx, int stencil, int steps, int tile_w, int sms);
 constexpr size_t visit_counter_words(int ny, int nx) {
     return kRowCounterStride + (size_t)(ny / (kTile - 16) + 2) * ((nx + 31) / 32);
+}
+constexpr size_t cc_visit_counter_words(int ny, int nx) {
+    return kRowCounterStride + (size_t)(ny / (kTile - 16) + 2) * (nx / 56 + 2);
 }
 cudaError_t visit_prepare(int stencil);
 cudaError_t launch_tc_f16_visits(const GridGeom &g, int stencil, const float *B, uint16_t *in,
