@@ -69,6 +69,11 @@ struct PackArgs {
     float scale;
     SplitScale *sc;
     int y0, y1, x0, x1;
+    // launched right behind max_abs_scale_kernel on the same cells, which lets
+    // it start only once all work before both has completed: the cells are
+    // loaded beside that pass (past L1), before the wait for its scale (256
+    // split grids of a mixed batch: 12.0 -> 9.2 us per upload)
+    bool behind_max;
 };
 
 template <int MODE>
@@ -81,7 +86,7 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(const PackArgs a) {
     const BlockPos b = block_pos(a.p, a.q0);
     const int X = (b.pan - 1) * CPP + lane;  // this lane's first cell: X, X + 32, ...
     pdl_launch_dependents();
-    pdl_wait();
+    if (MODE != kPackSplit || !a.behind_max) pdl_wait();
     float v[K][N];
 #pragma unroll
     for (int k = 0; k < K; k++) {
@@ -92,7 +97,7 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(const PackArgs a) {
         const float *src = a.in + (size_t)(row_in ? iy : 0) * a.nx;
         if (row_in && ix >= 0 && ix + CELLS <= a.nx) {
 #pragma unroll
-            for (int i = 0; i < N; i++) v[k][i] = src[ix + lane + 32 * i];
+            for (int i = 0; i < N; i++) v[k][i] = __ldcg(src + ix + lane + 32 * i);
         } else {
             // border and padding cells: the loads clamped to the row and the
             // values selected, so that they all are in flight at once
@@ -100,12 +105,13 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(const PackArgs a) {
 #pragma unroll
             for (int i = 0; i < N; i++) {
                 const int x = ix + lane + 32 * i;
-                const float c = row_in ? src[min(max(x, 0), a.nx - 1)] : 0.0f;
+                const float c = row_in ? __ldcg(src + min(max(x, 0), a.nx - 1)) : 0.0f;
                 const bool pad_in = row_pad && x >= -a.pad && x < a.nx + a.pad;
                 v[k][i] = row_in && x >= 0 && x < a.nx ? c : pad_in ? a.pad_value : 0.0f;
             }
         }
     }
+    if (MODE == kPackSplit && a.behind_max) pdl_wait();
     float scale = a.scale;
     bool border = false;  // the block may hold cells outside the update rectangle
     if (MODE == kPackSplit && a.sc) {
@@ -272,8 +278,8 @@ __global__ void __launch_bounds__(kThreads) max_abs_kernel(const float *__restri
 // scratch[1] (blocks done) zero for the next use.
 __global__ void __launch_bounds__(kThreads) max_abs_scale_kernel(const float *__restrict__ in, size_t n,
                                                                  unsigned *scratch, SplitScale *sc) {
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();  // (after the wait: see PackArgs::behind_max)
     const unsigned u = block_max_abs(in, n);
     if (threadIdx.x != 0) return;
     atomicMax(&scratch[0], u);
@@ -545,6 +551,7 @@ cudaError_t launch_split_upload(const float *in, const GridGeom &g, unsigned *sc
     PackArgs a = pack_args(in, g.ny, g.nx, 0, 0.0f, hi, 8);
     a.out_lo = lo;
     a.sc = sc;
+    a.behind_max = true;
     a.y0 = g.y0; a.y1 = g.y1; a.x0 = g.x0; a.x1 = g.x1;
     return launch_pack<kPackSplit>(a, s);
 }
