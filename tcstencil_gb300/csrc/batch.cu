@@ -149,8 +149,7 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
     using C = BatchCfg<SPLIT>;
     constexpr int NS = C::STAGES;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                                ~static_cast<uintptr_t>(1023));
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *stage_base = smem;  // [NS][planes | bands]
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)NS * C::STAGE_BYTES);
     // accumulator barriers: plain [2] slots, split [kBatchRingSlots] windows
@@ -630,8 +629,9 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                         mbar_arrive(&acc_empty[Gb % kBatchRingSlots]);
                     }
                     shift_block(u, ss);
-                    store_block_split(o, u, y, X0 + 16 * jb, fast, row_in, mx);
+                    store_block_split(o, u, y, X0 + 16 * jb, row_in, mx);
                 });
+                if (ok && !fast && !rows_out) copy_rows(o, y, X0, grp, C::GROUPS, nwin - 1);
                 if (ok && ss.k != 0 && !fast && !rows_out)
                     resplit_border(o, y, X0, grp, C::GROUPS, nwin - 1, ss);
                 G0 += nwin;

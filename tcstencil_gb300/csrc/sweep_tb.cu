@@ -22,8 +22,8 @@
 // (no other window reads those panels), and window w of the second step
 // waits for its two blocks: the second step follows the first a few windows
 // behind, and the tensor pipe does not drain between them.  Radius 2 runs at
-// the tensor pipe's 60 cycles per MMA (16386²: 371 -> 312 us per step against
-// one step per launch); radius 1 (356 -> 264) at 490 cycles per window of 360
+// the tensor pipe's 60 cycles per MMA (8196²: 104 -> 85 us per step against
+// one step per launch); radius 1 (102 -> 73) at 480 cycles per window of 360
 // cycles' MMAs, the five regions' turnaround.  An epilogue warp
 // waits once per block, on a barrier that both windows' commits arrive at.
 // (Waiting for windows, each released by all warps read or not, cost a warp
@@ -31,7 +31,11 @@
 // barriers per block; one range check per panel row instead of per pair
 // -> 292; both panels summed before the first is split -> 272; the groups
 // taking turns over both steps' blocks -> 264.  Reading each window the moment
-// it completes, for three groups of 128 registers, was slower: 309.)  (The form this
+// it completes, for three groups of 128 registers, was slower: 309.)  Rows
+// outside the update rectangle are left out of the blocks and copied after
+// them, and only panels that straddle its sides choose per cell: at 1026²,
+// where half of the tiles touch the border, 6.5 -> 4.95 us per step (8.0 a
+// step in single launches).  (The form this
 // replaces, with 80-column tiles, a second image for the intermediate and a
 // handoff per step, took 140 / 156 us per step at 8196², box2d1r / box2d2r.)
 // Two stages: the next tile loads while a tile runs both its steps.
@@ -47,13 +51,6 @@ using SG = StageLines;
 __device__ int g_tb_error = 0;
 
 constexpr int kTbStages = 2;
-constexpr int kTbRing = 5;
-constexpr int kTbRegion = 96;
-constexpr int kTbWindows = kTile / 16 + 1;  // of one step
-constexpr int kTbBlocks = kTile / 16 + 2;   // blocks -1 .. 8: the halo panels are -1 and 8
-constexpr int kTbHalo = 2;                  // rows given up at the top and bottom
-constexpr int kTbRows = kTile - 2 * kTbHalo;
-constexpr int kTbMapRows = 4;
 constexpr int kTbGroups = 4;                // epilogue block groups
 constexpr int kTbEpiWarps = 4 * kTbGroups;  // a lane quarter each
 // MMA issuer warps 1 .. 3 take the windows w with w % 3 == id of every step;
@@ -88,77 +85,12 @@ struct TbParams {
     float coef[25];
 };
 
-// Eight columns of a split block from its two windows' regions (TMEM columns
-// `a` and `b` of each part; b is ignored for the halo panels, which one window
-// alone reaches): the loads, and after tmem_ld_wait their sum u as
-// split_block_load forms it.
-__device__ __forceinline__ void panel_load(uint32_t a, uint32_t b, bool two, uint32_t (&v)[6][8]) {
-#pragma unroll
-    for (int part = 0; part < 3; part++) {
-        tmem_ld_x8(a + 32 * part, v[2 * part]);
-        if (two) tmem_ld_x8(b + 32 * part, v[2 * part + 1]);
-    }
-}
-__device__ __forceinline__ void panel_sum(const uint32_t (&v)[6][8], bool two, const StepScale &ss,
-                                          float (&u)[8]) {
-    auto pr = [&](int part, int c) {
-        return make_float2(__uint_as_float(v[part][c]), __uint_as_float(v[part][c + 1]));
-    };
-#pragma unroll
-    for (int c = 0; c < 8; c += 2) {
-        float2 main = pr(0, c), c1 = pr(2, c), c2 = pr(4, c);
-        if (two) {
-            main = __fadd2_rn(main, pr(1, c));
-            c1 = __fadd2_rn(c1, pr(3, c));
-            c2 = __fadd2_rn(c2, pr(5, c));
-        }
-        const float2 x = __ffma2_rn(main, make_float2(2048.0f, 2048.0f), __fadd2_rn(c1, c2));
-        u[c] = x.x;
-        u[c + 1] = x.y;
-    }
-    if (ss.k != 0) {
-        const float f = ss.s * (1.0f / 2048.0f);
-#pragma unroll
-        for (int c = 0; c < 8; c++) u[c] *= f;
-    }
-}
-
-// split_panel where not every cell is updated: cells outside [x0, x1) or of a
-// row outside the rectangle keep the old pair (re-split when `move`s scale
-// shifts).
-__device__ __forceinline__ PanelPair split_panel_edge(const float (&u)[8], const PanelPair &old, int xb,
-                                                   bool row_in, int x0, int x1, const StepScale &move,
-                                                   float &mx) {
-    const uint32_t ih[4] = {old.hi.x, old.hi.y, old.hi.z, old.hi.w};
-    const uint32_t il[4] = {old.lo.x, old.lo.y, old.lo.z, old.lo.w};
-    uint32_t hw[4], lw[4];
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        uint16_t hh[2], ll[2];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int x = xb + 2 * c + k;
-            if (row_in && x >= x0 && x < x1) {
-                split_fixed_u(u[2 * c + k], hh[k], ll[k], mx);
-            } else {
-                hh[k] = (uint16_t)(ih[c] >> (16 * k));
-                ll[k] = (uint16_t)(il[c] >> (16 * k));
-                if (move.k != 0) resplit_pair(hh[k], ll[k], move);
-            }
-        }
-        hw[c] = (uint32_t)hh[0] | ((uint32_t)hh[1] << 16);
-        lw[c] = (uint32_t)ll[0] | ((uint32_t)ll[1] << 16);
-    }
-    return PanelPair{make_uint4(hw[0], hw[1], hw[2], hw[3]), make_uint4(lw[0], lw[1], lw[2], lw[3])};
-}
-
 template <int S>
 __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid_constant__ TbParams p) {
     using C = TbCfg<S>;
     constexpr int R = C::R;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                                ~static_cast<uintptr_t>(1023));
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *stage_base = smem;  // [stage][hi, lo]
     uint8_t *band_base = smem + (size_t)kTbStages * 2 * SG::PLANE;
     uint64_t *bars = reinterpret_cast<uint64_t *>(band_base + C::BAND);
@@ -407,10 +339,6 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
             const int y = Yb + m;
             const bool top = ty == 0, bottom = ty == p.tiles_y - 1;
             const bool row_in = y >= g.y0 && y < g.y1;
-            // first step: all of the image's rows may be updated; second: the
-            // rows this tile owns
-            const bool rows1 = Yb >= g.y0 && Yb + kTile <= g.y1;
-            const bool rows2 = !top && !bottom && Yb + kTbHalo >= g.y0 && Yb + kTile - kTbHalo <= g.y1;
             const bool mine = (top || m >= kTbHalo) && (bottom || m < kTile - kTbHalo) && y < g.ny;
             const uint32_t img = smem_u32(stage_base) +
                                  (uint32_t)((i % kTbStages) * 2 * SG::PLANE + (m + SG::TOP) * 16);
@@ -422,11 +350,14 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                         const int xb = X0 - 8 + 8 * pan;
                         const uint32_t a = img + (uint32_t)(pan * SG::CHUNK);
                         PanelPair w;
-                        if (rows1 && xb >= g.x0 && xb + 8 <= g.x1) {
+                        if (!row_in) {  // a row that keeps its values
+                            if (ss1.k == 0) return;
+                            w = resplit_panel(PanelPair{lds128(a), lds128(a + SG::PLANE)}, ss1);
+                        } else if (xb >= g.x0 && xb + 8 <= g.x1) {
                             w = split_panel(u, mx1);
                         } else {
                             const PanelPair old{lds128(a), lds128(a + SG::PLANE)};
-                            w = split_panel_edge(u, old, xb, row_in, g.x0, g.x1, ss1, mx1);
+                            w = split_panel_edge(u, old, xb, g.x0, g.x1, ss1, mx1);
                         }
                         sts128(a, w.hi);
                         sts128(a + SG::PLANE, w.lo);
@@ -443,15 +374,15 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                     const int rb = r0 + 4 >= 5 ? r0 - 1 : r0 + 4;  // nine windows on
                     const bool ok = take_block(1, idx - kTbWindows, rb, i, ss2, [&](int pan, const float (&u)[8]) {
                         const int xb = X0 - 8 + 8 * pan;
-                        if (!mine || xb >= g.nx) return;
+                        if (!mine || !row_in || xb >= g.nx) return;
                         const size_t off = row0 + (size_t)pan * g.p16.nyp * 8;
                         PanelPair w;
-                        if (rows2 && xb >= g.x0 && xb + 8 <= g.x1) {
+                        if (xb >= g.x0 && xb + 8 <= g.x1) {
                             w = split_panel(u, mx2);
                         } else {
                             const PanelPair old{*reinterpret_cast<const uint4 *>(p.in_hi + off),
                                                 *reinterpret_cast<const uint4 *>(p.in_lo + off)};
-                            w = split_panel_edge(u, old, xb, row_in, g.x0, g.x1, cs2, mx2);
+                            w = split_panel_edge(u, old, xb, g.x0, g.x1, cs2, mx2);
                         }
                         *reinterpret_cast<uint4 *>(p.out_hi + off) = w.hi;
                         *reinterpret_cast<uint4 *>(p.out_lo + off) = w.lo;
@@ -460,6 +391,26 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                 }
             }
             r0 = r0 + 3 >= 5 ? r0 - 2 : r0 + 3;  // 18 windows on
+            // rows that keep their values: this group's panels (all loads before
+            // the first store)
+            if (!stop && mine && !row_in) {
+                PanelPair keep[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const size_t off = row0 + (size_t)(1 + grp + 4 * k) * g.p16.nyp * 8;
+                    keep[k] = PanelPair{*reinterpret_cast<const uint4 *>(p.in_hi + off),
+                                        *reinterpret_cast<const uint4 *>(p.in_lo + off)};
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int pan = 1 + grp + 4 * k;
+                    if (X0 - 8 + 8 * pan >= g.nx) break;
+                    const size_t off = row0 + (size_t)pan * g.p16.nyp * 8;
+                    const PanelPair w = cs2.k != 0 ? resplit_panel(keep[k], cs2) : keep[k];
+                    *reinterpret_cast<uint4 *>(p.out_hi + off) = w.hi;
+                    *reinterpret_cast<uint4 *>(p.out_lo + off) = w.lo;
+                }
+            }
         }
         if (!stop && p.scale) {  // tile 0 is CTA 0's
             cta_scale_flush<kTbEpiWarps>(cs, 0, p.scale, p.t0 + 1, ss1, mx1, blockIdx.x == 0);
@@ -503,7 +454,7 @@ cudaError_t launch_tb(const GridGeom &g, const float *B, const uint16_t *in_hi,
     if (e == cudaSuccess) e = encode_panel_map(in_lo, g.p16, &p.map_lo, kTile / 8 + 2, kTbMapRows);
     if (e != cudaSuccess) return e;
     p.tiles_x = (g.nx + kTile - 1) / kTile;
-    p.tiles_y = g.ny <= kTile ? 1 : (g.ny - 2 * kTbHalo + kTbRows - 1) / kTbRows;
+    p.tiles_y = tb_tiles_y(g.ny);
     p.n_tiles = p.tiles_x * p.tiles_y;
     p.in_hi = in_hi;
     p.in_lo = in_lo;

@@ -270,8 +270,7 @@ __global__ void __launch_bounds__(Sweep<S>::THREADS, 1) tc_sweep_kernel(const __
     constexpr int NP = M::PLANES;
 
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                                ~static_cast<uintptr_t>(1023));
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *stage_base = smem;                                    // [NS][NP][stage]
     uint8_t *band_base = smem + (size_t)NS * NP * SG::PLANE;     // [BAND_PLANES][NDY]
     uint64_t *bars =
@@ -567,8 +566,7 @@ __global__ void __launch_bounds__(Ring<MULTI>::THREADS, 1) tc_split_ring_kernel(
     constexpr int NP = M::PLANES;
 
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                                ~static_cast<uintptr_t>(1023));
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *stage_base = smem;                                 // [NS][NP][stage]
     uint8_t *band_base = smem + (size_t)NS * NP * SG::PLANE;  // NDY * 4 KB
     uint64_t *bars =
@@ -810,9 +808,10 @@ __global__ void __launch_bounds__(Ring<MULTI>::THREADS, 1) tc_split_ring_kernel(
                     mbar_arrive(&win_empty[Gb % kRingSlots]);
                 }
                 shift_block(u, ss);
-                store_block_split(o, u, y, X0 + 16 * j, fast, row_in, mx);
+                store_block_split(o, u, y, X0 + 16 * j, row_in, mx);
             });
             if (!ok) break;
+            if (!fast) copy_rows(o, y, X0, grp, kRingGroups, kTileWindows - 1);
             if (ss.k != 0 && !fast) resplit_border(o, y, X0, grp, kRingGroups, kTileWindows - 1, ss);
             // the step's last item of this warp: its maximum and the step's
             // exponent go out before the item is counted

@@ -250,8 +250,7 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
     constexpr int stage_bytes = visit_stage_bytes(W);
     constexpr int NS = kVisitStages;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                                ~static_cast<uintptr_t>(1023));
+    uint8_t *smem = align_smem(smem_raw);
     uint8_t *stage_base = smem;                          // [NS]
     uint8_t *band_base = smem + (size_t)NS * stage_bytes;  // [2R+1]
     uint64_t *bars = reinterpret_cast<uint64_t *>(band_base + (2 * R + 1) * kBandBytes);

@@ -290,39 +290,15 @@ __device__ __forceinline__ uint32_t pack_h2(float v0, float v1) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// split_fixed_u of two values into packed hi and lo words, with the same
+// split_fixed_u of a panel row's eight values into packed words, with the same
 // values and less conversion work: t = rint(u) is formed by the
 // add-and-subtract of 1.5 * 2^23 (round to nearest even for |u| < 2^22; a zero
 // t is +0).  While |t| <= 2^11, hi = t 2^-11 is exact in FP16 and lo = u - t is
 // exact; past that (|u| above 2048.5: the value slightly above 1, or NaN) hi
 // rounds in FP16 and split_fixed_u's rule is taken.  One comparison serves
-// both values, on the maximum that mx needs anyway.
-__device__ __forceinline__ void split_pair_u(float u0, float u1, uint32_t &hw, uint32_t &lw,
-                                             float &mx) {
-    constexpr float kRound = 12582912.0f;  // 1.5 * 2^23
-    const float2 u = make_float2(u0, u1);
-    const float m = fmaxf(fabsf(u0), fabsf(u1));
-    mx = fmaxf(mx, m);
-    // packed FP32 operations: each lane rounds as the scalar one would
-    const float2 t = __fadd2_rn(__fadd2_rn(u, make_float2(kRound, kRound)),
-                                make_float2(-kRound, -kRound));
-    if (m <= 2048.5f) {
-        const float2 h = __fmul2_rn(t, make_float2(1.0f / 2048.0f, 1.0f / 2048.0f));
-        const float2 l = __ffma2_rn(t, make_float2(-1.0f, -1.0f), u);  // u - t, exact
-        hw = pack_h2(h.x, h.y);
-        lw = pack_h2(l.x, l.y);
-    } else {
-        uint16_t h0, l0, h1, l1;
-        split_fixed_u(u0, h0, l0, mx);
-        split_fixed_u(u1, h1, l1, mx);
-        hw = (uint32_t)h0 | ((uint32_t)h1 << 16);
-        lw = (uint32_t)l0 | ((uint32_t)l1 << 16);
-    }
-}
-
-// split_pair_u of a panel row's eight values, with one range check for all
-// (a check per pair is a branch per pair: 550 cycles per panel row in the
-// blocked kernel, whose warps wait on each).
+// all eight, on the maximum that mx needs anyway (a check per pair is a branch
+// per pair: 550 cycles per panel row in the two-step kernel, whose warps wait
+// on each).
 struct PanelPair {
     uint4 hi, lo;
 };
@@ -456,6 +432,92 @@ __device__ __forceinline__ void split_block_load(uint32_t region_a, uint32_t reg
         u[c] = r.x;
         u[c + 1] = r.y;
     }
+}
+
+// Split tiles that are stepped twice per load (sweep_tb.cu, batch.cu): the
+// ring of window regions, and the windows and 16-column blocks of a step
+// (block b: columns X0-16+16b ..; 0 and 9 hold the halo panels).
+constexpr int kTbRing = 5;
+constexpr int kTbRegion = 96;
+constexpr int kTbWindows = kTile / 16 + 1;
+constexpr int kTbBlocks = kTile / 16 + 2;
+
+// Eight columns of a split block from its two windows' regions (TMEM columns
+// `a` and `b` of each part; b is ignored for the halo panels, which one window
+// alone reaches): the loads, and after tmem_ld_wait their sum u as
+// split_block_load forms it.
+__device__ __forceinline__ void panel_load(uint32_t a, uint32_t b, bool two, uint32_t (&v)[6][8]) {
+#pragma unroll
+    for (int part = 0; part < 3; part++) {
+        tmem_ld_x8(a + 32 * part, v[2 * part]);
+        if (two) tmem_ld_x8(b + 32 * part, v[2 * part + 1]);
+    }
+}
+__device__ __forceinline__ void panel_sum(const uint32_t (&v)[6][8], bool two, const StepScale &ss,
+                                          float (&u)[8]) {
+    auto pr = [&](int part, int c) {
+        return make_float2(__uint_as_float(v[part][c]), __uint_as_float(v[part][c + 1]));
+    };
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+        float2 main = pr(0, c), c1 = pr(2, c), c2 = pr(4, c);
+        if (two) {
+            main = __fadd2_rn(main, pr(1, c));
+            c1 = __fadd2_rn(c1, pr(3, c));
+            c2 = __fadd2_rn(c2, pr(5, c));
+        }
+        const float2 x = __ffma2_rn(main, make_float2(2048.0f, 2048.0f), __fadd2_rn(c1, c2));
+        u[c] = x.x;
+        u[c + 1] = x.y;
+    }
+    if (ss.k != 0) {
+        const float f = ss.s * (1.0f / 2048.0f);
+#pragma unroll
+        for (int c = 0; c < 8; c++) u[c] *= f;
+    }
+}
+
+// A panel row's old pair in units of the new scale.
+__device__ __forceinline__ PanelPair resplit_panel(const PanelPair &old, const StepScale &move) {
+    PanelPair o = old;
+    uint32_t *oh = &o.hi.x, *ol = &o.lo.x;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        uint16_t h[2], l[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            h[k] = (uint16_t)(oh[c] >> (16 * k));
+            l[k] = (uint16_t)(ol[c] >> (16 * k));
+            resplit_pair(h[k], l[k], move);
+        }
+        oh[c] = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
+        ol[c] = (uint32_t)l[0] | ((uint32_t)l[1] << 16);
+    }
+    return o;
+}
+
+// split_panel where not every column is updated: cells outside [x0, x1) keep
+// the old pair (re-split when `move`s scale shifts).  Their u counts as zero
+// and the words are merged by masks (a choice per cell took several times
+// split_panel's time).
+__device__ __forceinline__ PanelPair split_panel_edge(const float (&u)[8], const PanelPair &old, int xb,
+                                                   int x0, int x1, const StepScale &move, float &mx) {
+    const int a = x0 - xb, b = x1 - xb;  // updated cells of the panel: [a, b)
+    float v[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) v[c] = c >= a && c < b ? u[c] : 0.0f;
+    PanelPair w = split_panel(v, mx);
+    const PanelPair o = move.k != 0 ? resplit_panel(old, move) : old;
+    const uint32_t *oh = &o.hi.x, *ol = &o.lo.x;
+    uint32_t *wh = &w.hi.x, *wl = &w.lo.x;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const uint32_t m = (2 * c >= a && 2 * c < b ? 0xffffu : 0u) |
+                           (2 * c + 1 >= a && 2 * c + 1 < b ? 0xffff0000u : 0u);
+        wh[c] = (wh[c] & m) | (oh[c] & ~m);
+        wl[c] = (wl[c] & m) | (ol[c] & ~m);
+    }
+    return w;
 }
 
 // MMAs of window wg of a staged split tile (its panels 2wg, 2wg+1; the lo
@@ -663,48 +725,51 @@ __device__ __forceinline__ void resplit_border(const TileOut &o, int y, int X0, 
     }
 }
 
-// Splits and stores one 16-column block of u (units of the step's scale):
-// fast blocks split in pairs, others split each updated cell alone and copy
-// the rest (on a step whose copies change scale, resplit_border then rewrites
-// the grid's copied cells).  The largest |u| of the updated cells is kept in
-// mx (the border's share of the step maximum is the record's B; padding cells
-// never count).
+// A split block's values to the output planes, for rows of the update
+// rectangle: panels whose columns all lie in it are split and stored; in the
+// others (at the grid's sides) the rest keeps its input pair (re-split later
+// where the scale shifts: resplit_border).  Rows outside the rectangle are
+// copy_rows'.  (A choice per cell with both planes read, for every tile that
+// touches the border, as it was before: 512 mixed grids' split part 5.87 ms,
+// now 5.42; a 4096² radius-1 grid in one launch of single steps 26.4 -> 21.3
+// us per step, in which one range check per panel row has its share.)
 __device__ __forceinline__ void store_block_split(const TileOut &o, const float (&u)[16], int y,
-                                                  int xb, bool fast, bool row_in, float &mx) {
-    const size_t off0 = plane_index16(o.pg, y, xb);     // cells xb .. xb+7
-    const size_t off1 = off0 + (size_t)o.pg.nyp * 8;  // cells xb+8 .. xb+15
-    uint32_t hw[8], lw[8];
-    if (fast) {
+                                                  int xb, bool row_in, float &mx) {
+    if (!row_in) return;
 #pragma unroll
-        for (int c = 0; c < 8; c++) split_pair_u(u[2 * c], u[2 * c + 1], hw[c], lw[c], mx);
-    } else {
-        const uint4 i0 = *reinterpret_cast<const uint4 *>(o.in_hi + off0);
-        const uint4 i1 = *reinterpret_cast<const uint4 *>(o.in_hi + off1);
-        const uint4 l0 = *reinterpret_cast<const uint4 *>(o.in_lo + off0);
-        const uint4 l1 = *reinterpret_cast<const uint4 *>(o.in_lo + off1);
-        const uint32_t iw[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
-        const uint32_t il[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+    for (int h = 0; h < 2; h++) {
+        const int xh = xb + 8 * h;
+        const size_t off = plane_index16(o.pg, y, xb) + (size_t)h * o.pg.nyp * 8;
+        float v[8];
 #pragma unroll
-        for (int c = 0; c < 8; c++) {
-            uint16_t hh[2], ll[2];
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const int x = xb + 2 * c + k;
-                if (row_in && x >= o.x0 && x < o.x1) {
-                    split_fixed_u(u[2 * c + k], hh[k], ll[k], mx);
-                } else {
-                    hh[k] = (uint16_t)(iw[c] >> (16 * k));
-                    ll[k] = (uint16_t)(il[c] >> (16 * k));
-                }
-            }
-            hw[c] = (uint32_t)hh[0] | ((uint32_t)hh[1] << 16);
-            lw[c] = (uint32_t)ll[0] | ((uint32_t)ll[1] << 16);
+        for (int c = 0; c < 8; c++) v[c] = u[8 * h + c];
+        PanelPair w;
+        if (xh >= o.x0 && xh + 8 <= o.x1) {
+            w = split_panel(v, mx);
+        } else {
+            const PanelPair old{*reinterpret_cast<const uint4 *>(o.in_hi + off),
+                                *reinterpret_cast<const uint4 *>(o.in_lo + off)};
+            w = split_panel_edge(v, old, xh, o.x0, o.x1, StepScale{2048.0f, 0, 0}, mx);
         }
+        *reinterpret_cast<uint4 *>(o.out_hi + off) = w.hi;
+        *reinterpret_cast<uint4 *>(o.out_lo + off) = w.lo;
     }
-    *reinterpret_cast<uint4 *>(o.out_hi + off0) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-    *reinterpret_cast<uint4 *>(o.out_hi + off1) = make_uint4(hw[4], hw[5], hw[6], hw[7]);
-    *reinterpret_cast<uint4 *>(o.out_lo + off0) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-    *reinterpret_cast<uint4 *>(o.out_lo + off1) = make_uint4(lw[4], lw[5], lw[6], lw[7]);
+}
+
+// A tile's row outside the update rectangle: its blocks j0, j0 + dj, .. < nblk
+// copied from the input planes, off the accumulator ring's path.
+__device__ __forceinline__ void copy_rows(const TileOut &o, int y, int X0, int j0, int dj, int nblk) {
+    if (y >= o.y0 && y < o.y1) return;
+#pragma unroll 1
+    for (int j = j0; j < nblk; j += dj) {
+        const size_t a = plane_index16(o.pg, y, X0 + 16 * j), b = a + (size_t)o.pg.nyp * 8;
+        const uint4 h0 = *reinterpret_cast<const uint4 *>(o.in_hi + a), h1 = *reinterpret_cast<const uint4 *>(o.in_hi + b);
+        const uint4 l0 = *reinterpret_cast<const uint4 *>(o.in_lo + a), l1 = *reinterpret_cast<const uint4 *>(o.in_lo + b);
+        *reinterpret_cast<uint4 *>(o.out_hi + a) = h0;
+        *reinterpret_cast<uint4 *>(o.out_hi + b) = h1;
+        *reinterpret_cast<uint4 *>(o.out_lo + a) = l0;
+        *reinterpret_cast<uint4 *>(o.out_lo + b) = l1;
+    }
 }
 
 __device__ __forceinline__ bool tile_inside(const TileOut &o, int Y0, int X0) {

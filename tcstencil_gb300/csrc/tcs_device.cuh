@@ -138,6 +138,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     return ok != 0;
 }
 
+// The next 1024-byte boundary of the dynamic shared memory.  As an offset to
+// the array, not a rounded integer: the compiler then knows that accesses
+// through the result are to shared memory, and emits no generic ones (with
+// them: 8196² box2d2r FP16 41.8 us per step, 40.0 without; two-step split
+// 1026² 5.3, 5.1).
+__device__ __forceinline__ uint8_t *align_smem(uint8_t *raw) { return raw + (-smem_u32(raw) & 1023u); }
+
 // Waits for the phase of `parity` to complete.  Gives up (returns false) when
 // *abort becomes non-zero or after kWaitLimitNs; the caller then records the
 // error and leaves its loop.

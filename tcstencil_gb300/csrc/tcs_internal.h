@@ -60,6 +60,13 @@ constexpr int kPadRows = 8;
 
 __host__ __device__ constexpr int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
+// Tile rows of two split steps per load: each gives up kTbHalo rows at its top
+// and bottom; their copies start at multiples of kTbMapRows rows.
+constexpr int kTbHalo = 2;
+constexpr int kTbRows = kTile - 2 * kTbHalo;
+constexpr int kTbMapRows = 4;
+inline int tb_tiles_y(int ny) { return ny <= kTile ? 1 : (ny - 2 * kTbHalo + kTbRows - 1) / kTbRows; }
+
 struct PlaneGeom {
     int nyp;   // rows per panel, padding included
     int npan;  // panels, padding included
