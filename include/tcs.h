@@ -216,8 +216,8 @@ int tcs_plan_scale_exp(tcs_plan plan, int *scale_exp);
 int tcs_plan_set_coeffs(tcs_plan plan, const float *coeffs);
 /* Temporal blocking depth: 1 (single steps, the default) or 2 (two steps per
  * launch, intermediate kept on chip; split precision on the tensor engine,
- * faster there but for 2000 to 3000 columns and rows, where the one-launch form
- * of single steps is).  Results are bit-identical either way; the autotuner
+ * faster there but around 2900 columns and rows, where the one-launch form of
+ * single steps is).  Results are bit-identical either way; the autotuner
  * picks, tcs_sweep_host and pipes take depth 2 for split. */
 int tcs_plan_set_temporal_depth(tcs_plan plan, int depth);
 /* Tensor engine (FP16 or split, temporal depth 1): run(steps >= 2) as ONE

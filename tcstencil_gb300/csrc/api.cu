@@ -429,11 +429,11 @@ struct tcs_plan_s {
     // blocked pairs, with the same bits as single steps.  The one-call form,
     // pipes and autotuned plans of untuned sizes take it for every split grid:
     // box2d1r / box2d2r, us per step, best form of single steps -> pairs:
-    // 256² 6.65 -> 6.26 / 6.88 -> 6.46, 1026² 7.49 -> 6.53 / 8.91 -> 6.64, 4096²
-    // 26.5 -> 22.2 / 27.2 -> 25.1, 16386² 356 -> 264 / 371 -> 312.  Only around
-    // 2048² to 2900² is the one-launch form of single steps faster (2048² 10.3
-    // -> 11.3, 2896² 14.5 -> 15.5), where a pair's launches still weigh; the
-    // tuned table takes it there.
+    // 256² 6.53 -> 4.69 / 7.23 -> 5.19, 1026² 7.83 -> 5.00 / 9.21 -> 5.78, 1600²
+    // 9.25 -> 7.39 / 10.0 -> 8.23, 4096² 21.5 -> 21.0 / 25.2 -> 24.2, 8196² 89.4
+    // -> 73.6 / 101 -> 86.0.  Only around 2900² is the one-launch form of single
+    // steps no slower (12.2 / 12.4, 13.7 / 14.6), where a pair's launches still
+    // weigh; the tuned table takes it there.
     int temporal_depth = 1;
     bool pairs() const { return temporal_depth == 2; }
     void take_pairs() {
