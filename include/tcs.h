@@ -205,7 +205,8 @@ int tcs_plan_destroy(tcs_plan plan);
 int tcs_plan_upload(tcs_plan plan, const float *grid, int grid_on_host, void *stream);
 /* Writes the current state as an ny x nx FP32 row-major grid. */
 int tcs_plan_download(tcs_plan plan, float *grid, int grid_on_host, void *stream);
-/* Runs `steps` sweep steps.  use_graph != 0 replays a CUDA graph of the steps. */
+/* Runs `steps` sweep steps.  use_graph != 0 replays a CUDA graph of the steps
+ * (calls of up to eight launches, tcs_plan_launches, go out directly). */
 int tcs_plan_run(tcs_plan plan, int steps, int use_graph, void *stream);
 /* Device pointers of the current state planes (lo = NULL unless split), and
  * the bytes of one plane. */

@@ -794,7 +794,17 @@ int tcs_plan_scale_exp(tcs_plan p, int *scale_exp) {
 int tcs_plan_run(tcs_plan p, int steps, int use_graph, void *stream) {
     if (!p || steps < 0) return fail(TCS_ERR_INVALID, "tcs_plan_run: bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
-    if (!use_graph || steps <= 1) {
+    // Up to eight launches go out directly: a graph's start and end cost the
+    // device about 5 us more than theirs (solves of a resident grid, graph ->
+    // direct: 256² FP16 one launch 23.2 -> 20.5 us, 128² split 1 / 4 / 8 launches
+    // 26.7 -> 20.5 / 53 -> 48 / 89 -> 84), and the host is done with them before
+    // the device is (about 5 us a launch against 6 to 10); past sixteen a
+    // single-step launch is shorter than its host call (256² FP16, 24 launches:
+    // 115 -> 120 us) and the graph keeps the host free.
+    int launches = 0;
+    int lst = tcs_plan_launches(p, steps, &launches);
+    if (lst) return lst;
+    if (!use_graph || launches <= 8) {
         int to = p->cur;
         const int st = p->enqueue(steps, p->cur, s, &to);
         if (!st) p->cur = to;
