@@ -119,7 +119,8 @@ __device__ __forceinline__ void walk_blocks(uint32_t col, Sink &&sink) {
         uint32_t v[2][16];
         tmem_ld_x16(col + 16 * g, v[0]);
         if (g + 1 < G) tmem_ld_x16(col + 16 * (g + 1), v[1]);
-        tmem_ld_wait();
+        if (g + 1 < G) tmem_ld_wait(v);
+        else tmem_ld_wait(v[0]);
 #pragma unroll
         for (int p = 2 * g; p < 2 * g + 4 && p < 2 * G; p++)
             sink(p, pack_panel(v[(p >> 1) - g] + 8 * (p & 1)));
@@ -162,7 +163,7 @@ __device__ __forceinline__ void step_to_image(const WarpTile &c, int half, int t
         tmem_ld_x8(c.ecol, e);
         const uint4 old = lds128(c.eimg);
         const uint4 m = lds128(c.mask + 16 * (half ? 9 + eb : ea));
-        tmem_ld_wait();
+        tmem_ld_wait(e);
         if (row) sts128(c.eimg, blend(pack_panel(e), old, m));
         walk_blocks<G>(c.col, [&](int p, const uint4 &w) {
             if (row) sts128(c.img + p * SG::CHUNK, w);
@@ -173,7 +174,7 @@ __device__ __forceinline__ void step_to_image(const WarpTile &c, int half, int t
             tmem_ld_x8(c.ecol, e);
             const uint4 old = lds128(c.eimg);
             const uint4 m = cells_mask(c.mask, max(ea, c.ea), min(eb, c.eb));
-            tmem_ld_wait();
+            tmem_ld_wait(e);
             if (row) sts128(c.eimg, blend(pack_panel(e), old, m));
         }
         walk_blocks<G>(c.col, [&](int p, const uint4 &w) {

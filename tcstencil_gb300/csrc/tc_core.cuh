@@ -418,7 +418,7 @@ __device__ __forceinline__ void split_block_load(uint32_t region_a, uint32_t reg
         tmem_ld_x16(region_a + 16 + 32 * part, v[2 * part]);
         tmem_ld_x16(region_b + 32 * part, v[2 * part + 1]);
     }
-    tmem_ld_wait();
+    tmem_ld_wait(v);
     // two columns per packed FP32 operation (each lane rounds as the scalar
     // one would)
     auto pr = [&](int part, int c) {
@@ -603,7 +603,7 @@ __device__ __forceinline__ void epilogue_load(uint32_t lane_col, int half,
     uint32_t v[G][16];
 #pragma unroll
     for (int gg = 0; gg < G; gg++) tmem_ld_x16(lane_col + 16 * (half * G + gg + 1), v[gg]);
-    tmem_ld_wait();
+    tmem_ld_wait(v);
 #pragma unroll
     for (int gg = 0; gg < G; gg++)
 #pragma unroll
@@ -811,7 +811,7 @@ __device__ __forceinline__ void plain_epilogue(const TileOut &o, uint32_t lane_c
     uint32_t v[G][16];
 #pragma unroll
     for (int gg = 0; gg < G; gg++) tmem_ld_x16(lane_col + 16 * (j0 + gg + 1), v[gg]);
-    tmem_ld_wait();
+    tmem_ld_wait(v);
     release();
 #pragma unroll
     for (int gg = 0; gg < G; gg++) {

@@ -278,8 +278,21 @@ __device__ __forceinline__ void tmem_ld_x8(uint32_t taddr, uint32_t (&v)[8]) {
         : "r"(taddr));
 }
 
-__device__ __forceinline__ void tmem_ld_wait() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// Waits for this thread's tcgen05.ld's.  The words they loaded pass through an
+// empty asm that depends on the wait, so that no use of one can be moved
+// before it (the loads return at once, and to the compiler their results are
+// there).
+__device__ __forceinline__ void tmem_loaded(uint32_t &v, uint32_t waited) { asm("" : "+r"(v) : "r"(waited)); }
+template <typename T, int N>
+__device__ __forceinline__ void tmem_loaded(T (&v)[N], uint32_t waited) {
+#pragma unroll
+    for (int i = 0; i < N; i++) tmem_loaded(v[i], waited);
+}
+template <typename... V>
+__device__ __forceinline__ void tmem_ld_wait(V &...v) {
+    uint32_t waited;
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n\tmov.u32 %0, 0;" : "=r"(waited)::"memory");
+    (tmem_loaded(v, waited), ...);
 }
 
 // Shared-memory matrix descriptor, no swizzle.  The operand is made of
