@@ -429,9 +429,9 @@ struct tcs_plan_s {
     // blocked pairs, with the same bits as single steps.  The one-call form,
     // pipes and autotuned plans of untuned sizes take it for every split grid:
     // box2d1r / box2d2r, us per step, best form of single steps -> pairs:
-    // 256² 6.53 -> 4.69 / 7.23 -> 5.19, 1026² 7.83 -> 5.00 / 9.21 -> 5.78, 1600²
-    // 9.25 -> 7.39 / 10.0 -> 8.23, 4096² 21.5 -> 21.0 / 25.2 -> 24.2, 8196² 89.4
-    // -> 73.6 / 101 -> 86.0.  Only around 2900² is the one-launch form of single
+    // 256² 6.38 -> 3.15 / 7.10 -> 3.48, 1026² 7.67 -> 4.42 / 9.05 -> 5.31, 1600²
+    // 9.11 -> 5.91 / 10.0 -> 7.04, 4096² 21.5 -> 21.0 / 25.2 -> 24.2, 8196² 89.4
+    // -> 73.5 / 101 -> 85.3.  Only around 2900² is the one-launch form of single
     // steps no slower (12.2 / 12.4, 13.7 / 14.6), where a pair's launches still
     // weigh; the tuned table takes it there.
     int temporal_depth = 1;

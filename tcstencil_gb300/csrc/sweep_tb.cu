@@ -3,7 +3,8 @@
 // rate takes twice as long as a radius-1 tile's MMAs and as long as a
 // radius-2 tile's; two steps per load and store halve the traffic.
 //
-// Tile.  As in the single-step split kernel (sweep_tc.cu): the stage holds
+// Tile.  As in the single-step split kernel (sweep_tc.cu), W = 128, 80 or 32
+// columns wide (tb_width; the numbers here are for 128): the stage holds
 // rows Yb-4 .. Yb+131 of the panels X0-8 .. X0+135, hi and lo, and one step's
 // nine windows give rows Yb .. Yb+127 of the columns X0-16 .. X0+143.  The
 // first step's values go back over the staged image (X0-8 .. X0+135: the
@@ -34,8 +35,8 @@
 // it completes, for three groups of 128 registers, was slower: 309.)  Rows
 // outside the update rectangle are left out of the blocks and copied after
 // them, and only panels that straddle its sides choose per cell: at 1026²,
-// where half of the tiles touch the border, 6.5 -> 4.95 us per step (8.0 a
-// step in single launches).  (The form this
+// where half of the tiles touch the border, 6.5 -> 4.95 us per step, and 4.32
+// with 80 columns (8.0 a step in single launches).  (The form this
 // replaces, with 80-column tiles, a second image for the intermediate and a
 // handoff per step, took 140 / 156 us per step at 8196², box2d1r / box2d2r.)
 // Two stages: the next tile loads while a tile runs both its steps.
@@ -85,10 +86,12 @@ struct TbParams {
     float coef[25];
 };
 
-template <int S>
+template <int S, int W>
 __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid_constant__ TbParams p) {
     using C = TbCfg<S>;
     constexpr int R = C::R;
+    constexpr int WIN = W / 16 + 1, BLK = W / 16 + 2, PANELS = W / 8 + 2;
+    static_assert(WIN % kTbIssuers == 0 && 2 * WIN > kTbRing, "an issuer's windows and the barriers' phases");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = align_smem(smem_raw);
     uint8_t *stage_base = smem;  // [stage][hi, lo]
@@ -97,9 +100,9 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
     uint64_t *full = bars;                          // [stages]
     uint64_t *empty = full + kTbStages;             // [stages]
     uint64_t *win_empty = empty + kTbStages;        // [kTbRing] region read by its blocks' groups
-    uint64_t *blk_full = win_empty + kTbRing;       // [2][kTbBlocks] a step's block: its windows complete
-    uint64_t *blk_ready = blk_full + 2 * kTbBlocks; // [kTbBlocks] first-step values in the image
-    uint64_t *drain = blk_ready + kTbBlocks;        // [1]
+    uint64_t *blk_full = win_empty + kTbRing;       // [2][BLK] a step's block: its windows complete
+    uint64_t *blk_ready = blk_full + 2 * BLK; // [BLK] first-step values in the image
+    uint64_t *drain = blk_ready + BLK;        // [1]
     CtaScale cs;                                    // the CTA's side of the scale
     cs.bar = drain + 1;                             // [2]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(cs.bar + 2);
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
     cs.cnt = cs.max + 2;                            // [2]
     cs.ss = reinterpret_cast<StepScale *>(cs.cnt + 2);  // [2]
     uint32_t *issued = reinterpret_cast<uint32_t *>(cs.ss + 2);  // [kTbIssuers] 1 + its last window
-    static_assert((2 * kTbStages + kTbRing + 3 * kTbBlocks + 3) * 8 + 24 + 2 * sizeof(StepScale) +
+    static_assert((2 * kTbStages + kTbRing + 3 * BLK + 3) * 8 + 24 + 2 * sizeof(StepScale) +
                           4 * kTbIssuers <= C::BARS,
                   "barrier area");
 
@@ -122,10 +125,10 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
             mbar_init(&empty[s], kTbIssuers);
         }
         for (int r = 0; r < kTbRing; r++) mbar_init(&win_empty[r], 8);  // two groups
-        for (int b = 0; b < kTbBlocks; b++) {
+        for (int b = 0; b < BLK; b++) {
             // the halo blocks have one window
             for (int st = 0; st < 2; st++)
-                mbar_init(&blk_full[st * kTbBlocks + b], b == 0 || b == kTbBlocks - 1 ? 1 : 2);
+                mbar_init(&blk_full[st * BLK + b], b == 0 || b == BLK - 1 ? 1 : 2);
             mbar_init(&blk_ready[b], 4);
         }
         for (int k = 0; k < kTbIssuers; k++) issued[k] = 0;
@@ -168,10 +171,10 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                 const int t = (int)blockIdx.x + i * (int)gridDim.x;
                 const int ty = t / p.tiles_x, tx = t - ty * p.tiles_x;
                 uint8_t *st = stage_base + (size_t)s * 2 * SG::PLANE;
-                mbar_arrive_expect_tx(&full[s], 2 * SG::PLANE);
-                tma_load_3d(st, &p.map_hi, &full[s], 0, ty * kTbRows / kTbMapRows, tx * (kTile / 8));
+                mbar_arrive_expect_tx(&full[s], 2 * PANELS * SG::CHUNK);
+                tma_load_3d(st, &p.map_hi, &full[s], 0, ty * kTbRows / kTbMapRows, tx * (W / 8));
                 tma_load_3d(st + SG::PLANE, &p.map_lo, &full[s], 0, ty * kTbRows / kTbMapRows,
-                            tx * (kTile / 8));
+                            tx * (W / 8));
                 last_issued = i;
             }
             for (int k = 0; k < kTbStages && last_issued - k >= 0; k++) {
@@ -193,7 +196,6 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
             bool stop = false;
             // global window, its region, the region's uses before it
             int G = id, r = id % kTbRing, uses = id / kTbRing;
-            static_assert(2 * kTbWindows % kTbIssuers == 0, "an issuer's windows are the same in every tile");
             const int before = (id + kTbIssuers - kTbRing % kTbIssuers) % kTbIssuers;  // issuer of G - 5
             // bounded wait until issuer k has issued window G
             auto issued_by = [&](int k, int G) {
@@ -211,9 +213,9 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                 }
                 const uint64_t a_hi0 =
                     smem_desc(smem_u32(stage_base + (size_t)s * 2 * SG::PLANE), SG::CHUNK, 128);
-                for (int sw = id; sw < 2 * kTbWindows; sw += kTbIssuers) {
-                    const bool second = sw >= kTbWindows;
-                    const int w = second ? sw - kTbWindows : sw;
+                for (int sw = id; sw < 2 * WIN; sw += kTbIssuers) {
+                    const bool second = sw >= WIN;
+                    const int w = second ? sw - WIN : sw;
                     // window w's blocks are w and w + 1
                     if ((G >= kTbRing && !issued_by(before, G - kTbRing)) ||
                         !mbar_wait(&win_empty[r], (uses & 1) ^ 1, abort_flag) ||
@@ -227,9 +229,9 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                     issue_split_window<R, SG>(a_hi0, band, tmem_base + r * kTbRegion, w);
                     st_release_cta(&issued[id], (uint32_t)G + 1);
                     // the window's two blocks (the second step has no halo blocks)
-                    uint64_t *bf = blk_full + (second ? kTbBlocks : 0);
+                    uint64_t *bf = blk_full + (second ? BLK : 0);
                     if (!second || w > 0) umma_commit(&bf[w]);
-                    if (!second || w < kTbWindows - 1) umma_commit(&bf[w + 1]);
+                    if (!second || w < WIN - 1) umma_commit(&bf[w + 1]);
                     G += kTbIssuers;
                     r += kTbIssuers;
                     while (r >= kTbRing) {
@@ -281,7 +283,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
         // windows back, and sink each panel (its index in the image, its
         // eight values).  rb: region of the step's window 0, at most 4.
         auto take_block = [&](int st, int b, int rb, int i, const StepScale &ss, auto &&sink) {
-            bool ok = mbar_wait(&blk_full[st * kTbBlocks + b], i & 1, abort_flag);
+            bool ok = mbar_wait(&blk_full[st * BLK + b], i & 1, abort_flag);
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) fail(kErrWaitResult);
                 return false;
@@ -300,16 +302,16 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                 if (lane == 0) {
                     // in the second step the outer windows have one block
                     if (b > 0) mbar_arrive_n(&win_empty[wa], st == 1 && b == 1 ? 2 : 1);
-                    if (b < kTbBlocks - 1) mbar_arrive_n(&win_empty[wb], st == 1 && b == kTbBlocks - 2 ? 2 : 1);
+                    if (b < BLK - 1) mbar_arrive_n(&win_empty[wb], st == 1 && b == BLK - 2 ? 2 : 1);
                 }
             };
             float u[8];
             uint32_t v[6][8];
-            if (b == 0 || b == kTbBlocks - 1) {
+            if (b == 0 || b == BLK - 1) {
                 // halo panel: the inner one of the block; cells that lack a
                 // column of the input are zero (nothing valid reads them)
                 panel_load(b == 0 ? tb + 8 : ta, 0, false, v);
-                tmem_ld_wait();
+                tmem_ld_wait(v);
                 release();
                 panel_sum(v, false, ss, u);
 #pragma unroll
@@ -321,10 +323,10 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                 // five regions the windows wait for this release)
                 float u2[8];
                 panel_load(ta, tb, true, v);
-                tmem_ld_wait();
+                tmem_ld_wait(v);
                 panel_sum(v, true, ss, u);
                 panel_load(ta + 8, tb + 8, true, v);
-                tmem_ld_wait();
+                tmem_ld_wait(v);
                 release();
                 panel_sum(v, true, ss, u2);
                 sink(2 * b - 1, u);
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
         for (int i = 0; i < n_mine && !stop; i++) {
             const int t = (int)blockIdx.x + i * (int)gridDim.x;
             const int ty = t / p.tiles_x, tx = t - ty * p.tiles_x;
-            const int Yb = ty * kTbRows, X0 = tx * kTile;
+            const int Yb = ty * kTbRows, X0 = tx * W;
             const int y = Yb + m;
             const bool top = ty == 0, bottom = ty == p.tiles_y - 1;
             const bool row_in = y >= g.y0 && y < g.y1;
@@ -343,8 +345,10 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
             const uint32_t img = smem_u32(stage_base) +
                                  (uint32_t)((i % kTbStages) * 2 * SG::PLANE + (m + SG::TOP) * 16);
             const size_t row0 = plane_index16(g.p16, mine ? y : 0, X0 - 8);
-            for (int idx = grp; idx < 2 * kTbWindows && !stop; idx += kTbGroups) {
-                if (idx < kTbBlocks) {
+            // (rolled: unrolled, as it would be for 80 columns, it spills registers)
+#pragma unroll 1
+            for (int idx = grp; idx < 2 * WIN && !stop; idx += kTbGroups) {
+                if (idx < BLK) {
                     // first step -> the image
                     const bool ok = take_block(0, idx, r0, i, ss1, [&](int pan, const float (&u)[8]) {
                         const int xb = X0 - 8 + 8 * pan;
@@ -371,8 +375,8 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                     if (lane == 0) mbar_arrive(&blk_ready[idx]);
                 } else {
                     // second step -> the output planes
-                    const int rb = r0 + 4 >= 5 ? r0 - 1 : r0 + 4;  // nine windows on
-                    const bool ok = take_block(1, idx - kTbWindows, rb, i, ss2, [&](int pan, const float (&u)[8]) {
+                    const int rb = (r0 + WIN) % kTbRing;
+                    const bool ok = take_block(1, idx - WIN, rb, i, ss2, [&](int pan, const float (&u)[8]) {
                         const int xb = X0 - 8 + 8 * pan;
                         if (!mine || !row_in || xb >= g.nx) return;
                         const size_t off = row0 + (size_t)pan * g.p16.nyp * 8;
@@ -388,29 +392,23 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
                         *reinterpret_cast<uint4 *>(p.out_lo + off) = w.lo;
                     });
                     if (!ok) stop = true;
+                    __syncwarp();  // rows may have parted; warp-wide TMEM loads next
                 }
             }
-            r0 = r0 + 3 >= 5 ? r0 - 2 : r0 + 3;  // 18 windows on
-            // rows that keep their values: this group's panels (all loads before
-            // the first store)
+            r0 = (r0 + 2 * WIN) % kTbRing;
+            // rows that keep their values: this group's panels
             if (!stop && mine && !row_in) {
-                PanelPair keep[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const size_t off = row0 + (size_t)(1 + grp + 4 * k) * g.p16.nyp * 8;
-                    keep[k] = PanelPair{*reinterpret_cast<const uint4 *>(p.in_hi + off),
-                                        *reinterpret_cast<const uint4 *>(p.in_lo + off)};
-                }
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const int pan = 1 + grp + 4 * k;
-                    if (X0 - 8 + 8 * pan >= g.nx) break;
+#pragma unroll 1
+                for (int pan = 1 + grp; pan <= W / 8 && X0 - 8 + 8 * pan < g.nx; pan += kTbGroups) {
                     const size_t off = row0 + (size_t)pan * g.p16.nyp * 8;
-                    const PanelPair w = cs2.k != 0 ? resplit_panel(keep[k], cs2) : keep[k];
+                    PanelPair w{*reinterpret_cast<const uint4 *>(p.in_hi + off),
+                                *reinterpret_cast<const uint4 *>(p.in_lo + off)};
+                    if (cs2.k != 0) w = resplit_panel(w, cs2);
                     *reinterpret_cast<uint4 *>(p.out_hi + off) = w.hi;
                     *reinterpret_cast<uint4 *>(p.out_lo + off) = w.lo;
                 }
             }
+            __syncwarp();
         }
         if (!stop && p.scale) {  // tile 0 is CTA 0's
             cta_scale_flush<kTbEpiWarps>(cs, 0, p.scale, p.t0 + 1, ss1, mx1, blockIdx.x == 0);
@@ -429,19 +427,51 @@ __global__ void __launch_bounds__(kTbThreads, 1) tc_split_tb_kernel(const __grid
 
 int g_tb_sms = 0;
 
-template <int S>
-cudaError_t launch_tb(const GridGeom &g, const float *B, const uint16_t *in_hi,
-                      const uint16_t *in_lo, uint16_t *out_hi, uint16_t *out_lo, cudaStream_t s,
-                      SplitScale *scale, int t0) {
+// Tile columns: what a launch takes is about its waves of tiles times a tile's
+// windows (2 (W/16 + 1), one after another), so a grid of few tiles is cut
+// narrower; a tie goes to the wider tile, which recomputes less halo.  32
+// columns only while they leave half of the SMs free: past that their loads
+// and launches, 1.5 times as many bytes per cell, take back what the shorter
+// chain gives.  us per step of a pair, W = 128 / 80 / 32 (box2d1r; box2d2r):
+// 256² 4.72 / 3.82 / 3.15 (5.26 / 4.14 / 3.48), 512² 4.79 / 3.78 / 3.55, 724²
+// 4.78 / 3.87 / 3.89 (5.28 / 4.23 / 4.81), 1024² 4.75 / 4.36 / 4.99, 1600² 7.51
+// / 5.91 / 7.77 (8.43 / 7.04 / 9.53), 2048² 7.61 / 7.70 / 11.1, 4096² 20.8 /
+// 22.6 / 34.1, 8196² 73.1 / 75.4 / 129.  (A tile takes 3, 6 or 9 windows a step:
+// a multiple of the issuers, so that an issuer's windows are the same in every
+// tile.)
+int tb_width(const GridGeom &g) {
+    const int ty = tb_tiles_y(g.ny);
+    auto tiles = [&](int w) { return (long long)((g.nx + w - 1) / w) * ty; };
+    auto waves = [&](int w) { return (tiles(w) + g_tb_sms - 1) / g_tb_sms; };
+    if (tiles(32) <= g_tb_sms / 2) return 32;
+    return waves(80) * 6 < waves(128) * 9 ? 80 : 128;
+}
+
+template <int S, int W>
+cudaError_t launch_tb_w(TbParams &p, cudaStream_t s) {
     using C = TbCfg<S>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(tc_split_tb_kernel<S>,
+        cudaError_t e = cudaFuncSetAttribute(tc_split_tb_kernel<S, W>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(C::SMEM));
         if (e != cudaSuccess) return e;
         configured = true;
     }
+    cudaError_t e = encode_panel_map(p.in_hi, p.g.p16, &p.map_hi, W / 8 + 2, kTbMapRows);
+    if (e == cudaSuccess) e = encode_panel_map(p.in_lo, p.g.p16, &p.map_lo, W / 8 + 2, kTbMapRows);
+    if (e != cudaSuccess) return e;
+    p.tiles_x = (p.g.nx + W - 1) / W;
+    p.n_tiles = p.tiles_x * p.tiles_y;
+    const int grid = p.n_tiles < g_tb_sms ? p.n_tiles : g_tb_sms;
+    return launch_step(tc_split_tb_kernel<S, W>, grid, kTbThreads, C::SMEM, s, p);
+}
+
+template <int S>
+cudaError_t launch_tb(const GridGeom &g, const float *B, const uint16_t *in_hi,
+                      const uint16_t *in_lo, uint16_t *out_hi, uint16_t *out_lo, cudaStream_t s,
+                      SplitScale *scale, int t0) {
+    using C = TbCfg<S>;
     if (!g_tb_sms) {
         int dev = 0;
         cudaGetDevice(&dev);
@@ -450,12 +480,7 @@ cudaError_t launch_tb(const GridGeom &g, const float *B, const uint16_t *in_hi,
     }
     TbParams p;
     p.g = g;
-    cudaError_t e = encode_panel_map(in_hi, g.p16, &p.map_hi, kTile / 8 + 2, kTbMapRows);
-    if (e == cudaSuccess) e = encode_panel_map(in_lo, g.p16, &p.map_lo, kTile / 8 + 2, kTbMapRows);
-    if (e != cudaSuccess) return e;
-    p.tiles_x = (g.nx + kTile - 1) / kTile;
     p.tiles_y = tb_tiles_y(g.ny);
-    p.n_tiles = p.tiles_x * p.tiles_y;
     p.in_hi = in_hi;
     p.in_lo = in_lo;
     p.out_hi = out_hi;
@@ -463,8 +488,11 @@ cudaError_t launch_tb(const GridGeom &g, const float *B, const uint16_t *in_hi,
     p.scale = scale;
     p.t0 = t0;
     for (int k = 0; k < 25; k++) p.coef[k] = k < C::NDY * C::NDY ? B[k] : 0.0f;
-    const int grid = p.n_tiles < g_tb_sms ? p.n_tiles : g_tb_sms;
-    return launch_step(tc_split_tb_kernel<S>, grid, kTbThreads, C::SMEM, s, p);
+    switch (tb_width(g)) {
+    case 32: return launch_tb_w<S, 32>(p, s);
+    case 80: return launch_tb_w<S, 80>(p, s);
+    default: return launch_tb_w<S, 128>(p, s);
+    }
 }
 
 }  // namespace
