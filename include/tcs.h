@@ -252,7 +252,10 @@ int tcs_plan_launches(tcs_plan plan, int steps, int *launches);
 
 /* One-call form: host FP32 grid in, `steps` steps, host FP32 grid out.  Device
  * state is kept in a per-thread cache keyed by shape and mode, so repeated
- * calls of one shape do not reallocate. */
+ * calls of one shape do not reallocate.  Large FP16 and FP32 grids go through
+ * in row bands whose copies and sweeps overlap (the same bits; the device holds
+ * the grid twice in FP32 beside its planes, or the call falls back to the grid
+ * as a whole). */
 int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *problem, int steps);
 /* Frees the calling thread's cached plans. */
 void tcs_release_cache(void);

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <algorithm>
 #include <map>
+#include <mutex>
 #include <memory>
 #include <string>
 #include <tuple>
@@ -141,6 +142,35 @@ int run_step(const GridGeom &g, int stencil, int engine, int precision, const fl
 using namespace tcs;
 
 // ================================================================ C-ABI ==
+namespace errors {
+
+// The kernels' error words, one per translation unit, are read and cleared by
+// one tiny kernel into a mapped host word: five blocking copies took 40 us, a
+// third of a small one-call sweep.
+constexpr int kErrorWords = 5;
+struct ErrorWords {
+    int *p[kErrorWords] = {};
+};
+struct {
+    std::mutex mu;
+    std::map<int, ErrorWords> words;  // by device
+    int *code = nullptr;
+} g_errors;
+
+__global__ void take_errors_kernel(const ErrorWords w, int *code) {
+    int c = 0;
+    for (int k = 0; k < kErrorWords; k++) {
+        const int v = *reinterpret_cast<volatile int *>(w.p[k]);
+        if (!v) continue;
+        atomicExch(w.p[k], 0);
+        if (!c) c = v;
+    }
+    *code = c;
+    __threadfence_system();
+}
+
+}  // namespace errors
+
 extern "C" {
 
 const char *tcs_status_string(int status) {
@@ -175,22 +205,27 @@ size_t tcs_plane_elems(int ny, int nx, int precision) {
 int tcs_device_error(int *code) {
     int st = cuda_status(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     if (st) return st;
-    int c = 0;
-    st = cuda_status(tc_take_error(&c), "reading the device error word");
+    using namespace errors;
+    int dev = 0, c = 0;
+    st = cuda_status(cudaGetDevice(&dev), "cudaGetDevice");
     if (st) return st;
-    int cb = 0;
-    st = cuda_status(batch_take_error(&cb), "reading the batch error word");
+    std::lock_guard<std::mutex> lk(g_errors.mu);
+    ErrorWords &w = g_errors.words[dev];
+    if (!w.p[0]) {
+        cudaError_t (*const word[])(int **) = {tc_error_word, batch_error_word, tb_error_word, visit_error_word,
+                                               cc_error_word};
+        for (int k = 0; k < kErrorWords && !st; k++) st = cuda_status(word[k](&w.p[k]), "device error word");
+        if (st) w.p[0] = nullptr;
+    }
+    if (!st && !g_errors.code)
+        st = cuda_status(cudaHostAlloc(&g_errors.code, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped),
+                         "cudaHostAlloc(device error)");
     if (st) return st;
-    if (!c) c = cb;
-    st = cuda_status(tb_take_error(&cb), "reading the blocked-sweep error word");
+    take_errors_kernel<<<1, 1>>>(w, g_errors.code);
+    st = cuda_status(cudaGetLastError(), "error word launch");
+    if (!st) st = cuda_status(cudaStreamSynchronize(nullptr), "reading the device error words");
     if (st) return st;
-    if (!c) c = cb;
-    st = cuda_status(visit_take_error(&cb), "reading the visit-sweep error word");
-    if (st) return st;
-    if (!c) c = cb;
-    st = cuda_status(cc_take_error(&cb), "reading the CUDA-core error word");
-    if (st) return st;
-    if (!c) c = cb;
+    c = *const_cast<volatile int *>(g_errors.code);
     if (code) *code = c;
     return c ? fail(TCS_ERR_TIMEOUT, "device wait timed out (code %d)", c) : TCS_OK;
 }
@@ -847,15 +882,155 @@ int tcs_plan_run(tcs_plan p, int steps, int use_graph, void *stream) {
 namespace {
 
 using CacheKey = std::tuple<int, int, int, int, int, int, int, int, int>;
+// A large grid in row bands, each a plan of its own rows and `halo` >= r steps
+// more on either side (wrong values creep in by r rows a step from a band's
+// cut edges), so that one band's sweep runs while the next is copied in and
+// the last copied out: the copies, most of a call, take both directions of the
+// link at once.  The halo rows are swept twice; every cell is the same sum.
+struct HostBands {
+    struct Band {
+        int a, b, lo, hi;  // its rows [a, b), swept as the grid [lo, hi)
+        tcs_plan plan = nullptr;
+        cudaEvent_t in = nullptr, done = nullptr;
+    };
+    int halo = 0;
+    std::vector<Band> bands;
+    float *in = nullptr, *out = nullptr;  // the grid, FP32
+    cudaStream_t up = nullptr, run = nullptr, down = nullptr;  // (blocking: ordered with the default stream)
+    ~HostBands() {
+        for (Band &b : bands) {
+            if (b.plan) tcs_plan_destroy(b.plan);
+            if (b.in) cudaEventDestroy(b.in);
+            if (b.done) cudaEventDestroy(b.done);
+        }
+        for (float *p : {in, out})
+            if (p) dev_free(p);
+        for (cudaStream_t t : {up, run, down})
+            if (t) cudaStreamDestroy(t);
+    }
+};
+
 struct PlanCache {
     std::map<CacheKey, tcs_plan> plans;
+    std::map<CacheKey, HostBands *> bands;
     ~PlanCache() {
         // Device memory is released by the driver at process exit; freeing it
         // from a static destructor could run after the CUDA runtime is gone.
         plans.clear();
+        bands.clear();
     }
 };
 thread_local PlanCache t_cache;
+
+// Bands of a one-call sweep (1: the grid as a whole), and the halo (a power of
+// two, so that calls of near step counts share one set): from 16 MB on, bands
+// at least four halos high, as many as a model of the call's time favours.
+// Copies: 200 GB/s one way, 330 both ways at once; a step: its cells at the
+// rate the engine reaches on a large grid, or the shortest step, with a tenth
+// more for a band's partial last wave.  Whole grid: in, sweep, out; bands: the
+// first in, the slower of the copies and the sweeps, the last out.  Measured,
+// us, before -> bands: 3000 x 5003 box2d1r FP16 20 steps 927 -> 620, 8196² 3741
+// -> 2446, 60 steps 5414 -> 2578; where the model keeps the grid whole, 2100 x
+// 2000 box2d2r FP32 20 steps, bands took 547, the whole 470.  Split grids share
+// one scale over the whole grid, step by step, so they are not cut.
+int host_bands(const tcs_problem *pr, const GridGeom &g, int steps, int *halo) {
+    const int r = stencil_r(pr->stencil);
+    const size_t bytes = (size_t)g.ny * g.nx * sizeof(float);
+    if (pr->precision == TCS_PREC_SPLIT || steps < 1 || steps > 512 || bytes < ((size_t)16 << 20) || g.y0 != r ||
+        g.y1 != g.ny - r)
+        return 1;
+    int h = 16;
+    while (h < r * steps) h *= 2;
+    *halo = h;
+    // cells per us and shortest step, by stencil (star2d1r, star2d2r, box2d1r, box2d2r)
+    static const double tensor[4] = {2.4e6, 1.65e6, 2.4e6, 1.65e6}, f16[4] = {2.2e6, 1.5e6, 1.65e6, 0.82e6},
+                        f32[4] = {1.75e6, 1.03e6, 1.16e6, 0.5e6};
+    const bool tc = pr->engine == TCS_ENGINE_TENSOR, box2 = pr->stencil == TCS_BOX2D2R;
+    const double rate = (tc ? tensor : pr->precision == TCS_PREC_F32 ? f32 : f16)[pr->stencil];
+    const double shortest = tc ? 1.7 : box2 ? 4.0 : 2.2;
+    const double copy = bytes / 200e3, both = 2 * bytes / 330e3;  // us
+    auto sweep = [&](double rows) { return steps * std::max(shortest, rows * g.nx / rate); };
+    int best = 1;
+    double t_best = 0.95 * (2 * copy + sweep(g.ny));
+    for (int k = 2; k <= 4; k++) {
+        if (g.ny / k < 4 * h) break;
+        const double t = 2 * copy / k + std::max(both * (k - 1) / k, 1.1 * k * sweep(g.ny / (double)k + 2 * h));
+        if (t < t_best) {
+            t_best = t;
+            best = k;
+        }
+    }
+    return best;
+}
+
+int make_host_bands(const tcs_problem *pr, int n, int halo, HostBands **out) {
+    std::unique_ptr<HostBands> hb(new HostBands());
+    hb->halo = halo;
+    const size_t bytes = (size_t)pr->ny * pr->nx * sizeof(float);
+    int st = dev_alloc_t(&hb->in, bytes, "staging");
+    if (!st) st = dev_alloc_t(&hb->out, bytes, "staging");
+    for (cudaStream_t *t : {&hb->up, &hb->run, &hb->down})
+        if (!st) st = cuda_status(cudaStreamCreate(t), "cudaStreamCreate");
+    for (int k = 0; k < n && !st; k++) {
+        HostBands::Band b;
+        b.a = (int)((long long)pr->ny * k / n);
+        b.b = (int)((long long)pr->ny * (k + 1) / n);
+        b.lo = std::max(0, b.a - halo);
+        b.hi = std::min(pr->ny, b.b + halo);
+        tcs_problem q = *pr;
+        q.ny = b.hi - b.lo;
+        if (q.y0 || q.y1 || q.x0 || q.x1) {  // the whole interior in rows (host_bands)
+            q.y0 = stencil_r(pr->stencil);
+            q.y1 = q.ny - q.y0;
+        }
+        st = tcs_plan_create(&q, &b.plan);
+        if (!st) st = cuda_status(cudaEventCreateWithFlags(&b.in, cudaEventDisableTiming), "cudaEventCreate");
+        if (!st) st = cuda_status(cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming), "cudaEventCreate");
+        hb->bands.push_back(b);
+    }
+    if (!st) *out = hb.release();
+    return st;
+}
+
+int sweep_host_bands(HostBands *hb, const float *h_in, float *h_out, const tcs_problem *pr, int steps) {
+    const size_t nx = (size_t)pr->nx;
+    const bool f32 = pr->precision == TCS_PREC_F32;
+    int st = TCS_OK, copied = 0;
+    auto check = [&](cudaError_t e, const char *what) {
+        if (!st) st = cuda_status(e, what);
+    };
+    auto give = [&](const HostBands::Band &b) {
+        check(cudaStreamWaitEvent(hb->down, b.done, 0), "cudaStreamWaitEvent");
+        check(cudaMemcpyAsync(h_out + b.a * nx, hb->out + b.a * nx, (size_t)(b.b - b.a) * nx * sizeof(float),
+                              cudaMemcpyDeviceToHost, hb->down), "download copy");
+    };
+    for (size_t k = 0; k < hb->bands.size() && !st; k++) {
+        HostBands::Band &b = hb->bands[k];
+        check(cudaMemcpyAsync(hb->in + copied * nx, h_in + copied * nx, (size_t)(b.hi - copied) * nx * sizeof(float),
+                              cudaMemcpyHostToDevice, hb->up), "upload copy");
+        check(cudaEventRecord(b.in, hb->up), "cudaEventRecord");
+        check(cudaStreamWaitEvent(hb->run, b.in, 0), "cudaStreamWaitEvent");
+        copied = b.hi;
+        if (!st) st = tcs_plan_set_coeffs(b.plan, pr->coeffs);
+        if (!st) st = tcs_plan_upload(b.plan, hb->in + b.lo * nx, 0, hb->run);
+        if (!st) st = tcs_plan_run(b.plan, steps, 1, hb->run);
+        if (!st)
+            check(launch_unpack_rows(b.plan->buf[b.plan->cur][0], b.hi - b.lo, pr->nx, f32, hb->out + b.lo * nx,
+                                     b.a - b.lo + kPadTop, b.b - b.lo + kPadTop, hb->run), "unpack launch");
+        check(cudaEventRecord(b.done, hb->run), "cudaEventRecord");
+        // (a copy to pageable memory holds the host until it is done: behind
+        // the next band's launches)
+        if (k > 0 && !st) give(hb->bands[k - 1]);
+    }
+    if (!st) give(hb->bands.back());
+    // the caller's buffers stay in use until all streams are done, also after
+    // an error
+    for (cudaStream_t t : {hb->up, hb->run, hb->down}) {
+        const cudaError_t e = cudaStreamSynchronize(t);
+        check(e, "cudaStreamSynchronize");
+    }
+    return st;
+}
 
 }  // namespace
 
@@ -866,6 +1041,28 @@ int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *pr, int s
         return fail(TCS_ERR_INVALID, "tcs_sweep_host: bad arguments");
     const CacheKey key{pr->ny, pr->nx, pr->stencil, pr->engine, pr->precision,
                        pr->y0, pr->y1, pr->x0, pr->x1};
+    GridGeom g;
+    int halo = 0;
+    if (make_geom(pr->ny, pr->nx, pr->stencil, pr->y0, pr->y1, pr->x0, pr->x1, &g) == TCS_OK) {
+        const int n = host_bands(pr, g, steps, &halo);
+        const size_t cells = (size_t)pr->ny * pr->nx;
+        // (bands read ahead of what they write: the same buffer or separate ones)
+        const bool apart = h_out == h_in || h_out + cells <= h_in || h_in + cells <= h_out;
+        if (n > 1 && apart) {
+            HostBands *&hb = t_cache.bands[key];
+            if (hb && (hb->halo != halo || (int)hb->bands.size() != n)) {
+                delete hb;
+                hb = nullptr;
+            }
+            // (short of memory for the bands: the grid as a whole)
+            if (hb || make_host_bands(pr, n, halo, &hb) == TCS_OK) {
+                int st = sweep_host_bands(hb, h_in, h_out, pr, steps);
+                if (!st) st = tcs_device_error(nullptr);
+                return st;
+            }
+            cudaGetLastError();
+        }
+    }
     tcs_plan p;
     auto it = t_cache.plans.find(key);
     if (it == t_cache.plans.end()) {
@@ -888,6 +1085,8 @@ int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *pr, int s
 void tcs_release_cache(void) {
     for (auto &kv : t_cache.plans) tcs_plan_destroy(kv.second);
     t_cache.plans.clear();
+    for (auto &kv : t_cache.bands) delete kv.second;
+    t_cache.bands.clear();
 }
 
 }  // extern "C"

@@ -755,11 +755,8 @@ cudaError_t launch_build_bands(const float *coef, int r, bool box, bool split, u
     return cudaGetLastError();
 }
 
-cudaError_t batch_take_error(int *code) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbol(code, g_batch_error, sizeof(int));
-    if (e != cudaSuccess) return e;
-    return *code ? cudaMemcpyToSymbol(g_batch_error, &zero, sizeof(int)) : cudaSuccess;
+cudaError_t batch_error_word(int **word) {
+    return cudaGetSymbolAddress(reinterpret_cast<void **>(word), g_batch_error);
 }
 
 }  // namespace tcs

@@ -122,6 +122,6 @@ cudaError_t launch_batch(const BatchParams &p, bool split, int num_sms, cudaStre
 // Bands of one stencil (coefficients n x n row-major, n = 2r+1) into dst.
 cudaError_t launch_build_bands(const float *coef, int r, bool box, bool split, uint16_t *dst,
                                cudaStream_t s);
-cudaError_t batch_take_error(int *code);
+cudaError_t batch_error_word(int **word);
 
 }  // namespace tcs

@@ -826,11 +826,8 @@ cudaError_t launch_cc_visits(const GridGeom &g, int stencil, bool f32, const Tap
                : dispatch_cv<false>(stencil, v.ppl, v.warps, p, c, sms, s);
 }
 
-cudaError_t cc_take_error(int *code) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbol(code, g_cc_error, sizeof(int));
-    if (e != cudaSuccess) return e;
-    return *code ? cudaMemcpyToSymbol(g_cc_error, &zero, sizeof(int)) : cudaSuccess;
+cudaError_t cc_error_word(int **word) {
+    return cudaGetSymbolAddress(reinterpret_cast<void **>(word), g_cc_error);
 }
 
 }  // namespace tcs

@@ -509,11 +509,8 @@ cudaError_t launch_tc_split2(const GridGeom &g, int stencil, const float *B, con
     }
 }
 
-cudaError_t tb_take_error(int *code) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbol(code, g_tb_error, sizeof(int));
-    if (e != cudaSuccess) return e;
-    return *code ? cudaMemcpyToSymbol(g_tb_error, &zero, sizeof(int)) : cudaSuccess;
+cudaError_t tb_error_word(int **word) {
+    return cudaGetSymbolAddress(reinterpret_cast<void **>(word), g_tb_error);
 }
 
 }  // namespace tcs

@@ -947,11 +947,8 @@ cudaError_t tc_prepare(int stencil, bool split) {
     }
 }
 
-cudaError_t tc_take_error(int *code) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbol(code, g_tc_error, sizeof(int));
-    if (e != cudaSuccess) return e;
-    return *code ? cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int)) : cudaSuccess;
+cudaError_t tc_error_word(int **word) {
+    return cudaGetSymbolAddress(reinterpret_cast<void **>(word), g_tc_error);
 }
 
 cudaError_t launch_tc_f16(const GridGeom &g, int stencil, const float *B, const uint16_t *in,

@@ -624,11 +624,8 @@ cudaError_t launch_tc_f16_visits(const GridGeom &g, int stencil, const float *B,
     }
 }
 
-cudaError_t visit_take_error(int *code) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbol(code, g_visit_error, sizeof(int));
-    if (e != cudaSuccess) return e;
-    return *code ? cudaMemcpyToSymbol(g_visit_error, &zero, sizeof(int)) : cudaSuccess;
+cudaError_t visit_error_word(int **word) {
+    return cudaGetSymbolAddress(reinterpret_cast<void **>(word), g_visit_error);
 }
 
 }  // namespace tcs

@@ -169,8 +169,8 @@ cudaError_t launch_cc_visits(const GridGeom &g, int stencil, bool f32, const Tap
                              void *out, int steps, const CcVisitShape &v, unsigned *counters,
                              cudaStream_t s, int sms);
 
-// Reads and clears the tensor kernels' device error word.
-cudaError_t tc_take_error(int *code);
+// The kernels' device error words (tcs_device_error reads and clears them).
+cudaError_t tc_error_word(int **word);
 struct SplitScale;
 // Split launches take the grid's per-step scale (SplitScale below; null: the
 // fixed scale of the planes as packed) and t0, the steps of the current run
@@ -179,9 +179,9 @@ struct SplitScale;
 cudaError_t launch_tc_split2(const GridGeom &g, int stencil, const float *B, const uint16_t *in_hi,
                              const uint16_t *in_lo, uint16_t *out_hi, uint16_t *out_lo,
                              cudaStream_t s, SplitScale *scale = nullptr, int t0 = 0);
-cudaError_t tb_take_error(int *code);
+cudaError_t tb_error_word(int **word);
 // Reads and clears the CUDA-core kernels' device error word.
-cudaError_t cc_take_error(int *code);
+cudaError_t cc_error_word(int **word);
 // Configures the tensor kernel of (stencil, split) ahead of its first launch.
 cudaError_t tc_prepare(int stencil, bool split);
 
@@ -210,7 +210,7 @@ cudaError_t visit_prepare(int stencil);
 cudaError_t launch_tc_f16_visits(const GridGeom &g, int stencil, const float *B, uint16_t *in,
                                  uint16_t *out, int steps, const VisitShape &v,
                                  unsigned *counters, cudaStream_t s, int sms);
-cudaError_t visit_take_error(int *code);
+cudaError_t visit_error_word(int **word);
 cudaError_t launch_tc_split_steps(const GridGeom &g, int stencil, const float *B,
                                   const uint16_t *in_hi, const uint16_t *in_lo, uint16_t *out_hi,
                                   uint16_t *out_lo, int steps, unsigned *rows_done, cudaStream_t s,
