@@ -470,6 +470,21 @@ struct CvParams {
     unsigned *ended, *done;   // CTAs at their end; [tiles] finished visits (zeros)
 };
 
+// The last CTA whose tiles need no counter any more leaves them zero for the
+// next launch: as leave_counters of sweep_visit.cu.  Called by a whole warp.
+__device__ __forceinline__ void cv_leave_counters(const CvParams &p, int lane) {
+    if (p.visits < 2) return;
+    int last = 0;
+    if (lane == 0) {
+        fence_acq_rel_gpu();
+        last = atomicAdd(p.ended, 1u) == gridDim.x - 1;
+        fence_acq_rel_gpu();
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    for (int t = lane; t < p.tiles_x * p.tiles_y; t += 32) p.done[t] = 0;
+    if (lane == 0) *p.ended = 0;
+}
+
 template <int S, bool F32, int PPL, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
     cc_visit_kernel(const __grid_constant__ CvParams p, const __grid_constant__ TapCoeffs c) {
@@ -495,6 +510,7 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
     __syncthreads();
 
     uint32_t phase = 0;
+    bool counted = false;  // (warp 0)
     for (int k = blockIdx.x; k < n_items; k += gridDim.x, phase ^= 1) {
         const int visit = k / n_tiles, tile = k - visit * n_tiles;
         const int ty = tile / p.tiles_x, tx = tile - ty * p.tiles_x;
@@ -516,6 +532,11 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
                         break;
                     }
                 }
+            }
+            // no counter is read or added to for this CTA's other tiles any more
+            if (ok && k + (int)gridDim.x >= n_items) {
+                cv_leave_counters(p, lane);
+                counted = true;
             }
             if (lane == 0) {
                 if (ok) {
@@ -630,20 +651,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
             }
         }
     }
-    // the last CTA to end leaves the counters zero for the next launch
-    if (p.visits > 1) {
-        __shared__ int last;
-        if (threadIdx.x == 0) {
-            fence_acq_rel_gpu();
-            last = atomicAdd(p.ended, 1u) == gridDim.x - 1;
-            fence_acq_rel_gpu();
-        }
-        __syncthreads();
-        if (last) {
-            for (int t = threadIdx.x; t < n_tiles; t += WARPS * 32) p.done[t] = 0;
-            if (threadIdx.x == 0) *p.ended = 0;
-        }
-    }
+    // an early exit did not leave the counters
+    if (!counted && warp == 0) cv_leave_counters(p, lane);
 }
 
 template <int S, bool F32, int PPL, int WARPS>

@@ -232,6 +232,25 @@ __device__ __forceinline__ bool wait_neighbours(const unsigned *done, const Tile
     return true;
 }
 
+// The last CTA whose tiles need no counter any more leaves them zero for the
+// next launch (a memset before each launch took a tenth of a 256², 10-step
+// run).  By then every tile's last addition has been made: a tile's last visit
+// waits for its own, and the CTAs count here after their last waits, beside
+// their last visits' steps (at the kernel's end it was 1 us of a small
+// launch).  Called by a whole warp.
+__device__ __forceinline__ void leave_counters(const VisitParams &p, int lane) {
+    if (p.visits < 2) return;
+    int last = 0;
+    if (lane == 0) {
+        fence_acq_rel_gpu();
+        last = atomicAdd(p.ended, 1u) == gridDim.x - 1;
+        fence_acq_rel_gpu();
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    for (int t = lane; t < p.tiles_x * p.tiles_y; t += 32) p.done[t] = 0;
+    if (lane == 0) *p.ended = 0;
+}
+
 // mbar_wait that polls for a while before it sleeps between polls: a step's
 // waits end within a microsecond, and a sleep that outlasts one costs a
 // quarter of a step.
@@ -263,7 +282,8 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     unsigned *stored = tmem_slot + 2;             // [slots] warps that stored their last step
-    static_assert((2 * NS + 2 * kVisitSlots + 1) * 8 + 8 + 4 * kVisitSlots <= kBarBytes, "barrier area");
+    volatile unsigned *left_over = stored + kVisitSlots;  // the producer gave up
+    static_assert((2 * NS + 2 * kVisitSlots + 1) * 8 + 12 + 4 * kVisitSlots <= kBarBytes, "barrier area");
     uint32_t *masks = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(bars) + kBarBytes);
 
     const int warp = threadIdx.x >> 5;
@@ -281,7 +301,12 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
         }
         mbar_init(drain, kVisitSlots);
         *abort_flag = 0;
+        *left_over = 0;
         fence_mbar_init();
+        // the first tile's load runs beside the rest of the set-up
+        mbar_arrive_expect_tx(&full[0], (uint32_t)stage_bytes);
+        tma_load_3d(stage_base, &p.map[0], &full[0], 0, (int)blockIdx.x / p.tiles_x * (kTile - 2 * p.halo) / p.map_rows,
+                    (int)blockIdx.x % p.tiles_x * W / 8);
     }
     if (warp == 1) {
         __syncwarp();
@@ -308,10 +333,11 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
 
     if (warp == 0) {
         // ------------------------------------------------------ producer ---
-        int i = 0, last_issued = -1;
+        int i = 0, last_issued = 0;
         TileWalk w;
         w.init(blockIdx.x, grid, tiles_x, tiles_y);
         for (int k = blockIdx.x; k < n_items; k += grid, i++, w.advance()) {
+            if (i == 0) continue;  // loaded above
             const int s = i % NS;
             if (w.step > 0 && !wait_neighbours(p.done, w, lane, abort_flag)) {
                 if (lane == 0) fail(kErrWaitDep);
@@ -332,6 +358,9 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
             if (!__shfl_sync(0xffffffffu, ok, 0)) break;
             last_issued = i;
         }
+        // no counter is read or added to by this CTA from here on
+        if (i * grid + (int)blockIdx.x >= n_items) leave_counters(p, lane);
+        else if (lane == 0) *left_over = 1;
         // every stage armed last must have landed before exit
         if (lane == 0) {
             for (int k = 0; k < NS && last_issued - k >= 0; k++) {
@@ -474,20 +503,8 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
         __syncwarp();
         tmem_dealloc(tmem_base, kTmemCols);
     }
-    // The last CTA to end leaves the counters zero for the next launch (a
-    // memset before each launch took a tenth of a 256², 10-step run).
-    if (p.visits > 1) {
-        if (threadIdx.x == 0) {
-            fence_acq_rel_gpu();
-            *tmem_slot = atomicAdd(p.ended, 1u) == (unsigned)grid - 1;
-            fence_acq_rel_gpu();
-        }
-        __syncthreads();
-        if (*tmem_slot) {
-            for (int t = threadIdx.x; t < tiles_x * tiles_y; t += kVisitThreads) p.done[t] = 0;
-            if (threadIdx.x == 0) *p.ended = 0;
-        }
-    }
+    // a producer that gave up did not leave the counters
+    if (*left_over && warp == 0) leave_counters(p, lane);
 }
 
 // One CTA per SM: two would share TMEM, of which each takes all, and the CTAs
