@@ -485,13 +485,13 @@ __device__ __forceinline__ void cv_leave_counters(const CvParams &p, int lane) {
     if (lane == 0) *p.ended = 0;
 }
 
-template <int S, bool F32, int PPL, int WARPS>
+template <int S, bool F32, int PPL, int WARPS, int TR>
 __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
     cc_visit_kernel(const __grid_constant__ CvParams p, const __grid_constant__ TapCoeffs c) {
     using L = CcLane<S, F32, PPL>;
     constexpr int V = L::V, H = L::H, W = L::W, R = L::R;
     constexpr int PANELS = L::PANELS;
-    constexpr int ROWS = kCcTileRows / WARPS, PAIRS = ROWS / 2;  // of a warp
+    constexpr int ROWS = TR / WARPS, PAIRS = ROWS / 2;  // of a warp
     using T = typename L::T;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
@@ -514,9 +514,9 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
     for (int k = blockIdx.x; k < n_items; k += gridDim.x, phase ^= 1) {
         const int visit = k / n_tiles, tile = k - visit * n_tiles;
         const int ty = tile / p.tiles_x, tx = tile - ty * p.tiles_x;
-        const int Yb = ty * (kCcTileRows - 2 * p.halo);
+        const int Yb = ty * (TR - 2 * p.halo);
         const int chunk0 = tx * (PANELS - 2);  // first panel of the tile
-        const int rows = min(kCcRunRows, p.p.nyp - Yb);
+        const int rows = min(TR + 8, p.p.nyp - Yb);
         if (warp == 0) {
             bool ok = true;
             if (visit > 0) {
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
         if (threadIdx.x == 0) {
             T *out = static_cast<T *>(p.plane[(visit & 1) ^ 1]);
             const int top = ty == 0 ? 0 : p.halo;  // tile rows [top, bottom)
-            const int bottom = min(ty == p.tiles_y - 1 ? kCcTileRows : kCcTileRows - p.halo, rows - 4);
+            const int bottom = min(ty == p.tiles_y - 1 ? TR : TR - p.halo, rows - 4);
             const int q0 = tx == 0 ? 1 : 2;
             const int q1 = min(tx == p.tiles_x - 1 ? PANELS + 1 : PANELS, p.p.npan - chunk0);
             for (int q = q0; q < q1; q++)
@@ -655,15 +655,15 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
     if (!counted && warp == 0) cv_leave_counters(p, lane);
 }
 
-template <int S, bool F32, int PPL, int WARPS>
+template <int S, bool F32, int PPL, int WARPS, int TR>
 cudaError_t launch_cv(const CvParams &p, const TapCoeffs &c, int sms, cudaStream_t s) {
     static int per_sm = 0;
     if (!per_sm) {
-        cudaError_t e = cudaFuncSetAttribute(cc_visit_kernel<S, F32, PPL, WARPS>,
+        cudaError_t e = cudaFuncSetAttribute(cc_visit_kernel<S, F32, PPL, WARPS, TR>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, cv_smem<PPL>());
         int n = 0;
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, cc_visit_kernel<S, F32, PPL, WARPS>,
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, cc_visit_kernel<S, F32, PPL, WARPS, TR>,
                                                               WARPS * 32, cv_smem<PPL>());
         if (e != cudaSuccess) return e;
         if (n < 1) return cudaErrorInvalidConfiguration;
@@ -681,22 +681,24 @@ cudaError_t launch_cv(const CvParams &p, const TapCoeffs &c, int sms, cudaStream
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, cc_visit_kernel<S, F32, PPL, WARPS>, p, c);
+    return cudaLaunchKernelEx(&cfg, cc_visit_kernel<S, F32, PPL, WARPS, TR>, p, c);
 }
 
 template <int S, bool F32>
-cudaError_t dispatch_cv(int ppl, int warps, const CvParams &p, const TapCoeffs &c, int sms, cudaStream_t s) {
-    if (ppl == 2) return launch_cv<S, F32, 2, 8>(p, c, sms, s);
-    return warps == 16 ? launch_cv<S, F32, 1, 16>(p, c, sms, s) : launch_cv<S, F32, 1, 8>(p, c, sms, s);
+cudaError_t dispatch_cv(const CcVisitShape &v, const CvParams &p, const TapCoeffs &c, int sms, cudaStream_t s) {
+    if (v.ppl == 2) return launch_cv<S, F32, 2, 8, 128>(p, c, sms, s);
+    if (v.warps == 8) return launch_cv<S, F32, 1, 8, 128>(p, c, sms, s);
+    if (v.rows == 32) return launch_cv<S, F32, 1, 16, 32>(p, c, sms, s);
+    return v.rows == 64 ? launch_cv<S, F32, 1, 16, 64>(p, c, sms, s) : launch_cv<S, F32, 1, 16, 128>(p, c, sms, s);
 }
 template <bool F32>
-cudaError_t dispatch_cv(int stencil, int ppl, int warps, const CvParams &p, const TapCoeffs &c, int sms,
+cudaError_t dispatch_cv(int stencil, const CcVisitShape &v, const CvParams &p, const TapCoeffs &c, int sms,
                         cudaStream_t s) {
     switch (stencil) {
-    case TCS_STAR2D1R: return dispatch_cv<TCS_STAR2D1R, F32>(ppl, warps, p, c, sms, s);
-    case TCS_STAR2D2R: return dispatch_cv<TCS_STAR2D2R, F32>(ppl, warps, p, c, sms, s);
-    case TCS_BOX2D1R: return dispatch_cv<TCS_BOX2D1R, F32>(ppl, warps, p, c, sms, s);
-    case TCS_BOX2D2R: return dispatch_cv<TCS_BOX2D2R, F32>(ppl, warps, p, c, sms, s);
+    case TCS_STAR2D1R: return dispatch_cv<TCS_STAR2D1R, F32>(v, p, c, sms, s);
+    case TCS_STAR2D2R: return dispatch_cv<TCS_STAR2D2R, F32>(v, p, c, sms, s);
+    case TCS_BOX2D1R: return dispatch_cv<TCS_BOX2D1R, F32>(v, p, c, sms, s);
+    case TCS_BOX2D2R: return dispatch_cv<TCS_BOX2D2R, F32>(v, p, c, sms, s);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -746,12 +748,19 @@ cudaError_t launch_cc_f32(const GridGeom &g, int stencil, const TapCoeffs &c, co
 }
 
 // The form of a sweep's visits by its tiles per SM (n, of half-panel-lane
-// tiles).  Few tiles: sixteen warps each, so that a step's row sequence is
-// short (FP16 with halo 8, more steps per visit); a few per SM: eight warps,
+// tiles).  Few tiles: sixteen warps each (FP16 with halo 8, more steps per
+// visit), and on grids below about a wave of them tiles of 64 or 32 rows, as
+// a step takes an SM as long as its rows have instructions; a few per SM: eight warps,
 // two or three CTAs per SM; many: whole-panel lanes, which spend fewer
 // instructions per cell on halo words and overlap tiles by less.  With many
 // tiles the radius-2 boxes (25 taps, bound by their FMAs, of which a visit's
 // overlap computes a fifth twice) are faster in single steps: visits = 0.
+// us per step of 128 / 64 / 32 rows: FP16 star2d1r 256² 1.54 / 1.09 / 0.89,
+// box2d2r 3.63 / 2.29 / 1.54; 700² (n = 0.9 of 64 rows, 2.0 of 32) 1.59 / 1.12 /
+// 1.12, 3.68 / 2.35 / 2.76; 1026² (1.45 of 64) 1.63 / 1.54, 1500² (2.9) 1.96 /
+// 2.71; FP32 star2d1r 256² 1.43 / 1.13 / 0.96, 512² (1.25 of 32) 1.48 / 1.14 /
+// 1.09, 700² (1.1 of 64) 1.43 / 1.28, 800² (1.5) 1.45 / 1.59.  (Thirty-two warps
+// instead of sixteen: 256² 1.55 -> 1.91.)
 // Measured on GB300, us per step, one step per launch -> 16 warps / 8 warps /
 // whole panels (FP16 halo 8 / 4 / 4; FP32 4):
 //   FP16 star2d1r  700² 6.09 -> 1.56 / 1.95 / 3.38, 2048² 6.76 -> 3.48 / 3.32
@@ -770,17 +779,20 @@ CcVisitShape cc_visit_shape(const GridGeom &g, int stencil, bool f32, int steps,
     const int r = stencil_r(stencil);
     const bool box2 = stencil == TCS_BOX2D2R;
     const int cpp = f32 ? 4 : 8, nchunks = (g.nx + cpp - 1) / cpp;
-    auto shape = [&](int ppl, int warps, int halo) {
-        const int panels = 16 * ppl, rows = kCcTileRows - 2 * halo;
+    auto shape = [&](int ppl, int warps, int halo, int tile_rows = kCcTileRows) {
+        const int panels = 16 * ppl, rows = tile_rows - 2 * halo;
+        v.rows = tile_rows;
         v.ppl = ppl;
         v.warps = warps;
         v.halo = halo;
         v.tiles_x = nchunks <= panels ? 1 : (nchunks - 2 + panels - 3) / (panels - 2);
-        v.tiles_y = g.ny <= kCcTileRows ? 1 : (g.ny - 2 * halo + rows - 1) / rows;
+        v.tiles_y = g.ny <= tile_rows ? 1 : (g.ny - 2 * halo + rows - 1) / rows;
         const int depth = halo / r + 1;
         v.visits = (steps + depth - 1) / depth;
         return (double)v.tiles_x * v.tiles_y / sms;
     };
+    if (shape(1, 16, f32 ? 4 : 8, 32) <= (f32 ? 1.25 : 1.05)) return v;
+    if (shape(1, 16, f32 ? 4 : 8, 64) <= (f32 ? 1.2 : 1.5)) return v;
     if (f32) {
         const double n = shape(1, 8, 4);
         if (n <= 1.4) {
@@ -804,10 +816,9 @@ CcVisitShape cc_visit_shape(const GridGeom &g, int stencil, bool f32, int steps,
 cudaError_t cc_visit_prepare(int stencil, bool f32) {
     CvParams p{};
     const TapCoeffs c{};
-    for (int form = 0; form < 3; form++) {
-        const int ppl = form == 2 ? 2 : 1, warps = form == 1 ? 16 : 8;
-        const cudaError_t e = f32 ? dispatch_cv<true>(stencil, ppl, warps, p, c, 1, nullptr)
-                                  : dispatch_cv<false>(stencil, ppl, warps, p, c, 1, nullptr);
+    for (const CcVisitShape &v : {CcVisitShape{1, 8, 128}, CcVisitShape{1, 16, 128}, CcVisitShape{1, 16, 64}, CcVisitShape{1, 16, 32}, CcVisitShape{2, 8, 128}}) {
+        const cudaError_t e = f32 ? dispatch_cv<true>(stencil, v, p, c, 1, nullptr)
+                                  : dispatch_cv<false>(stencil, v, p, c, 1, nullptr);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -831,8 +842,8 @@ cudaError_t launch_cc_visits(const GridGeom &g, int stencil, bool f32, const Tap
     p.plane[1] = out;
     p.ended = counters;
     p.done = counters + kRowCounterStride;
-    return f32 ? dispatch_cv<true>(stencil, v.ppl, v.warps, p, c, sms, s)
-               : dispatch_cv<false>(stencil, v.ppl, v.warps, p, c, sms, s);
+    return f32 ? dispatch_cv<true>(stencil, v, p, c, sms, s)
+               : dispatch_cv<false>(stencil, v, p, c, sms, s);
 }
 
 cudaError_t cc_error_word(int **word) {

@@ -161,7 +161,7 @@ cudaError_t launch_cc_f32(const GridGeom &g, int stencil, const TapCoeffs &c, co
 // one flip per visit; visits = 0: single steps are faster); counters:
 // cc_visit_counter_words of zeros, which a launch leaves zero again.
 struct CcVisitShape {
-    int ppl, warps, halo, tiles_x, tiles_y, visits;
+    int ppl, warps, rows, halo, tiles_x, tiles_y, visits;
 };
 CcVisitShape cc_visit_shape(const GridGeom &g, int stencil, bool f32, int steps, int sms);
 cudaError_t cc_visit_prepare(int stencil, bool f32);
@@ -204,7 +204,8 @@ constexpr size_t visit_counter_words(int ny, int nx) {
     return kRowCounterStride + (size_t)(ny / (kTile - 16) + 2) * ((nx + 31) / 32);
 }
 constexpr size_t cc_visit_counter_words(int ny, int nx) {
-    return kRowCounterStride + (size_t)(ny / (kTile - 16) + 2) * (nx / 56 + 2);
+    // 128-row tiles, or 64-row ones where there are fewer of them than SMs
+    return kRowCounterStride + (size_t)(ny / (kTile - 16) + 2) * (nx / 56 + 2) + 1024;
 }
 cudaError_t visit_prepare(int stencil);
 cudaError_t launch_tc_f16_visits(const GridGeom &g, int stencil, const float *B, uint16_t *in,

@@ -1,8 +1,9 @@
 """CUDA-core steps taken several per tile visit (the one-launch form of larger
 grids) against one launch per step: each cell is computed by itself in the same
 order, so the same bits, also with infinities and NaN, in every form the size
-rule takes (few, some and many tiles per SM, FP16 and FP32), at tile edges
-(rows 112, 120, 128; columns 112, 240 FP16 and 56, 120 FP32), with update
+rule takes (few, some and many tiles per SM of 32, 64 and 128 rows, FP16 and
+FP32), at tile edges (rows 16, 24, 48, 56, 112, 120, 128; columns 112, 240 FP16
+and 56, 120 FP32), with update
 rectangles and over repeated runs; FP32 storage also against gold."""
 import zlib
 
@@ -44,7 +45,8 @@ def _case(stencil, shape):
 
 @pytest.mark.parametrize("prec", ["f16", "f32"])
 @pytest.mark.parametrize("stencil", STENCILS)
-@pytest.mark.parametrize("shape", [(129, 800), (241, 649), (361, 561), (8, 1300), (1400, 9), (249, 728), (505, 513), (64, 70)])
+@pytest.mark.parametrize("shape", [(129, 800), (241, 649), (361, 561), (8, 1300), (1400, 9), (249, 728), (505, 513), (64, 70),
+                                   (33, 129), (49, 241), (177, 340), (225, 121), (529, 700), (611, 130), (729, 64)])
 @pytest.mark.parametrize("runs", [(2, 11), (11, 4, 12)])
 def test_visits_equal_single_steps(tcs, torch_cuda, stencil, prec, shape, runs):
     A, B = _case(stencil, shape)
