@@ -45,6 +45,9 @@
 // one infinity or NaN makes every output of its windows in the reaching rows
 // NaN, here as in single steps; which further cells it reaches over several
 // steps depends on the visit's halo.
+#include <algorithm>
+#include <cmath>
+
 #include "tc_core.cuh"
 #include "tile_walk.h"
 
@@ -548,17 +551,21 @@ cudaError_t prepare_visit() {
 
 }  // namespace
 
-// The tile width and halo of a sweep, from a model of a step's SM cycles that
-// was fitted to sweeps of 128² to 16386² (M: a tile's MMAs; L: from the last
-// MMA of a step to the slot's next one; B: from a visit's last step to the
-// next visit's first MMA; n tiles per SM):
-//   step = max(n M, M + L, n (M + L) / 2),  visit = T step + B (2 B / n, n > 2)
+// The tile width and halo of a sweep, from a model of its SM cycles that was
+// fitted to 2640 sweeps of 256² to 4096² in 2 to 64 steps (M: a tile's MMAs; L:
+// from the last MMA of a step to the slot's next one; n tiles per SM; I: the
+// visits a CTA makes, between their average and that of the CTAs with one tile
+// more, as neighbours wait for one another):
+//   one tile after another:  visits (T (M + L) + 3417)
+//   two slots at a time:     I (T max(M, 0.575 (M + L)) + 243)
+// of which the larger.
 // Narrow tiles have short steps and more SMs, wide ones fewer MMAs per cell;
 // halo 8 takes more steps per visit, halo 4 fewer rows twice, and halo 2
 // (whose copies move half lines) pays only for radius 2 with many tiles,
-// where T = 2 already takes the sweep off the memory bound.  The model's
-// choice measured within 3 % of the best of W = 32, 64, 96, 128 with every
-// halo at all but one of 30 grids (6 % at 1026², 10 steps, box2d2r); box2d2r,
+// where T = 2 already takes the sweep off the memory bound.  Over the sweeps
+// above the choice costs 1.1 % over the best of W = 32, 64, 96, 128 with every
+// halo, 15 % at most (a model of n without I, fitted to runs of many steps: 3.2
+// %, and 31 %: 1300² box2d2r 4 steps 17.0 us, 12.9 now).  box2d2r,
 // us per step, W 32 / 64 / 96 / 128: 256² 1.47 / 1.90 / 2.34 / 2.88, 1026²
 // 1.70 / 2.13 / 2.36 / 2.82, 2048² 4.05 / 3.08 / 3.15 / 3.41, 8196² - / - /
 // 40.0 / 40.7.  The best form against one launch per step (radius 1 star /
@@ -582,15 +589,14 @@ VisitShape visit_shape(int ny, int nx, int stencil, int steps, int tile_w, int s
             const int by_rows = halo / r + 1, by_cols = 8 / r;
             const int depth = by_rows < by_cols ? by_rows : by_cols;
             v.visits = (steps + depth - 1) / depth;
-            double n = (double)v.tiles_x * v.tiles_y / sms;
-            if (n < 1.0) n = 1.0;
+            const double n = (double)v.tiles_x * v.tiles_y / sms;
             if (halo == 2 && (r == 1 || n <= 4.0)) continue;
-            const double per_mma = r == 1 ? 66.0 : w == 96 ? 61.0 : 64.0;
-            const double m = per_mma * (w / 16 + 1) * (2 * r + 1), l = 800.0 + 9.0 * w;
-            double step = n * m;
-            if (step < m + l) step = m + l;
-            if (step < n * (m + l) / 2) step = n * (m + l) / 2;
-            const double cost = steps * step + v.visits * 4750.0 * (n > 2.0 ? 2.0 / n : 1.0);
+            const double t = (double)steps / v.visits;
+            const double m = 61.7 * (w / 16 + 1) * (2 * r + 1) - 50.0, l = 586.0 + 8.0 * w;
+            const double per_cta = std::max(std::ceil(v.visits * n), v.visits * (n + 0.42 * (std::ceil(n) - n)));
+            const double chain = v.visits * (t * (m + l) + 3417.0);
+            const double slots = per_cta * (t * std::max(m, 0.575 * (m + l)) + 243.0);
+            const double cost = std::max(chain, slots);
             if (!best.visits || cost < best_cost) {
                 best = v;
                 best_cost = cost;
