@@ -24,7 +24,7 @@ INCLUDE = os.path.join(ROOT, "include")
 OUT = os.path.join(PKG, "_build")
 
 CU_SOURCES = ["layout.cu", "sweep_cc.cu", "sweep_tc.cu", "sweep_visit.cu", "api.cu", "sweep_noalloc.cu", "batch.cu", "server.cu", "sweep_tb.cu", "drift.cu", "memory.cu"]
-HEADERS = ["tcs_device.cuh", "tcs_internal.h", "tc_core.cuh", "batch.h", "tile_walk.h"]
+HEADERS = ["tcs_device.cuh", "tcs_internal.h", "tc_core.cuh", "batch.h", "tile_walk.h", "visit_tile.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-Wall",
                      "--expt-relaxed-constexpr", "-I", INCLUDE]

@@ -1,31 +1,41 @@
 // Batched sweeps: many grids of different sizes, stencils, coefficients,
 // precisions (FP16 or split) and step counts advanced by ONE persistent
-// tensor-core launch.
+// tensor-core launch per precision.
 //
-// Work list.  Every (grid, step, tile) is one item; items are ordered step
-// major (all grids' first steps, then all second steps, ...) and decoded from
+// Work list.  Every (grid, turn, tile) is one item: a turn is a split step, or
+// an FP16 visit of up to five (radius 1) or three steps taken on the tile in
+// shared memory (sweep_visit.cu; batch.h).  Items are ordered turn major (all
+// grids' first turns, then all second turns, ...) and decoded from
 // their index on the device (BatchParams), so a run's description is a few
 // small tables however many items it has.  Each CTA (one per SM) takes the
 // next index from a global counter, so items are taken in order, and only by
-// running CTAs.  An item of step t > 0 needs every
-// tile of its grid's step t - 1: the producer waits (bounded) on a
-// per-(grid, step) completion counter that the epilogue warps increment after
-// their stores (release reductions, one per run of consecutive items of the
-// same grid and step; the producer polls with acquire loads, once per run of
-// items of the same grid and step).  Those items come earlier in the list and
+// running CTAs.  An item of turn t > 0 needs every
+// tile of its grid's turn t - 1: the producer waits (bounded) on a
+// per-(grid, turn) completion counter that is added to after the epilogue
+// warps' stores (release reductions, one per run of consecutive items of the
+// same grid and turn; the producer polls with acquire loads, once per run of
+// items of the same grid and turn).  Those items come earlier in the list and
 // so were taken by
 // running CTAs; the earliest unfinished item always has its inputs ready, so
 // the launch cannot deadlock, whatever else shares the GPU.
-// The same counters also guard the ping-pong's write-after-read hazard: step
-// t+1 overwrites the plane step t-1 read, and starts only after all of step t,
-// hence all of step t-1, finished.
+// The same counters also guard the ping-pong's write-after-read hazard: turn
+// t+1 overwrites the plane turn t-1 read, and starts only after all of turn t,
+// hence all of turn t-1, finished.
+//
+// What a turn costs besides its tiles is the way from its last store to the
+// next load, 2 us, and a load and a store, so FP16 grids take several steps
+// between: 256 mixed FP16 grids 2.08 -> 1.50 ms, 256 of 512², 10 steps, 477 ->
+// 336 us (box2d1r) and 497 -> 492 (box2d2r, bound by its MMAs either way),
+// and 256 of 124² 75 -> 41.  (Two split steps per item, as sweep_tb.cu:
+// 8196² 112 -> 86 us per step, but 256 mixed split grids 5.42 -> 5.95 ms: tiles
+// of 124 rows are more of them, and an item's 96 registers spill or reload.)
 //
 // Per item the producer loads the tile's input panels (one tensor-map load per
 // plane, from the grid's maps in device memory) AND bulk-copies the grid's
 // coefficient bands (prebuilt in global memory by build_bands_kernel) into the
 // stage, so the MMA issuers need nothing else; stencil radius and precision
 // select one of four fully unrolled MMA sequences (tc_core.cuh), the same code
-// the single-grid kernel runs, so every grid gets the same bits alone and in
+// the single-grid kernels run, so every grid gets the same bits alone and in
 // a batch.  The run ends with a tiny kernel that flips each grid's ping-pong
 // state, so a captured graph can be replayed to advance the batch again.
 #include <algorithm>
@@ -36,6 +46,7 @@
 
 #include "batch.h"
 #include "tc_core.cuh"
+#include "visit_tile.cuh"
 
 namespace tcs {
 
@@ -46,16 +57,17 @@ using SG = StageLines;  // line-aligned staging, as the single-grid kernels
 
 __device__ int g_batch_error = 0;
 
-// Per-precision launch shapes.  FP16 items: three stages of one plane plus
-// bands, two accumulator slots, eight epilogue warps (the single-grid plain
-// kernel's shape).  Split items: two stages of hi+lo plus bands, the window
-// ring of the single-grid split kernel, twelve epilogue warps in three groups.
+// Per-precision launch shapes.  FP16 items (visits): four stages of one plane
+// plus bands, two accumulator slots, each with its own issuer and eight
+// epilogue warps (the single-grid visit kernel's shape).  Split items: two
+// stages of hi+lo plus bands, the window ring of the single-grid split kernel,
+// twelve epilogue warps in three groups.
 constexpr int kRing = 8;  // published work items in flight
 // The work layout (step offsets, tile prefix) is copied into shared memory
 // when it fits, so decoding an item costs no global round trip.
 constexpr int kTableInts = 2048;
-// barriers, the item ring and the per-slot scale words, before the tables
-constexpr int kBarrierArea = 832;
+// barriers, the item ring, the per-slot words and the masks, before the tables
+constexpr int kBarrierArea = 2048;
 template <bool SPLIT>
 struct BatchCfg {
     // FP16: four stages, a multiple of the two issuers, so stage i % 4 holds
@@ -64,14 +76,16 @@ struct BatchCfg {
     static constexpr int PLANES = SPLIT ? 2 : 1;
     static constexpr int BAND_BYTES = (SPLIT ? 4 : 1) * 5 * kBandBytes;  // radius 2
     static constexpr int STAGE_BYTES = PLANES * SG::PLANE + BAND_BYTES;
-    static constexpr int GROUPS = SPLIT ? 3 : 2;
+    static constexpr int GROUPS = SPLIT ? 3 : 4;
     static constexpr int EPI_WARPS = 4 * GROUPS;
-    // MMA issuer warps 1 and 2 (one issues while the other waits on a region
-    // or slot, or commits): split items alternate windows between them, FP16
-    // items alternate whole items
+    static constexpr int ITEM_WARPS = SPLIT ? EPI_WARPS : EPI_WARPS / 2;  // that take one item
+    // MMA issuer warps 1 and 2: split items alternate windows between them
+    // (one issues while the other waits on a region, or commits), FP16 items
+    // alternate whole items
     static constexpr int ISSUERS = 2;
-    // commits that free a stage: both issuers' (split), the item's issuer's (FP16)
-    static constexpr int STAGE_RELEASES = SPLIT ? 2 : 1;
+    // what frees a stage: both issuers' commits (split), the item's epilogue
+    // warps (FP16)
+    static constexpr int STAGE_RELEASES = SPLIT ? 2 : ITEM_WARPS;
     static constexpr int EPI_WARP0 = 1 + ISSUERS;
     static constexpr int SIGNAL_WARP = EPI_WARP0 + EPI_WARPS;
     static constexpr int THREADS = 32 * (SIGNAL_WARP + 1);
@@ -80,6 +94,7 @@ struct BatchCfg {
     static_assert(SMEM <= 232448, "shared memory budget");
     static_assert(STAGE_BYTES % 16 == 0, "bulk copy alignment");
 };
+constexpr int kBatchSlotCols = 256;  // FP16: TMEM columns per slot (160 used)
 constexpr int kBatchRingSlots = 5;  // split window regions in TMEM
 constexpr int kBatchRegion = 96;
 
@@ -94,15 +109,15 @@ __device__ __forceinline__ void batch_fail(const BatchParams &p, int code) {
 
 // Work index k -> (grid, step, tile) from the step offsets and tile prefix
 // (shared or global memory); see BatchParams.
-__device__ __forceinline__ BatchItem decode_item(const int *step_off, const int *tile_prefix,
-                                                 int n_steps, int n_grids, int k) {
-    int lo = 0, hi = n_steps;  // step_off[lo] <= k < step_off[hi]
+__device__ __forceinline__ BatchItem decode_item(const int *turn_off, const int *tile_prefix,
+                                                 int n_turns, int n_grids, int k) {
+    int lo = 0, hi = n_turns;  // turn_off[lo] <= k < turn_off[hi]
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (step_off[mid] <= k) lo = mid;
+        if (turn_off[mid] <= k) lo = mid;
         else hi = mid;
     }
-    const int local = k - step_off[lo];
+    const int local = k - turn_off[lo];
     int a = 0, b = n_grids;  // tile_prefix[a] <= local < tile_prefix[b]
     while (b - a > 1) {
         const int mid = (a + b) >> 1;
@@ -115,10 +130,10 @@ __device__ __forceinline__ BatchItem decode_item(const int *step_off, const int 
 // The item after `it` (index k + 1), from two table reads: the next tile of
 // the grid, else the first tile of the next grid still running at this step,
 // else the first tile of the next step.
-__device__ __forceinline__ BatchItem next_item(const BatchItem &it, const int *step_off,
+__device__ __forceinline__ BatchItem next_item(const BatchItem &it, const int *turn_off,
                                                const int *tile_prefix) {
     const int local = tile_prefix[it.g] + it.tile + 1;  // within step it.t
-    if (local < step_off[it.t + 1] - step_off[it.t]) {
+    if (local < turn_off[it.t + 1] - turn_off[it.t]) {
         if (local < tile_prefix[it.g + 1]) return BatchItem{it.g, it.t, it.tile + 1};
         return BatchItem{it.g + 1, it.t, 0};
     }
@@ -141,7 +156,7 @@ __global__ void build_one_band_kernel(const BandArgs a, int r, int box, int spli
 
 __global__ void flip_states_kernel(BatchGrid *grids, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) grids[i].state ^= grids[i].steps & 1;
+    if (i < n) grids[i].state ^= grids[i].turns & 1;
 }
 
 template <bool SPLIT>
@@ -152,7 +167,8 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
     uint8_t *smem = align_smem(smem_raw);
     uint8_t *stage_base = smem;  // [NS][planes | bands]
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)NS * C::STAGE_BYTES);
-    // accumulator barriers: plain [2] slots, split [kBatchRingSlots] windows
+    // accumulator barriers: FP16 [2] slots (a step's MMAs complete; its results
+    // in the image), split [kBatchRingSlots] windows (complete; read)
     constexpr int NACC = SPLIT ? kBatchRingSlots : 2;
     uint64_t *full = bars;                        // [NS]
     uint64_t *empty = bars + NS;                  // [NS]
@@ -171,12 +187,15 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
     uint64_t *item_scaled = reinterpret_cast<uint64_t *>(tmem_slot + 2);  // [kRing]
     ItemScale *ring_scale = reinterpret_cast<ItemScale *>(item_scaled + kRing);  // [kRing]
     unsigned *item_max = reinterpret_cast<unsigned *>(ring_scale + kRing);       // [kRing]
+    // FP16: per ring slot, the item's grid; the mask table
+    constexpr int kVisitAt = ((2 * NS + 2 * NACC + 1 + 4 * kRing) * 8 + 8 +
+                              kRing * (int)(sizeof(BatchItem) + sizeof(ItemScale) + 4) + 15) / 16 * 16;
+    VisitItem *ring_visit = reinterpret_cast<VisitItem *>(reinterpret_cast<uint8_t *>(bars) + kVisitAt);  // [kRing]
+    uint32_t *masks = reinterpret_cast<uint32_t *>(ring_visit + kRing);
     volatile int *grid_error = p.error;
-    static_assert((2 * NS + 2 * NACC + 1 + 3 * kRing) * 8 + kRing * sizeof(BatchItem) + 8 +
-                          kRing * (8 + sizeof(ItemScale) + 4) <= kBarrierArea,
-                  "barrier area");
+    static_assert(kVisitAt + kRing * sizeof(VisitItem) + kMaskBytes <= kBarrierArea, "barrier area");
     int *tables = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(bars) + kBarrierArea);
-    const int n_table = p.n_steps + 1 + p.n_grids + 1;
+    const int n_table = p.n_turns + 1 + p.n_grids + 1;
     const bool tables_in_smem = n_table <= kTableInts;
 
     const int warp = threadIdx.x >> 5;
@@ -191,12 +210,12 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
         }
         for (int b = 0; b < NACC; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], C::EPI_WARPS);
+            mbar_init(&acc_empty[b], C::ITEM_WARPS);
         }
         mbar_init(drain, C::ISSUERS);
         for (int j = 0; j < kRing; j++) {
             mbar_init(&item_ready[j], 1);
-            mbar_init(&item_done[j], C::EPI_WARPS);
+            mbar_init(&item_done[j], C::ITEM_WARPS);
             mbar_init(&ring_free[j], 1);
             mbar_init(&item_scaled[j], 1);
             item_max[j] = 0u;
@@ -209,10 +228,11 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
         tmem_alloc(tmem_slot, kTmemCols);
         tmem_relinquish();
     }
+    if (!SPLIT) build_masks(masks, threadIdx.x);
     if (tables_in_smem) {
-        for (int i = threadIdx.x; i <= p.n_steps; i += blockDim.x) tables[i] = p.step_off[i];
+        for (int i = threadIdx.x; i <= p.n_turns; i += blockDim.x) tables[i] = p.turn_off[i];
         for (int i = threadIdx.x; i <= p.n_grids; i += blockDim.x)
-            tables[p.n_steps + 1 + i] = p.tile_prefix[i];
+            tables[p.n_turns + 1 + i] = p.tile_prefix[i];
     }
     tc_fence_before();
     __syncthreads();
@@ -229,8 +249,8 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
         // group, the group after the next one requested), so those latencies
         // overlap the stage and ring waits of the next iteration.
         if (lane == 0) {
-            const int *step_off = tables_in_smem ? tables : p.step_off;
-            const int *tile_prefix = tables_in_smem ? tables + p.n_steps + 1 : p.tile_prefix;
+            const int *turn_off = tables_in_smem ? tables : p.turn_off;
+            const int *tile_prefix = tables_in_smem ? tables + p.n_turns + 1 : p.tile_prefix;
             int last_issued = -1;
             // (grid, step) whose dependency this thread has already seen met;
             // later items of the same pair need no further poll or fence
@@ -265,7 +285,7 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
             BatchItem it{};
             BatchGrid g{};
             if (k < p.n_items) {
-                it = decode_item(step_off, tile_prefix, p.n_steps, p.n_grids, k);
+                it = decode_item(turn_off, tile_prefix, p.n_turns, p.n_grids, k);
                 g = p.grids[it.g];
                 k_next = (int)atomicAdd(p.work_counter, (unsigned)grab);
             }
@@ -286,17 +306,30 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                 // the tile's row and column, once, for every role
                 it.ty = it.tile / g.tiles_x;
                 it.tx = it.tile - it.ty * g.tiles_x;
+                const int in = (g.state + it.t) & 1;
                 ring[j] = it;
+                if constexpr (!SPLIT) {
+                    VisitItem &q = ring_visit[j];
+                    q.out = in ? g.plane[0][0] : g.plane[1][0];
+                    q.pg = g.pg;
+                    q.ny = g.ny; q.nx = g.nx;
+                    q.y0 = g.y0; q.y1 = g.y1; q.x0 = g.x0; q.x1 = g.x1;
+                    q.r = g.r;
+                    const int base = g.steps / g.turns;
+                    q.steps = base + (it.t < g.steps - base * g.turns ? 1 : 0);
+                    q.nwin = tile_windows(g.nx, it.tx * kTile);
+                    q.bottom = it.ty == g.tiles_y - 1;
+                }
                 mbar_arrive(&item_ready[j]);
-                // step t > 0: every tile of the grid's previous step is stored;
-                // step 0 of a gated grid: the external gate is open
+                // turn t > 0: every tile of the grid's previous turn is stored;
+                // turn 0 of a gated grid: the external gate is open
                 const unsigned *ctr = nullptr;
                 unsigned target = 0;
                 if (it.g == met_g && it.t == met_t) {
                     // met before, and the proxy fence after that poll still orders the copies below
                 } else if (it.t > 0) {
                     ctr = p.counters + (size_t)(g.ctr_base + it.t - 1) * kRowCounterStride;
-                    target = (unsigned)(g.n_tiles * C::EPI_WARPS);
+                    target = (unsigned)(g.n_tiles * C::ITEM_WARPS);
                 } else if (g.gate) {
                     ctr = g.gate;
                     target = g.gate_value;
@@ -332,9 +365,9 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                 const int band_bytes = batch_band_elems(g.r, SPLIT) * 2;
                 uint8_t *st = stage_base + (size_t)s * C::STAGE_BYTES;
                 mbar_arrive_expect_tx(&full[s], C::PLANES * SG::PLANE + band_bytes);
-                const int in = (g.state + it.t) & 1;
                 const CUtensorMap *maps = g.maps + 2 * in;
-                load_tile_map(maps, maps + 1, C::PLANES, it.ty * kTile, it.tx * kTile, st, &full[s]);
+                load_tile_map(maps, maps + 1, C::PLANES, it.ty * (SPLIT ? kTile : kBatchRows), it.tx * kTile, st,
+                              &full[s]);
                 bulk_load(st + C::PLANES * SG::PLANE, p.bands + g.band_base, band_bytes, &full[s]);
                 if (SPLIT) {
                     pub_j = j;
@@ -356,11 +389,11 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                     k = k_next;
                     k_end = k + grab;
                     if (k < p.n_items) {
-                        it = decode_item(step_off, tile_prefix, p.n_steps, p.n_grids, k);
+                        it = decode_item(turn_off, tile_prefix, p.n_turns, p.n_grids, k);
                         k_next = (int)atomicAdd(p.work_counter, (unsigned)grab);
                     }
                 } else if (k < p.n_items) {
-                    it = next_item(it, step_off, tile_prefix);
+                    it = next_item(it, turn_off, tile_prefix);
                 }
                 if (k < p.n_items) {
                     if (it.g != g_prev) g = p.grids[it.g];
@@ -384,17 +417,18 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
         // --------------------------------------------------- MMA issuers ---
         // Both issuers read every published item, in order (the slot sequence
         // and the stop sentinel).  Split: both wait for every stage fill and
-        // issue alternate windows.  FP16: item i's issuer is i % 2 and it alone
-        // waits for the item's stage: with four stages a stage only holds one
-        // issuer's items, so each stage's fills are waited for by one thread in
-        // order (an mbarrier parity wait also succeeds for the phase before the
-        // current one, so a thread must never skip a fill it later waits past).
+        // issue alternate windows.  FP16: item i's issuer and accumulator slot
+        // are i % 2, and it alone waits for the item's stage: with four stages
+        // a stage only holds one issuer's items, so each stage's fills are
+        // waited for by one thread in order (an mbarrier parity wait also
+        // succeeds for the phase before the current one, so a thread must
+        // never skip a fill it later waits past).
         // A ring slot is republished only after the signal warp finished its
         // item, which needs a lagging issuer's own earlier item, so neither
         // issuer can be lapped on the ring.
         if (lane == 0) {
             const int id = warp - 1;  // split: windows G % 2 == id; FP16: items i % 2 == id
-            AccSlots slots;  // FP16: walks every item, so both see the same slot uses
+            uint32_t e = 0;  // FP16: the slot's steps so far
             int G = 0;       // split: global window counter of the ring
             bool stop = false;
             for (int i = 0; !stop; i++) {
@@ -406,24 +440,17 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                 }
                 const BatchItem it = ring[i % kRing];
                 if (it.g < 0) break;
-                uint32_t col = 0, mask = 0;
-                if constexpr (!SPLIT) {
-                    mask = slots.take(false, col);
-                    if ((i & 1) != id) {
-                        slots.used(mask);
-                        continue;
-                    }
-                }
+                if (!SPLIT && (i & 1) != id) continue;
                 if (!mbar_wait(&full[s], (i / NS) & 1, abort_flag, wait_lim)) {
                     batch_fail(p, kErrWaitFull);
                     *abort_flag = 1;
                     break;
                 }
-                const BatchGrid g = p.grids[it.g];  // one batch of loads, before any barrier
                 uint8_t *st = stage_base + (size_t)s * C::STAGE_BYTES;
                 const uint64_t a_hi0 = smem_desc(smem_u32(st), SG::CHUNK, 128);
                 const uint32_t band = smem_u32(st + C::PLANES * SG::PLANE);
                 if constexpr (SPLIT) {
+                    const BatchGrid g = p.grids[it.g];  // one batch of loads, before any barrier
                     const int nwin = tile_windows(g.nx, it.tx * kTile);
 #pragma unroll 1
                     for (int w = 0; w < nwin; w++, G++) {
@@ -442,22 +469,25 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                         umma_commit(&acc_full[r]);
                     }
                 } else {
-                    if (!slots.acquire(acc_empty, mask, abort_flag, wait_lim)) {
-                        batch_fail(p, kErrWaitAccum);
-                        *abort_flag = 1;
-                        stop = true;
-                    } else {
+                    const int r = ring_visit[i % kRing].r, T = ring_visit[i % kRing].steps;
+                    const int nwin = ring_visit[i % kRing].nwin;
+                    const uint32_t d = tmem_base + (uint32_t)(id * kBatchSlotCols);
+                    for (int t = 0; t < T; t++, e++) {
+                        // the slot's previous step has been read out (and,
+                        // within a visit, written to the image)
+                        if (e > 0 && !mbar_wait_soon(&acc_empty[id], (e - 1) & 1, abort_flag, wait_lim)) {
+                            batch_fail(p, kErrWaitAccum);
+                            *abort_flag = 1;
+                            stop = true;
+                            break;
+                        }
                         tc_fence_after();
-                        const uint32_t d = tmem_base + col;
-                        // all windows: FP16 items are bound by the producer, and a
-                        // second MMA sequence for edge tiles measured slower
-                        if (g.r == 1) issue_plain_windows<1, SG>(a_hi0, band, d);
-                        else issue_plain_windows<2, SG>(a_hi0, band, d);
-                        slots.commit(acc_full, mask);
-                        slots.used(mask);
+                        if (r == 1) issue_visit_tile<1, kTile / 16 + 1>(a_hi0, band, d, nwin);
+                        else issue_visit_tile<2, kTile / 16 + 1>(a_hi0, band, d, nwin);
+                        umma_commit(&acc_full[id]);
                     }
                 }
-                if (!stop) umma_commit(&empty[s]);
+                if (SPLIT && !stop) umma_commit(&empty[s]);
             }
             // every issuer commits (one with nothing in flight completes at
             // once), so the drain phase always completes
@@ -532,16 +562,18 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                 }
                 mbar_arrive(&ring_free[j]);
                 pend = ctr;
-                n_pend += C::EPI_WARPS;
+                n_pend += C::ITEM_WARPS;
             }
             if (n_pend) release();
         }
     } else {
         // ------------------------------------------------------ epilogue ---
         const int q = warp & 3;
-        const int grp = (warp - C::EPI_WARP0) >> 2;  // plain: column half; split: block group
+        // split: block group; FP16: slot and column half
+        const int grp = (warp - C::EPI_WARP0) >> 2;
+        const int slot = grp >> 1, half = grp & 1;
         const int m = q * 32 + lane;
-        AccSlots slots;
+        uint32_t e = 0;  // FP16: the slot's steps so far
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
         int G0 = 0;  // split: first ring window of the item
         bool stop = false;
@@ -561,24 +593,24 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
             }
             const BatchItem it = ring[j];
             if (it.g < 0) break;
-            const BatchGrid g = p.grids[it.g];  // one batch of loads, before any barrier
-            const int in = (g.state + it.t) & 1;
-            TileOut o;
-            // (selects, not a runtime index, keep the descriptor in registers)
-            o.in_hi = in ? g.plane[1][0] : g.plane[0][0];
-            o.in_lo = in ? g.plane[1][1] : g.plane[0][1];
-            o.out_hi = in ? g.plane[0][0] : g.plane[1][0];
-            o.out_lo = in ? g.plane[0][1] : g.plane[1][1];
-            o.pg = g.pg;
-            o.y0 = g.y0; o.y1 = g.y1; o.x0 = g.x0; o.x1 = g.x1;
-            o.ny = g.ny; o.nx = g.nx;
-            const int Y0 = it.ty * kTile;
-            const int X0 = it.tx * kTile;
-            // this warp's 32 rows all lie in the plane's padding below the grid:
-            // nothing of them to load or store (padding only has to stay finite,
-            // and it does: it keeps what it holds)
-            const bool rows_out = Y0 + 32 * q >= g.ny;
             if constexpr (SPLIT) {
+                const BatchGrid g = p.grids[it.g];  // one batch of loads, before any barrier
+                const int in = (g.state + it.t) & 1;
+                TileOut o;
+                // (selects, not a runtime index, keep the descriptor in registers)
+                o.in_hi = in ? g.plane[1][0] : g.plane[0][0];
+                o.in_lo = in ? g.plane[1][1] : g.plane[0][1];
+                o.out_hi = in ? g.plane[0][0] : g.plane[1][0];
+                o.out_lo = in ? g.plane[0][1] : g.plane[1][1];
+                o.pg = g.pg;
+                o.y0 = g.y0; o.y1 = g.y1; o.x0 = g.x0; o.x1 = g.x1;
+                o.ny = g.ny; o.nx = g.nx;
+                const int Y0 = it.ty * kTile;
+                const int X0 = it.tx * kTile;
+                // this warp's 32 rows all lie in the plane's padding below the grid:
+                // nothing of them to load or store (padding only has to stay finite,
+                // and it does: it keeps what it holds)
+                const bool rows_out = Y0 + 32 * q >= g.ny;
                 const int y = Y0 + m;
                 const bool fast = tile_inside(o, Y0, X0);
                 const bool row_in = y >= o.y0 && y < o.y1;
@@ -646,29 +678,58 @@ __global__ void __launch_bounds__(BatchCfg<SPLIT>::THREADS, 1) tc_batch_kernel(c
                     if (lane == 0) atomicMax(&item_max[j], __float_as_uint(mx * (1.0f / 2048.0f)));
                 }
             } else {
-                uint32_t col;
-                const uint32_t mask = slots.take(false, col);
-                ok = slots.ready(acc_full, mask, abort_flag, wait_lim);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) {
-                    fail_result();
-                    stop = true;
-                    break;
+                if ((i & 1) != slot) continue;
+                // (as an epilogue warp of sweep_visit.cu)
+                const VisitItem &g = ring_visit[j];
+                constexpr int G = kTile / 32;
+                const int s = i % NS, T = g.steps, r = g.r;
+                const int X0 = it.tx * kTile, y = it.ty * kBatchRows + m;
+                const bool top = it.ty == 0, bottom = g.bottom;
+                WarpTile c;
+                c.col = lane_base + (uint32_t)(slot * kBatchSlotCols) + 16 * (half * G + 1);
+                c.ecol = lane_base + (uint32_t)(slot * kBatchSlotCols) + (half ? 16 + kTile : 8);
+                c.mask = smem_u32(masks);
+                c.xf = X0 + 16 * half * G;
+                c.ex = half ? X0 + kTile : X0 - 8;
+                const uint32_t row0 = smem_u32(stage_base) + (uint32_t)(s * C::STAGE_BYTES + (m + SG::TOP) * 16);
+                c.img = row0 + (uint32_t)((1 + 2 * half * G) * SG::CHUNK);
+                c.eimg = row0 + (uint32_t)((half ? 4 * G + 1 : 0) * SG::CHUNK);
+                c.inner = min(c.xf, c.ex) >= g.x0 && max(c.xf + 16 * G, c.ex + 8) <= g.x1;
+                if (!c.inner) {
+                    c.q0 = (g.x0 - c.xf) >> 3;
+                    c.p0 = (g.x0 - c.xf + 7) >> 3;
+                    c.p1 = (g.x1 - c.xf) >> 3;
+                    c.q1 = (g.x1 - c.xf + 7) >> 3;
+                    c.ea = clamp8(g.x0 - c.ex);
+                    c.eb = clamp8(g.x1 - c.ex);
                 }
-                if (rows_out || X0 + 64 * grp >= g.nx) {  // this half is all padding
-                    __syncwarp();
-                    if (lane == 0) slots.release(acc_empty, mask);
-                    slots.used(mask);
-                } else {
+                c.tmax = y >= g.y0 && y < g.y1
+                             ? min(top ? kTile : m / r + 1, bottom ? kTile : (kTile - 1 - m) / r + 1)
+                             : 0;
+                for (int t = 1; t <= T; t++, e++) {
+                    const bool ok = mbar_wait_soon(&acc_full[slot], e & 1, abort_flag, wait_lim);
+                    if (!__all_sync(0xffffffffu, ok)) {
+                        fail_result();
+                        stop = true;
+                        break;
+                    }
                     tc_fence_after();
-                    float f[Mode<false>::SUB_BLOCKS / 2][16];
-                    epilogue_load(lane_base + col, grp, f);
+                    if (t < T) {
+                        step_to_image<G>(c, half, t, r, g.x0, g.x1);
+                        fence_proxy_async_smem();  // the next step's MMAs read the image
+                    } else {
+                        const bool owned = y < g.ny && (top || m >= kBatchHalo) && (bottom || m < kTile - kBatchHalo);
+                        uint4 *dst = reinterpret_cast<uint4 *>(g.out + plane_index16(g.pg, owned ? y : 0, c.xf));
+                        step_to_plane<G>(c, t, g.x0, g.x1, g.nx, owned, dst, g.pg.nyp);
+                    }
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) slots.release(acc_empty, mask);
-                    epilogue_store(o, f, grp, m, Y0, X0);
-                    slots.used(mask);
+                    if (lane == 0) {
+                        mbar_arrive(&acc_empty[slot]);
+                        if (t == T) mbar_arrive(&empty[s]);
+                    }
                 }
+                if (stop) break;
             }
             // this warp's stores are issued: the signal warp publishes them
             __syncwarp();
@@ -787,10 +848,10 @@ struct tcs_batch_s {
     int n_grids = 0;
     struct Part {
         int first = 0, n_grids = 0;
-        int *d_layout = nullptr;        // step_off then tile_prefix
-        unsigned *d_counters = nullptr; // per (grid, step), then work counter, error word;
+        int *d_layout = nullptr;        // turn_off then tile_prefix
+        unsigned *d_counters = nullptr; // per (grid, turn), then work counter, error word;
                                         // each on its own 128-byte line (kRowCounterStride)
-        int n_items = 0, n_steps = 0, n_counters = 0;
+        int n_items = 0, n_turns = 0, n_counters = 0;
     } part[2];                          // [FP16, split]
     uint16_t *d_bands = nullptr;
     float *d_coefs = nullptr;
@@ -816,7 +877,9 @@ struct tcs_batch_s {
             if (p) dev_free(p);
     }
 
-    int state_of(const Entry &e) const { return (runs * (e.steps & 1)) & 1; }
+    int state_of(const Entry &e) const {
+        return (runs & batch_turns(e.prob.precision == TCS_PREC_SPLIT, stencil_r(e.prob.stencil), e.steps)) & 1;
+    }
 };
 
 namespace {
@@ -868,11 +931,15 @@ int batch_build(tcs_batch b) {
     auto is_split = [&](int i) { return b->entries[i].prob.precision == TCS_PREC_SPLIT; };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
         if (is_split(x) != is_split(y)) return !is_split(x);
-        return b->entries[x].steps > b->entries[y].steps;
+        auto turns_of = [&](int i) {
+            const auto &e = b->entries[i];
+            return batch_turns(is_split(i), stencil_r(e.prob.stencil), e.steps);
+        };
+        return turns_of(x) > turns_of(y);
     });
     std::vector<BatchGrid> grids(n);
     std::vector<float> coefs(25 * (size_t)n, 0.0f);
-    std::vector<int> steps(n), tiles(n);
+    std::vector<int> turns(n), tiles(n);
     int band = 0;
     int ctr[2] = {0, 0};
     for (int i = 0; i < n; i++) {
@@ -887,21 +954,20 @@ int batch_build(tcs_batch b) {
         G.ny = e.g.ny;
         G.nx = e.g.nx;
         G.y0 = e.g.y0; G.y1 = e.g.y1; G.x0 = e.g.x0; G.x1 = e.g.x1;
-        G.tiles_x = (e.g.nx + kTile - 1) / kTile;
-        G.n_tiles = G.tiles_x * ((e.g.ny + kTile - 1) / kTile);
         G.r = stencil_r(e.prob.stencil);
         G.box = stencil_box(e.prob.stencil);
         G.split = split;
         G.steps = e.steps;
+        batch_shape(G);
         G.ctr_base = ctr[split];
         G.band_base = band;
         G.state = 0;
         G.gate = e.gate;
         G.gate_value = e.gate_value;
         G.scale = split ? b->d_scales + order[i] : nullptr;
-        steps[i] = e.steps;
+        turns[i] = G.turns;
         tiles[i] = G.n_tiles;
-        ctr[split] += std::max(e.steps, 1);
+        ctr[split] += std::max(G.turns, 1);
         band += batch_band_elems(G.r, split);
         std::memcpy(&coefs[25 * (size_t)i], e.coeffs, sizeof(e.coeffs));
         b->point_updates += (long long)(e.g.y1 - e.g.y0) * (e.g.x1 - e.g.x0) * e.steps;
@@ -914,13 +980,13 @@ int batch_build(tcs_batch b) {
         P.n_grids = 0;
         while (first + P.n_grids < n && (int)grids[first + P.n_grids].split == k) P.n_grids++;
         first += P.n_grids;
-        P.n_steps = P.n_grids ? steps[P.first] : 0;
+        P.n_turns = P.n_grids ? turns[P.first] : 0;
         P.n_counters = ctr[k];
         if (!P.n_grids) continue;
-        std::vector<int> layout(P.n_steps + 1 + P.n_grids + 1);
-        const long long n_items = batch_layout(steps.data() + P.first, tiles.data() + P.first,
+        std::vector<int> layout(P.n_turns + 1 + P.n_grids + 1);
+        const long long n_items = batch_layout(turns.data() + P.first, tiles.data() + P.first,
                                                P.n_grids, layout.data(),
-                                               layout.data() + P.n_steps + 1);
+                                               layout.data() + P.n_turns + 1);
         if (n_items < 0) return fail(TCS_ERR_INVALID, "tcs_batch: more than 2^31 work items per run");
         P.n_items = (int)n_items;
         st = dev_alloc_t(&P.d_layout, layout.size() * sizeof(int), "layout");
@@ -961,9 +1027,9 @@ int batch_enqueue(tcs_batch b, cudaStream_t s) {
         if (st) return st;
         BatchParams p;
         p.grids = b->d_grids + P.first;
-        p.step_off = P.d_layout;
-        p.tile_prefix = P.d_layout + P.n_steps + 1;
-        p.n_steps = P.n_steps;
+        p.turn_off = P.d_layout;
+        p.tile_prefix = P.d_layout + P.n_turns + 1;
+        p.n_turns = P.n_turns;
         p.n_grids = P.n_grids;
         p.n_items = P.n_items;
         p.counters = P.d_counters;
@@ -971,7 +1037,7 @@ int batch_enqueue(tcs_batch b, cudaStream_t s) {
         p.error = reinterpret_cast<int *>(P.d_counters + (size_t)(P.n_counters + 1) * kRowCounterStride);
         p.bands = b->d_bands;
         p.wait_ns = b->wait_ns;
-        p.grab = batch_grab(k == 1);
+        p.grab = kBatchGrab;
         st = cuda_status(launch_batch(p, k == 1, g_sms, s), "batch kernel launch");
         if (st) return st;
     }
@@ -1139,7 +1205,12 @@ int tcs_batch_info(tcs_batch b, long long *point_updates, int *items, int *grids
     int st = batch_build(b);
     if (st) return st;
     if (point_updates) *point_updates = b->point_updates;
-    if (items) *items = b->part[0].n_items + b->part[1].n_items;
+    if (items) {  // 128 x 128 tiles, one step each
+        long long n = 0;
+        for (const auto &e : b->entries)
+            n += (long long)((e.g.ny + kTile - 1) / kTile) * ((e.g.nx + kTile - 1) / kTile) * e.steps;
+        *items = (int)std::min(n, 0x7fffffffLL);
+    }
     if (grids) *grids = (int)b->entries.size();
     return TCS_OK;
 }

@@ -14,14 +14,15 @@ struct BatchGrid {
     PlaneGeom pg;
     int ny, nx;             // cells (beyond them: plane padding)
     int y0, y1, x0, x1;
-    int tiles_x;
+    int tiles_x, tiles_y;
     int n_tiles;
     int r, box, split;
     int steps;      // steps in one run
-    int ctr_base;   // completion counter of step 0 of the run
+    int turns;      // turns in one run (batch_turns)
+    int ctr_base;   // completion counter of turn 0 of the run
     int band_base;  // first band element in the band buffer
     int state;      // which plane holds the current state
-    // external gate: step 0 starts once *gate >= gate_value (null: no gate)
+    // external gate: turn 0 starts once *gate >= gate_value (null: no gate)
     const unsigned *gate;
     unsigned gate_value;
     // tensor maps of the planes in device memory, [state][hi, lo] (lo = hi for
@@ -30,6 +31,28 @@ struct BatchGrid {
     // split grids: the per-step scale (SplitScale; step t of a run is slot t+1)
     SplitScale *scale;
 };
+
+// A turn is what a tile does between two waits on its grid's other tiles, and
+// flips the ping-pong once: a split step, or the steps of an FP16 visit, up to
+// five (radius 1) or three on a tile that owns 120 rows (sweep_visit.cu, halo
+// 4).  A run's steps are spread evenly over its turns, the first ones taking
+// one more.
+constexpr int kBatchHalo = 4;
+constexpr int kBatchRows = kTile - 2 * kBatchHalo;
+constexpr int batch_depth(int r) { return kBatchHalo / r + 1; }
+inline int batch_turns(bool split, int r, int steps) {
+    return split ? steps : (steps + batch_depth(r) - 1) / batch_depth(r);
+}
+
+// The tiling and turns of a grid whose size, stencil, precision and steps are
+// set.
+inline void batch_shape(BatchGrid &g) {
+    g.tiles_x = (g.nx + kTile - 1) / kTile;
+    g.tiles_y = g.split || g.ny <= kTile ? (g.ny + kTile - 1) / kTile
+                                         : (g.ny - 2 * kBatchHalo + kBatchRows - 1) / kBatchRows;
+    g.n_tiles = g.tiles_x * g.tiles_y;
+    g.turns = batch_turns(g.split, g.r, g.steps);
+}
 
 // Encodes the four tensor maps of a grid's planes ([state][hi, lo]).
 inline cudaError_t encode_grid_maps(const BatchGrid &g, CUtensorMap out[4]) {
@@ -43,8 +66,20 @@ inline cudaError_t encode_grid_maps(const BatchGrid &g, CUtensorMap out[4]) {
 }
 
 struct BatchItem {
-    int g, t, tile;  // grid, step within the run, tile
+    int g, t, tile;  // grid, turn within the run, tile
     int ty, tx;      // the tile's row and column (set by the producer when it publishes)
+};
+
+// A published FP16 item: what its issuer and epilogue warps need of the grid,
+// copied by the producer (which holds the grid's descriptor anyway).
+struct alignas(16) VisitItem {
+    uint16_t *out;
+    PlaneGeom pg;
+    int ny, nx, y0, y1, x0, x1;
+    int r;
+    int steps;       // of the visit
+    int nwin;        // windows the tile needs (tile_windows)
+    int bottom;      // last tile row
 };
 
 // Split items: the step's scale (StepScale of tc_core.cuh, as s, k, e) and
@@ -56,53 +91,50 @@ struct ItemScale {
     SplitScale *sc;
 };
 
-// One run's work: items are ordered step major and, within a step, by grid
-// then tile.  Grids are sorted by step count (descending), so the grids still
-// running at step t are a prefix of the array: step t holds the first
+// One run's work: items are ordered turn major and, within a turn, by grid
+// then tile.  Grids are sorted by turns (descending), so the grids still
+// running at turn t are a prefix of the array: turn t holds the first
 // tile_prefix[G_t] tiles of the concatenated grids, and work index k decodes
-// with two binary searches (step_off, then tile_prefix).
+// with two binary searches (turn_off, then tile_prefix).
 struct BatchParams {
-    const BatchGrid *grids;  // [n_grids], steps descending
-    const int *step_off;     // [n_steps + 1]: first work index of each step
-    const int *tile_prefix;  // [n_grids + 1]: first tile of each grid within a step
-    int n_steps, n_grids, n_items;
-    unsigned *counters;      // one per (grid, step), kRowCounterStride apart, zero at launch
+    const BatchGrid *grids;  // [n_grids], turns descending
+    const int *turn_off;     // [n_turns + 1]: first work index of each turn
+    const int *tile_prefix;  // [n_grids + 1]: first tile of each grid within a turn
+    int n_turns, n_grids, n_items;
+    unsigned *counters;      // one per (grid, turn), kRowCounterStride apart, zero at launch
     unsigned *work_counter;  // next work index, zero at launch
     int *error;              // first failed wait of this launch (0 = none)
     const uint16_t *bands;
     unsigned long long wait_ns;  // limit of the dependency and gate waits
-    int grab;                    // work indices taken per atomic (batch_grab)
+    int grab;                    // work indices taken per atomic (kBatchGrab)
 };
 
-// Work indices a CTA takes per atomic: consecutive items mostly share a grid
-// (one dependency poll, incremental decode), but a small grid's tiles then
-// run on fewer SMs one after another, lengthening its step-to-step chain.
-// Measured on GB300 with 512 mixed grids: 4 for FP16 items, BATCH_GRAB_SPLIT
-// for the longer split items.
-#ifndef BATCH_GRAB_SPLIT
-#define BATCH_GRAB_SPLIT 1
-#endif
-constexpr int batch_grab(bool split) { return split ? BATCH_GRAB_SPLIT : 4; }
+// Work indices a CTA takes per atomic: more would share a dependency poll and
+// the decode, but a small grid's tiles then run on fewer SMs one after another.
+// Measured on GB300, FP16 items, 4 -> 1 per atomic: 24 grids of 600 x 500, 80
+// star2d2r steps 616 -> 391 us, 256 mixed grids 1.52 -> 1.50 ms (single-step
+// items, a third as long, preferred 4).
+constexpr int kBatchGrab = 1;
 
 // Default limit of a batched run's dependency and gate waits: one second.
 constexpr unsigned long long kBatchWaitNs = 1000000000ull;
 
-// Fills step_off and tile_prefix for grids whose run steps (descending) and
+// Fills turn_off and tile_prefix for grids whose run turns (descending) and
 // tile counts are given; returns the number of work items, or -1 when it
 // would not fit an int.
-inline long long batch_layout(const int *steps, const int *tiles, int n_grids, int *step_off,
+inline long long batch_layout(const int *turns, const int *tiles, int n_grids, int *turn_off,
                               int *tile_prefix) {
     tile_prefix[0] = 0;
     for (int i = 0; i < n_grids; i++) tile_prefix[i + 1] = tile_prefix[i] + tiles[i];
-    const int n_steps = n_grids ? steps[0] : 0;
+    const int n_turns = n_grids ? turns[0] : 0;
     long long off = 0;
-    int g = n_grids;  // grids with steps > t
-    step_off[0] = 0;
-    for (int t = 0; t < n_steps; t++) {
-        while (g > 0 && steps[g - 1] <= t) g--;
+    int g = n_grids;  // grids with turns > t
+    turn_off[0] = 0;
+    for (int t = 0; t < n_turns; t++) {
+        while (g > 0 && turns[g - 1] <= t) g--;
         off += tile_prefix[g];
         if (off > 0x7fffffffLL) return -1;
-        step_off[t + 1] = static_cast<int>(off);
+        turn_off[t + 1] = static_cast<int>(off);
     }
     return off;
 }

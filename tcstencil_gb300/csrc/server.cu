@@ -115,6 +115,7 @@ struct Request {
     float coeffs[25];
     GridGeom g;
     int steps = 0, done_steps = 0;
+    int cur = 0;  // which planes hold the state (one flip per turn)
     const float *h_in = nullptr;
     float *h_out = nullptr;
     size_t plane_bytes = 0, bytes = 0, off = 0;
@@ -171,7 +172,7 @@ struct tcs_server_s {
     // double-buffered round descriptors
     struct RoundBuf {
         BatchGrid *h_grids = nullptr, *d_grids = nullptr;
-        int *h_layout = nullptr, *d_layout = nullptr;  // step_off then tile_prefix
+        int *h_layout = nullptr, *d_layout = nullptr;  // turn_off then tile_prefix
         unsigned *d_counters = nullptr;
         size_t cap_hg = 0, cap_hl = 0, cap_dg = 0, cap_dl = 0, cap_dc = 0;
         cudaEvent_t start = nullptr, end = nullptr;
@@ -461,27 +462,30 @@ bool tcs_server_s::launch_round() {
     if (part.empty()) return false;
 
     // FP16 grids first, then split grids (one batched launch each), each part
-    // sorted by this round's steps, descending (stable: admission order)
-    std::vector<int> run_steps(part.size());
+    // sorted by this round's turns, descending (stable: admission order)
+    std::vector<int> run_steps(part.size()), turns(part.size());
     for (size_t i = 0; i < part.size(); i++) {
         const int rem = part[i]->steps - part[i]->done_steps;
         run_steps[i] = cfg.round_steps > 0 ? std::min(rem, cfg.round_steps) : rem;
+        turns[i] = batch_turns(part[i]->split, part[i]->r, run_steps[i]);
     }
     std::vector<size_t> order(part.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) {
         if (part[x]->split != part[y]->split) return !part[x]->split;
-        return run_steps[x] > run_steps[y];
+        return turns[x] > turns[y];
     });
     {
         std::vector<Request *> p2(part.size());
-        std::vector<int> s2(part.size());
+        std::vector<int> s2(part.size()), t2(part.size());
         for (size_t i = 0; i < order.size(); i++) {
             p2[i] = part[order[i]];
             s2[i] = run_steps[order[i]];
+            t2[i] = turns[order[i]];
         }
         part.swap(p2);
         run_steps.swap(s2);
+        turns.swap(t2);
     }
     const int n = (int)part.size();
     int first[2] = {0, 0}, count[2] = {0, 0};
@@ -490,15 +494,21 @@ bool tcs_server_s::launch_round() {
     size_t n_ctr = 0;
     std::vector<int> tiles(n);
     for (int i = 0; i < n; i++) {
-        const Request *q = part[i];
-        tiles[i] = ((q->g.ny + kTile - 1) / kTile) * ((q->g.nx + kTile - 1) / kTile);
-        n_ctr += run_steps[i];
+        BatchGrid G{};
+        G.ny = part[i]->g.ny;
+        G.nx = part[i]->g.nx;
+        G.r = part[i]->r;
+        G.split = part[i]->split;
+        G.steps = run_steps[i];
+        batch_shape(G);
+        tiles[i] = G.n_tiles;
+        n_ctr += turns[i];
     }
-    // layouts: part k's step_off then tile_prefix at lay_off[k]
+    // layouts: part k's turn_off then tile_prefix at lay_off[k]
     size_t lay_off[2], n_layout = 0;
     for (int k = 0; k < 2; k++) {
         lay_off[k] = n_layout;
-        if (count[k]) n_layout += (size_t)run_steps[first[k]] + 1 + count[k] + 1;
+        if (count[k]) n_layout += (size_t)turns[first[k]] + 1 + count[k] + 1;
     }
     // buffer b is idle (its last round completed), so it may be regrown
     int st = grow_pinned(&b.h_grids, &b.cap_hg, part.size(), retired);
@@ -509,8 +519,8 @@ bool tcs_server_s::launch_round() {
     long long n_items[2] = {0, 0};
     for (int k = 0; k < 2 && !st; k++) {
         if (!count[k]) continue;
-        const int ms = run_steps[first[k]];
-        n_items[k] = batch_layout(run_steps.data() + first[k], tiles.data() + first[k], count[k],
+        const int ms = turns[first[k]];
+        n_items[k] = batch_layout(turns.data() + first[k], tiles.data() + first[k], count[k],
                                   b.h_layout + lay_off[k], b.h_layout + lay_off[k] + ms + 1);
         if (n_items[k] < 0) st = fail(TCS_ERR_INVALID, "round of more than 2^31 work items");
     }
@@ -530,20 +540,19 @@ bool tcs_server_s::launch_round() {
         G.ny = q->g.ny;
         G.nx = q->g.nx;
         G.y0 = q->g.y0; G.y1 = q->g.y1; G.x0 = q->g.x0; G.x1 = q->g.x1;
-        G.tiles_x = (q->g.nx + kTile - 1) / kTile;
-        G.n_tiles = tiles[i];
         G.r = q->r;
         G.box = q->box;
         G.split = q->split;
         G.steps = run_steps[i];
+        batch_shape(G);
         G.ctr_base = ctr;
         G.band_base = q->slot * kBatchMaxBandElems;
-        G.state = q->done_steps & 1;
+        G.state = q->cur;
         G.gate = nullptr;
         G.gate_value = 0;
         G.maps = d_maps + 4 * (size_t)q->slot;
         G.scale = q->split ? d_scale + q->slot : nullptr;
-        ctr += run_steps[i];
+        ctr += turns[i];
     }
 
     const double t_built = now();
@@ -558,12 +567,12 @@ bool tcs_server_s::launch_round() {
     if (!st) st = cuda_status(cudaEventRecord(b.start, compute), "cudaEventRecord");
     for (int k = 0; k < 2 && !st; k++) {
         if (!count[k]) continue;
-        const int ms = run_steps[first[k]];
+        const int ms = turns[first[k]];
         BatchParams p;
         p.grids = b.d_grids + first[k];
-        p.step_off = b.d_layout + lay_off[k];
+        p.turn_off = b.d_layout + lay_off[k];
         p.tile_prefix = b.d_layout + lay_off[k] + ms + 1;
-        p.n_steps = ms;
+        p.n_turns = ms;
         p.n_grids = count[k];
         p.n_items = (int)n_items[k];
         p.counters = b.d_counters;  // ctr_base is absolute across both parts
@@ -571,7 +580,7 @@ bool tcs_server_s::launch_round() {
         p.error = d_err;
         p.bands = d_bands;
         p.wait_ns = kBatchWaitNs;
-        p.grab = batch_grab(k == 1);
+        p.grab = kBatchGrab;
         st = cuda_status(launch_batch(p, k == 1, sms, compute), "batch launch");
     }
     if (!st) st = cuda_status(cudaEventRecord(b.end, compute), "cudaEventRecord");
@@ -587,6 +596,7 @@ bool tcs_server_s::launch_round() {
     for (size_t i = 0; i < part.size(); i++) {
         Request *q = part[i];
         q->done_steps += run_steps[i];
+        q->cur ^= turns[i] & 1;
         if (q->done_steps < q->steps) continue;
         {
             // a cancellation asked for before now wins: no download
@@ -595,7 +605,7 @@ bool tcs_server_s::launch_round() {
             q->finishing = true;
         }
         // finished in this round: unpack and download behind it
-        const int rs = finish(q, q->done_steps & 1, !waited_round, b.end);
+        const int rs = finish(q, q->cur, !waited_round, b.end);
         waited_round = true;
         if (rs) fail_request(q, rs);
     }
@@ -714,10 +724,10 @@ int tcs_server_create(const tcs_server_config *config, tcs_server *out) {
     }
     for (auto &b : s->rb) {
         if (!st) st = grow_pinned(&b.h_grids, &b.cap_hg, (size_t)slots, s->retired);
-        if (!st) st = grow_pinned(&b.h_layout, &b.cap_hl, (size_t)slots + 1024, s->retired);
+        if (!st) st = grow_pinned(&b.h_layout, &b.cap_hl, (size_t)slots + 256, s->retired);
         if (!st) st = grow_device(&b.d_grids, &b.cap_dg, (size_t)slots, s->retired);
-        if (!st) st = grow_device(&b.d_layout, &b.cap_dl, (size_t)slots + 1024, s->retired);
-        if (!st) st = grow_device(&b.d_counters, &b.cap_dc, (size_t)1 << 16, s->retired);
+        if (!st) st = grow_device(&b.d_layout, &b.cap_dl, (size_t)slots + 256, s->retired);
+        if (!st) st = grow_device(&b.d_counters, &b.cap_dc, (size_t)1 << 14, s->retired);
     }
     if (st) {
         tcs_server_destroy(s.release());
