@@ -30,7 +30,6 @@ constexpr int kBandElems = 32 * 16;             // one 16(K) x 32(N) FP16 band
 constexpr int kBandBytes = kBandElems * 2;
 constexpr int kEpiWarps = 8;                    // plain: two warpgroups, one per column half
 constexpr int kTmemCols = 512;                  // two accumulator slots of 256 columns
-constexpr int kSlotCols = 256;                  // AccSlots: two slots of the batched FP16 items
 constexpr uint32_t kIdesc = idesc_f16_f32(128, 32);
 constexpr uint32_t kIdescStack = idesc_f16_f32(128, 96);
 
@@ -49,64 +48,7 @@ struct Mode {
     static constexpr int PLANES = SPLIT ? 2 : 1;          // hi (and lo) data planes
     static constexpr int BAND_PLANES = SPLIT ? 4 : 1;     // band bytes per row, in kBandBytes
 };
-static_assert(Mode<false>::ACC <= kSlotCols, "TMEM layout");
-
-// Which accumulator slots a sub-tile holds: plain sub-tiles alternate between
-// the two slots, a split sub-tile takes both.  The MMA issuer and the
-// epilogue walk the same sequence, so both see the same slots, and each slot
-// counts its own uses for the barrier parities.
-struct AccSlots {
-    uint32_t uses[2] = {0, 0};
-    int next = 0;
-    // Returns the slot mask (bit s = slot s) and the first column.
-    __device__ __forceinline__ uint32_t take(bool split, uint32_t &col) {
-        if (split) {
-            next = 0;
-            col = 0;
-            return 3u;
-        }
-        const int s = next;
-        next ^= 1;
-        col = (uint32_t)(s * kSlotCols);
-        return 1u << s;
-    }
-    __device__ __forceinline__ void used(uint32_t mask) {
-        if (mask & 1u) uses[0]++;
-        if (mask & 2u) uses[1]++;
-    }
-    // MMA issuer: waits until every slot of the mask is free (bounded).
-    __device__ __forceinline__ bool acquire(uint64_t *acc_empty, uint32_t mask,
-                                            const volatile int *abort,
-                                            uint64_t limit_ns = kWaitLimitNs) const {
-#pragma unroll
-        for (int s = 0; s < 2; s++)
-            if ((mask >> s) & 1u)
-                if (!mbar_wait(&acc_empty[s], (uses[s] & 1u) ^ 1u, abort, limit_ns)) return false;
-        return true;
-    }
-    // MMA issuer: the slots' accumulators are complete when the MMAs are.
-    __device__ __forceinline__ void commit(uint64_t *acc_full, uint32_t mask) const {
-#pragma unroll
-        for (int s = 0; s < 2; s++)
-            if ((mask >> s) & 1u) umma_commit(&acc_full[s]);
-    }
-    // Epilogue: waits until the slots' accumulators are complete (bounded).
-    __device__ __forceinline__ bool ready(uint64_t *acc_full, uint32_t mask,
-                                          const volatile int *abort,
-                                          uint64_t limit_ns = kWaitLimitNs) const {
-#pragma unroll
-        for (int s = 0; s < 2; s++)
-            if ((mask >> s) & 1u)
-                if (!mbar_wait(&acc_full[s], uses[s] & 1u, abort, limit_ns)) return false;
-        return true;
-    }
-    // Epilogue (one lane per warp): this warp is done reading the slots.
-    __device__ __forceinline__ void release(uint64_t *acc_empty, uint32_t mask) const {
-#pragma unroll
-        for (int s = 0; s < 2; s++)
-            if ((mask >> s) & 1u) mbar_arrive(&acc_empty[s]);
-    }
-};
+static_assert(2 * Mode<false>::ACC <= kTmemCols, "TMEM layout");
 
 // plane_index of an FP16 (or split) plane, 8 cells per panel row: the
 // panel and the cell in it by shifts, not by a division by the plane's cpp
@@ -591,25 +533,6 @@ __device__ __forceinline__ void issue_plain_tile(uint64_t a_hi0, uint32_t band, 
     else issue_plain_windows<R, SG>(a_hi0, band, d);
 }
 
-// Epilogue of a whole plain tile, first half: this warp's accumulators into
-// registers, one FP32 value per output (lanes = tile rows of the warp's lane
-// quarter, `half` = which half of the tile's column blocks).  lane_col is the
-// TMEM address of the warp's lane quarter at the tile's first column.  After
-// it returns the accumulator may be reused.
-__device__ __forceinline__ void epilogue_load(uint32_t lane_col, int half,
-                                              float (&f)[Mode<false>::SUB_BLOCKS / 2][16]) {
-    constexpr int G = Mode<false>::SUB_BLOCKS / 2;
-    // output block j is accumulator columns 16(j+1) .. 16(j+1)+15
-    uint32_t v[G][16];
-#pragma unroll
-    for (int gg = 0; gg < G; gg++) tmem_ld_x16(lane_col + 16 * (half * G + gg + 1), v[gg]);
-    tmem_ld_wait(v);
-#pragma unroll
-    for (int gg = 0; gg < G; gg++)
-#pragma unroll
-        for (int c = 0; c < 16; c++) f[gg][c] = __uint_as_float(v[gg][c]);
-}
-
 // Output of one tile: planes, geometry and the update rectangle.
 struct TileOut {
     const uint16_t *in_hi, *in_lo;  // input planes (cells outside the rectangle)
@@ -774,20 +697,6 @@ __device__ __forceinline__ void copy_rows(const TileOut &o, int y, int X0, int j
 
 __device__ __forceinline__ bool tile_inside(const TileOut &o, int Y0, int X0) {
     return Y0 >= o.y0 && Y0 + kTile <= o.y1 && X0 >= o.x0 && X0 + kTile <= o.x1;
-}
-
-// Epilogue of a whole plain tile, second half: converts and stores this
-// warp's outputs (tile row m).
-__device__ __forceinline__ void epilogue_store(const TileOut &o,
-                                               const float (&f)[Mode<false>::SUB_BLOCKS / 2][16],
-                                               int half, int m, int Y0, int X0) {
-    constexpr int G = Mode<false>::SUB_BLOCKS / 2;
-    const int y = Y0 + m;
-    const bool fast = tile_inside(o, Y0, X0);
-    const bool row_in = y >= o.y0 && y < o.y1;
-#pragma unroll
-    for (int gg = 0; gg < G; gg++)
-        store_block(o, f[gg], y, X0 + 16 * (half * G + gg), fast, row_in);
 }
 
 // Plain tiles of W = 64, 96 or 128 columns (the plain sweep kernel's
