@@ -485,8 +485,8 @@ __device__ __forceinline__ void cv_leave_counters(const CvParams &p, int lane) {
     if (lane == 0) *p.ended = 0;
 }
 
-template <int S, bool F32, int PPL, int WARPS, int TR>
-__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
+template <int S, bool F32, int PPL, int WARPS, int TR, int CTAS>
+__global__ void __launch_bounds__(WARPS * 32, CTAS)
     cc_visit_kernel(const __grid_constant__ CvParams p, const __grid_constant__ TapCoeffs c) {
     using L = CcLane<S, F32, PPL>;
     constexpr int V = L::V, H = L::H, W = L::W, R = L::R;
@@ -655,15 +655,15 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
     if (!counted && warp == 0) cv_leave_counters(p, lane);
 }
 
-template <int S, bool F32, int PPL, int WARPS, int TR>
+template <int S, bool F32, int PPL, int WARPS, int TR, int CTAS>
 cudaError_t launch_cv(const CvParams &p, const TapCoeffs &c, int sms, cudaStream_t s) {
     static int per_sm = 0;
     if (!per_sm) {
-        cudaError_t e = cudaFuncSetAttribute(cc_visit_kernel<S, F32, PPL, WARPS, TR>,
+        cudaError_t e = cudaFuncSetAttribute(cc_visit_kernel<S, F32, PPL, WARPS, TR, CTAS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, cv_smem<PPL>());
         int n = 0;
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, cc_visit_kernel<S, F32, PPL, WARPS, TR>,
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, cc_visit_kernel<S, F32, PPL, WARPS, TR, CTAS>,
                                                               WARPS * 32, cv_smem<PPL>());
         if (e != cudaSuccess) return e;
         if (n < 1) return cudaErrorInvalidConfiguration;
@@ -681,15 +681,30 @@ cudaError_t launch_cv(const CvParams &p, const TapCoeffs &c, int sms, cudaStream
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, cc_visit_kernel<S, F32, PPL, WARPS, TR>, p, c);
+    return cudaLaunchKernelEx(&cfg, cc_visit_kernel<S, F32, PPL, WARPS, TR, CTAS>, p, c);
 }
 
 template <int S, bool F32>
 cudaError_t dispatch_cv(const CcVisitShape &v, const CvParams &p, const TapCoeffs &c, int sms, cudaStream_t s) {
-    if (v.ppl == 2) return launch_cv<S, F32, 2, 8, 128>(p, c, sms, s);
-    if (v.warps == 8) return launch_cv<S, F32, 1, 8, 128>(p, c, sms, s);
-    if (v.rows == 32) return launch_cv<S, F32, 1, 16, 32>(p, c, sms, s);
-    return v.rows == 64 ? launch_cv<S, F32, 1, 16, 64>(p, c, sms, s) : launch_cv<S, F32, 1, 16, 128>(p, c, sms, s);
+    if (v.ppl == 2) {
+        // Where a whole-panel FP32 lane fits 80 registers, 24 warps on an SM
+        // instead of 16, from three tiles per SM on (us per step: 8196²
+        // star2d1r 39.7 -> 37.5, box2d1r 60.0 -> 55.9, 3000² 6.07 -> 5.80, 8.75
+        // -> 8.42); with fewer tiles the tighter code is the slower one (2500²
+        // box2d1r 6.28 -> 6.59).
+        if constexpr (F32 && (S == TCS_STAR2D1R || S == TCS_BOX2D1R)) {
+            const int tiles = p.tiles_x * p.tiles_y;
+            if (tiles > 3 * sms) return launch_cv<S, F32, 2, 8, 128, 3>(p, c, sms, s);
+            if (!tiles) {  // preparation of both
+                const cudaError_t e = launch_cv<S, F32, 2, 8, 128, 3>(p, c, sms, s);
+                if (e != cudaSuccess) return e;
+            }
+        }
+        return launch_cv<S, F32, 2, 8, 128, 2>(p, c, sms, s);
+    }
+    if (v.warps == 8) return launch_cv<S, F32, 1, 8, 128, 2>(p, c, sms, s);
+    if (v.rows == 32) return launch_cv<S, F32, 1, 16, 32, 1>(p, c, sms, s);
+    return v.rows == 64 ? launch_cv<S, F32, 1, 16, 64, 1>(p, c, sms, s) : launch_cv<S, F32, 1, 16, 128, 1>(p, c, sms, s);
 }
 template <bool F32>
 cudaError_t dispatch_cv(int stencil, const CcVisitShape &v, const CvParams &p, const TapCoeffs &c, int sms,

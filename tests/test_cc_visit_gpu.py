@@ -53,11 +53,11 @@ def test_visits_equal_single_steps(tcs, torch_cuda, stencil, prec, shape, runs):
     _same(tcs, A, B, stencil, prec, runs)
 
 
-@pytest.mark.parametrize("prec,shape", [("f16", (1900, 2300)), ("f32", (1300, 1500)), ("f16", (4200, 3900)), ("f32", (2300, 2500))])
+@pytest.mark.parametrize("prec,shape", [("f16", (1900, 2300)), ("f32", (1300, 1500)), ("f16", (4200, 3900)), ("f32", (2300, 2500)), ("f32", (3100, 2700))])
 @pytest.mark.parametrize("stencil", STENCILS)
 def test_forms_for_more_tiles_per_sm(tcs, torch_cuda, stencil, prec, shape):
     A, B = _case(stencil, shape)
-    if stencil == "box2d2r" and shape[0] == 4200:
+    if stencil == "box2d2r" and shape[0] > 3000:
         p = tcs.Plan(*shape, stencil, B, engine="cudacore", precision=prec)
         assert p.launches(5) == 5  # many tiles: its FMAs bound it
         p.close()
