@@ -104,6 +104,13 @@ struct CcLane {
     static constexpr int NT = tap_count(S);
     static constexpr bool BOX = stencil_box(S);
     static constexpr int PANELS = 16 * PPL;          // of a warp's row
+    // Taps of odd dx in scalar operations: their cell pairs straddle two
+    // register pairs, and the two moves that align one cost more than packing
+    // saves (8196² visits, us per step, FP16 star2d1r 30.9 -> 27.9, star2d2r 45.0
+    // -> 42.7, box2d1r 41.3 -> 38.8; FP32 star2d1r 37.5 -> 35.4, star2d2r 72.0 ->
+    // 67.4, box2d2r 130 -> 122 a single step).  The FP32 box2d1r's single steps
+    // are faster packed (24.3 against 25.1 at 4096²).
+    static constexpr bool ODD_SCALAR = !(F32 && BOX && R == 1);
     using T = typename std::conditional<F32, float, uint16_t>::type;
 
     // shared address of tile row 0 of this lane's cells, and of the outer
@@ -217,6 +224,16 @@ struct CcLane {
                     for (int i = 0; i < H; i += 2) {
                         const float2 x2 = make_float2(x[R + i + dx], x[R + i + 1 + dx]);
                         const float2 a = k == 0 ? make_float2(0.0f, 0.0f) : a2[q][i / 2];
+                        if (ODD_SCALAR && dx % 2 != 0) {
+                            // the pair straddles two register pairs
+                            if constexpr (F32) {
+                                const float2 p = make_float2(__fmul_rn(x2.x, cc.x), __fmul_rn(x2.y, cc.x));
+                                a2[q][i / 2] = k == 0 && !BOX ? p : make_float2(__fadd_rn(a.x, p.x), __fadd_rn(a.y, p.y));
+                            } else {
+                                a2[q][i / 2] = make_float2(fmaf(x2.x, cc.x, a.x), fmaf(x2.y, cc.x, a.y));
+                            }
+                            continue;
+                        }
                         if constexpr (F32) {
                             const float2 p = __ffma2_rn(x2, cc, make_float2(neg0, neg0));
                             a2[q][i / 2] = k == 0 && !BOX ? p : __fadd2_rn(a, p);
@@ -672,7 +689,11 @@ cudaError_t launch_cv(const CvParams &p, const TapCoeffs &c, int sms, cudaStream
     const int tiles = p.tiles_x * p.tiles_y;
     if (!tiles) return cudaSuccess;  // preparation only
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles < per_sm * sms ? tiles : per_sm * sms));
+    // (up to three tiles per SM, two CTAs each: where three fit, some SMs would
+    // have three tiles' steps and others one or two; FP16 2048² star2d1r 3.31 ->
+    // 2.94 us per step, box2d1r 4.44 -> 3.88, FP32 1500² box2d1r 3.72 -> 3.32)
+    const int ctas = (WARPS == 8 && tiles <= 3 * sms && per_sm > 2 ? 2 : per_sm) * sms;
+    cfg.gridDim = dim3((unsigned)(tiles < ctas ? tiles : ctas));
     cfg.blockDim = dim3(WARPS * 32);
     cfg.dynamicSmemBytes = cv_smem<PPL>();
     cfg.stream = s;
