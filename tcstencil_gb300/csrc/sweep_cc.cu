@@ -189,21 +189,22 @@ struct CcLane {
 
     // Rows y0, y0+1 from the window rows y0-2 .. y0+3, held as three row
     // pairs p0, p1, p2, in gold's tap order.
+    template <bool PACK = true>
     __device__ __forceinline__ void compute(const TapCoeffs &c, const float (&p0)[2][W],
                                             const float (&p1)[2][W], const float (&p2)[2][W],
                                             float (&acc)[2][H]) const {
         auto row = [&](int wr) -> const float (&)[W] {
             return wr < 2 ? p0[wr] : wr < 4 ? p1[wr - 2] : p2[wr - 4];
         };
-        if constexpr (F32 ? !(PPL == 2 && BOX && R == 1) : R == 1 || !BOX) {
+        if constexpr (PACK && !(F32 && PPL == 2 && BOX && R == 1)) {
             // packed FP32 operations on cell pairs, taps outside the rows so
             // that one coefficient pair serves both rows; each lane rounds as
             // the scalar operation does, so the bits are the same (measured
             // at 8196², us per step, one step per launch: star2d1r 61.4 ->
             // 57.9 and box2d1r 66.4 -> 63.4 before the interior path,
-            // star2d2r 55.0 -> 51.8 after it; the FP16 box2d2r keeps the
-            // scalar chain: 83.0 -> 92.5 with its taps spilling registers,
-            // and 96 -> 109 in the visit kernel, which has the registers).
+            // star2d2r 55.0 -> 51.8 after it; the FP16 box2d2r since its odd
+            // taps are scalar: 80.9 -> 73.3, 4096² 25.7 -> 21.8, though not on
+            // visits of 64-row tiles, 700² 2.50 -> 2.62).
             // FP32 storage wants gold's unfused products: x c + -0 rounds as
             // x c does, and with the -0 a run-time value the compiler cannot
             // make one fused operation of it and the sum (it does of a packed
@@ -252,8 +253,8 @@ struct CcLane {
                 }
             return;
         }
-        // scalar chains: the FP16 box2d2r, and the FP32 box2d1r of whole-panel
-        // lanes
+        // scalar chains: the FP16 box2d2r of short tiles, and the FP32 box2d1r
+        // of whole-panel lanes
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             constexpr int dy0 = tap_dy(S, 0), dx0 = tap_dx(S, 0);
@@ -614,7 +615,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS)
                 }
                 const float (&own)[2][W] = win[(u + 1) % 3];
                 float acc[2][H];
-                ln.compute(c, win[u % 3], own, n, acc);
+                ln.template compute<F32 || S != TCS_BOX2D2R || TR == kCcTileRows>(c, win[u % 3], own, n, acc);
 #pragma unroll
                 for (int q = 0; q < 2; q++) {
                     if constexpr (decltype(all)::value) {
@@ -798,7 +799,7 @@ cudaError_t launch_cc_f32(const GridGeom &g, int stencil, const TapCoeffs &c, co
 // 1.09, 700² (1.1 of 64) 1.43 / 1.28, 800² (1.5) 1.45 / 1.59.  (Thirty-two warps
 // instead of sixteen: 256² 1.55 -> 1.91.)
 // Measured on GB300, us per step, one step per launch -> 16 warps / 8 warps /
-// whole panels (FP16 halo 8 / 4 / 4; FP32 4):
+// whole panels, 128 rows (FP16 halo 8 / 4 / 4; FP32 4), when the lines were drawn:
 //   FP16 star2d1r  700² 6.09 -> 1.56 / 1.95 / 3.38, 2048² 6.76 -> 3.48 / 3.32
 //        / 4.00, 4096² 12.7 -> 11.7 / 8.66 / 7.90, 8196² 47.6 -> 46.6 / 32.0 / 29.7
 //   FP16 star2d2r  700² 6.51 -> 2.11 / 2.66 / 4.61, 8196² 51.3 -> - / 51.9 /
@@ -810,6 +811,9 @@ cudaError_t launch_cc_f32(const GridGeom &g, int stencil, const TapCoeffs &c, co
 //        box2d1r 87.2 -> - / 68.6 / 57.8
 //   FP32 box2d2r   1026² 7.28 -> 4.10 / 5.68 / 6.20, 2500² 17.6 -> - / 16.4 /
 //        14.9, 4096² 37.0 -> - / 44.7 / 38.9
+// Since the odd taps are scalar (compute), at 8196²: FP16 star2d1r 27.9, star2d2r
+// 42.7, box2d1r 38.8, box2d2r 73.4 (single steps; 3600² 19.2 in visits, 19.3
+// single), FP32 35.4, 67.4, 55.9, 122 (single).
 CcVisitShape cc_visit_shape(const GridGeom &g, int stencil, bool f32, int steps, int sms) {
     CcVisitShape v{};
     const int r = stencil_r(stencil);
