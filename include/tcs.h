@@ -218,8 +218,9 @@ int tcs_plan_set_coeffs(tcs_plan plan, const float *coeffs);
 /* Temporal blocking depth: 1 (single steps, the default) or 2 (two steps per
  * launch, intermediate kept on chip; split precision on the tensor engine,
  * faster there but around 2900 columns and rows, where the one-launch form of
- * single steps is).  Results are bit-identical either way; the autotuner
- * picks, tcs_sweep_host and pipes take depth 2 for split. */
+ * single steps is).  Results are bit-identical either way for grids of finite
+ * values (tcs_plan_set_multistep says what others do); the autotuner picks,
+ * tcs_sweep_host and pipes take depth 2 for split. */
 int tcs_plan_set_temporal_depth(tcs_plan plan, int depth);
 /* Tensor engine (FP16 or split, temporal depth 1): run(steps >= 2) as ONE
  * launch instead of one launch per step.  FP16 tiles take up to eight
@@ -281,7 +282,8 @@ int tcs_pipe_wait(tcs_pipe pipe);
  * coefficients, FP16 or split precision, and step counts) with ONE persistent
  * tensor-core launch per run: every (grid, step, tile) is a work item, and a
  * tile of step t starts once its grid's step t-1 is stored.  Each grid gets
- * the same bits as a tcs_plan of the same problem run alone.  No reference
+ * the same bits as a tcs_plan of the same problem run alone (finite values, as
+ * tcs_plan_set_multistep).  No reference
  * counterpart: the reference runs one grid per process (main_1r.cu /
  * main_2r.cu); batches serve many small problems at once.
  *
