@@ -613,19 +613,22 @@ int tcs_plan_create(const tcs_problem *pr, tcs_plan *out) {
     p->prob.coeffs = p->coeffs;
     const size_t elems = tcs_plane_elems(pr->ny, pr->nx, pr->precision);
     p->plane_bytes = elems * (pr->precision == TCS_PREC_F32 ? 4 : 2);
+    SetUp up;
+    st = up.open();
+    if (st) return st;
     // Zeroed, so that padding cells, which no sweep writes, are finite: a
     // zero band entry times a NaN would still poison an MMA sum.
     for (int s = 0; s < 2; s++)
         for (int pl = 0; pl < p->planes(); pl++) {
             st = dev_alloc_t(&p->buf[s][pl], p->plane_bytes, "plane");
-            if (!st) st = cuda_status(cudaMemset(p->buf[s][pl], 0, p->plane_bytes), "cudaMemset(plane)");
+            if (!st) st = up.zero(p->buf[s][pl], p->plane_bytes, "plane clear");
             if (st) return st;
         }
     if (pr->precision == TCS_PREC_SPLIT) {
         st = dev_alloc_t(&p->d_scale, sizeof(SplitScale), "scale");
-        if (!st) st = cuda_status(cudaMemset(p->d_scale, 0, sizeof(SplitScale)), "cudaMemset(scale)");
+        if (!st) st = up.zero(p->d_scale, sizeof(SplitScale), "scale clear");
         if (!st) st = dev_alloc_t(&p->d_upload, kUploadScratch * sizeof(unsigned), "max");
-        if (!st) st = cuda_status(cudaMemset(p->d_upload, 0, kUploadScratch * sizeof(unsigned)), "cudaMemset(max)");
+        if (!st) st = up.zero(p->d_upload, kUploadScratch * sizeof(unsigned), "max clear");
         if (st) return st;
     }
     size_t words = cc_visit_counter_words(pr->ny, pr->nx);
@@ -643,7 +646,8 @@ int tcs_plan_create(const tcs_problem *pr, tcs_plan *out) {
         if (st) return st;
     }
     st = dev_alloc_t(&p->rows_done, words * sizeof(unsigned), "row counters");
-    if (!st) st = cuda_status(cudaMemset(p->rows_done, 0, words * sizeof(unsigned)), "cudaMemset(counters)");
+    if (!st) st = up.zero(p->rows_done, words * sizeof(unsigned), "counter clear");
+    if (!st) st = up.finish();
     if (st) return st;
     *out = p.release();
     return TCS_OK;

@@ -910,17 +910,19 @@ int batch_build(tcs_batch b) {
         gaps.push_back(total);
         total += gel;
     }
-    int st = dev_alloc_t(&b->pool, total * sizeof(uint16_t), "batch planes");
-    if (!st) st = cuda_status(cudaMemset(b->pool, 0, total * sizeof(uint16_t)), "cudaMemset(batch planes)");
+    SetUp up;
+    int st = up.open();
+    if (!st) st = dev_alloc_t(&b->pool, total * sizeof(uint16_t), "batch planes");
+    if (!st) st = up.zero(b->pool, total * sizeof(uint16_t), "batch plane clear");
     for (size_t k = 0; k < gaps.size() && !st; k++) {
-        st = guard_place(b->pool + gaps[k], gel * sizeof(uint16_t), "batch plane guard", 0);
+        st = guard_place(b->pool + gaps[k], gel * sizeof(uint16_t), "batch plane guard", up.stream());
         if (!st) b->guards.push_back(b->pool + gaps[k]);
     }
     if (!st) st = dev_alloc_t(&b->d_scales, b->entries.size() * sizeof(SplitScale), "scales");
-    if (!st) st = cuda_status(cudaMemset(b->d_scales, 0, b->entries.size() * sizeof(SplitScale)), "cudaMemset(scales)");
+    if (!st) st = up.zero(b->d_scales, b->entries.size() * sizeof(SplitScale), "scale clear");
     const size_t upload_bytes = b->entries.size() * kUploadScratch * sizeof(unsigned);
     if (!st) st = dev_alloc_t(&b->d_upload, upload_bytes, "max");
-    if (!st) st = cuda_status(cudaMemset(b->d_upload, 0, upload_bytes), "cudaMemset(max)");
+    if (!st) st = up.zero(b->d_upload, upload_bytes, "max clear");
     if (st) return st;
     b->pool_elems = total;
     // descriptors (FP16 grids then split grids, each sorted by steps,
@@ -991,7 +993,7 @@ int batch_build(tcs_batch b) {
         P.n_items = (int)n_items;
         st = dev_alloc_t(&P.d_layout, layout.size() * sizeof(int), "layout");
         if (!st) st = dev_alloc_t(&P.d_counters, (size_t)(P.n_counters + 2) * kRowCounterStride * sizeof(unsigned), "counters");
-        if (!st) st = cuda_status(cudaMemcpy(P.d_layout, layout.data(), layout.size() * sizeof(int), cudaMemcpyHostToDevice), "layout copy");
+        if (!st) st = up.copy(P.d_layout, layout.data(), layout.size() * sizeof(int), "layout copy");
         if (st) return st;
     }
     // tensor maps of every grid's planes, then the descriptors that point at them
@@ -1001,16 +1003,17 @@ int batch_build(tcs_batch b) {
         st = cuda_status(encode_grid_maps(grids[i], &maps[4 * i]), "tensor map encode");
         grids[i].maps = b->d_maps + 4 * i;
     }
-    if (!st) st = cuda_status(cudaMemcpy(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice), "maps copy");
+    if (!st) st = up.copy(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), "maps copy");
     if (st) return st;
     st = dev_alloc_t(&b->d_grids, grids.size() * sizeof(BatchGrid), "grids");
     if (!st) st = dev_alloc_t(&b->d_bands, std::max(band, 1) * sizeof(uint16_t), "bands");
     if (!st) st = dev_alloc_t(&b->d_coefs, coefs.size() * sizeof(float), "coefs");
-    if (!st) st = cuda_status(cudaMemcpy(b->d_grids, grids.data(), grids.size() * sizeof(BatchGrid), cudaMemcpyHostToDevice), "grids copy");
-    if (!st) st = cuda_status(cudaMemcpy(b->d_coefs, coefs.data(), coefs.size() * sizeof(float), cudaMemcpyHostToDevice), "coefs copy");
+    if (!st) st = up.copy(b->d_grids, grids.data(), grids.size() * sizeof(BatchGrid), "grids copy");
+    if (!st) st = up.copy(b->d_coefs, coefs.data(), coefs.size() * sizeof(float), "coefs copy");
     if (st) return st;
-    build_bands_kernel<<<(unsigned)grids.size(), 256>>>(b->d_grids, b->d_coefs, b->d_bands);
+    build_bands_kernel<<<(unsigned)grids.size(), 256, 0, up.stream()>>>(b->d_grids, b->d_coefs, b->d_bands);
     st = cuda_status(cudaGetLastError(), "band build launch");
+    if (!st) st = up.finish();
     if (st) return st;
     st = cuda_status(batch_prepare(nullptr), "batch kernel set-up");
     if (st) return st;

@@ -179,6 +179,13 @@ int host_alloc(void **p, size_t bytes, const char *what) { return allocate(p, by
 void dev_free(void *p) { release(p, false); }
 void host_free(void *p) { release(p, true); }
 
+int SetUp::open() { return cuda_status(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking), "cudaStreamCreate"); }
+int SetUp::zero(void *p, size_t bytes, const char *what) { return cuda_status(cudaMemsetAsync(p, 0, bytes, s_), what); }
+int SetUp::copy(void *dst, const void *host, size_t bytes, const char *what) {
+    return cuda_status(cudaMemcpyAsync(dst, host, bytes, cudaMemcpyHostToDevice, s_), what);
+}
+int SetUp::finish() { return cuda_status(cudaStreamSynchronize(s_), "set-up"); }
+
 }  // namespace tcs
 
 using namespace tcs;

@@ -697,7 +697,9 @@ int tcs_server_create(const tcs_server_config *config, tcs_server *out) {
     s->cfg = *config;
     if (s->cfg.max_active == 0) s->cfg.max_active = 1024;
     s->cfg.hbm_budget_bytes = align_up(s->cfg.hbm_budget_bytes);
+    SetUp up;
     int st = cuda_status(batch_prepare(&s->sms), "batch kernel set-up");
+    if (!st) st = up.open();
     if (!st) st = dev_alloc_t(&s->pool, s->cfg.hbm_budget_bytes, "server budget");
     if (st) return st;
     s->alloc.reset(s->cfg.hbm_budget_bytes);
@@ -706,10 +708,11 @@ int tcs_server_create(const tcs_server_config *config, tcs_server *out) {
     if (!st) st = dev_alloc_t(&s->d_maps, (size_t)slots * 4 * sizeof(CUtensorMap), "maps");
     if (!st) st = host_alloc_t(&s->h_maps, (size_t)slots * 4 * sizeof(CUtensorMap), "maps");
     if (!st) st = dev_alloc_t(&s->d_upload, kUploadScratch * (size_t)slots * sizeof(unsigned), "max");
-    if (!st) st = cuda_status(cudaMemset(s->d_upload, 0, kUploadScratch * (size_t)slots * sizeof(unsigned)), "cudaMemset(max)");
+    if (!st) st = up.zero(s->d_upload, kUploadScratch * (size_t)slots * sizeof(unsigned), "max clear");
     if (!st) st = dev_alloc_t(&s->d_scale, slots * sizeof(SplitScale), "scales");
     if (!st) st = dev_alloc_t(&s->d_err, sizeof(int), "error");
-    if (!st) st = cuda_status(cudaMemset(s->d_err, 0, sizeof(int)), "cudaMemset(error)");
+    if (!st) st = up.zero(s->d_err, sizeof(int), "error clear");
+    if (!st) st = up.finish();
     if (!st) st = host_alloc_t(&s->h_slot_err, slots * sizeof(int), "errors");
     if (!st) st = cuda_status(cudaStreamCreateWithFlags(&s->compute, cudaStreamNonBlocking), "cudaStreamCreate");
     if (!st) st = cuda_status(cudaStreamCreateWithFlags(&s->upload, cudaStreamNonBlocking), "cudaStreamCreate");

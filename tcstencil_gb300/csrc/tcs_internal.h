@@ -122,6 +122,26 @@ int dev_alloc(void **p, size_t bytes, const char *what);
 int host_alloc(void **p, size_t bytes, const char *what);
 void dev_free(void *p);
 void host_free(void *p);
+// What the creation of an object puts into its device memory (zeroed planes,
+// counters and scratch, tables), on a stream of its own and complete once
+// finish returns: the object's first use may be on any stream, also one that
+// the default stream does not order, and does not wait for what the caller has
+// queued on the default stream, as cudaMemset would.
+class SetUp {
+public:
+    ~SetUp() {
+        if (s_) cudaStreamDestroy(s_);
+    }
+    int open();
+    int zero(void *p, size_t bytes, const char *what);
+    int copy(void *dst, const void *host, size_t bytes, const char *what);
+    cudaStream_t stream() const { return s_; }
+    int finish();
+
+private:
+    cudaStream_t s_ = nullptr;
+};
+
 // Guard regions inside the library's own memory: the guard size in force
 // (0: off); guard_place fills bytes at p with the canary on stream s and
 // has tcs_guard_check watch them; guard_forget stops watching, after
