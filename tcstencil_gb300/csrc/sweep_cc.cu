@@ -499,6 +499,7 @@ __device__ __forceinline__ void cv_leave_counters(const CvParams &p, int lane) {
         fence_acq_rel_gpu();
     }
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __syncwarp();
     for (int t = lane; t < p.tiles_x * p.tiles_y; t += 32) p.done[t] = 0;
     if (lane == 0) *p.ended = 0;
 }
@@ -550,6 +551,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS)
                         break;
                     }
                 }
+                __syncwarp();  // all lanes' acquires before lane 0's copies (a vote orders no memory)
             }
             // no counter is read or added to for this CTA's other tiles any more
             if (ok && k + (int)gridDim.x >= n_items) {

@@ -100,6 +100,9 @@ __device__ __forceinline__ bool wait_neighbours(const unsigned *done, const Tile
                           global_timer_ns() - t0 > kWaitLimitNs;
         if (__any_sync(0xffffffffu, stop)) return false;
     }
+    // (a vote orders no memory: the barrier puts every lane's acquire before
+    // what lane 0 does next)
+    __syncwarp();
     return true;
 }
 
@@ -118,6 +121,7 @@ __device__ __forceinline__ void leave_counters(const VisitParams &p, int lane) {
         fence_acq_rel_gpu();
     }
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __syncwarp();  // lane 0's acquire before the other lanes' stores
     for (int t = lane; t < p.tiles_x * p.tiles_y; t += 32) p.done[t] = 0;
     if (lane == 0) *p.ended = 0;
 }
