@@ -16,6 +16,7 @@
 
 #include "batch.h"
 #include "tcs_internal.h"
+#include "tile_walk.h"
 
 namespace tcs {
 
@@ -524,19 +525,39 @@ struct tcs_plan_s {
     VisitShape visit_shape(int steps) const {
         return tcs::visit_shape(g.ny, g.nx, prob.stencil, steps, tile_w, device_sms());
     }
-    int steps_in_one(int steps, int from, cudaStream_t s) {
-        if (prob.engine == TCS_ENGINE_CUDACORE)
+    // The next launch of a run with `left` steps to go: all of them, but for
+    // runs of more items than a launch may have (tile_walk.h).
+    Launch take(int left) const {
+        if (prob.engine == TCS_ENGINE_CUDACORE) {
+            const CcVisitShape v = cc_shape(left);
+            return next_launch(left, v.visits, v.depth, (long long)v.tiles_x * v.tiles_y);
+        }
+        if (visits()) {
+            const VisitShape v = visit_shape(left);
+            return next_launch(left, v.visits, v.depth, (long long)v.tiles_x * v.tiles_y);
+        }
+        return next_launch(left, left, 1, tiles());
+    }
+    // One launch of a run with `left` steps to go; t0: the run's steps before it.
+    int steps_in_one(int left, const Launch &l, int t0, int from, cudaStream_t s) {
+        if (prob.engine == TCS_ENGINE_CUDACORE) {
+            CcVisitShape v = cc_shape(left);
+            v.visits = l.turns;
             return cuda_status(
                 launch_cc_visits(g, prob.stencil, prob.precision == TCS_PREC_F32,
                                  tap_coeffs(prob.stencil, coeffs), buf[from][0], buf[1 - from][0],
-                                 steps, cc_shape(steps), rows_done, s, device_sms()),
+                                 l.steps, v, rows_done, s, device_sms()),
                 "multi-step sweep launch");
-        if (visits())
+        }
+        if (visits()) {
+            VisitShape v = visit_shape(left);
+            v.visits = l.turns;
             return cuda_status(
                 launch_tc_f16_visits(g, prob.stencil, coeffs, static_cast<uint16_t *>(buf[from][0]),
-                                     static_cast<uint16_t *>(buf[1 - from][0]), steps,
-                                     visit_shape(steps), rows_done, s, device_sms()),
+                                     static_cast<uint16_t *>(buf[1 - from][0]), l.steps, v, rows_done, s,
+                                     device_sms()),
                 "multi-step sweep launch");
+        }
         const int tiles_y = (g.ny + kTile - 1) / kTile;
         int st = cuda_status(
             cudaMemsetAsync(rows_done, 0, (size_t)tiles_y * kRowCounterStride * sizeof(unsigned), s),
@@ -546,16 +567,21 @@ struct tcs_plan_s {
             launch_tc_split_steps(g, prob.stencil, coeffs, static_cast<const uint16_t *>(buf[from][0]),
                                   static_cast<const uint16_t *>(buf[from][1]),
                                   static_cast<uint16_t *>(buf[1 - from][0]),
-                                  static_cast<uint16_t *>(buf[1 - from][1]), steps, rows_done, s,
-                                  d_scale, 0),
+                                  static_cast<uint16_t *>(buf[1 - from][1]), l.steps, rows_done, s,
+                                  d_scale, t0),
             "multi-step sweep launch");
     }
     // The state `steps` steps from `from` ends in: one flip per step, step
     // pair or visit.
     int final_state(int steps, int from) const {
-        if (multi(steps) && prob.engine == TCS_ENGINE_CUDACORE)
-            return from ^ (cc_shape(steps).visits & 1);
-        if (multi(steps) && visits()) return from ^ (visit_shape(steps).visits & 1);
+        if (multi(steps)) {
+            for (int left = steps; left > 0;) {
+                const Launch l = take(left);
+                from ^= l.turns & 1;
+                left -= l.steps;
+            }
+            return from;
+        }
         const int launches = pairs() ? steps / 2 + steps % 2 : steps;
         return from ^ (launches & 1);
     }
@@ -565,8 +591,12 @@ struct tcs_plan_s {
     int enqueue(int steps, int from, cudaStream_t s, int *to) {
         int st = TCS_OK;
         if (multi(steps)) {
-            *to = final_state(steps, from);
-            st = steps_in_one(steps, from, s);
+            for (int t = 0; t < steps && !st;) {
+                const Launch l = take(steps - t);
+                st = steps_in_one(steps - t, l, t, from, s);
+                from ^= l.turns & 1;
+                t += l.steps;
+            }
         } else {
             for (int t = 0; t < steps && !st;) {
                 if (pairs() && steps - t >= 2) {
@@ -578,8 +608,8 @@ struct tcs_plan_s {
                 }
                 from ^= 1;
             }
-            *to = from;
         }
+        *to = from;
         if (!st && d_scale)
             st = cuda_status(launch_split_scale_end_run(d_scale, steps, s), "scale end of run");
         return st;
@@ -808,7 +838,9 @@ int tcs_plan_tile_width(tcs_plan p, int *tile_w) {
 
 int tcs_plan_launches(tcs_plan p, int steps, int *launches) {
     if (!p || steps < 0 || !launches) return fail(TCS_ERR_INVALID, "tcs_plan_launches: bad arguments");
-    if (p->multi(steps)) *launches = 1;
+    *launches = 0;
+    if (p->multi(steps))
+        for (int left = steps; left > 0; left -= p->take(left).steps) ++*launches;
     else *launches = p->pairs() ? steps / 2 + steps % 2 : steps;
     return TCS_OK;
 }

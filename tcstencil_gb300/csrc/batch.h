@@ -41,7 +41,7 @@ constexpr int kBatchHalo = 4;
 constexpr int kBatchRows = kTile - 2 * kBatchHalo;
 constexpr int batch_depth(int r) { return kBatchHalo / r + 1; }
 inline int batch_turns(bool split, int r, int steps) {
-    return split ? steps : (steps + batch_depth(r) - 1) / batch_depth(r);
+    return split || steps <= 0 ? steps : (steps - 1) / batch_depth(r) + 1;
 }
 
 // The tiling and turns of a grid whose size, stencil, precision and steps are

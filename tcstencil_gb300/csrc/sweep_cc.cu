@@ -829,8 +829,8 @@ CcVisitShape cc_visit_shape(const GridGeom &g, int stencil, bool f32, int steps,
         v.halo = halo;
         v.tiles_x = nchunks <= panels ? 1 : (nchunks - 2 + panels - 3) / (panels - 2);
         v.tiles_y = g.ny <= tile_rows ? 1 : (g.ny - 2 * halo + rows - 1) / rows;
-        const int depth = halo / r + 1;
-        v.visits = (steps + depth - 1) / depth;
+        v.depth = halo / r + 1;
+        v.visits = steps > 0 ? (steps - 1) / v.depth + 1 : 0;
         return (double)v.tiles_x * v.tiles_y / sms;
     };
     if (shape(1, 16, f32 ? 4 : 8, 32) <= (f32 ? 1.25 : 1.05)) return v;

@@ -448,8 +448,8 @@ VisitShape visit_shape(int ny, int nx, int stencil, int steps, int tile_w, int s
             v.tiles_x = (nx + w - 1) / w;
             v.tiles_y = ny <= kTile ? 1 : (ny - 2 * halo + h - 1) / h;
             const int by_rows = halo / r + 1, by_cols = 8 / r;
-            const int depth = by_rows < by_cols ? by_rows : by_cols;
-            v.visits = (steps + depth - 1) / depth;
+            v.depth = by_rows < by_cols ? by_rows : by_cols;
+            v.visits = steps > 0 ? (steps - 1) / v.depth + 1 : 0;
             const double n = (double)v.tiles_x * v.tiles_y / sms;
             if (halo == 2 && (r == 1 || n <= 4.0)) continue;
             const double t = (double)steps / v.visits;

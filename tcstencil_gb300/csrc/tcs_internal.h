@@ -182,6 +182,7 @@ cudaError_t launch_cc_f32(const GridGeom &g, int stencil, const TapCoeffs &c, co
 // cc_visit_counter_words of zeros, which a launch leaves zero again.
 struct CcVisitShape {
     int ppl, warps, rows, halo, tiles_x, tiles_y, visits;
+    int depth;  // steps of a visit at most
 };
 CcVisitShape cc_visit_shape(const GridGeom &g, int stencil, bool f32, int steps, int sms);
 cudaError_t cc_visit_prepare(int stencil, bool f32);
@@ -218,6 +219,7 @@ constexpr int kRowCounterStride = 32;
 // zeros, which a launch leaves zero again.
 struct VisitShape {
     int tile_w, tiles_x, tiles_y, halo, visits;
+    int depth;  // steps of a visit at most
 };
 VisitShape visit_shape(int ny, int nx, int stencil, int steps, int tile_w, int sms);
 constexpr size_t visit_counter_words(int ny, int nx) {

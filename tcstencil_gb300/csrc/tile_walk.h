@@ -12,6 +12,25 @@
 
 namespace tcs {
 
+// The kernels count a launch's items in an int, past its last one by up to a
+// few grid widths, and their completions (16 of an item at most) in an
+// unsigned: launches are kept to kMaxItems items, and a run of more goes out in
+// several.
+constexpr int kMaxItems = 1 << 27;
+
+// A run's next launch: of `turns` turns (visits or steps) of up to `depth`
+// steps on `tiles` tiles, how many it makes, and the steps they take out of
+// `left`.
+struct Launch {
+    int turns, steps;
+};
+inline Launch next_launch(int left, int turns, int depth, long long tiles) {
+    const long long most = kMaxItems / tiles > 1 ? kMaxItems / tiles : 1;
+    if (turns <= most) return Launch{turns, left};
+    const long long steps = most * depth;
+    return Launch{static_cast<int>(most), static_cast<int>(steps < left ? steps : left)};
+}
+
 struct TileWalk {
     int step, ty, tx, dy, dx, tiles_x, tiles_y;
 
