@@ -253,7 +253,8 @@ int tcs_plan_launches(tcs_plan plan, int steps, int *launches);
 
 /* One-call form: host FP32 grid in, `steps` steps, host FP32 grid out.  Device
  * state is kept in a per-thread cache keyed by shape and mode, so repeated
- * calls of one shape do not reallocate.  Large FP16 and FP32 grids go through
+ * calls of one shape do not reallocate (a shape's row bands, below, are made
+ * anew for a step count above all before it, at most five times).  Large FP16 and FP32 grids go through
  * in row bands whose copies and sweeps overlap (the same bits; the device holds
  * the grid twice in FP32 beside its planes, or the call falls back to the grid
  * as a whole). */

@@ -930,25 +930,36 @@ struct HostBands {
         cudaEvent_t in = nullptr, done = nullptr;
     };
     int halo = 0;
+    bool refused = false;  // short of memory for it: the grid as a whole, until the cache is released
     std::vector<Band> bands;
     float *in = nullptr, *out = nullptr;  // the grid, FP32
     cudaStream_t up = nullptr, run = nullptr, down = nullptr;  // (blocking: ordered with the default stream)
-    ~HostBands() {
+    void drop_bands() {
         for (Band &b : bands) {
             if (b.plan) tcs_plan_destroy(b.plan);
             if (b.in) cudaEventDestroy(b.in);
             if (b.done) cudaEventDestroy(b.done);
         }
-        for (float *p : {in, out})
-            if (p) dev_free(p);
-        for (cudaStream_t t : {up, run, down})
-            if (t) cudaStreamDestroy(t);
+        bands.clear();
+        halo = 0;
     }
+    void clear() {
+        drop_bands();
+        for (float **p : {&in, &out}) {
+            if (*p) dev_free(*p);
+            *p = nullptr;
+        }
+        for (cudaStream_t *t : {&up, &run, &down}) {
+            if (*t) cudaStreamDestroy(*t);
+            *t = nullptr;
+        }
+    }
+    ~HostBands() { clear(); }
 };
 
 struct PlanCache {
     std::map<CacheKey, tcs_plan> plans;
-    std::map<CacheKey, HostBands *> bands;
+    std::map<CacheKey, HostBands *> bands;  // one set of a shape; it only ever grows its halo
     ~PlanCache() {
         // Device memory is released by the driver at process exit; freeing it
         // from a static destructor could run after the CUDA runtime is gone.
@@ -958,39 +969,45 @@ struct PlanCache {
 };
 thread_local PlanCache t_cache;
 
-// Bands of a one-call sweep (1: the grid as a whole), and the halo (a power of
-// two, so that calls of near step counts share one set): from 16 MB on, bands
-// at least four halos high, as many as a model of the call's time favours.
+// A model of a one-call sweep's time (us) as a whole (n = 1) or in n bands.
 // Copies: 200 GB/s one way, 330 both ways at once; a step: its cells at the
 // rate the engine reaches on a large grid, or the shortest step, with a tenth
 // more for a band's partial last wave.  Whole grid: in, sweep, out; bands: the
-// first in, the slower of the copies and the sweeps, the last out.  Measured,
-// us, before -> bands: 3000 x 5003 box2d1r FP16 20 steps 927 -> 620, 8196² 3741
-// -> 2446, 60 steps 5414 -> 2578; where the model keeps the grid whole, 2100 x
-// 2000 box2d2r FP32 20 steps, bands took 547, the whole 470.  Split grids share
-// one scale over the whole grid, step by step, so they are not cut.
-int host_bands(const tcs_problem *pr, const GridGeom &g, int steps, int *halo) {
-    const int r = stencil_r(pr->stencil);
-    const size_t bytes = (size_t)g.ny * g.nx * sizeof(float);
-    if (pr->precision == TCS_PREC_SPLIT || steps < 1 || steps > 512 || bytes < ((size_t)16 << 20) || g.y0 != r ||
-        g.y1 != g.ny - r)
-        return 1;
-    int h = 16;
-    while (h < r * steps) h *= 2;
-    *halo = h;
+// first in, the slower of the copies and the sweeps, the last out.
+double host_time(const tcs_problem *pr, const GridGeom &g, int steps, int n, int halo) {
     // cells per us and shortest step, by stencil (star2d1r, star2d2r, box2d1r, box2d2r)
     static const double tensor[4] = {2.4e6, 1.65e6, 2.4e6, 1.65e6}, f16[4] = {2.2e6, 1.5e6, 1.65e6, 0.82e6},
                         f32[4] = {1.75e6, 1.03e6, 1.16e6, 0.5e6};
     const bool tc = pr->engine == TCS_ENGINE_TENSOR, box2 = pr->stencil == TCS_BOX2D2R;
     const double rate = (tc ? tensor : pr->precision == TCS_PREC_F32 ? f32 : f16)[pr->stencil];
     const double shortest = tc ? 1.7 : box2 ? 4.0 : 2.2;
-    const double copy = bytes / 200e3, both = 2 * bytes / 330e3;  // us
+    const double bytes = (double)g.ny * g.nx * sizeof(float);
+    const double copy = bytes / 200e3, both = 2 * bytes / 330e3;
     auto sweep = [&](double rows) { return steps * std::max(shortest, rows * g.nx / rate); };
-    int best = 1;
-    double t_best = 0.95 * (2 * copy + sweep(g.ny));
-    for (int k = 2; k <= 4; k++) {
-        if (g.ny / k < 4 * h) break;
-        const double t = 2 * copy / k + std::max(both * (k - 1) / k, 1.1 * k * sweep(g.ny / (double)k + 2 * h));
+    if (n == 1) return 2 * copy + sweep(g.ny);
+    return 2 * copy / n + std::max(both * (n - 1) / n, 1.1 * n * sweep(g.ny / (double)n + 2 * halo));
+}
+// Grids that may go in bands: from 16 MB on, updated from the first to the
+// last row.  Split grids share one scale over the whole grid, step by step.
+bool may_band(const tcs_problem *pr, const GridGeom &g, int steps) {
+    const int r = stencil_r(pr->stencil);
+    return pr->precision != TCS_PREC_SPLIT && steps >= 1 && steps <= 512 &&
+           (size_t)g.ny * g.nx * sizeof(float) >= ((size_t)16 << 20) && g.y0 == r && g.y1 == g.ny - r;
+}
+constexpr double kBandGain = 0.95;  // of the whole grid's time: bands that promise less are not used
+
+// Bands of a one-call sweep (1: the grid as a whole) and their halo, a power
+// of two: bands at least four halos high, as many as the model favours.
+// Measured, us, before -> bands: 3000 x 5003 box2d1r FP16 20 steps 927 -> 620,
+// 8196² 3741 -> 2446, 60 steps 5414 -> 2578; where the model keeps the grid
+// whole, 2100 x 2000 box2d2r FP32 20 steps, bands took 547, the whole 470.
+int host_bands(const tcs_problem *pr, const GridGeom &g, int steps, int *halo) {
+    int h = 16, best = 1;
+    while (h < stencil_r(pr->stencil) * steps) h *= 2;
+    *halo = h;
+    double t_best = kBandGain * host_time(pr, g, steps, 1, 0);
+    for (int k = 2; k <= 4 && g.ny / k >= 4 * h; k++) {
+        const double t = host_time(pr, g, steps, k, h);
         if (t < t_best) {
             t_best = t;
             best = k;
@@ -998,15 +1015,22 @@ int host_bands(const tcs_problem *pr, const GridGeom &g, int steps, int *halo) {
     }
     return best;
 }
+// Whether a set made for another step count serves this one: a larger halo is
+// only swept for longer.
+bool bands_serve(const HostBands &hb, const tcs_problem *pr, const GridGeom &g, int steps) {
+    const int n = (int)hb.bands.size();
+    return n > 1 && hb.halo >= stencil_r(pr->stencil) * steps &&
+           host_time(pr, g, steps, n, hb.halo) < kBandGain * host_time(pr, g, steps, 1, 0);
+}
 
-int make_host_bands(const tcs_problem *pr, int n, int halo, HostBands **out) {
-    std::unique_ptr<HostBands> hb(new HostBands());
+int make_host_bands(const tcs_problem *pr, int n, int halo, HostBands *hb) {
+    hb->drop_bands();
     hb->halo = halo;
     const size_t bytes = (size_t)pr->ny * pr->nx * sizeof(float);
-    int st = dev_alloc_t(&hb->in, bytes, "staging");
-    if (!st) st = dev_alloc_t(&hb->out, bytes, "staging");
+    int st = hb->in ? TCS_OK : dev_alloc_t(&hb->in, bytes, "staging");
+    if (!st && !hb->out) st = dev_alloc_t(&hb->out, bytes, "staging");
     for (cudaStream_t *t : {&hb->up, &hb->run, &hb->down})
-        if (!st) st = cuda_status(cudaStreamCreate(t), "cudaStreamCreate");
+        if (!st && !*t) st = cuda_status(cudaStreamCreate(t), "cudaStreamCreate");
     for (int k = 0; k < n && !st; k++) {
         HostBands::Band b;
         b.a = (int)((long long)pr->ny * k / n);
@@ -1024,7 +1048,6 @@ int make_host_bands(const tcs_problem *pr, int n, int halo, HostBands **out) {
         if (!st) st = cuda_status(cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming), "cudaEventCreate");
         hb->bands.push_back(b);
     }
-    if (!st) *out = hb.release();
     return st;
 }
 
@@ -1080,23 +1103,30 @@ int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *pr, int s
     GridGeom g;
     int halo = 0;
     if (make_geom(pr->ny, pr->nx, pr->stencil, pr->y0, pr->y1, pr->x0, pr->x1, &g) == TCS_OK) {
-        const int n = host_bands(pr, g, steps, &halo);
         const size_t cells = (size_t)pr->ny * pr->nx;
         // (bands read ahead of what they write: the same buffer or separate ones)
         const bool apart = h_out == h_in || h_out + cells <= h_in || h_in + cells <= h_out;
-        if (n > 1 && apart) {
-            HostBands *&hb = t_cache.bands[key];
-            if (hb && (hb->halo != halo || (int)hb->bands.size() != n)) {
-                delete hb;
-                hb = nullptr;
+        if (apart && may_band(pr, g, steps)) {
+            const int n = host_bands(pr, g, steps, &halo);
+            const auto at = t_cache.bands.find(key);
+            HostBands *hb = at == t_cache.bands.end() ? nullptr : at->second;
+            bool use = hb && bands_serve(*hb, pr, g, steps);
+            // A set is made anew only for a larger halo, so that calls of
+            // changing step counts settle on one set and allocate no more.
+            if (!use && n > 1 && (!hb || (hb->halo < halo && !hb->refused))) {
+                if (!hb) hb = t_cache.bands[key] = new HostBands();
+                use = make_host_bands(pr, n, halo, hb) == TCS_OK;
+                if (!use) {
+                    hb->clear();
+                    hb->refused = true;
+                    cudaGetLastError();
+                }
             }
-            // (short of memory for the bands: the grid as a whole)
-            if (hb || make_host_bands(pr, n, halo, &hb) == TCS_OK) {
+            if (use) {
                 int st = sweep_host_bands(hb, h_in, h_out, pr, steps);
                 if (!st) st = tcs_device_error(nullptr);
                 return st;
             }
-            cudaGetLastError();
         }
     }
     tcs_plan p;
