@@ -1129,18 +1129,28 @@ int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *pr, int s
             }
         }
     }
-    tcs_plan p;
-    auto it = t_cache.plans.find(key);
-    if (it == t_cache.plans.end()) {
-        int st = tcs_plan_create(pr, &p);
-        if (st) return st;
-        p->take_pairs();
-        t_cache.plans.emplace(key, p);
-    } else {
-        p = it->second;
+    tcs_plan p = nullptr;
+    auto upload = [&]() {  // (what may allocate)
+        auto it = t_cache.plans.find(key);
+        if (it == t_cache.plans.end()) {
+            int st = tcs_plan_create(pr, &p);
+            if (st) return st;
+            p->take_pairs();
+            t_cache.plans.emplace(key, p);
+        } else {
+            p = it->second;
+        }
+        int st = tcs_plan_set_coeffs(p, pr->coeffs);
+        return st ? st : tcs_plan_upload(p, h_in, 1, nullptr);
+    };
+    int st = upload();
+    const auto at = t_cache.bands.find(key);
+    if (st == TCS_ERR_NOMEM && at != t_cache.bands.end() && at->second->in) {
+        // the shape's bands, kept from calls of other step counts, make room
+        at->second->clear();
+        at->second->refused = true;
+        st = upload();
     }
-    int st = tcs_plan_set_coeffs(p, pr->coeffs);
-    if (!st) st = tcs_plan_upload(p, h_in, 1, nullptr);
     if (!st) st = tcs_plan_run(p, steps, 1, nullptr);
     if (!st) st = tcs_plan_download(p, h_out, 1, nullptr);
     if (!st) st = cuda_status(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");

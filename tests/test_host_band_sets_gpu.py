@@ -65,6 +65,27 @@ def test_changing_step_counts_settle(tcs, allocations):
     assert allocations == []
 
 
+def test_bands_give_way_to_the_whole_grid(tcs, torch_cuda):
+    """Where the device has no room for the grid as a whole beside its cached
+    bands (a hook refuses what would pass a budget), the bands go; later calls
+    that could take bands again go as a whole."""
+    A, c = _case("box2d1r", (2200, 2100))
+    ref = {n: _plan(tcs, A, "box2d1r", c, n, "tensor", "f16") for n in (16, 600)}
+    tcs.lib().tcs_release_cache()
+    base = tcs.alloc_stats()[1]
+    np.testing.assert_array_equal(tcs.sweep_host(A, 16, "box2d1r", c), ref[16])  # three bands
+    budget = tcs.alloc_stats()[1] + (16 << 20)  # room for less than a whole plan
+    assert tcs.alloc_stats()[1] - base > 2 * A.nbytes
+    tcs.set_alloc_hook(lambda n, what: tcs.alloc_stats()[1] + n > budget)
+    try:
+        np.testing.assert_array_equal(tcs.sweep_host(A, 600, "box2d1r", c), ref[600])  # above 512: as a whole
+        np.testing.assert_array_equal(tcs.sweep_host(A, 16, "box2d1r", c), ref[16])
+    finally:
+        tcs.set_alloc_hook(None)
+        tcs.lib().tcs_release_cache()
+    assert tcs.alloc_stats()[1] == base
+
+
 def test_two_threads_band_their_own_grids(tcs, torch_cuda):
     cases = [_case("star2d1r", (2300, 2000)), _case("box2d2r", (2400, 2100))]
     names, steps = ("star2d1r", "box2d2r"), (15, 7)
