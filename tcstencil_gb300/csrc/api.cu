@@ -146,19 +146,18 @@ using namespace tcs;
 namespace errors {
 
 // The kernels' error words, one per translation unit, are read and cleared by
-// one tiny kernel into a mapped host word: five blocking copies took 40 us, a
-// third of a small one-call sweep.
+// one tiny kernel that leaves the first in a word of its own, read back with
+// one blocking copy: a copy per word took 40 us, a third of a small one-call
+// sweep.  Nothing is kept between calls: no memory of the host's, and no
+// address, which a reset of the device would make stale.
 constexpr int kErrorWords = 5;
 struct ErrorWords {
     int *p[kErrorWords] = {};
 };
-struct {
-    std::mutex mu;
-    std::map<int, ErrorWords> words;  // by device
-    int *code = nullptr;
-} g_errors;
+__device__ int g_taken = 0;
+std::mutex g_taken_mu;
 
-__global__ void take_errors_kernel(const ErrorWords w, int *code) {
+__global__ void take_errors_kernel(const ErrorWords w) {
     int c = 0;
     for (int k = 0; k < kErrorWords; k++) {
         const int v = *reinterpret_cast<volatile int *>(w.p[k]);
@@ -166,8 +165,7 @@ __global__ void take_errors_kernel(const ErrorWords w, int *code) {
         atomicExch(w.p[k], 0);
         if (!c) c = v;
     }
-    *code = c;
-    __threadfence_system();
+    g_taken = c;
 }
 
 }  // namespace errors
@@ -207,26 +205,17 @@ int tcs_device_error(int *code) {
     int st = cuda_status(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     if (st) return st;
     using namespace errors;
-    int dev = 0, c = 0;
-    st = cuda_status(cudaGetDevice(&dev), "cudaGetDevice");
+    ErrorWords w;
+    cudaError_t (*const word[])(int **) = {tc_error_word, batch_error_word, tb_error_word, visit_error_word,
+                                           cc_error_word};
+    for (int k = 0; k < kErrorWords && !st; k++) st = cuda_status(word[k](&w.p[k]), "device error word");
     if (st) return st;
-    std::lock_guard<std::mutex> lk(g_errors.mu);
-    ErrorWords &w = g_errors.words[dev];
-    if (!w.p[0]) {
-        cudaError_t (*const word[])(int **) = {tc_error_word, batch_error_word, tb_error_word, visit_error_word,
-                                               cc_error_word};
-        for (int k = 0; k < kErrorWords && !st; k++) st = cuda_status(word[k](&w.p[k]), "device error word");
-        if (st) w.p[0] = nullptr;
-    }
-    if (!st && !g_errors.code)
-        st = cuda_status(cudaHostAlloc(&g_errors.code, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped),
-                         "cudaHostAlloc(device error)");
-    if (st) return st;
-    take_errors_kernel<<<1, 1>>>(w, g_errors.code);
+    int c = 0;
+    std::lock_guard<std::mutex> lk(g_taken_mu);
+    take_errors_kernel<<<1, 1>>>(w);
     st = cuda_status(cudaGetLastError(), "error word launch");
-    if (!st) st = cuda_status(cudaStreamSynchronize(nullptr), "reading the device error words");
+    if (!st) st = cuda_status(cudaMemcpyFromSymbol(&c, g_taken, sizeof(int)), "reading the device error words");
     if (st) return st;
-    c = *const_cast<volatile int *>(g_errors.code);
     if (code) *code = c;
     return c ? fail(TCS_ERR_TIMEOUT, "device wait timed out (code %d)", c) : TCS_OK;
 }
@@ -1153,8 +1142,7 @@ int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *pr, int s
     }
     if (!st) st = tcs_plan_run(p, steps, 1, nullptr);
     if (!st) st = tcs_plan_download(p, h_out, 1, nullptr);
-    if (!st) st = cuda_status(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
-    if (!st) st = tcs_device_error(nullptr);
+    if (!st) st = tcs_device_error(nullptr);  // (waits for the device)
     return st;
 }
 
