@@ -233,9 +233,11 @@ __device__ __forceinline__ uint32_t pack_h2(float v0, float v1) {
 }
 
 // split_fixed_u of a panel row's eight values into packed words, with the same
-// values and less conversion work: t = rint(u) is formed by the
+// bits and less conversion work: t = rint(u) is formed by the
 // add-and-subtract of 1.5 * 2^23 (round to nearest even for |u| < 2^22; a zero
-// t is +0).  While |t| <= 2^11, hi = t 2^-11 is exact in FP16 and lo = u - t is
+// t is +0).  hi takes 2^-40 of u - t along: lost in the rounding where t is not
+// zero, and the -0 of rint for small negative u where it is (a sign copied to t
+// instead: 2 % of a 16386² radius-1 solve).  While |t| <= 2^11, hi = t 2^-11 is exact in FP16 and lo = u - t is
 // exact; past that (|u| above 2048.5: the value slightly above 1, or NaN) hi
 // rounds in FP16 and split_fixed_u's rule is taken.  One comparison serves
 // all eight, on the maximum that mx needs anyway (a check per pair is a branch
@@ -246,6 +248,7 @@ struct PanelPair {
 };
 __device__ __forceinline__ PanelPair split_panel(const float (&u)[8], float &mx) {
     constexpr float kRound = 12582912.0f;  // 1.5 * 2^23
+    constexpr float kTiny = 1.0f / (1 << 20) / (1 << 20);
     uint32_t hw[4], lw[4];
     float m = 0.0f;
 #pragma unroll
@@ -254,8 +257,9 @@ __device__ __forceinline__ PanelPair split_panel(const float (&u)[8], float &mx)
         m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
         const float2 t = __fadd2_rn(__fadd2_rn(v, make_float2(kRound, kRound)),
                                     make_float2(-kRound, -kRound));
-        const float2 h = __fmul2_rn(t, make_float2(1.0f / 2048.0f, 1.0f / 2048.0f));
         const float2 l = __ffma2_rn(t, make_float2(-1.0f, -1.0f), v);  // exact
+        const float2 h = __ffma2_rn(l, make_float2(kTiny, kTiny),
+                                    __fmul2_rn(t, make_float2(1.0f / 2048.0f, 1.0f / 2048.0f)));
         hw[c] = pack_h2(h.x, h.y);
         lw[c] = pack_h2(l.x, l.y);
     }
