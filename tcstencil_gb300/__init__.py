@@ -305,9 +305,10 @@ class Plan:
                  precision: str = "f16", rect=None, temporal_depth: int | None = None,
                  tile_w: int | None = None):
         """engine "auto" takes the autotuner's choice for this problem class
-        (engine, temporal depth, launch form and tile width); temporal_depth 2
-        runs steps in blocked pairs (split precision, tensor engine); tile_w
-        (128, 96 or 64) is the tile width of plain FP16 tensor sweeps."""
+        (engine, temporal depth, launch form and, with one launch per step, tile
+        width); temporal_depth 2 runs steps in blocked pairs (split precision,
+        tensor engine); tile_w (128, 96 or 64) is the tile width of plain FP16
+        tensor sweeps."""
         tuned_launch = -1
         if engine == "auto":
             from .autotune import best_config, best_launch, best_tile_width
@@ -318,7 +319,11 @@ class Plan:
                 temporal_depth = 2 if precision == "split" and tuned_launch < 0 else tuned_depth
             if tuned_launch < 0 and precision == "f16":
                 tuned_launch = 1  # every tuned FP16 class takes one launch for all steps
-            if tile_w is None and engine == "tensor" and precision == "f16":
+            # One-launch runs choose their width by the grid and the steps, within
+            # about 1 % of the best; a class's width would hold for all its sizes
+            # and step counts (box2d2r 6500², 20 steps, the class's 96 columns
+            # 25.5 us per step, free 23.5; box2d1r 2048², 64 columns 2.48, 2.36).
+            if tile_w is None and engine == "tensor" and precision == "f16" and tuned_launch != 1:
                 tile_w = best_tile_width(stencil, ny, nx)
         self._c = _coeffs(coeffs, stencil)
         y0, y1, x0, x1 = _rect(rect)

@@ -208,7 +208,8 @@ def best_launch(stencil: str, precision: str, ny: int, nx: int, cache: Cache | N
 
 def best_tile_width(stencil: str, ny: int, nx: int, cache: Cache | None = None) -> int:
     """The tuned tile width of plain FP16 tensor sweeps for this problem class
-    (128 when not tuned)."""
+    (128 when not tuned).  Plan(engine="auto") takes it where the tuned form is
+    one launch per step; one-launch runs choose their own."""
     cache = cache or Cache()
     e = cache.lookup("sweep", sweep_key(stencil, "f16", ny, nx))
     return int(e.get("tile_w", 128)) if e else 128
