@@ -66,7 +66,6 @@ constexpr int kVisitStages = 4;                 // a multiple of the slots
 constexpr int kVisitEpi0 = 1 + kVisitSlots;     // first epilogue warp
 constexpr int kVisitEpi = 8;                    // epilogue warps per slot
 constexpr int kVisitThreads = 32 * (kVisitEpi0 + kVisitSlots * kVisitEpi);
-constexpr int kVisitSlotCols = 256;             // TMEM columns per slot (160 used)
 constexpr int kBarBytes = 256;                  // barriers and flags, before the masks
 
 struct VisitParams {
@@ -81,6 +80,9 @@ struct VisitParams {
     float coef[25];
 };
 
+// TMEM columns of a slot (16 (W/16 + 2) used): all there are between the two,
+// or, beside another launch's CTA, what 32-column tiles need.
+__host__ __device__ constexpr int visit_slot_cols(int ctas) { return ctas == 2 ? 64 : kTmemCols / kVisitSlots; }
 __host__ __device__ constexpr int visit_stage_bytes(int W) { return (W / 8 + 2) * SG::CHUNK; }
 
 // Waits (bounded) for visit w.step - 1 of the tile and its neighbours: lane l
@@ -127,12 +129,15 @@ __device__ __forceinline__ void leave_counters(const VisitParams &p, int lane) {
 }
 
 // G: a tile is W = 32 G columns wide, G blocks of 16 for each column half.
-template <int S, int G>
-__global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid_constant__ VisitParams p) {
+// CTAS: 2 leaves room on an SM for a CTA of another launch (launch_visit).
+template <int S, int G, int CTAS>
+__global__ void __launch_bounds__(kVisitThreads, CTAS) tc_visit_kernel(const __grid_constant__ VisitParams p) {
     constexpr int R = stencil_r(S);
     constexpr int W = 32 * G;
     constexpr int stage_bytes = visit_stage_bytes(W);
     constexpr int NS = kVisitStages;
+    constexpr int slot_cols = visit_slot_cols(CTAS);
+    static_assert(16 * (W / 16 + 2) <= slot_cols, "TMEM slot");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = align_smem(smem_raw);
     uint8_t *stage_base = smem;                          // [NS]
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
     }
     if (warp == 1) {
         __syncwarp();
-        tmem_alloc(tmem_slot, kTmemCols);
+        tmem_alloc(tmem_slot, kVisitSlots * slot_cols);
         tmem_relinquish();
     }
     build_bands(reinterpret_cast<uint16_t *>(band_base), p.coef, R, stencil_box(S), false,
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
         if (lane == 0) {
             const int id = warp - 1;  // its slot: tiles i with i % slots == id
             const uint32_t band = smem_u32(band_base);
-            const uint32_t d = tmem_base + (uint32_t)(id * kVisitSlotCols);
+            const uint32_t d = tmem_base + (uint32_t)(id * slot_cols);
             bool stop = false;
             uint32_t e = 0;  // the slot's steps so far
             TileWalk w;
@@ -288,7 +293,7 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
         const int q = warp & 3;       // TMEM lane quarter
         const int m = q * 32 + lane;  // tile row
         const uint32_t lane_col =
-            tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(slot * kVisitSlotCols);
+            tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(slot * slot_cols);
         const GridGeom &g = p.g;
         uint32_t e = 0;  // the slot's steps so far
         bool stop = false;
@@ -368,44 +373,61 @@ __global__ void __launch_bounds__(kVisitThreads, 1) tc_visit_kernel(const __grid
     tc_fence_after();
     if (warp == 1) {
         __syncwarp();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc(tmem_base, kVisitSlots * slot_cols);
     }
     // a producer that gave up did not leave the counters
     if (*left_over && warp == 0) leave_counters(p, lane);
 }
 
-// One CTA per SM: two would share TMEM, of which each takes all, and the CTAs
-// of a launch wait on one another.
+// A launch's CTAs wait on one another, so none may wait for TMEM that a CTA
+// which itself waits holds.  One CTA per SM takes all of TMEM, and more than
+// half of the shared memory, so that it stands alone.  The form for two takes
+// 128 of the 512 columns and just under half: two of them fit, but neither fits
+// beside any other kernel that takes TMEM (tc_sweep_kernel, the smallest, has
+// 121 KB and up).
+template <int CTAS>
 size_t visit_smem(int R, int W) {
     const size_t need = 1024 + (size_t)kVisitStages * visit_stage_bytes(W) + (2 * R + 1) * kBandBytes + kBarBytes + kMaskBytes;
-    return need > 120 * 1024 ? need : 120 * 1024;
+    const size_t least = (CTAS == 2 ? 110 : 120) * 1024;
+    return need > least ? need : least;
 }
 
-template <int S, int G>
+template <int S, int G, int CTAS = 1>
 cudaError_t launch_visit_w(VisitParams &p, int sms, cudaStream_t s) {
     const int tiles = p.tiles_x * p.tiles_y;
     const int grid = tiles < sms ? tiles : sms;
-    return launch_step(tc_visit_kernel<S, G>, grid, kVisitThreads, visit_smem(stencil_r(S), 32 * G),
+    return launch_step(tc_visit_kernel<S, G, CTAS>, grid, kVisitThreads, visit_smem<CTAS>(stencil_r(S), 32 * G),
                        s, p, true);
 }
+// 32-column tiles that leave a quarter of the SMs free go out in the form that
+// shares an SM with another launch's: plans in several streams then run side by
+// side, two launches to an SM, where whole-SM launches of more than half of the
+// SMs take turns.  512² in 20 steps, us per step of one of 8 plans in 8 streams
+// (a launch per step / whole SMs / shared): star2d1r 0.64 / 0.93 / 0.38,
+// box2d2r 0.72 / 1.32 / 0.55.  Its 48 registers instead of 84 cost one plan
+// alone 1 to 3 % up to 512² (64 steps: star2d1r 0.989 -> 1.000, box2d2r 1.41 ->
+// 1.45 us per step) and 5 % above, where the tiles fill the SMs (700² box2d2r 1.44 ->
+// 1.52) and a launch per step takes turns as well.
 template <int S>
 cudaError_t launch_visit(VisitParams &p, int w, int sms, cudaStream_t s) {
+    if (w == 32 && 4 * p.tiles_x * p.tiles_y <= 3 * sms) return launch_visit_w<S, 1, 2>(p, sms, s);
     return w == 128  ? launch_visit_w<S, 4>(p, sms, s)
            : w == 96 ? launch_visit_w<S, 3>(p, sms, s)
            : w == 64 ? launch_visit_w<S, 2>(p, sms, s)
                      : launch_visit_w<S, 1>(p, sms, s);
 }
 
-template <int S, int G>
+template <int S, int G, int CTAS = 1>
 cudaError_t prepare_visit_w() {
-    return cudaFuncSetAttribute(tc_visit_kernel<S, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)visit_smem(stencil_r(S), 32 * G));
+    return cudaFuncSetAttribute(tc_visit_kernel<S, G, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)visit_smem<CTAS>(stencil_r(S), 32 * G));
 }
 template <int S>
 cudaError_t prepare_visit() {
     static bool configured = false;
     if (configured) return cudaSuccess;
     cudaError_t e = prepare_visit_w<S, 1>();
+    if (e == cudaSuccess) e = prepare_visit_w<S, 1, 2>();
     if (e == cudaSuccess) e = prepare_visit_w<S, 2>();
     if (e == cudaSuccess) e = prepare_visit_w<S, 3>();
     if (e == cudaSuccess) e = prepare_visit_w<S, 4>();
