@@ -106,15 +106,7 @@ struct BatchParams {
     int *error;              // first failed wait of this launch (0 = none)
     const uint16_t *bands;
     unsigned long long wait_ns;  // limit of the dependency and gate waits
-    int grab;                    // work indices taken per atomic (kBatchGrab)
 };
-
-// Work indices a CTA takes per atomic: more would share a dependency poll and
-// the decode, but a small grid's tiles then run on fewer SMs one after another.
-// Measured on GB300, FP16 items, 4 -> 1 per atomic: 24 grids of 600 x 500, 80
-// star2d2r steps 616 -> 391 us, 256 mixed grids 1.52 -> 1.50 ms (single-step
-// items, a third as long, preferred 4).
-constexpr int kBatchGrab = 1;
 
 // Default limit of a batched run's dependency and gate waits: one second.
 constexpr unsigned long long kBatchWaitNs = 1000000000ull;

@@ -580,7 +580,6 @@ bool tcs_server_s::launch_round() {
         p.error = d_err;
         p.bands = d_bands;
         p.wait_ns = kBatchWaitNs;
-        p.grab = kBatchGrab;
         st = cuda_status(launch_batch(p, k == 1, sms, compute), "batch launch");
     }
     if (!st) st = cuda_status(cudaEventRecord(b.end, compute), "cudaEventRecord");

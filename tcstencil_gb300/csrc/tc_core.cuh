@@ -380,13 +380,10 @@ __device__ __forceinline__ void split_block_load(uint32_t region_a, uint32_t reg
     }
 }
 
-// Split tiles that are stepped twice per load (sweep_tb.cu, batch.cu): the
-// ring of window regions, and the windows and 16-column blocks of a step
-// (block b: columns X0-16+16b ..; 0 and 9 hold the halo panels).
+// Split tiles that are stepped twice per load (sweep_tb.cu): the ring of window
+// regions.
 constexpr int kTbRing = 5;
 constexpr int kTbRegion = 96;
-constexpr int kTbWindows = kTile / 16 + 1;
-constexpr int kTbBlocks = kTile / 16 + 2;
 
 // Eight columns of a split block from its two windows' regions (TMEM columns
 // `a` and `b` of each part; b is ignored for the halo panels, which one window
