@@ -259,6 +259,9 @@ __device__ __forceinline__ bool wait_all_rows(const unsigned *rows_done, int til
         __nanosleep(128);
     }
     fence_acq_rel_gpu();
+    // (a vote orders no memory: every lane's polls and fence before what one
+    // of them reads next)
+    __syncwarp(mask);
     return true;
 }
 
