@@ -393,6 +393,25 @@ struct tcs_plan_s {
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (steps, start state)
     unsigned *rows_done = nullptr;  // tensor form: counters of the multi-step launches
 
+    // Whether the upload's pack lets the first step's launch start beside it.
+    // A CUDA-core step's CTAs, five to an SM, then go where the pack's blocks
+    // leave room instead of evenly: solves of one step in a row, us each, with
+    // it -> without: box2d2r FP32 1026² 20.0 -> 12.9, 4000 x 91 18.9 -> 11.8, FP16
+    // 2000 x 2100 26.7 -> 20.2.  With so few CTAs that there is room anyway it is
+    // 0.2 us better.
+    bool early_step() const { return prob.engine == TCS_ENGINE_TENSOR || tiles() <= 4; }
+    // Whether the download's unpack lets the next solve's upload start beside
+    // it.  Where single steps follow, the pack's and the step's CTAs then wait
+    // through the unpack on the SMs that happen to be free, and run there (FP16
+    // box2d2r 1026², 1 step 17.6 -> 12.7 without it); one launch of all steps
+    // takes no such place (2000 x 2100 star2d1r, 2 steps 20.9 with it, 22.5
+    // without).  Split: better up to about 1026² (2 steps 24.6 -> 25.4 without),
+    // worse for large grids (4097 x 4100 128 -> 122).
+    bool single_steps = false;  // the last run's launches were single FP16 tensor steps
+    bool early_upload() const {
+        return prob.precision == TCS_PREC_SPLIT ? (long long)prob.ny * prob.nx < (1LL << 22) : !single_steps;
+    }
+
     int planes() const { return prob.precision == TCS_PREC_SPLIT ? 2 : 1; }
 
     void drop_graphs() {
@@ -711,7 +730,7 @@ int tcs_plan_upload(tcs_plan p, const float *grid, int on_host, void *stream) {
             if (!st) st = cuda_status(cudaStreamWaitEvent(p->aux, p->band_ev[k], 0), "cudaStreamWaitEvent");
             if (!st)
                 st = cuda_status(launch_pack_rows(p->staging, p->prob.ny, p->prob.nx, f32,
-                                                  p->buf[0][0], q0, q1, p->aux), "pack launch");
+                                                  p->buf[0][0], q0, q1, p->aux, p->early_step()), "pack launch");
         }
         if (!st) st = cuda_status(cudaEventRecord(p->band_ev[tcs_plan_s::kBands], p->aux), "cudaEventRecord");
         if (!st) st = cuda_status(cudaStreamWaitEvent(s, p->band_ev[tcs_plan_s::kBands], 0), "cudaStreamWaitEvent");
@@ -728,7 +747,8 @@ int tcs_plan_upload(tcs_plan p, const float *grid, int on_host, void *stream) {
     p->cur = 0;
     cudaError_t e;
     if (p->prob.precision == TCS_PREC_F32)
-        e = launch_pack_f32(src, p->prob.ny, p->prob.nx, 0, 0.0f, static_cast<float *>(p->buf[0][0]), s);
+        e = launch_pack_f32(src, p->prob.ny, p->prob.nx, 0, 0.0f, static_cast<float *>(p->buf[0][0]), s,
+                            p->early_step());
     else if (p->prob.precision == TCS_PREC_SPLIT) {
         // scaled so that max |x| 2^-E < 1, all on the device
         e = launch_split_upload(src, p->g, p->d_upload, p->d_scale,
@@ -736,7 +756,8 @@ int tcs_plan_upload(tcs_plan p, const float *grid, int on_host, void *stream) {
                                 static_cast<uint16_t *>(p->buf[0][1]), s);
     }
     else
-        e = launch_pack_f16(src, p->prob.ny, p->prob.nx, 0, 0.0f, static_cast<uint16_t *>(p->buf[0][0]), s);
+        e = launch_pack_f16(src, p->prob.ny, p->prob.nx, 0, 0.0f, static_cast<uint16_t *>(p->buf[0][0]), s,
+                            p->early_step());
     return cuda_status(e, "pack launch");
 }
 
@@ -774,12 +795,15 @@ int tcs_plan_download(tcs_plan p, float *grid, int on_host, void *stream) {
     cudaError_t e;
     const int c = p->cur;
     if (p->prob.precision == TCS_PREC_F32)
-        e = launch_unpack_f32(static_cast<float *>(p->buf[c][0]), p->prob.ny, p->prob.nx, 0, dst, s);
+        e = launch_unpack_f32(static_cast<float *>(p->buf[c][0]), p->prob.ny, p->prob.nx, 0, dst, s,
+                              p->early_upload());
     else if (p->prob.precision == TCS_PREC_SPLIT)
         e = launch_unpack_split_dev(static_cast<uint16_t *>(p->buf[c][0]), static_cast<uint16_t *>(p->buf[c][1]),
-                                    p->prob.ny, p->prob.nx, split_scale_exp_ptr(p->d_scale), dst, s);
+                                    p->prob.ny, p->prob.nx, split_scale_exp_ptr(p->d_scale), dst, s,
+                                    p->early_upload());
     else
-        e = launch_unpack_f16(static_cast<uint16_t *>(p->buf[c][0]), p->prob.ny, p->prob.nx, 0, dst, s);
+        e = launch_unpack_f16(static_cast<uint16_t *>(p->buf[c][0]), p->prob.ny, p->prob.nx, 0, dst, s,
+                              p->early_upload());
     int st = cuda_status(e, "unpack launch");
     if (st || !on_host) return st;
     return cuda_status(cudaMemcpyAsync(grid, p->staging, (size_t)p->prob.ny * p->prob.nx * sizeof(float),
@@ -864,6 +888,7 @@ int tcs_plan_run(tcs_plan p, int steps, int use_graph, void *stream) {
     int launches = 0;
     int lst = tcs_plan_launches(p, steps, &launches);
     if (lst) return lst;
+    if (steps > 0) p->single_steps = p->prob.engine == TCS_ENGINE_TENSOR && p->visits() && !p->multi(steps);
     if (!use_graph || launches <= 8) {
         int to = p->cur;
         const int st = p->enqueue(steps, p->cur, s, &to);

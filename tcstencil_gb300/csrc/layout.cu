@@ -74,6 +74,7 @@ struct PackArgs {
     // loaded beside that pass (past L1), before the wait for its scale (256
     // split grids of a mixed batch: 12.0 -> 9.2 us per upload)
     bool behind_max;
+    bool early;  // lets the next kernel's launch start beside it (tcs_internal.h)
 };
 
 template <int MODE>
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(const PackArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const BlockPos b = block_pos(a.p, a.q0);
     const int X = (b.pan - 1) * CPP + lane;  // this lane's first cell: X, X + 32, ...
-    pdl_launch_dependents();
+    if (a.early) pdl_launch_dependents();
     if (MODE != kPackSplit || !a.behind_max) pdl_wait();
     float v[K][N];
 #pragma unroll
@@ -172,6 +173,7 @@ struct UnpackArgs {
     int q0, q1;
     float scale;
     const int *exp;
+    bool early;  // as PackArgs
 };
 
 template <int MODE>
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(kThreads) unpack_kernel(const UnpackArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const BlockPos b = block_pos(a.p, a.q0);
     const int row = min(b.row + lane, a.q1 - 1);
-    pdl_launch_dependents();
+    if (a.early) pdl_launch_dependents();
     pdl_wait();
     uint4 v[K], l[K];
 #pragma unroll
@@ -452,6 +454,7 @@ PackArgs pack_args(const float *in, int ny, int nx, int pad, float pad_value, vo
     a.p = plane_geom(ny + 2 * pad, nx + 2 * pad, cpp);
     a.q1 = a.p.nyp;
     a.scale = 1.0f;
+    a.early = true;
     return a;
 }
 UnpackArgs unpack_args(const void *in, int ny, int nx, int pad, float *out, int cpp) {
@@ -477,13 +480,17 @@ unsigned max_abs_blocks(size_t n) {
 }  // namespace
 
 cudaError_t launch_pack_f16(const float *in, int ny, int nx, int pad, float pad_value,
-                            uint16_t *plane, cudaStream_t s) {
-    return launch_pack<kPackF16>(pack_args(in, ny, nx, pad, pad_value, plane, 8), s);
+                            uint16_t *plane, cudaStream_t s, bool early) {
+    PackArgs a = pack_args(in, ny, nx, pad, pad_value, plane, 8);
+    a.early = early;
+    return launch_pack<kPackF16>(a, s);
 }
 
 cudaError_t launch_unpack_f16(const uint16_t *plane, int ny, int nx, int pad, float *out,
-                              cudaStream_t s) {
-    return launch_unpack<kPackF16>(unpack_args(plane, ny, nx, pad, out, 8), s);
+                              cudaStream_t s, bool early) {
+    UnpackArgs a = unpack_args(plane, ny, nx, pad, out, 8);
+    a.early = early;
+    return launch_unpack<kPackF16>(a, s);
 }
 
 __global__ void split_scale_end_run_kernel(SplitScale *sc, int steps) {
@@ -505,21 +512,26 @@ cudaError_t launch_split_scale_end_run(SplitScale *sc, int steps, cudaStream_t s
 }
 
 cudaError_t launch_pack_f32(const float *in, int ny, int nx, int pad, float pad_value,
-                            float *plane, cudaStream_t s) {
-    return launch_pack<kPackF32>(pack_args(in, ny, nx, pad, pad_value, plane, 4), s);
+                            float *plane, cudaStream_t s, bool early) {
+    PackArgs a = pack_args(in, ny, nx, pad, pad_value, plane, 4);
+    a.early = early;
+    return launch_pack<kPackF32>(a, s);
 }
 
 cudaError_t launch_unpack_f32(const float *plane, int ny, int nx, int pad, float *out,
-                              cudaStream_t s) {
-    return launch_unpack<kPackF32>(unpack_args(plane, ny, nx, pad, out, 4), s);
+                              cudaStream_t s, bool early) {
+    UnpackArgs a = unpack_args(plane, ny, nx, pad, out, 4);
+    a.early = early;
+    return launch_unpack<kPackF32>(a, s);
 }
 
 // Plane rows [q0, q1) only (every panel), pad 0: the grid rows they hold are
 // [q0 - 4, q1 - 4) clipped to the grid; the pad rows above and below belong
 // to the first and last ranges.
 cudaError_t launch_pack_rows(const float *in, int ny, int nx, bool f32, void *plane, int q0,
-                             int q1, cudaStream_t s) {
+                             int q1, cudaStream_t s, bool early) {
     PackArgs a = pack_args(in, ny, nx, 0, 0.0f, plane, f32 ? 4 : 8);
+    a.early = early;
     if (q0 < 0 || q1 > a.p.nyp || q0 >= q1) return cudaErrorInvalidValue;
     a.q0 = q0;
     a.q1 = q1;
@@ -565,8 +577,9 @@ cudaError_t launch_unpack_split(const uint16_t *hi, const uint16_t *lo, int ny, 
 }
 
 cudaError_t launch_unpack_split_dev(const uint16_t *hi, const uint16_t *lo, int ny, int nx,
-                                    const int *exp_in, float *out, cudaStream_t s) {
+                                    const int *exp_in, float *out, cudaStream_t s, bool early) {
     UnpackArgs a = unpack_args(hi, ny, nx, 0, out, 8);
+    a.early = early;
     a.in_lo = lo;
     a.exp = exp_in;
     return launch_unpack<kPackSplit>(a, s);

@@ -399,18 +399,19 @@ cudaError_t launch_visit_w(VisitParams &p, int sms, cudaStream_t s) {
     return launch_step(tc_visit_kernel<S, G, CTAS>, grid, kVisitThreads, visit_smem<CTAS>(stencil_r(S), 32 * G),
                        s, p, true);
 }
-// 32-column tiles that leave a quarter of the SMs free go out in the form that
-// shares an SM with another launch's: plans in several streams then run side by
-// side, two launches to an SM, where whole-SM launches of more than half of the
-// SMs take turns.  512² in 20 steps, us per step of one of 8 plans in 8 streams
-// (a launch per step / whole SMs / shared): star2d1r 0.64 / 0.93 / 0.38,
-// box2d2r 0.72 / 1.32 / 0.55.  Its 48 registers instead of 84 cost one plan
-// alone 1 to 3 % up to 512² (64 steps: star2d1r 0.989 -> 1.000, box2d2r 1.41 ->
-// 1.45 us per step) and 5 % above, where the tiles fill the SMs (700² box2d2r 1.44 ->
-// 1.52) and a launch per step takes turns as well.
+// 32-column tiles on more than half of the SMs, but not on nearly all, go out in
+// the form that shares an SM with another launch's: plans in several streams
+// then run side by side, two launches to an SM, where such whole-SM launches
+// take turns (smaller ones have room beside one another).  512² in 20 steps, us
+// per step of one of 8 plans in 8 streams (a launch per step / whole SMs /
+// shared): star2d1r 0.64 / 0.93 / 0.38, box2d2r 0.72 / 1.32 / 0.55.  Its 48
+// registers instead of 84 cost one plan alone 0 to 3 % (512², 64 steps: star2d1r
+// 0.994 -> 0.997, box2d2r 1.41 -> 1.44 us per step), and 5 % with more tiles (700²
+// box2d2r 1.44 -> 1.52), where a launch per step takes turns as well.
 template <int S>
 cudaError_t launch_visit(VisitParams &p, int w, int sms, cudaStream_t s) {
-    if (w == 32 && 4 * p.tiles_x * p.tiles_y <= 3 * sms) return launch_visit_w<S, 1, 2>(p, sms, s);
+    const int tiles = p.tiles_x * p.tiles_y;
+    if (w == 32 && 2 * tiles > sms && 4 * tiles <= 3 * sms) return launch_visit_w<S, 1, 2>(p, sms, s);
     return w == 128  ? launch_visit_w<S, 4>(p, sms, s)
            : w == 96 ? launch_visit_w<S, 3>(p, sms, s)
            : w == 64 ? launch_visit_w<S, 2>(p, sms, s)

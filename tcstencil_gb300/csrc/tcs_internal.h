@@ -245,15 +245,17 @@ cudaError_t launch_tc_split(const GridGeom &g, int stencil, const float *B, cons
 // --- layout kernels -------------------------------------------------------
 // pack/unpack between an FP32 row-major grid and an engine plane of the
 // (ny + 2 pad) x (nx + 2 pad) padded grid; every plane cell is written by
-// pack (cells outside the padded grid are 0).
+// pack (cells outside the padded grid are 0).  early: the next kernel, where it
+// is launched with programmatic stream serialization, may take its place on the
+// SMs beside this one.
 cudaError_t launch_pack_f16(const float *in, int ny, int nx, int pad, float pad_value,
-                            uint16_t *plane, cudaStream_t s);
+                            uint16_t *plane, cudaStream_t s, bool early = true);
 cudaError_t launch_unpack_f16(const uint16_t *plane, int ny, int nx, int pad, float *out,
-                              cudaStream_t s);
+                              cudaStream_t s, bool early = false);
 cudaError_t launch_pack_f32(const float *in, int ny, int nx, int pad, float pad_value,
-                            float *plane, cudaStream_t s);
+                            float *plane, cudaStream_t s, bool early = true);
 cudaError_t launch_unpack_f32(const float *plane, int ny, int nx, int pad, float *out,
-                              cudaStream_t s);
+                              cudaStream_t s, bool early = false);
 cudaError_t launch_pack_split(const float *in, int ny, int nx, int pad, float pad_value,
                               int scale_exp, uint16_t *hi, uint16_t *lo, cudaStream_t s);
 cudaError_t launch_unpack_split(const uint16_t *hi, const uint16_t *lo, int ny, int nx, int pad,
@@ -268,14 +270,14 @@ cudaError_t launch_split_upload(const float *in, const GridGeom &g, unsigned *sc
                                 SplitScale *sc, uint16_t *hi, uint16_t *lo, cudaStream_t s);
 // Unpack with the scale exponent kept in device memory.
 cudaError_t launch_unpack_split_dev(const uint16_t *hi, const uint16_t *lo, int ny, int nx,
-                                    const int *exp_in, float *out, cudaStream_t s);
+                                    const int *exp_in, float *out, cudaStream_t s, bool early = false);
 // max |x| over n floats into *out_bits (float bits; *out_bits must start at 0).
 cudaError_t launch_max_abs(const float *in, size_t n, unsigned *out_bits, cudaStream_t s);
 // FP16 (f32 false) or FP32 plane rows [q0, q1) from / to an ny x nx
 // row-major grid, no padding; the grid rows involved are [q0 - 4, q1 - 4)
 // clipped to [0, ny).
 cudaError_t launch_pack_rows(const float *in, int ny, int nx, bool f32, void *plane, int q0,
-                             int q1, cudaStream_t s);
+                             int q1, cudaStream_t s, bool early = true);
 cudaError_t launch_unpack_rows(const void *plane, int ny, int nx, bool f32, float *out, int q0,
                                int q1, cudaStream_t s);
 
