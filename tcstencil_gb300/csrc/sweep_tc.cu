@@ -798,6 +798,13 @@ __global__ void __launch_bounds__(Ring<MULTI>::THREADS, 1) tc_split_ring_kernel(
             const int y = Y0 + m;
             const bool fast = tile_inside(o, Y0, X0);
             const bool row_in = y >= o.y0 && y < o.y1;
+            // The border rows.  One step per launch: beside the tile's load and
+            // first MMAs (behind its blocks they were at the end of a small grid's
+            // step: 128² box2d2r 6.97 -> 6.28 us per step), and those below the grid
+            // only for a caller's planes: both of a plan's (those with a scale
+            // record) hold zeros there (1026² star2d1r 7.70 -> 7.35, 64² 6.74 -> 6.46).
+            // With several steps, only its windows say that the step before is there.
+            if (!MULTI && !fast && (!p.scale || y < o.ny)) copy_rows(o, y, X0, grp, kRingGroups, kTileWindows - 1);
             const bool ok = walk_windows(grp, kRingGroups, kTileWindows, ready, release, [&](int j) {
                 const int Ga = G0 + j, Gb = Ga + 1;
                 tc_fence_after();
@@ -814,7 +821,7 @@ __global__ void __launch_bounds__(Ring<MULTI>::THREADS, 1) tc_split_ring_kernel(
                 store_block_split(o, u, y, X0 + 16 * j, row_in, mx);
             });
             if (!ok) break;
-            if (!fast) copy_rows(o, y, X0, grp, kRingGroups, kTileWindows - 1);
+            if (MULTI && !fast) copy_rows(o, y, X0, grp, kRingGroups, kTileWindows - 1);
             if (ss.k != 0 && !fast) resplit_border(o, y, X0, grp, kRingGroups, kTileWindows - 1, ss);
             // the step's last item of this warp: its maximum and the step's
             // exponent go out before the item is counted
