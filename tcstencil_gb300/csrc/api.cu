@@ -473,11 +473,11 @@ struct tcs_plan_s {
     // blocked pairs, with the same bits as single steps.  The one-call form,
     // pipes and autotuned plans of untuned sizes take it for every split grid:
     // box2d1r / box2d2r, us per step, best form of single steps -> pairs:
-    // 256² 6.38 -> 3.15 / 7.10 -> 3.48, 1026² 7.67 -> 4.42 / 9.05 -> 5.31, 1600²
-    // 9.11 -> 5.91 / 10.0 -> 7.04, 4096² 21.5 -> 21.0 / 25.2 -> 24.2, 8196² 89.4
-    // -> 73.5 / 101 -> 85.3.  Only around 2900² is the one-launch form of single
-    // steps no slower (12.2 / 12.4, 13.7 / 14.6), where a pair's launches still
-    // weigh; the tuned table takes it there.
+    // 256² 5.94 -> 3.21 / 6.50 -> 3.59, 1026² 7.39 -> 4.40 / 8.73 -> 5.23, 1600²
+    // 9.27 -> 5.96 / 10.1 -> 7.09, 4096² 22.1 -> 20.8 / 25.5 -> 24.0, 8196² 89.0
+    // -> 72.7 / 98.6 -> 85.0, 16386² 337 -> 270 / 355 -> 317.  Only around 2900² is
+    // the one-launch form of single steps no slower (12.2 / 12.2, 13.7 / 14.4),
+    // where a pair's launches still weigh; the tuned table takes it there.
     int temporal_depth = 1;
     bool pairs() const { return temporal_depth == 2; }
     void take_pairs() {
@@ -510,10 +510,9 @@ struct tcs_plan_s {
             return multistep < 0 && several(steps) && cc_shape(steps).visits > 0;
         if (multistep >= 0) return multistep == 1;
         // Split, us per step, one launch per step -> one launch (box2d1r /
-        // box2d2r): 2400² 16.5 -> 11.8 / 16.5 -> 12.6, 3200² 22.2 -> 16.3 /
-        // 23.0 -> 17.2, 4800² 51.8 -> 46.2 / 53.0 -> 47.0, 6400² 65.9 -> 60.5
-        // / 66.4 -> 64.3, 8196² 104.0 -> 100.8 / 104.7 -> 107.2, 12000² 206.0
-        // -> 208.9 / 207.5 -> 222.3, 16386² 378.6 -> 391.1 / 380.1 -> 416.9:
+        // box2d2r): 1600² 10.1 -> 9.3 / 10.9 -> 10.1, 2900² 16.4 -> 12.2 / 18.3
+        // -> 13.7, 4096² 27.3 -> 22.1 / 29.4 -> 25.5, 8196² 95.8 -> 89.0 / 98.6
+        // -> 102, 16386² 337 -> 346 / 355 -> 398:
         // the multi-step kernel spends a little more per tile, which the step
         // overheads repay up to about 20 tiles per SM.
         if (prob.precision == TCS_PREC_SPLIT) return tiles > sms && tiles <= 20 * sms;
@@ -546,26 +545,41 @@ struct tcs_plan_s {
         }
         return next_launch(left, left, 1, tiles());
     }
-    // One launch of a run with `left` steps to go; t0: the run's steps before it.
-    int steps_in_one(int left, const Launch &l, int t0, int from, cudaStream_t s) {
+    // How many launches they are.  (The choice of a shape takes a microsecond of a
+    // small call; a grid has fewer tiles than counters.)
+    int several_launches(int steps) const {
+        const size_t tiles = prob.engine == TCS_ENGINE_CUDACORE ? cc_visit_counter_words(g.ny, g.nx)
+                             : visits()                         ? visit_counter_words(g.ny, g.nx)
+                                                                : (size_t)this->tiles();
+        if ((double)tiles * steps <= kMaxItems) return 1;
+        int n = 0;
+        for (int left = steps; left > 0; left -= take(left).steps) n++;
+        return n;
+    }
+    // The next launch (*l) of a run with `left` steps to go, out on stream s; t0:
+    // the run's steps before it.
+    int steps_in_one(int left, Launch *l, int t0, int from, cudaStream_t s) {
         if (prob.engine == TCS_ENGINE_CUDACORE) {
             CcVisitShape v = cc_shape(left);
-            v.visits = l.turns;
+            *l = next_launch(left, v.visits, v.depth, (long long)v.tiles_x * v.tiles_y);
+            v.visits = l->turns;
             return cuda_status(
                 launch_cc_visits(g, prob.stencil, prob.precision == TCS_PREC_F32,
                                  tap_coeffs(prob.stencil, coeffs), buf[from][0], buf[1 - from][0],
-                                 l.steps, v, rows_done, s, device_sms()),
+                                 l->steps, v, rows_done, s, device_sms()),
                 "multi-step sweep launch");
         }
         if (visits()) {
             VisitShape v = visit_shape(left);
-            v.visits = l.turns;
+            *l = next_launch(left, v.visits, v.depth, (long long)v.tiles_x * v.tiles_y);
+            v.visits = l->turns;
             return cuda_status(
                 launch_tc_f16_visits(g, prob.stencil, coeffs, static_cast<uint16_t *>(buf[from][0]),
-                                     static_cast<uint16_t *>(buf[1 - from][0]), l.steps, v, rows_done, s,
+                                     static_cast<uint16_t *>(buf[1 - from][0]), l->steps, v, rows_done, s,
                                      device_sms()),
                 "multi-step sweep launch");
         }
+        *l = take(left);
         const int tiles_y = (g.ny + kTile - 1) / kTile;
         int st = cuda_status(
             cudaMemsetAsync(rows_done, 0, (size_t)tiles_y * kRowCounterStride * sizeof(unsigned), s),
@@ -575,7 +589,7 @@ struct tcs_plan_s {
             launch_tc_split_steps(g, prob.stencil, coeffs, static_cast<const uint16_t *>(buf[from][0]),
                                   static_cast<const uint16_t *>(buf[from][1]),
                                   static_cast<uint16_t *>(buf[1 - from][0]),
-                                  static_cast<uint16_t *>(buf[1 - from][1]), l.steps, rows_done, s,
+                                  static_cast<uint16_t *>(buf[1 - from][1]), l->steps, rows_done, s,
                                   d_scale, t0),
             "multi-step sweep launch");
     }
@@ -600,8 +614,8 @@ struct tcs_plan_s {
         int st = TCS_OK;
         if (multi(steps)) {
             for (int t = 0; t < steps && !st;) {
-                const Launch l = take(steps - t);
-                st = steps_in_one(steps - t, l, t, from, s);
+                Launch l;
+                st = steps_in_one(steps - t, &l, t, from, s);
                 from ^= l.turns & 1;
                 t += l.steps;
             }
@@ -851,9 +865,7 @@ int tcs_plan_tile_width(tcs_plan p, int *tile_w) {
 
 int tcs_plan_launches(tcs_plan p, int steps, int *launches) {
     if (!p || steps < 0 || !launches) return fail(TCS_ERR_INVALID, "tcs_plan_launches: bad arguments");
-    *launches = 0;
-    if (p->multi(steps))
-        for (int left = steps; left > 0; left -= p->take(left).steps) ++*launches;
+    if (p->multi(steps)) *launches = p->several_launches(steps);
     else *launches = p->pairs() ? steps / 2 + steps % 2 : steps;
     return TCS_OK;
 }
@@ -888,7 +900,7 @@ int tcs_plan_run(tcs_plan p, int steps, int use_graph, void *stream) {
     int launches = 0;
     int lst = tcs_plan_launches(p, steps, &launches);
     if (lst) return lst;
-    if (steps > 0) p->single_steps = p->prob.engine == TCS_ENGINE_TENSOR && p->visits() && !p->multi(steps);
+    if (steps > 0) p->single_steps = p->prob.engine == TCS_ENGINE_TENSOR && p->visits() && launches == steps;
     if (!use_graph || launches <= 8) {
         int to = p->cur;
         const int st = p->enqueue(steps, p->cur, s, &to);
