@@ -230,7 +230,10 @@ int tcs_plan_set_temporal_depth(tcs_plan plan, int depth);
  * than nine tiles of 128 x 128 or calls of more than ten steps, split grids of
  * more than one and at most 20 tiles per SM; 0: never; 1: always.  CUDA-core
  * plans take the one-launch form in mode -1 too, by the FP16 rule where it is
- * faster (the radius-2 box up to about seven tiles per SM), not in mode 1.
+ * faster (the radius-2 box up to about seven tiles per SM), not in mode 1.  For
+ * four and more CUDA-core plans at once in several streams, mode 0 is the
+ * faster one (single steps fill the SMs between them, and one-launch runs of
+ * more than half of the SMs take turns).
  * Results are bit-identical either way for grids of finite values (on the
  * tensor engine an infinity or NaN spreads by whole 16-column windows a step,
  * and over several steps of a visit not past its tile's halo).  TCS_MULTI=0 in
@@ -248,7 +251,8 @@ int tcs_plan_set_multistep(tcs_plan plan, int mode);
 int tcs_plan_set_tile_width(tcs_plan plan, int tile_w);
 int tcs_plan_tile_width(tcs_plan plan, int *tile_w);
 /* Kernel launches tcs_plan_run(plan, steps, ...) makes (the device work of
- * one call: 1 for a multi-step launch, else one per step or step pair). */
+ * one call: 1 for a multi-step launch, or more where it would have more than
+ * 2^27 tile visits; else one per step or step pair). */
 int tcs_plan_launches(tcs_plan plan, int steps, int *launches);
 
 /* One-call form: host FP32 grid in, `steps` steps, host FP32 grid out.  Device
@@ -305,7 +309,9 @@ int tcs_batch_download(tcs_batch batch, int index, float *grid, int grid_on_host
 /* One run: every grid advances by its step count.  use_graph != 0 replays a
  * captured CUDA graph of the run. */
 int tcs_batch_run(tcs_batch batch, int use_graph, void *stream);
-/* Point updates per run, work items per run and the number of grids. */
+/* Point updates per run, 128 x 128 tiles times steps per run (the launch takes
+ * FP16 tiles for several steps at a time, so it has fewer work items) and the
+ * number of grids. */
 int tcs_batch_info(tcs_batch batch, long long *point_updates, int *items, int *grids);
 /* External gate: grid `index` starts its first step only once the device
  * word *d_flag is >= value (written by another stream, kernel or copy), so a

@@ -475,7 +475,7 @@ struct tcs_plan_s {
     // box2d1r / box2d2r, us per step, best form of single steps -> pairs:
     // 256² 5.94 -> 3.21 / 6.50 -> 3.59, 1026² 7.39 -> 4.40 / 8.73 -> 5.23, 1600²
     // 9.27 -> 5.96 / 10.1 -> 7.09, 4096² 22.1 -> 20.8 / 25.5 -> 24.0, 8196² 89.0
-    // -> 72.7 / 98.6 -> 85.0, 16386² 337 -> 270 / 355 -> 317.  Only around 2900² is
+    // -> 72.7 / 98.6 -> 85.0, 16386² 337 -> 269 / 355 -> 317.  Only around 2900² is
     // the one-launch form of single steps no slower (12.2 / 12.2, 13.7 / 14.4),
     // where a pair's launches still weigh; the tuned table takes it there.
     int temporal_depth = 1;

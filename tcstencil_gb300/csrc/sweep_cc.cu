@@ -800,8 +800,9 @@ cudaError_t launch_cc_f32(const GridGeom &g, int stencil, const TapCoeffs &c, co
 // 2.71; FP32 star2d1r 256² 1.43 / 1.13 / 0.96, 512² (1.25 of 32) 1.48 / 1.14 /
 // 1.09, 700² (1.1 of 64) 1.43 / 1.28, 800² (1.5) 1.45 / 1.59.  (Thirty-two warps
 // instead of sixteen: 256² 1.55 -> 1.91.)
-// Measured on GB300, us per step, one step per launch -> 16 warps / 8 warps /
-// whole panels, 128 rows (FP16 halo 8 / 4 / 4; FP32 4), when the lines were drawn:
+// What the lines were drawn from, before the odd taps were scalar (compute), us
+// per step, one step per launch -> 16 warps / 8 warps / whole panels, 128 rows
+// (FP16 halo 8 / 4 / 4; FP32 4):
 //   FP16 star2d1r  700² 6.09 -> 1.56 / 1.95 / 3.38, 2048² 6.76 -> 3.48 / 3.32
 //        / 4.00, 4096² 12.7 -> 11.7 / 8.66 / 7.90, 8196² 47.6 -> 46.6 / 32.0 / 29.7
 //   FP16 star2d2r  700² 6.51 -> 2.11 / 2.66 / 4.61, 8196² 51.3 -> - / 51.9 /
@@ -813,9 +814,25 @@ cudaError_t launch_cc_f32(const GridGeom &g, int stencil, const TapCoeffs &c, co
 //        box2d1r 87.2 -> - / 68.6 / 57.8
 //   FP32 box2d2r   1026² 7.28 -> 4.10 / 5.68 / 6.20, 2500² 17.6 -> - / 16.4 /
 //        14.9, 4096² 37.0 -> - / 44.7 / 38.9
-// Since the odd taps are scalar (compute), at 8196²: FP16 star2d1r 27.9, star2d2r
-// 42.7, box2d1r 38.8, box2d2r 73.4 (single steps; 3600² 19.2 in visits, 19.3
-// single), FP32 35.4, 67.4, 55.9, 122 (single).
+// With scalar odd taps, the chosen form in calls of 50 steps (one step per launch
+// -> visits):
+//   FP16 star2d1r  256² 5.68 -> 0.79, 1026² 5.79 -> 1.36, 2048² 6.62 -> 2.54, 4096²
+//        12.5 -> 7.24, 8196² 47.2 -> 28.0
+//   FP16 star2d2r  6.12 -> 1.12, 6.24 -> 1.98, 7.27 -> 3.80, 14.1 -> 10.4, 48.5 -> 42.2
+//   FP16 box2d1r   5.99 -> 0.95, 6.12 -> 1.65, 7.35 -> 3.36, 13.9 -> 9.85, 48.8 -> 37.8
+//   FP16 box2d2r   7.42 -> 1.50, 7.55 -> 3.17, 9.27 -> 6.86, 3000² 14.3 -> 13.1, then
+//        single steps: 4096² 21.6, 8196² 73.1
+//   FP32 star2d1r  4.56 -> 0.91, 4.64 -> 1.57, 6.69 -> 2.88, 22.5 -> 9.34, 85.7 -> 36.3
+//   FP32 star2d2r  5.09 -> 1.44, 5.25 -> 2.55, 7.77 -> 4.82, 24.1 -> 17.5, 87.2 -> 67.0
+//   FP32 box2d1r   5.05 -> 1.03, 5.18 -> 2.02, 7.72 -> 4.72, 24.1 -> 14.6, 87.1 -> 55.3
+//   FP32 box2d2r   6.44 -> 1.87, 7.08 -> 4.19, 12.5 -> 11.1, then single steps: 3000²
+//        20.9, 4096² 34.9, 8196² 122
+// One plan at a time, that is: plans in several streams fill the SMs in single
+// steps too, and do not compute a visit's overlap.  us per step of one of 4 / 8
+// plans in as many streams, single steps -> visits: FP16 star2d1r 1026² 1.73 ->
+// 1.56 / 1.02 -> 1.56, box2d2r 2.69 -> 3.21 / 1.81 -> 3.21, FP32 box2d2r 512² 1.70
+// -> 2.40 / 1.10 -> 2.40, 2048² 7.79 -> 11.3 / 7.80 -> 11.3.  (Forms of 64
+// registers for two launches to an SM: one plan 10 to 25 % slower.)
 CcVisitShape cc_visit_shape(const GridGeom &g, int stencil, bool f32, int steps, int sms) {
     CcVisitShape v{};
     const int r = stencil_r(stencil);

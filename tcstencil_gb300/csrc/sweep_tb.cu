@@ -23,8 +23,8 @@
 // (no other window reads those panels), and window w of the second step
 // waits for its two blocks: the second step follows the first a few windows
 // behind, and the tensor pipe does not drain between them.  Radius 2 runs at
-// the tensor pipe's 60 cycles per MMA (8196²: 104 -> 85 us per step against
-// one step per launch); radius 1 (102 -> 73) at 480 cycles per window of 360
+// the tensor pipe's 60 cycles per MMA (8196²: 98.6 -> 84.6 us per step against
+// one step per launch); radius 1 (95.8 -> 72.5) at 480 cycles per window of 360
 // cycles' MMAs, the five regions' turnaround.  An epilogue warp
 // waits once per block, on a barrier that both windows' commits arrive at.
 // (Waiting for windows, each released by all warps read or not, cost a warp

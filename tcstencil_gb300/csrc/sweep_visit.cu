@@ -449,17 +449,15 @@ cudaError_t prepare_visit() {
 // Narrow tiles have short steps and more SMs, wide ones fewer MMAs per cell;
 // halo 8 takes more steps per visit, halo 4 fewer rows twice, and halo 2
 // (whose copies move half lines) pays only for radius 2 with many tiles,
-// where T = 2 already takes the sweep off the memory bound.  Over the sweeps
-// above the choice costs 1.1 % over the best of W = 32, 64, 96, 128 with every
-// halo, 15 % at most (a model of n without I, fitted to runs of many steps: 3.2
-// %, and 31 %: 1300² box2d2r 4 steps 17.0 us, 12.9 now).  box2d2r,
-// us per step, W 32 / 64 / 96 / 128: 256² 1.47 / 1.90 / 2.34 / 2.88, 1026²
-// 1.70 / 2.13 / 2.36 / 2.82, 2048² 4.05 / 3.08 / 3.15 / 3.41, 8196² - / - /
-// 40.0 / 40.7.  The best form against one launch per step (radius 1 star /
-// radius 2 box): 256² 3.50 -> 1.03 / 3.79 -> 1.47, 1026² 4.09 -> 1.32 /
-// 4.52 -> 1.70, 4096² 11.2 -> 6.96 / 12.7 -> 10.0; against one step per tile
-// visit in one launch: 8196² 42.1 -> 26.9 / 41.5 -> 40.0, 16386² 169 -> 107 /
-// 167 -> 158 (5792², radius 2, whose planes nearly fit L2: 19.75 -> 20.0).
+// where T = 2 already takes the sweep off the memory bound.  Against widths of
+// 64 and 96 columns set by the caller, over 13 grids of 256² to 8196², four
+// stencils and calls of 4 to 100 steps, the choice is 1.0 % behind the best on
+// average; where it misses most is radius 2 at 2048² (100 steps: 3.55 us per
+// step, 64 columns 2.85) and in calls of four steps around 1300² (3.7, 3.1);
+// profiles/visit_widths.md has all.  us per step in calls of 100 steps, against
+// one launch per step, star2d1r / box2d2r: 256² 4.45 -> 0.98 / 5.06 -> 1.40, 1026²
+// 4.83 -> 1.23 / 5.43 -> 1.58, 4096² 11.1 -> 6.81 / 12.8 -> 9.39, 8196² 46.4 ->
+// 26.7 / 47.9 -> 36.8.
 VisitShape visit_shape(int ny, int nx, int stencil, int steps, int tile_w, int sms) {
     const int r = stencil_r(stencil);
     VisitShape best{};
