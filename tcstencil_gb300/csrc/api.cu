@@ -146,10 +146,12 @@ using namespace tcs;
 namespace errors {
 
 // The kernels' error words, one per translation unit, are read and cleared by
-// one tiny kernel that leaves the first in a word of its own, read back with
-// one blocking copy: a copy per word took 40 us, a third of a small one-call
-// sweep.  Nothing is kept between calls: no memory of the host's, and no
-// address, which a reset of the device would make stale.
+// one tiny kernel that leaves the first in one word (a copy per word took 40 us,
+// a third of a small one-call sweep).  Nothing is kept between calls of
+// tcs_device_error, whose word is a device one read back by a blocking copy: no
+// memory of the host's, and no address, which a reset of the device would make
+// stale.  The one-call form has a pinned word beside its cached plans, which
+// the kernel writes itself: 13 us instead of 17.
 constexpr int kErrorWords = 5;
 struct ErrorWords {
     int *p[kErrorWords] = {};
@@ -157,7 +159,7 @@ struct ErrorWords {
 __device__ int g_taken = 0;
 std::mutex g_taken_mu;
 
-__global__ void take_errors_kernel(const ErrorWords w) {
+__global__ void take_errors_kernel(const ErrorWords w, int *taken) {
     int c = 0;
     for (int k = 0; k < kErrorWords; k++) {
         const int v = *reinterpret_cast<volatile int *>(w.p[k]);
@@ -165,7 +167,38 @@ __global__ void take_errors_kernel(const ErrorWords w) {
         atomicExch(w.p[k], 0);
         if (!c) c = v;
     }
-    g_taken = c;
+    *taken = c;
+    __threadfence_system();
+}
+
+// The first error since the last call into *c (0: none), by way of the pinned
+// word if there is one.  Waits for the device.
+int take(int *c, int *pinned) {
+    int st = cuda_status(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+    ErrorWords w;
+    cudaError_t (*const word[])(int **) = {tc_error_word, batch_error_word, tb_error_word, visit_error_word,
+                                           cc_error_word};
+    for (int k = 0; k < kErrorWords && !st; k++) st = cuda_status(word[k](&w.p[k]), "device error word");
+    if (st) return st;
+    std::unique_lock<std::mutex> lk(g_taken_mu, std::defer_lock);
+    int *to = pinned;
+    if (!pinned) {
+        lk.lock();
+        st = cuda_status(cudaGetSymbolAddress(reinterpret_cast<void **>(&to), g_taken), "device error word");
+        if (st) return st;
+    }
+    take_errors_kernel<<<1, 1>>>(w, to);
+    st = cuda_status(cudaGetLastError(), "error word launch");
+    if (st) return st;
+    if (!pinned) return cuda_status(cudaMemcpy(c, to, sizeof(int), cudaMemcpyDeviceToHost), "reading the device error words");
+    st = cuda_status(cudaStreamSynchronize(nullptr), "reading the device error words");
+    *c = *const_cast<volatile int *>(pinned);
+    return st;
+}
+
+int report(int st, int c) {
+    if (st) return st;
+    return c ? fail(TCS_ERR_TIMEOUT, "device wait timed out (code %d)", c) : TCS_OK;
 }
 
 }  // namespace errors
@@ -202,22 +235,10 @@ size_t tcs_plane_elems(int ny, int nx, int precision) {
 }
 
 int tcs_device_error(int *code) {
-    int st = cuda_status(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
-    if (st) return st;
-    using namespace errors;
-    ErrorWords w;
-    cudaError_t (*const word[])(int **) = {tc_error_word, batch_error_word, tb_error_word, visit_error_word,
-                                           cc_error_word};
-    for (int k = 0; k < kErrorWords && !st; k++) st = cuda_status(word[k](&w.p[k]), "device error word");
-    if (st) return st;
     int c = 0;
-    std::lock_guard<std::mutex> lk(g_taken_mu);
-    take_errors_kernel<<<1, 1>>>(w);
-    st = cuda_status(cudaGetLastError(), "error word launch");
-    if (!st) st = cuda_status(cudaMemcpyFromSymbol(&c, g_taken, sizeof(int)), "reading the device error words");
-    if (st) return st;
-    if (code) *code = c;
-    return c ? fail(TCS_ERR_TIMEOUT, "device wait timed out (code %d)", c) : TCS_OK;
+    const int st = errors::take(&c, nullptr);
+    if (!st && code) *code = c;
+    return errors::report(st, c);
 }
 
 // ----------------------------------------------------- layout transforms --
@@ -986,6 +1007,8 @@ struct HostBands {
 struct PlanCache {
     std::map<CacheKey, tcs_plan> plans;
     std::map<CacheKey, HostBands *> bands;  // one set of a shape; it only ever grows its halo
+    int *error = nullptr;        // pinned: errors::take
+    bool error_refused = false;  // (no memory for it: until the cache is released)
     ~PlanCache() {
         // Device memory is released by the driver at process exit; freeing it
         // from a static destructor could run after the CUDA runtime is gone.
@@ -1117,6 +1140,15 @@ int sweep_host_bands(HostBands *hb, const float *h_in, float *h_out, const tcs_p
     return st;
 }
 
+// tcs_device_error at the end of a one-call sweep.
+int host_errors() {
+    if (!t_cache.error && !t_cache.error_refused)
+        t_cache.error_refused = host_alloc_t(&t_cache.error, sizeof(int), "error word") != TCS_OK;
+    int c = 0;
+    const int st = errors::take(&c, t_cache.error);
+    return errors::report(st, c);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1150,8 +1182,7 @@ int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *pr, int s
             }
             if (use) {
                 int st = sweep_host_bands(hb, h_in, h_out, pr, steps);
-                if (!st) st = tcs_device_error(nullptr);
-                return st;
+                return st ? st : host_errors();
             }
         }
     }
@@ -1179,8 +1210,7 @@ int tcs_sweep_host(const float *h_in, float *h_out, const tcs_problem *pr, int s
     }
     if (!st) st = tcs_plan_run(p, steps, 1, nullptr);
     if (!st) st = tcs_plan_download(p, h_out, 1, nullptr);
-    if (!st) st = tcs_device_error(nullptr);  // (waits for the device)
-    return st;
+    return st ? st : host_errors();  // (waits for the device)
 }
 
 void tcs_release_cache(void) {
@@ -1188,6 +1218,9 @@ void tcs_release_cache(void) {
     t_cache.plans.clear();
     for (auto &kv : t_cache.bands) delete kv.second;
     t_cache.bands.clear();
+    if (t_cache.error) host_free(t_cache.error);
+    t_cache.error = nullptr;
+    t_cache.error_refused = false;
 }
 
 }  // extern "C"
