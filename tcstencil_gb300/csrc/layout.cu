@@ -74,10 +74,13 @@ struct PackArgs {
     // loaded beside that pass (past L1), before the wait for its scale (256
     // split grids of a mixed batch: 12.0 -> 9.2 us per upload)
     bool behind_max;
-    bool early;  // lets the next kernel's launch start beside it (tcs_internal.h)
+    bool early;  // EARLY of the kernel
 };
 
-template <int MODE>
+// EARLY: lets the next kernel's launch start beside it (tcs_internal.h), as its
+// first instruction (behind the load of an argument that says so it came late:
+// 803 x 219 star2d1r, 2 steps 11.3 -> 12.1 us a solve).
+template <int MODE, bool EARLY>
 __global__ void __launch_bounds__(kThreads) pack_kernel(const PackArgs a) {
     constexpr int CPP = MODE == kPackF32 ? 4 : 8;
     constexpr int CELLS = kBlkPans * CPP;  // of a block's row
@@ -86,7 +89,7 @@ __global__ void __launch_bounds__(kThreads) pack_kernel(const PackArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const BlockPos b = block_pos(a.p, a.q0);
     const int X = (b.pan - 1) * CPP + lane;  // this lane's first cell: X, X + 32, ...
-    if (a.early) pdl_launch_dependents();
+    if (EARLY) pdl_launch_dependents();
     if (MODE != kPackSplit || !a.behind_max) pdl_wait();
     float v[K][N];
 #pragma unroll
@@ -176,7 +179,7 @@ struct UnpackArgs {
     bool early;  // as PackArgs
 };
 
-template <int MODE>
+template <int MODE, bool EARLY>
 __global__ void __launch_bounds__(kThreads) unpack_kernel(const UnpackArgs a) {
     constexpr int CPP = MODE == kPackF32 ? 4 : 8;
     constexpr int CELLS = kBlkPans * CPP;
@@ -185,7 +188,7 @@ __global__ void __launch_bounds__(kThreads) unpack_kernel(const UnpackArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const BlockPos b = block_pos(a.p, a.q0);
     const int row = min(b.row + lane, a.q1 - 1);
-    if (a.early) pdl_launch_dependents();
+    if (EARLY) pdl_launch_dependents();
     pdl_wait();
     uint4 v[K], l[K];
 #pragma unroll
@@ -434,13 +437,14 @@ template <int MODE>
 cudaError_t launch_pack(PackArgs a, cudaStream_t s) {
     const unsigned blocks = (unsigned)((a.q1 - a.q0 + kBlkRows - 1) / kBlkRows) *
                             (unsigned)((a.p.npan + kBlkPans - 1) / kBlkPans);
-    return launch_pdl(pack_kernel<MODE>, blocks, s, a);
+    return a.early ? launch_pdl(pack_kernel<MODE, true>, blocks, s, a) : launch_pdl(pack_kernel<MODE, false>, blocks, s, a);
 }
 template <int MODE>
 cudaError_t launch_unpack(UnpackArgs a, cudaStream_t s) {
     const unsigned blocks = (unsigned)((a.q1 - a.q0 + kBlkRows - 1) / kBlkRows) *
                             (unsigned)((a.p.npan + kBlkPans - 1) / kBlkPans);
-    return launch_pdl(unpack_kernel<MODE>, blocks, s, a);
+    return a.early ? launch_pdl(unpack_kernel<MODE, true>, blocks, s, a)
+                   : launch_pdl(unpack_kernel<MODE, false>, blocks, s, a);
 }
 
 PackArgs pack_args(const float *in, int ny, int nx, int pad, float pad_value, void *out, int cpp) {
